@@ -15,6 +15,7 @@
 #include "topo_p1.cuh"
 #include "topo_p2.cuh"
 #include "topo_p1march.cuh"
+#include "topo_dens.cuh"
 #include "topo_setup.h"
 #include "topo_fluid.cuh"
 #include "topo_fluid_setup.h"
@@ -214,6 +215,42 @@ P2Params<T> p2params(int nx, int ny, double hx, double hy, double lam, double mu
 }  // namespace
 
 extern "C" {
+
+// density filter: w / s by the integer quotient, and y = W x or W^T x through the table
+void emu_dens_quotient(long n, const double* w, const double* s, double* q) {
+  for (long i = 0; i < n; ++i) q[i] = dens_quotient(w[i], s[i], dens_reciprocal(s[i]));
+}
+
+int emu_dens_filter(int Nx, int Ny, double W, double H, double radius, int transpose, const double* x, double* y) {
+  const double sx = Nx > 1 ? W / double(Nx - 1) : 0.0, sy = Ny > 1 ? H / double(Ny - 1) : 0.0;
+  const int rx = Nx > 1 ? int(std::min<double>(Nx, std::floor(radius / sx) + 1.0)) : 0;
+  const int ry = Ny > 1 ? int(std::min<double>(Ny, std::floor(radius / sy) + 1.0)) : 0;
+  DensAxis X, Y;
+  if (!dens_axis(Nx, W, sx, rx, X) || !dens_axis(Ny, H, sy, ry, Y)) return 1;
+  const std::vector<int> half = dens_half_widths(X, Y, radius);
+  const size_t ncx = X.value.size();
+  std::vector<double> w(ncx * Y.value.size());
+  for (size_t i = 0; i < w.size(); ++i) {
+    const double dx = X.value[i % ncx], dy = Y.value[i / ncx], d = std::sqrt(dx * dx + dy * dy);
+    w[i] = d <= radius ? radius - d : -1.0;
+  }
+  const DensTable T{Nx, Ny, X.reach, Y.reach, int(ncx), X.cls.data(), Y.cls.data(), half.data(), w.data()};
+  std::vector<DensRow> rows(size_t(Nx) * Ny);
+  for (int i = 0; i < Nx * Ny; ++i) {
+    double s = 0.0;
+    dens_table_row(T, i, [&](int, double v) { s += v; });
+    rows[i] = DensRow{dens_reciprocal(s), s};
+  }
+  for (int i = 0; i < Nx * Ny; ++i) {
+    double acc = 0.0;
+    dens_table_row(T, i, [&](int j, double v) {
+      const DensRow R = transpose ? rows[j] : rows[i];
+      acc += dens_quotient(v, R.s, R.r) * x[j];
+    });
+    y[i] = acc;
+  }
+  return 0;
+}
 
 long emu_lean_warps() { return lean_warps; }
 void emu_set_segment(int seg) { seg_override = seg; }
