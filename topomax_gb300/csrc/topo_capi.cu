@@ -363,7 +363,7 @@ struct topo_ctx {
   }
 
   double dot64(const double* a, const double* b, size_t n, cudaStream_t s) {
-    k_dot<double, double><<<red.blocks, kVecThreads, 0, s>>>(a, b, n, red.partials, red.counter, red.out);
+    k_dot<double, double><<<red.blocks_for(n), kVecThreads, 0, s>>>(a, b, n, red.partials, red.counter, red.out);
     cudaMemcpyAsync(red.host, red.out, sizeof(double), cudaMemcpyDeviceToHost, s);
     cudaStreamSynchronize(s);
     return red.host[0];
@@ -533,8 +533,8 @@ int fgmres_ir(topo_ctx* C, MG<float>& mg, Apply64 apply64, const double* b, doub
   double* hbuf = C->red.host;
   auto multidot = [&](int count, const double* w) {
 #define TOPO_MD(K)                                                                                            \
-  k_multidot<double, double, K><<<C->red.blocks, kVecThreads, 0, s>>>(W.V, n, w, n, C->red.partials, C->red.counter, \
-                                                                     C->red.out)
+  k_multidot<double, double, K><<<C->red.blocks_for(n), kVecThreads, 0, s>>>(W.V, n, w, n, C->red.partials, \
+                                                                         C->red.counter, C->red.out)
     TOPO_DISPATCH_COUNT(count, TOPO_MD)
 #undef TOPO_MD
     cudaMemcpyAsync(hbuf, C->red.out, (count + 1) * sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -1041,7 +1041,7 @@ int topo_compliance(topo_ctx* ctx, const double* u, double* compliance, topo_str
     if (!u || !compliance) return ctx->fail(TOPO_ERR_ARG, "invalid compliance arguments");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     ctx->launches += 1;
-    k_dot<double, double><<<ctx->red.blocks, kVecThreads, 0, s>>>(ctx->load, u, 2 * ctx->nn2, ctx->red.partials,
+    k_dot<double, double><<<ctx->red.blocks_for(2 * ctx->nn2), kVecThreads, 0, s>>>(ctx->load, u, 2 * ctx->nn2, ctx->red.partials,
                                                                 ctx->red.counter, compliance);
     return ctx->cuda_check("compliance");
   });
@@ -1106,10 +1106,10 @@ int topo_emd_step(topo_ctx* ctx, const double* psi_prev, const double* g, double
         if (launched == 0 && k == 0) {
           // the clock times the first evaluation (later launches of a chunk may find Newton done)
           KClock kc(s, "Newton evaluation (volume and its derivative)", 0, 2.0 * n * 8.0);
-          k_newton<<<ctx->red.blocks, kVecThreads, 0, s>>>(ctx->half, ctx->ehalf, ctx->vw, n, volume, 1e-12, maxit,
+          k_newton<<<ctx->red.blocks_for(4 * n), kVecThreads, 0, s>>>(ctx->half, ctx->ehalf, ctx->vw, n, volume, 1e-12, maxit,
                                                             ctx->red.partials, ctx->red.counter, ctx->nstate);
         } else {
-          k_newton<<<ctx->red.blocks, kVecThreads, 0, s>>>(ctx->half, ctx->ehalf, ctx->vw, n, volume, 1e-12, maxit,
+          k_newton<<<ctx->red.blocks_for(4 * n), kVecThreads, 0, s>>>(ctx->half, ctx->ehalf, ctx->vw, n, volume, 1e-12, maxit,
                                                             ctx->red.partials, ctx->red.counter, ctx->nstate);
         }
       }
@@ -1123,7 +1123,7 @@ int topo_emd_step(topo_ctx* ctx, const double* psi_prev, const double* g, double
       // bracketing fallback (src/utils.py:138-157): grow [-r, r] from 2 while r <= 2000
       auto F = [&](double cc) {
         ctx->launches += 1;
-        k_eval_volume<<<ctx->red.blocks, kVecThreads, 0, s>>>(ctx->half, ctx->vw, n, cc, ctx->red.partials,
+        k_eval_volume<<<ctx->red.blocks_for(4 * n), kVecThreads, 0, s>>>(ctx->half, ctx->vw, n, cc, ctx->red.partials,
                                                                 ctx->red.counter, ctx->red.out);
         cudaMemcpyAsync(ctx->red.host, ctx->red.out, sizeof(double), cudaMemcpyDeviceToHost, s);
         cudaStreamSynchronize(s);
@@ -1172,7 +1172,7 @@ int topo_emd_finish(topo_ctx* ctx, const double* psi, const double* psi_prev, do
     if (!psi) return ctx->fail(TOPO_ERR_ARG, "invalid arguments");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     ctx->launches += 1;
-    k_emd_finish<<<ctx->red.blocks, kVecThreads, 0, s>>>(psi, psi_prev, ctx->vw, rho, ctx->nv, ctx->red.partials,
+    k_emd_finish<<<ctx->red.blocks_for(4 * ctx->nv), kVecThreads, 0, s>>>(psi, psi_prev, ctx->vw, rho, ctx->nv, ctx->red.partials,
                                                          ctx->red.counter, ctx->red.out);
     if (psi_prev && delta) {
       cudaMemcpyAsync(ctx->red.host, ctx->red.out, sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -1188,7 +1188,7 @@ int topo_integrate(topo_ctx* ctx, const double* f, double* out, topo_stream_t st
     if (!f || !out) return ctx->fail(TOPO_ERR_ARG, "invalid integrate arguments");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     ctx->launches += 1;
-    k_dot<double, double><<<ctx->red.blocks, kVecThreads, 0, s>>>(ctx->vw, f, ctx->nv, ctx->red.partials,
+    k_dot<double, double><<<ctx->red.blocks_for(ctx->nv), kVecThreads, 0, s>>>(ctx->vw, f, ctx->nv, ctx->red.partials,
                                                                 ctx->red.counter, out);
     return ctx->cuda_check("integrate");
   });

@@ -282,7 +282,7 @@ struct topo_fluid_ctx {
   double* pp(double* v) const { return v + 2 * n2; }
 
   double dot(const double* a, const double* b, size_t m, cudaStream_t s) {
-    k_dot<double, double><<<red.blocks, kVecThreads, 0, s>>>(a, b, m, red.partials, red.counter, red.out);
+    k_dot<double, double><<<red.blocks_for(m), kVecThreads, 0, s>>>(a, b, m, red.partials, red.counter, red.out);
     ++launches;
     cudaMemcpyAsync(red.host, red.out, sizeof(double), cudaMemcpyDeviceToHost, s);
     cudaStreamSynchronize(s);
@@ -290,7 +290,7 @@ struct topo_fluid_ctx {
   }
   // y = x - mean(x) on the pressure block (device-side mean)
   void center(const double* xp, double* yp, cudaStream_t s) {
-    k_dot<double, double><<<red.blocks, kVecThreads, 0, s>>>(xp, ones, nv, red.partials, red.counter, red.out);
+    k_dot<double, double><<<red.blocks_for(nv), kVecThreads, 0, s>>>(xp, ones, nv, red.partials, red.counter, red.out);
     k_fluid_center<<<grid(nv), kVecThreads, 0, s>>>(xp, yp, nv, red.out);
     launches += 2;
   }
@@ -351,7 +351,7 @@ void multidot(topo_fluid_ctx* C, int count, const double* w, double* h, double& 
     const int c = std::min(8, count - i0);
     const double* Vb = C->V + size_t(i0) * C->n;
 #define TOPO_MD(K) \
-  k_multidot<double, double, K><<<C->red.blocks, kVecThreads, 0, s>>>(Vb, C->n, w, C->n, C->red.partials, C->red.counter, C->red.out)
+  k_multidot<double, double, K><<<C->red.blocks_for(C->n), kVecThreads, 0, s>>>(Vb, C->n, w, C->n, C->red.partials, C->red.counter, C->red.out)
     TOPO_DISPATCH_COUNT(c, TOPO_MD)
 #undef TOPO_MD
     ++C->launches;
@@ -708,7 +708,7 @@ int topo_fluid_objective(topo_fluid_ctx* ctx, const double* rho, const double* u
     if (!ctx->penal_set) return ctx->fail(TOPO_ERR_STATE, "You must set penalization before calling penalizer");
     if (!rho || !u || !objective) return ctx->fail(TOPO_ERR_ARG, "invalid objective arguments");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    k_fluid_objective<<<ctx->red.blocks, kVecThreads, 0, s>>>(ctx->nx, ctx->ny, ctx->tab, ctx->pen, ctx->viscosity,
+    k_fluid_objective<<<ctx->red.blocks_for(size_t(8) * ctx->nx * ctx->ny), kVecThreads, 0, s>>>(ctx->nx, ctx->ny, ctx->tab, ctx->pen, ctx->viscosity,
                                                               rho, u, ctx->red.partials, ctx->red.counter, objective);
     ++ctx->launches;
     return ctx->cuda_check("fluid objective");

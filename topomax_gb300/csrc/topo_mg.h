@@ -91,6 +91,12 @@ struct Reducer {
   int sms = 148;
   int blocks = 0;
   void init(Arena& a, int sms);
+  // blocks of a reduction over n values: four values a thread at least (each block costs
+  // an atomic on one counter and its share of the last block's sum)
+  int blocks_for(size_t n) const {
+    const size_t b = (n + 1023) / 1024;
+    return b < 1 ? 1 : b < size_t(blocks) ? int(b) : blocks;
+  }
 };
 
 // Device-resident scalars of one preconditioned-CG solve (read back once at the end).

@@ -1216,7 +1216,7 @@ void MG<T>::diag_of(int l, T* d, cudaStream_t s) {
 template <class T>
 double MG<T>::dot(const T* a, const T* b, size_t n, cudaStream_t s) {
   ++launches;
-  k_dot<T, T><<<red_->blocks, kVecThreads, 0, s>>>(a, b, n, red_->partials, red_->counter, red_->out);
+  k_dot<T, T><<<red_->blocks_for(n), kVecThreads, 0, s>>>(a, b, n, red_->partials, red_->counter, red_->out);
   cudaMemcpyAsync(red_->host, red_->out, sizeof(double), cudaMemcpyDeviceToHost, s);
   cudaStreamSynchronize(s);
   return red_->host[0];
@@ -1245,14 +1245,14 @@ double MG<T>::estimate_lmax(int l, cudaStream_t s) {
     k_mul<T><<<g, kVecThreads, 0, s>>>(x, v.dinv, y, n);
     launches += 1;
     if (it % 4 == 3 || it + 1 == iters) {  // rescale to unit length (on the device)
-      k_dot<T, T><<<red_->blocks, kVecThreads, 0, s>>>(x, x, n, red_->partials, red_->counter, red_->out);
+      k_dot<T, T><<<red_->blocks_for(n), kVecThreads, 0, s>>>(x, x, n, red_->partials, red_->counter, red_->out);
       k_scale_unit<T><<<g, kVecThreads, 0, s>>>(x, red_->out, n);
       launches += 2;
     }
   }
   apply(l, x, y, s);
   k_mul<T><<<g, kVecThreads, 0, s>>>(v.t, v.diag, x, n);
-  k_dot2<T><<<red_->blocks, kVecThreads, 0, s>>>(x, y, x, v.t, n, red_->partials, red_->counter, red_->out);
+  k_dot2<T><<<red_->blocks_for(n), kVecThreads, 0, s>>>(x, y, x, v.t, n, red_->partials, red_->counter, red_->out);
   launches += 2;
   cudaMemcpyAsync(red_->host, red_->out, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
   cudaStreamSynchronize(s);
@@ -1668,10 +1668,10 @@ void MG<T>::pcg_prologue(bool warm, cudaStream_t s) {
     cudaMemcpyAsync(r, bi, n * sizeof(T), cudaMemcpyDeviceToDevice, s);
   }
   if (xacc_) launches += 1;
-  k_dot<T, T><<<red_->blocks, kVecThreads, 0, s>>>(bi, bi, n, red_->partials, red_->counter, &dev_->bb);
-  k_dot<T, T><<<red_->blocks, kVecThreads, 0, s>>>(r, r, n, red_->partials, red_->counter, &dev_->rr);
+  k_dot<T, T><<<red_->blocks_for(n), kVecThreads, 0, s>>>(bi, bi, n, red_->partials, red_->counter, &dev_->bb);
+  k_dot<T, T><<<red_->blocks_for(n), kVecThreads, 0, s>>>(r, r, n, red_->partials, red_->counter, &dev_->rr);
   vcycle(r, z, s);
-  k_dot<T, T><<<red_->blocks, kVecThreads, 0, s>>>(r, z, n, red_->partials, red_->counter, &dev_->rz);
+  k_dot<T, T><<<red_->blocks_for(n), kVecThreads, 0, s>>>(r, z, n, red_->partials, red_->counter, &dev_->rz);
   cudaMemcpyAsync(p, z, n * sizeof(T), cudaMemcpyDeviceToDevice, s);
   launches += 5;
 }
@@ -1732,14 +1732,14 @@ void MG<T>::pcg_body(cudaStream_t s, cudaGraphConditionalHandle h, int use_cond)
   apply(0, p, q, s, true);
   {
     KClock kc(s, "CG dot p.q", 0, 2.0 * n * sizeof(T));
-    launch_pdl(k_dot<T, T>, red_->blocks, kVecThreads, 0, s, static_cast<const T*>(p), static_cast<const T*>(q), n,
+    launch_pdl(k_dot<T, T>, red_->blocks_for(n), kVecThreads, 0, s, static_cast<const T*>(p), static_cast<const T*>(q), n,
                red_->partials, red_->counter, &dev_->pq);
   }
   pcg_xr(g, s);
   vcycle(r, z, s);
   {
     KClock kc(s, "CG dots r.r, r.z", 0, 2.0 * n * sizeof(T));
-    launch_pdl(k_dot2<T>, red_->blocks, kVecThreads, 0, s, static_cast<const T*>(r), static_cast<const T*>(r),
+    launch_pdl(k_dot2<T>, red_->blocks_for(n), kVecThreads, 0, s, static_cast<const T*>(r), static_cast<const T*>(r),
                static_cast<const T*>(r), static_cast<const T*>(z), n, red_->partials, red_->counter, &dev_->rr);
   }
   launch_pdl(k_pcg_check, 1, 1, 0, s, dev_, h, use_cond);

@@ -76,51 +76,76 @@ __device__ __forceinline__ R warp_sum(R v) {
   return v;
 }
 
-template <class R>
-__device__ __forceinline__ R block_sum(R v, R* sh) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  v = warp_sum(v);
-  if (lane == 0) sh[w] = v;
+// Sums of NV values per thread over the block (at most kVecThreads threads), in
+// res[0..NV) (shared, FP64) after the barrier at the end.  FP32 values go through warp
+// shuffles.  FP64 values go through shared memory, one warp per value: an FP64 addition
+// holds the SM's FP64 pipe for 16 cycles whatever the number of useful lanes, and a
+// shuffle tree in every warp issues 5 NV of them per warp where this issues nw + 5 per
+// value (eight warps, nine values: 117 instead of 387, 1.0 instead of 2.9 us a block).
+template <int NV, class R>
+__device__ __forceinline__ void block_sums(const R (&v)[NV], double* res) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  if constexpr (sizeof(R) == 4) {
+    __shared__ R sh[NV * 32];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const R s = warp_sum(v[k]);
+      if (lane == 0) sh[k * 32 + w] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x < NV) {
+      double s = 0.0;
+      for (int i = 0; i < nw; ++i) s += double(sh[threadIdx.x * 32 + i]);
+      res[threadIdx.x] = s;
+    }
+  } else {
+    __shared__ R sh[NV * kVecThreads];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh[k * kVecThreads + threadIdx.x] = v[k];
+    __syncthreads();
+    for (int k = w; k < NV; k += nw) {
+      R s = sh[k * kVecThreads + lane];
+      for (int i = 1; i < nw; ++i) s += sh[k * kVecThreads + 32 * i + lane];
+      s = warp_sum(s);
+      if (lane == 0) res[k] = s;
+    }
+  }
   __syncthreads();
-  const int nw = (blockDim.x + 31) >> 5;
-  v = (threadIdx.x < nw) ? sh[threadIdx.x] : R(0);
-  if (w == 0) v = warp_sum(v);
-  __syncthreads();
-  return v;  // valid in thread 0
 }
 
-// Finishes a reduction of NV values per block (1D or 2D grids).  Returns true
-// in thread 0 of the last block, with the totals in tot[].  The in-block tree
-// runs in R (float for FP32 data: FP64 arithmetic is scarce on this GPU), the
-// per-block partials and their final combination in FP64.
+// Finishes a reduction of NV values per block (1D or 2D grids, blocks of whole warps, at
+// most kVecThreads threads).  Returns true in thread 0 of the last block, with the totals
+// in tot[].  The in-block sums run in R (float for FP32 data) up to the warps, the
+// combination of warps and blocks in FP64, always in the same order.
 template <int NV, class R>
 __device__ bool finish_reduction(const R (&v)[NV], double* partials, unsigned* counter, double (&tot)[NV]) {
-  __shared__ R shr[32];
-  __shared__ double sh[32];
+  __shared__ double res[NV];
   __shared__ bool last;
   const unsigned bid = blockIdx.y * gridDim.x + blockIdx.x, nb = gridDim.x * gridDim.y;
-  for (int k = 0; k < NV; ++k) {
-    const R s = block_sum(v[k], shr);
-    if (threadIdx.x == 0) partials[size_t(bid) * NV + k] = double(s);
-  }
-  __threadfence();
-  if (threadIdx.x == 0) {
-    const unsigned prev = atomicAdd(counter, 1u);
-    last = (prev == nb - 1);
-  }
-  __syncthreads();
-  if (!last) return false;
-  __threadfence();
-  for (int k = 0; k < NV; ++k) {
-    double s = 0.0;
+  block_sums<NV, R>(v, res);
+  if (nb > 1) {
+    if (threadIdx.x < NV) {
+      partials[size_t(bid) * NV + threadIdx.x] = res[threadIdx.x];
+      __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == nb - 1;
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    double s[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) s[k] = 0.0;
     for (unsigned b = threadIdx.x; b < nb; b += blockDim.x)
-      s += ((volatile double*)partials)[size_t(b) * NV + k];
-    // fixed-order combine: strided per-thread sums then a tree
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) tot[k] = s;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) s[k] += __ldcg(partials + size_t(b) * NV + k);
+    block_sums<NV, double>(s, res);
+    if (threadIdx.x == 0) *counter = 0u;
   }
-  if (threadIdx.x == 0) *counter = 0u;
-  return threadIdx.x == 0;
+  if (threadIdx.x != 0) return false;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) tot[k] = res[k];
+  return true;
 }
 
 // out[0] = sum a_i b_i (or sum a_i^2 when b == nullptr)
