@@ -7,6 +7,7 @@
 // __syncthreads give -- so the tiling and index logic can be compared with
 // the FP64 oracle without a GPU.  It is never linked into the product library.
 #include <cstring>
+#include <limits>
 #include <memory>
 #include <type_traits>
 #include <vector>
@@ -214,7 +215,109 @@ P2Params<T> p2params(int nx, int ny, double hx, double hy, double lam, double mu
 }
 }  // namespace
 
+namespace {
+// Both sweeps of a stencil level over all blocks, every thread of a phase before any of the
+// next; shared memory starts as NaN.
+template <class T, int NC>
+void level_sweeps(LevelSweep<T, NC> P, const T* b, const T* xin, const T* xc, T* xpre, T* bc, T* xpost) {
+  const T nan = std::numeric_limits<T>::quiet_NaN();
+  const int nt = 256;
+  for (int J0 = 0; J0 < P.NYc; J0 += P.cy)
+    for (int I0 = 0; I0 < P.NXc; I0 += P.cx) {
+      std::vector<T> sm(P.down_shared(), nan);
+      T *sx = sm.data(), *sd = sx + NC * P.down_w() * P.down_h();
+      std::vector<LevelNode<T, NC>> N(nt);
+      std::vector<char> on(nt);
+      for (int t = 0; t < nt; ++t) on[t] = LevelDown<T, NC>::start(P, I0, J0, t, N[t]);
+      for (int t = 0; t < nt; ++t) {
+        LevelDown<T, NC>::first(P, I0, J0, t, nt, b, sd);
+        if (on[t]) N[t].load_b(P, b);
+      }
+      for (int t = 0; t < nt; ++t)
+        if (on[t]) LevelDown<T, NC>::smooth(P, t, N[t], sd, sx, xpre);
+      for (int t = 0; t < nt; ++t)
+        if (on[t]) LevelDown<T, NC>::residual(P, t, N[t], sx, sd);
+      for (int t = 0; t < nt; ++t) LevelDown<T, NC>::restrict_to(P, I0, J0, t, nt, sd, bc);
+      sm.assign(P.up_shared(), nan);
+      sd = sm.data();
+      sx = sd + NC * P.up_w() * P.up_h();
+      std::vector<typename LevelUp<T, NC>::Node> U(nt);
+      for (int t = 0; t < nt; ++t) on[t] = LevelUp<T, NC>::start(P, I0, J0, t, U[t]);
+      for (int t = 0; t < nt; ++t) {
+        LevelUp<T, NC>::correct(P, I0, J0, t, nt, xin, xc, sx);
+        if (on[t]) U[t].load_b(P, b);
+      }
+      for (int t = 0; t < nt; ++t)
+        if (on[t]) LevelUp<T, NC>::first(P, t, U[t], sx, sd);
+      for (int t = 0; t < nt; ++t)
+        if (on[t] && LevelUp<T, NC>::owned(P, t, U[t])) LevelUp<T, NC>::second(P, t, U[t], sd, xpost);
+    }
+}
+
+template <class T, int NC>
+int emu_sweeps(int nx, int ny, double hx, double hy, double lam, double mu, const int* dir, const double* kK,
+               const double* kM, const double* cheb, int NXc, int NYc, const int* dirc, int cx, int cy,
+               const double* b, const double* dinv, const double* xin, const double* xc, double* xpre, double* bc,
+               double* xpost) {
+  const int NX = nx + 1, NY = ny + 1, SW = StencilLayout<NC>::stride;
+  const size_t n = size_t(NX) * NY;
+  const ElemRefs R = make_elem_refs(hx, hy, lam, mu);
+  P1Params<T, NC> Q;
+  std::memset(&Q, 0, sizeof(Q));
+  Q.nx = nx;
+  Q.ny = ny;
+  Q.dir = dir_from(dir);
+  for (int o = 0; o < 2; ++o) {
+    for (int a = 0; a < 3 * NC; ++a)
+      for (int c = 0; c < 3 * NC; ++c) Q.K[o][a][c] = T(NC == 2 ? R.K2[o][a][c] : R.K1[o][a][c]);
+    for (int a = 0; a < 3; ++a)
+      for (int c = 0; c < 3; ++c) Q.Mm[o][a][c] = T(R.M1[o][a][c]);
+  }
+  auto cast = [](const double* s, size_t m) { return std::vector<T>(s, s + m); };
+  const std::vector<T> k = cast(kK, size_t(2) * nx * ny), m = kM ? cast(kM, size_t(2) * nx * ny) : std::vector<T>();
+  Q.kK = k.data();
+  Q.kM = kM ? m.data() : nullptr;
+  Q.kM_c = (NC == 1 && !kM) ? T(1) : T(0);
+  std::vector<T> st(n * SW);
+  for (int j = 0; j < NY; ++j)
+    for (int i = 0; i < NX; ++i) p1_stencil_node<T, NC>(i, j, Q, st.data() + (size_t(j) * NX + i) * SW);
+  LevelSweep<T, NC> P;
+  std::memset(&P, 0, sizeof(P));
+  const std::vector<T> ch = cast(cheb, 3), di = cast(dinv, n * NC), bb = cast(b, n * NC), xi = cast(xin, n * NC),
+                       xcc = cast(xc, size_t(NXc) * NYc * NC);
+  P.NX = NX;
+  P.NY = NY;
+  P.NXc = NXc;
+  P.NYc = NYc;
+  P.cx = cx;
+  P.cy = cy;
+  P.st = st.data();
+  P.dinv = di.data();
+  P.cheb = ch.data();
+  P.dirf = Q.dir;
+  P.dirc = dir_from(dirc);
+  std::vector<T> o1(n * NC, T(-7)), o2(size_t(NXc) * NYc * NC, T(-7)), o3(n * NC, T(-7));
+  level_sweeps<T, NC>(P, bb.data(), xi.data(), xcc.data(), o1.data(), o2.data(), o3.data());
+  std::copy(o1.begin(), o1.end(), xpre);
+  std::copy(o2.begin(), o2.end(), bc);
+  std::copy(o3.begin(), o3.end(), xpost);
+  return 0;
+}
+}  // namespace
+
 extern "C" {
+
+// down and up sweep of a stencil level (prec 0 FP64, 1 FP32) with cx x cy coarse nodes a block
+int emu_level_sweeps(int prec, int NC, int nx, int ny, double hx, double hy, double lam, double mu, const int* dir,
+                     const double* kK, const double* kM, const double* cheb, int NXc, int NYc, const int* dirc, int cx,
+                     int cy, const double* b, const double* dinv, const double* xin, const double* xc, double* xpre,
+                     double* bc, double* xpost) {
+#define TOPO_EMU_SWEEP(T, K) \
+  emu_sweeps<T, K>(nx, ny, hx, hy, lam, mu, dir, kK, kM, cheb, NXc, NYc, dirc, cx, cy, b, dinv, xin, xc, xpre, bc, xpost)
+  if (NC == 2) return prec ? TOPO_EMU_SWEEP(float, 2) : TOPO_EMU_SWEEP(double, 2);
+  return prec ? TOPO_EMU_SWEEP(float, 1) : TOPO_EMU_SWEEP(double, 1);
+#undef TOPO_EMU_SWEEP
+}
 
 // density filter: w / s by the integer quotient, and y = W x or W^T x through the table
 void emu_dens_quotient(long n, const double* w, const double* s, double* q) {

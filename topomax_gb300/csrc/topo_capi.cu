@@ -303,21 +303,6 @@ struct topo_ctx {
             std::fprintf(stderr, "[topo profile] %s level %zu (%dx%d nodes): %lld V-cycle visits, %.3f ms incl, %.2f us/visit\n",
                          name, l, mg.spec(int(l)).NX, mg.spec(int(l)).NY, mg.level_calls[l], mg.level_ms[l],
                          1e3 * mg.level_ms[l] / mg.level_calls[l]);
-        std::vector<long long> cyc;
-        mg.tail_profile(cyc);
-        if (!cyc.empty() && cyc.back() > 0) {
-          const int nl = mg.levels() - mg.tail_level();
-          std::fprintf(stderr, "[topo profile] %s tail: levels %d.., %d levels, %lld launches; k-cycles per phase:",
-                       name, mg.tail_level(), nl, cyc.back());
-          int slot = 1;
-          auto pr = [&](const char* what, int l) {
-            std::fprintf(stderr, " %s%d=%.2f", what, l, 1e-3 * double(cyc[slot++]) / double(cyc.back()));
-          };
-          for (int l = 0; l + 1 < nl; ++l) { pr("pre", l); pr("res", l); pr("restr", l); }
-          pr("coarse", nl - 1);
-          for (int l = nl - 2; l >= 0; --l) { pr("prol", l); pr("first", l); pr("post", l); }
-          std::fprintf(stderr, "\n");
-        }
       };
       dump("state32", smg32);
       dump("state64", smg64);

@@ -27,15 +27,20 @@
 // launched without the programmatic attribute), then allow their own
 // successor to be scheduled; the successor launches once every block of this
 // grid has passed that point and overlaps its launch with this grid's drain.
+// A kernel that reads data no kernel of the chain writes may call TOPO_PDL_LAUNCH() first,
+// read them, and TOPO_PDL_WAIT() before it touches anything else.
 #if defined(__CUDA_ARCH__)
-#define TOPO_PDL_ENTRY()                                 \
-  do {                                                   \
-    asm volatile("griddepcontrol.wait;" ::: "memory");   \
-    asm volatile("griddepcontrol.launch_dependents;" :::); \
-  } while (0)
+#define TOPO_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
+#define TOPO_PDL_LAUNCH() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
 #else
-#define TOPO_PDL_ENTRY() ((void)0)
+#define TOPO_PDL_WAIT() ((void)0)
+#define TOPO_PDL_LAUNCH() ((void)0)
 #endif
+#define TOPO_PDL_ENTRY() \
+  do {                   \
+    TOPO_PDL_WAIT();     \
+    TOPO_PDL_LAUNCH();   \
+  } while (0)
 
 namespace topo {
 

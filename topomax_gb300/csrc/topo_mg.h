@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "topo_common.cuh"
+#include "topo_p1level.cuh"
 #include "topo_p2.cuh"
 
 namespace topo {
@@ -191,7 +192,6 @@ class MG {
   int coarse_cheb_max_degree = 16;
   int coarse_cheb_level() const { return cheb_coarse_; }
   int coarse_cheb_deg = 0;
-  bool use_p1_march = true;  // large P1 levels: column march (false: node-centric kernels)
   long long capture_failures = 0;  // recordings that failed (those solves ran host-driven)
   // opt-in level timing (host-driven mode only): inclusive ms per level, summed
   bool profile_levels = false;
@@ -199,10 +199,6 @@ class MG {
   std::vector<double> level_ms;
   std::vector<long long> level_calls;
   void flush_level_profile();
-  // tail phase timing (profile_levels only): SM cycles summed per phase in
-  // execution order, last entry = launches; empty without a tail
-  void tail_profile(std::vector<long long>& cycles) const;
-  int tail_level() const { return tail_; }
   // tune the segment length of this hierarchy's march kernels (level 0 if P2, the P1
   // levels without a stencil) once per family and grid; needs set-up data in place
   bool autotune = true;
@@ -255,7 +251,7 @@ class MG {
     long long prologue_nodes = 0, body_nodes = 0;
   } graph_[2];
   bool graph_valid_ = false;
-  void build_tail(Arena& arena);
+  void build_tail();
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> prof_events_;
   // truncated hierarchy: the V-cycle stops at level cheb_coarse_ and solves it
   // with a fixed-degree Chebyshev iteration in one CTA (CoarseChebDesc, device)
@@ -267,10 +263,9 @@ class MG {
   void* cc_buf_ = nullptr;
   T* inner_buf_ = nullptr;  // per level: one stencil row (detect_uniform_levels)
   bool cc_selected_ = false;
-  int tail_ = -1;              // first level run by the one-CTA shared-memory tail kernel
-  void* tail_desc_ = nullptr;  // TailDesc<T, NC> (device)
-  size_t tail_smem_ = 0;
-  long long* tail_trace_ = nullptr;
+  int tail_ = -1;  // first level run by the one-CTA tail kernel, described by
+  TailSweep<T, 1> tail1_{};
+  TailSweep<T, 2> tail2_{};
   // set by pcg_body around its V-cycle: the level-0 post-smoothing launch also
   // reduces r.r, r.z and runs the iteration's test
   bool stencils_ready_ = false;  // set once setup() has assembled the stencils

@@ -14,6 +14,7 @@
 #include "topo_kclock.h"
 #include "topo_mg.h"
 #include "topo_p1.cuh"
+#include "topo_p1level.cuh"
 #include "topo_p1march.cuh"
 #include "topo_p2.cuh"
 #include "topo_vec.cuh"
@@ -223,15 +224,60 @@ __global__ void __launch_bounds__(P2M_THREADS) k_p1_march(P1Params<T, NC> P, P1I
   }
 }
 
-template <class T, int NC, int MODE, class PP>
-__global__ void __launch_bounds__(kRowThreads_) k_p1_smooth(PP P, SmoothBufs<T> B) {
-  TOPO_PDL_ENTRY();
-  const int a = blockIdx.x * kRowThreads_ + threadIdx.x, b = blockIdx.y;
-  if (a > P.nx) return;
-  if (MODE == kP2Pre) P1Smooth<T, NC>::pre(a, b, P, B);
-  else if (MODE == kP2Res) P1Smooth<T, NC>::res(a, b, P, B);
-  else if (MODE == kP2First) P1Smooth<T, NC>::first(a, b, P, B);
-  else P1Smooth<T, NC>::post2(a, b, P, B);
+// The sweeps of a stencil level (see topo_p1level.cuh).  The rows, inverse diagonals and
+// smoothing coefficients are fixed during a solve, so they are read before the wait for
+// the predecessor; the successor may start its own such reads at once.  What the
+// predecessor wrote comes through pointers without __restrict__: a load that the compiler
+// takes to be from memory nobody writes may move above the wait.
+//
+// Measured on design evaluations (us): the six launches per level and the earlier one-block
+// tail of 30 to 35 us took 8,490 at 80x40, 31,000 at 303x101 and 25,470 at 1000x500; sweeps
+// and tail take 5,520, 17,100 and 18,300.
+// Tile: 10 x 4 coarse nodes, 253 threads for 160 fine nodes of its own down, 220 up.  On the
+// 1000x500 design evaluation 14 x 6 (465 threads, less recomputed) measured 18.8 ms against
+// 18.6, 6 x 6 19.2, 14 x 2 18.9; FP64 at 160x80 63.9 ms against 76.8, 66.1 and 66.2 (a tile's
+// recomputed ring costs FP64-pipe time, a large tile leaves SMs without a block).
+constexpr int kSweepTileX = 10, kSweepTileY = 4;
+constexpr int kSweepThreads = 256;
+
+template <class T, int NC>
+__global__ void __launch_bounds__(kSweepThreads)
+    k_level_down(LevelSweep<T, NC> P, const T* b, T* x, T* bc) {
+  extern __shared__ __align__(16) unsigned char sweep_raw[];
+  T* sx = reinterpret_cast<T*>(sweep_raw);
+  T* sd = sx + NC * P.down_w() * P.down_h();
+  const int tid = threadIdx.x, nt = blockDim.x, I0 = blockIdx.x * P.cx, J0 = blockIdx.y * P.cy;
+  TOPO_PDL_LAUNCH();
+  LevelNode<T, NC> N;
+  const bool on = LevelDown<T, NC>::start(P, I0, J0, tid, N);
+  TOPO_PDL_WAIT();
+  LevelDown<T, NC>::first(P, I0, J0, tid, nt, b, sd);
+  if (on) N.load_b(P, b);
+  __syncthreads();
+  if (on) LevelDown<T, NC>::smooth(P, tid, N, sd, sx, x);
+  __syncthreads();
+  if (on) LevelDown<T, NC>::residual(P, tid, N, sx, sd);
+  __syncthreads();
+  LevelDown<T, NC>::restrict_to(P, I0, J0, tid, nt, sd, bc);
+}
+
+template <class T, int NC>
+__global__ void __launch_bounds__(kSweepThreads)
+    k_level_up(LevelSweep<T, NC> P, const T* b, const T* xin, const T* xc, T* x) {
+  extern __shared__ __align__(16) unsigned char sweep_raw[];
+  T* sd = reinterpret_cast<T*>(sweep_raw);
+  T* sx = sd + NC * P.up_w() * P.up_h();
+  const int tid = threadIdx.x, nt = blockDim.x, I0 = blockIdx.x * P.cx, J0 = blockIdx.y * P.cy;
+  TOPO_PDL_LAUNCH();
+  typename LevelUp<T, NC>::Node N;
+  const bool on = LevelUp<T, NC>::start(P, I0, J0, tid, N);
+  TOPO_PDL_WAIT();
+  LevelUp<T, NC>::correct(P, I0, J0, tid, nt, xin, xc, sx);
+  if (on) N.load_b(P, b);
+  __syncthreads();
+  if (on) LevelUp<T, NC>::first(P, tid, N, sx, sd);
+  __syncthreads();
+  if (on && LevelUp<T, NC>::owned(P, tid, N)) LevelUp<T, NC>::second(P, tid, N, sd, x);
 }
 
 template <class T, int NC>
@@ -367,158 +413,140 @@ __global__ void k_dense_matvec(const T* __restrict__ Ainv, const T* __restrict__
   }
 }
 
-// ---------------------------------------------------------------------------
-// coarse-level tail: the V-cycle over the smallest levels runs in one CTA with
-// every work vector, the stencils and D^-1 resident in shared memory (one
-// launch instead of ~6 x levels; the phases touch no global memory)
-// ---------------------------------------------------------------------------
-constexpr int kTailThreads = 1024;
-constexpr int kTailMaxLevels = 10;
-constexpr size_t kTailSmemBudget = 196 * 1024;
-constexpr int kTailTraceSlots = 64;  // [0, 62]: SM cycles per phase, [63]: launches
+constexpr int kCoarseThreads = 1024;                   // one-CTA coarse Chebyshev solve
+constexpr size_t kCoarseSharedBudget = 196 * 1024;
 
+// The last levels of the V-cycle (see TailSweep): x = V-cycle(b) from its level 0 down.
+// Latency-bound: seven barriers per level.
 template <class T, int NC>
-struct TailLevel {
-  P1Stencil<T, NC> S;
-  Transfer X;  // to the next coarser level
-  const T* dinv;
-  const T* cheb;
-  int NX, nn, off;  // off: first of this level's five shared vectors x, b, r, d, x2 (NC*nn each)
-  int soff, doff;   // shared copies of the stencil (stride*nn) and of dinv (NC*nn)
-};
-
-template <class T, int NC>
-struct TailDesc {
-  int nlev, smem_elems;
-  const T* cinv;
-  long long* trace;  // opt-in phase timing (null: off)
-  TailLevel<T, NC> lv[kTailMaxLevels];
-};
-
-// Copies n values global -> shared with 16-byte accesses (both addresses 16-byte
-// aligned), the remainder one by one: the tail's per-launch staging issues a few
-// wide loads per thread instead of a long chain of scalar ones.
-template <class T>
-__device__ __forceinline__ void stage16(T* __restrict__ dst, const T* __restrict__ src, int n, int tid, int nt) {
-  constexpr int V = 16 / sizeof(T);
-  const int nv = n / V;
-  const float4* s4 = reinterpret_cast<const float4*>(src);
-  float4* d4 = reinterpret_cast<float4*>(dst);
-#pragma unroll 4
-  for (int i = tid; i < nv; i += nt) d4[i] = s4[i];
-  for (int i = nv * V + tid; i < n; i += nt) dst[i] = src[i];
-}
-
-template <class T, int NC>
-__global__ void __launch_bounds__(kTailThreads)
-    k_tail_vcycle(const TailDesc<T, NC>* __restrict__ D, const T* __restrict__ b_in, T* __restrict__ x_out) {
-  TOPO_PDL_ENTRY();
-  __shared__ TailLevel<T, NC> lv[kTailMaxLevels];
-  __shared__ __align__(16) T cinv[kCoarseMaxDofs * kCoarseMaxDofs];
-  extern __shared__ __align__(16) unsigned char tail_raw[];
-  T* sm = reinterpret_cast<T*>(tail_raw);
+__global__ void __launch_bounds__(kTailNodes)
+    k_level_tail(const __grid_constant__ TailSweep<T, NC> P, const T* b, T* x) {
+  constexpr int SW = StencilLayout<NC>::stride;
+  extern __shared__ __align__(16) unsigned char sweep_raw[];
+  T* sm = reinterpret_cast<T*>(sweep_raw);
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int nlev = D->nlev;
-  {
-    const int* src = reinterpret_cast<const int*>(D->lv);
-    int* dst = reinterpret_cast<int*>(lv);
-    const int words = int(sizeof(TailLevel<T, NC>) / sizeof(int)) * nlev;
-    for (int i = tid; i < words; i += nt) dst[i] = src[i];
-  }
-  __syncthreads();
-  // (stencil and diagonal offsets are multiples of 16 bytes, every source a separate allocation)
-  for (int l = 0; l < nlev; ++l) {
-    const TailLevel<T, NC>& L = lv[l];
-    stage16(sm + L.soff, L.S.s, StencilLayout<NC>::stride * L.nn, tid, nt);
-    stage16(sm + L.doff, L.dinv, NC * L.nn, tid, nt);
-  }
-  {
-    const int mc = NC * lv[nlev - 1].nn;
-    stage16(cinv, D->cinv, mc * mc, tid, nt);
-    const int m = NC * lv[0].nn;
-    T* b0 = sm + lv[0].off + m;  // (inside the level's five vectors: not 16-byte aligned)
-    for (int i = tid; i < m; i += nt) b0[i] = b_in[i];
-  }
-  __syncthreads();
-  if (tid == 0)
-    for (int l = 0; l < nlev; ++l) {
-      lv[l].S.s = sm + lv[l].soff;
-      lv[l].dinv = sm + lv[l].doff;
+  TOPO_PDL_LAUNCH();
+  // what no solve changes: rows, inverse diagonals, the coarsest inverse
+  for (int i = tid; i < P.vectors; i += nt) sm[i] = T(0);
+  for (int l = 1; l < P.nlev; ++l) {
+    const auto& L = P.lv[l];
+    for (int n = tid; n < L.NX * L.NY; n += nt) {
+      __align__(16) T st[SW];
+      load_row(L.st + size_t(n) * SW, st);
+      level_row<T, NC>(st);
+      copy_row<T, SW>(st, sm + L.row + n * SW);
+      for (int c = 0; c < NC; ++c) sm[L.di + NC * n + c] = L.dinv[NC * n + c];
     }
-  __syncthreads();
-  // opt-in timing: SM cycles of every phase in execution order
-  long long* const trace = tid == 0 ? D->trace : nullptr;
-  long long t_prev = clock64();
-  int slot = 1;
-  auto mark = [&]() {
+  }
+  const auto& C = P.lv[P.nlev];
+  const int m = C.NX * C.NY * NC;
+  for (int i = tid; i < m * m; i += nt) sm[P.inv + i] = P.cinv[i];
+  const auto& L0 = P.lv[0];
+  const bool on0 = tid < L0.NX * L0.NY;
+  const int n0 = on0 ? tid : 0;
+  T st0[SW], di0[NC], b0[NC];
+  load_row(L0.st + size_t(n0) * SW, st0);
+  level_row<T, NC>(st0);
+  for (int c = 0; c < NC; ++c) di0[c] = L0.dinv[NC * n0 + c];
+  TOPO_PDL_WAIT();
+  for (int c = 0; c < NC; ++c) b0[c] = b[NC * n0 + c];
+  __syncthreads();  // the zeros are in place
+  // level l's node of this thread: rows and so on from registers (level 0) or shared memory
+  auto with_node = [&](int l, auto&& f) {
+    const auto& L = P.lv[l];
+    const int n = tid;
+    if (n >= L.NX * L.NY) return;
+    const int j = n / L.NX, i = n - j * L.NX, w = L.NX + 2, p = (j + 1) * w + i + 1;
+    if (l == 0) {
+      f(L, n, i, j, w, p, st0, di0, b0);
+    } else {
+      __align__(16) T st[SW];
+      T di[NC], bl[NC];
+      copy_row<T, SW>(sm + L.row + n * SW, st);
+      for (int c = 0; c < NC; ++c) {
+        di[c] = sm[L.di + NC * n + c];
+        bl[c] = sm[L.b + NC * n + c];
+      }
+      f(L, n, i, j, w, p, st, di, bl);
+    }
+  };
+  auto down = [&](int l) {
+    with_node(l, [&](const auto& L, int, int, int, int, int p, const auto&, const auto& di, const auto& bl) {
+      const T c0 = L.cheb[0];
+      for (int c = 0; c < NC; ++c) sm[L.d + NC * p + c] = (c0 * di[c]) * bl[c];
+    });
     __syncthreads();
-    if (!trace) return;
-    const long long t = clock64();
-    if (slot < kTailTraceSlots - 1) trace[slot++] += t - t_prev;
-    t_prev = t;
+    with_node(l, [&](const auto& L, int, int, int, int w, int p, const auto& st, const auto& di, const auto& bl) {
+      T t[NC];
+      level_apply<T, NC>(st, sm + L.d, w, p, t);
+      const T c1 = L.cheb[1], c2 = L.cheb[2];
+      for (int c = 0; c < NC; ++c) {
+        const T u = sm[L.d + NC * p + c];
+        sm[L.x + NC * p + c] = level_step(u, c1, u, c2, di[c], bl[c] - t[c]);
+      }
+    });
+    __syncthreads();
+    with_node(l, [&](const auto& L, int, int, int, int w, int p, const auto& st, const auto&, const auto& bl) {
+      T t[NC];
+      level_apply<T, NC>(st, sm + L.x, w, p, t);
+      for (int c = 0; c < NC; ++c) sm[L.d + NC * p + c] = bl[c] - t[c];
+    });
+    __syncthreads();
+    const auto& L = P.lv[l];
+    const auto& K = P.lv[l + 1];
+    if (tid < K.NX * K.NY) {
+      const int J = tid / K.NX, I = tid - J * K.NX, w = L.NX + 2;
+      const bool zero = is_clamped(K.dir, I, J);
+      const T* r = sm + L.d + NC * ((2 * J + 1) * w + 2 * I + 1);
+      for (int c = 0; c < NC; ++c) sm[K.b + NC * tid + c] = zero ? T(0) : level_restrict<T, NC>(r + c, w);
+    }
+    __syncthreads();
   };
-  auto bufs = [&](int l) {
-    const int m = NC * lv[l].nn;
-    T* base = sm + lv[l].off;
-    return SmoothBufs<T>{base + m, lv[l].dinv, base, base + 4 * m, base + 2 * m, base + 3 * m, lv[l].cheb};
-  };
-  for (int l = 0; l + 1 < nlev; ++l) {
-    const TailLevel<T, NC>& L = lv[l];
-    const SmoothBufs<T> B = bufs(l);
-    for (int n = tid; n < L.nn; n += nt) {
-      const int b = n / L.NX, a = n - b * L.NX;
-      P1Smooth<T, NC>::pre(a, b, L.S, B);
-    }
-    mark();
-    for (int n = tid; n < L.nn; n += nt) {
-      const int b = n / L.NX, a = n - b * L.NX;
-      P1Smooth<T, NC>::res(a, b, L.S, B);
-    }
-    mark();
-    const TailLevel<T, NC>& C = lv[l + 1];
-    T* bc = sm + C.off + NC * C.nn;
-    for (int n = tid; n < C.nn; n += nt) {
-      const int J = n / C.NX, I = n - J * C.NX;
-      TransferKern<T, NC>::node_restrict(I, J, L.X, B.r, bc);
-    }
-    mark();
+  for (int l = 0; l < P.nlev; ++l) down(l);
+  if (tid < m) {  // the inverse is symmetric: column reads, one line per step
+    T s = T(0);
+    for (int k = 0; k < m; ++k) s = fma_t(sm[P.inv + k * m + tid], sm[C.b + k], s);
+    const int n = tid / NC, j = n / C.NX, i = n - j * C.NX;
+    sm[C.x + NC * ((j + 1) * (C.NX + 2) + i + 1) + tid % NC] = s;
   }
-  {  // coarsest level: dense inverse
-    const TailLevel<T, NC>& C = lv[nlev - 1];
-    const int m = NC * C.nn;
-    const T* bc = sm + C.off + m;
-    T* xc = sm + C.off;
-    for (int i = tid; i < m; i += nt) {
-      T acc = T(0);
-#pragma unroll 8
-      for (int j = 0; j < m; ++j) acc += cinv[i * m + j] * bc[j];
-      xc[i] = acc;
-    }
-    mark();
+  __syncthreads();
+  for (int l = P.nlev - 1; l >= 0; --l) {
+    T r0[NC], d0[NC], x2[NC];
+    with_node(l, [&](const auto& L, int, int i, int j, int, int p, const auto&, const auto&, const auto&) {
+      const auto& K = P.lv[l + 1];
+      if (is_clamped(L.dir, i, j)) return;
+      const int wc = K.NX + 2;
+      const int m0 = ((j >> 1) + 1) * wc + (i >> 1) + 1, m1 = (((j + 1) >> 1) + 1) * wc + ((i + 1) >> 1) + 1;
+      for (int c = 0; c < NC; ++c) {
+        const T u = sm[K.x + NC * m0 + c], v = sm[K.x + NC * m1 + c];
+        sm[L.x + NC * p + c] += m0 == m1 ? u : T(0.5) * (u + v);
+      }
+    });
+    __syncthreads();
+    with_node(l, [&](const auto& L, int, int, int, int w, int p, const auto& st, const auto& di, const auto& bl) {
+      T t[NC];
+      level_apply<T, NC>(st, sm + L.x, w, p, t);
+      const T c0 = L.cheb[0];
+      for (int c = 0; c < NC; ++c) {
+        r0[c] = bl[c] - t[c];
+        d0[c] = (c0 * di[c]) * r0[c];
+        x2[c] = sm[L.x + NC * p + c] + d0[c];
+        sm[L.d + NC * p + c] = d0[c];
+      }
+    });
+    __syncthreads();
+    with_node(l, [&](const auto& L, int n, int, int, int w, int p, const auto& st, const auto& di, const auto&) {
+      T t[NC];
+      level_apply<T, NC>(st, sm + L.d, w, p, t);
+      const T c1 = L.cheb[1], c2 = L.cheb[2];
+      for (int c = 0; c < NC; ++c) {
+        const T v = level_step(x2[c], c1, d0[c], c2, di[c], r0[c] - t[c]);
+        if (l == 0) x[NC * n + c] = v;
+        else sm[L.x + NC * p + c] = v;
+      }
+    });
+    if (l) __syncthreads();
   }
-  for (int l = nlev - 2; l >= 0; --l) {
-    const TailLevel<T, NC>& L = lv[l];
-    const SmoothBufs<T> B = bufs(l);
-    const T* xc = sm + lv[l + 1].off;
-    for (int n = tid; n < L.nn; n += nt) {
-      const int b = n / L.NX, a = n - b * L.NX;
-      TransferKern<T, NC>::node_prolong_add(a, b, L.X, xc, B.x);
-    }
-    mark();
-    for (int n = tid; n < L.nn; n += nt) {
-      const int b = n / L.NX, a = n - b * L.NX;
-      P1Smooth<T, NC>::first(a, b, L.S, B);
-    }
-    mark();
-    for (int n = tid; n < L.nn; n += nt) {
-      const int b = n / L.NX, a = n - b * L.NX;
-      P1Smooth<T, NC>::post2(a, b, L.S, B);
-      if (l == 0)
-        for (int c = 0; c < NC; ++c) x_out[NC * n + c] = B.x[NC * n + c];
-    }
-    mark();
-  }
-  if (trace) trace[kTailTraceSlots - 1] += 1;
 }
 
 template <class T, int NC>
@@ -544,7 +572,7 @@ constexpr int coarse_cheb_npt() {
 }
 
 template <class T>
-__global__ void __launch_bounds__(kTailThreads)
+__global__ void __launch_bounds__(kCoarseThreads)
     k_coarse_cheb(const CoarseChebDesc<T, 1>* __restrict__ D, const T* __restrict__ b, T* __restrict__ x_out) {
   TOPO_PDL_ENTRY();
   constexpr int NP = coarse_cheb_npt<T>(), SW = StencilLayout<1>::stride;
@@ -836,6 +864,26 @@ static inline Transfer make_transfer(const LevelSpec& f, const LevelSpec& c) {
   return X;
 }
 
+template <class T, int NC>
+inline LevelSweep<T, NC> level_sweep(const LevelSpec& S, const Transfer& X, const T* st, const T* inner, const T* dinv,
+                                     const T* cheb) {
+  LevelSweep<T, NC> P;
+  std::memset(&P, 0, sizeof(P));
+  P.NX = S.NX;
+  P.NY = S.NY;
+  P.NXc = X.NXc;
+  P.NYc = X.NYc;
+  P.cx = kSweepTileX;
+  P.cy = kSweepTileY;
+  P.st = st;
+  P.inner = inner;
+  P.dinv = dinv;
+  P.cheb = cheb;
+  P.dirf = X.dirf;
+  P.dirc = X.dirc;
+  return P;
+}
+
 // ---------------------------------------------------------------------------
 // graph-resident CG scalars
 // ---------------------------------------------------------------------------
@@ -967,7 +1015,7 @@ void MG<T>::init(const std::vector<LevelSpec>& specs, const ElemRefs* refs, doub
   for (auto& e : ev_)
     if (!e) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
   graph_valid_ = false;
-  build_tail(arena);
+  build_tail();
   cc_buf_ = arena.alloc(sizeof(CoarseChebDesc<T, 1>));
   inner_buf_ = arena.alloc_n<T>(specs.size() * StencilLayout<1>::stride);
 }
@@ -1026,7 +1074,7 @@ void MG<T>::select_coarse_cheb(cudaStream_t s) {
     const LevelSpec& S = specs_[l];
     if (S.p2 || S.NC != 1 || !lv_[l].st || !kK64_[l] || !kM64_[l]) continue;
     const size_t smem = 2 * S.nn() * sizeof(T);  // the two direction buffers
-    if (S.nn() > size_t(kTailThreads) * coarse_cheb_npt<T>() || smem > kTailSmemBudget) continue;
+    if (S.nn() > size_t(kCoarseThreads) * coarse_cheb_npt<T>() || smem > kCoarseSharedBudget) continue;
     const size_t nt = S.ntri();
     std::vector<double> kk(nt), km(nt);
     if (cudaMemcpyAsync(kk.data(), kK64_[l], nt * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -1062,7 +1110,7 @@ void MG<T>::select_coarse_cheb(cudaStream_t s) {
       h.C.c1[k] = T(c1[k]);
       h.C.c2[k] = T(c2[k]);
     }
-    const int limit = int(kTailSmemBudget);
+    const int limit = int(kCoarseSharedBudget);
     if (cudaMemcpyAsync(cc_buf_, &h, sizeof(h), cudaMemcpyHostToDevice, s) != cudaSuccess ||
         cudaFuncSetAttribute(k_coarse_cheb<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
       cudaGetLastError();
@@ -1077,78 +1125,35 @@ void MG<T>::select_coarse_cheb(cudaStream_t s) {
   if (cheb_coarse_ != prev) graph_valid_ = false;
 }
 
-// Chooses the tail levels (smallest levels whose shared vectors fit the
-// budget, never level 0) and uploads their descriptor.
+// Chooses the levels of k_level_tail (FP32): from the first level with at most kTailNodes
+// nodes (never level 0) whose shared memory fits, down to the coarsest.
 template <class T>
-void MG<T>::build_tail(Arena& arena) {
+void MG<T>::build_tail() {
   tail_ = -1;
-  tail_desc_ = nullptr;
-  tail_smem_ = 0;
   const int L = levels();
-  const int stride = specs_[L - 1].NC == 2 ? StencilLayout<2>::stride : StencilLayout<1>::stride;
-  size_t bytes = 0;
-  int first = L;
-  for (int l = L - 1; l >= 1; --l) {
-    // five vectors, the inverse diagonal and the stencil
-    const size_t add = (6 * specs_[l].ndof() + size_t(stride) * specs_[l].nn()) * sizeof(T);
-    if (specs_[l].p2 || !lv_[l].st || bytes + add > kTailSmemBudget || L - l > kTailMaxLevels) break;
-    bytes += add;
-    first = l;
-  }
-  if (first >= L - 1) return;  // fewer than two levels: nothing to gain
-  auto build = [&](auto nc_tag) {
-    constexpr int NC = decltype(nc_tag)::value;
-    TailDesc<T, NC> h;
-    std::memset(&h, 0, sizeof(h));
-    h.nlev = L - first;
-    h.cinv = cinv_;
-    int off = 0;
-    constexpr int kAlign = 16 / int(sizeof(T));  // shared offsets in 16-byte units (stage16)
-    auto align = [&](int o) { return (o + kAlign - 1) / kAlign * kAlign; };
-    for (int k = 0; k < h.nlev; ++k) {
-      const int l = first + k;
-      TailLevel<T, NC>& d = h.lv[k];
-      d.S = P1Stencil<T, NC>{specs_[l].nx, specs_[l].ny, specs_[l].dir, lv_[l].st};
-      if (l + 1 < L) d.X = make_transfer(specs_[l], specs_[l + 1]);
+  auto plan = [&](auto& P, int first) {
+    std::memset(&P, 0, sizeof(P));
+    P.nlev = L - 1 - first;
+    P.cinv = cinv_;
+    for (int l = first; l < L; ++l) {
+      auto& d = P.lv[l - first];
+      d.NX = specs_[l].NX;
+      d.NY = specs_[l].NY;
+      d.st = lv_[l].st;
       d.dinv = lv_[l].dinv;
       d.cheb = cheb_ + 8 * l;
-      d.NX = specs_[l].NX;
-      d.nn = int(specs_[l].nn());
-      d.off = off;
-      off += 5 * NC * d.nn;
+      d.dir = specs_[l].dir;
     }
-    for (int k = 0; k < h.nlev; ++k) {
-      TailLevel<T, NC>& d = h.lv[k];
-      d.soff = off = align(off);
-      off += StencilLayout<NC>::stride * d.nn;
-      d.doff = off = align(off);
-      off += NC * d.nn;
-    }
-    h.smem_elems = off;
-    h.trace = nullptr;
-    if (profile_levels) {
-      h.trace = static_cast<long long*>(arena.alloc(kTailTraceSlots * sizeof(long long)));
-      if (h.trace) cudaMemset(h.trace, 0, kTailTraceSlots * sizeof(long long));
-      tail_trace_ = h.trace;
-    }
-    void* p = arena.alloc(sizeof(h));
-    if (!p) return;
-    cudaMemcpy(p, &h, sizeof(h), cudaMemcpyHostToDevice);
-    // the limit is a property of the kernel, shared by every context in the
-    // process: always the budget, so that no context lowers another's
-    const int static_bytes = int(sizeof(TailLevel<T, NC>) * kTailMaxLevels + sizeof(T) * kCoarseMaxDofs * kCoarseMaxDofs);
-    const int limit = int(std::min<size_t>(kTailSmemBudget, size_t(227 * 1024 - static_bytes)));
-    if (size_t(off) * sizeof(T) > size_t(limit) ||
-        cudaFuncSetAttribute(k_tail_vcycle<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
-      cudaGetLastError();
-      return;
-    }
-    tail_desc_ = p;
-    tail_smem_ = size_t(off) * sizeof(T);
-    tail_ = first;
+    P.plan();
+    return size_t(P.shared) * sizeof(T) <= kTailShared;
   };
-  if (specs_[first].NC == 2) build(std::integral_constant<int, 2>{});
-  else build(std::integral_constant<int, 1>{});
+  if (sizeof(T) == 8) return;
+  for (int l = std::max(1, L - 1 - kTailMaxLevels); l + 1 < L && tail_ < 0; ++l) {
+    if (specs_[l].nn() > size_t(kTailNodes)) continue;
+    bool ok = true;
+    for (int k = l; k < L; ++k) ok &= !specs_[k].p2 && lv_[k].st;
+    if (ok && (specs_[l].NC == 2 ? plan(tail2_, l) : plan(tail1_, l))) tail_ = l;
+  }
 }
 
 template <class T>
@@ -1366,16 +1371,6 @@ int MG<T>::setup(cudaStream_t s) {
   return cudaStreamSynchronize(s) == cudaSuccess ? 0 : -5;
 }
 
-// One V-cycle from level l down: fused degree-2 Chebyshev pre-smoothing from
-// x = 0, residual restriction, coarse correction, fused post-smoothing.
-template <class T>
-void MG<T>::tail_profile(std::vector<long long>& cycles) const {
-  cycles.clear();
-  if (!tail_trace_) return;
-  cycles.resize(kTailTraceSlots);
-  cudaMemcpy(cycles.data(), tail_trace_, kTailTraceSlots * sizeof(long long), cudaMemcpyDeviceToHost);
-}
-
 template <class T>
 void MG<T>::flush_level_profile() {
   if (prof_events_.empty()) return;
@@ -1413,6 +1408,8 @@ void MG<T>::vcycle_level(int l, const T* b, T* x, cudaStream_t s) {
   vcycle_level_body(l, b, x, s);
 }
 
+// One V-cycle from level l down: fused degree-2 Chebyshev pre-smoothing from
+// x = 0, residual restriction, coarse correction, fused post-smoothing.
 template <class T>
 void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
   Lev& v = lv_[l];
@@ -1420,18 +1417,19 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
   const LevelSpec& S = specs_[l];
   if (l == cheb_coarse_ && cc_desc_) {
     KClock kc(s, "coarse Chebyshev (one CTA)", l, 0.0);
-    launch_pdl(k_coarse_cheb<T>, 1, kTailThreads, cc_smem_, s, static_cast<const CoarseChebDesc<T, 1>*>(cc_desc_), b, x);
+    launch_pdl(k_coarse_cheb<T>, 1, kCoarseThreads, cc_smem_, s, static_cast<const CoarseChebDesc<T, 1>*>(cc_desc_), b, x);
     ++launches;
     return;
   }
-  if (l == tail_ && tail_desc_ && use_tail) {
-    KClock kc(s, "tail V-cycle (one CTA)", l, 0.0);
-    if (S.NC == 2)
-      launch_pdl(k_tail_vcycle<T, 2>, 1, kTailThreads, tail_smem_, s, static_cast<const TailDesc<T, 2>*>(tail_desc_), b, x);
-    else
-      launch_pdl(k_tail_vcycle<T, 1>, 1, kTailThreads, tail_smem_, s, static_cast<const TailDesc<T, 1>*>(tail_desc_), b, x);
-    ++launches;
-    return;
+  if constexpr (sizeof(T) == 4) {
+    if (l == tail_ && use_tail) {
+      KClock kc(s, "V-cycle tail (one CTA)", l, 0.0);
+      const dim3 nt(unsigned(S.nn() + 31) / 32 * 32);
+      if (S.NC == 2) launch_pdl(k_level_tail<T, 2>, 1, nt, tail2_.shared * sizeof(T), s, tail2_, b, x);
+      else launch_pdl(k_level_tail<T, 1>, 1, nt, tail1_.shared * sizeof(T), s, tail1_, b, x);
+      ++launches;
+      return;
+    }
   }
   if (l == L - 1) {
     launch_pdl(k_dense_matvec<T>, 1, 256, 0, s, static_cast<const T*>(cinv_), b, x, int(S.ndof()));
@@ -1473,36 +1471,30 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
     launches += 2;
     return;
   }
-  // the level's operator: assembled stencil when there is one, else on the fly
-  // algorithmic bytes of the transfers and of a smoothing step on a stencil level
+  // algorithmic bytes of the transfers
   const double nf = double(S.nn()) * S.NC, ncrs = double(X.NXc) * X.NYc * S.NC;
   const double rbytes = (nf + ncrs) * sizeof(T), pbytes = (2 * nf + ncrs) * sizeof(T);
-  auto sbytes = [&](int mode) {
-    // the assembled stencil row of every node (7 NC x NC blocks, padded to 16 bytes), unless
-    // the level shares one interior row
-    const double row = double((7 * S.NC * S.NC * sizeof(T) + 15) / 16 * 16);
-    return mode_vectors(mode, false, false) * nf * sizeof(T) + (v.inner ? 0.0 : row * double(S.nn()));
-  };
-  auto run = [&](auto nc_tag, const auto& P) {
+  // per sweep: the stencil row of every node (7 NC x NC blocks, padded to 16 bytes; one row
+  // where the level shares it), down b, D^-1 read, x and the coarse residual written, up
+  // b, D^-1, x and the coarse correction read, x written
+  const double row = v.inner ? 0.0 : double((7 * S.NC * S.NC * sizeof(T) + 15) / 16 * 16) * double(S.nn());
+  auto run = [&](auto nc_tag) {
     constexpr int NC = decltype(nc_tag)::value;
-    using PP = std::decay_t<decltype(P)>;
-    constexpr bool ST = std::is_same<PP, P1Stencil<T, NC>>::value;
-    const char* fam_pre = ST ? "P1 stencil Pre" : "P1 node Pre";
-    const char* fam_res = ST ? "P1 stencil Res" : "P1 node Res";
-    const char* fam_first = ST ? "P1 stencil First" : "P1 node First";
-    const char* fam_post = ST ? "P1 stencil Post2" : "P1 node Post2";
-    { KClock kc(s, fam_pre, l, sbytes(kP2Pre)); launch_pdl(k_p1_smooth<T, NC, kP2Pre, PP>, gf, kRowThreads, 0, s, P, B); }
-    { KClock kc(s, fam_res, l, sbytes(kP2Res)); launch_pdl(k_p1_smooth<T, NC, kP2Res, PP>, gf, kRowThreads, 0, s, P, B); }
+    const LevelSweep<T, NC> P = level_sweep<T, NC>(S, X, v.st, v.inner, v.dinv, cheb_ + 8 * l);
+    const dim3 g((X.NXc + P.cx - 1) / P.cx, (X.NYc + P.cy - 1) / P.cy);
+    auto threads = [](int nodes) { return dim3(unsigned(nodes + 31) / 32 * 32); };
     {
-      KClock kc(s, "restriction", l, rbytes);
-      launch_pdl(k_restrict<T, NC>, gc, kRowThreads, 0, s, X, static_cast<const T*>(v.r), c.b, static_cast<const T*>(nullptr));
+      KClock kc(s, "P1 level down", l, row + (3 * nf + ncrs) * sizeof(T));
+      launch_pdl(k_level_down<T, NC>, g, threads(P.down_w() * P.down_h()), P.down_shared() * sizeof(T), s, P, b, v.x2,
+                 c.b);
     }
-    launches += 3;
     vcycle_level(l + 1, c.b, c.x, s);
-    { KClock kc(s, "prolongation", l, pbytes); launch_pdl(k_prolong_add<T, NC>, gf, kRowThreads, 0, s, X, static_cast<const T*>(c.x), x); }
-    { KClock kc(s, fam_first, l, sbytes(kP2First)); launch_pdl(k_p1_smooth<T, NC, kP2First, PP>, gf, kRowThreads, 0, s, P, B); }
-    { KClock kc(s, fam_post, l, sbytes(kP2Post2)); launch_pdl(k_p1_smooth<T, NC, kP2Post2, PP>, gf, kRowThreads, 0, s, P, B); }
-    launches += 3;
+    {
+      KClock kc(s, "P1 level up", l, row + (4 * nf + ncrs) * sizeof(T));
+      launch_pdl(k_level_up<T, NC>, g, threads(P.up_w() * P.up_h()), P.up_shared() * sizeof(T), s, P, b,
+                 static_cast<const T*>(v.x2), static_cast<const T*>(c.x), x);
+    }
+    launches += 2;
   };
   // large levels without a stencil: the column march (element products per cell)
   auto run_march = [&](auto nc_tag, const auto& P) {
@@ -1530,15 +1522,12 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
   };
   using I2 = std::integral_constant<int, 2>;
   using I1 = std::integral_constant<int, 1>;
-  const bool march = !v.st && use_p1_march;
   if (S.NC == 2) {
-    if (v.st) run(I2{}, P1Stencil<T, 2>{S.nx, S.ny, S.dir, v.st, v.inner});
-    else if (march) run_march(I2{}, make_p1<T, 2>(S, refs_[l], v.kK, nullptr));
-    else run(I2{}, make_p1<T, 2>(S, refs_[l], v.kK, nullptr));
+    if (v.st) run(I2{});
+    else run_march(I2{}, make_p1<T, 2>(S, refs_[l], v.kK, nullptr));
   } else {
-    if (v.st) run(I1{}, P1Stencil<T, 1>{S.nx, S.ny, S.dir, v.st, v.inner});
-    else if (march) run_march(I1{}, make_p1<T, 1>(S, refs_[l], v.kK, v.kM));
-    else run(I1{}, make_p1<T, 1>(S, refs_[l], v.kK, v.kM));
+    if (v.st) run(I1{});
+    else run_march(I1{}, make_p1<T, 1>(S, refs_[l], v.kK, v.kM));
   }
 }
 
@@ -1608,7 +1597,7 @@ void MG<T>::tune_marches(cudaStream_t s) {
   for (int l = 0; l < L; ++l) {
     const LevelSpec& S = specs_[l];
     Lev& v = lv_[l];
-    if (l == tail_ && tail_desc_ && use_tail) break;  // the tail runs the rest
+    if (l == tail_ && use_tail) break;  // the tail runs the rest
     if (l == cheb_coarse_ && cc_desc_) break;
     if (S.p2) {
       const size_t n = S.ndof();
@@ -1623,7 +1612,7 @@ void MG<T>::tune_marches(cudaStream_t s) {
       const size_t max_blocks = red_ ? size_t(red_->blocks) * 8 : 0;
       choose(march_family(true, sizeof(T), 2), S.nx, S.ny, p2_march_bps<T, kP2Apply>(), max_blocks,
              [&](int seg) { launch_p2_mode<T, kP2Apply>(p2_op_, xi_, io, s, seg); });
-    } else if (!v.st && use_p1_march && l + 1 < L) {
+    } else if (!v.st && l + 1 < L) {
       cudaMemsetAsync(v.x, 0, S.ndof() * sizeof(T), s);
       P1Io<T> io;
       std::memset(&io, 0, sizeof(io));
