@@ -795,6 +795,35 @@ void emu_fluid_apply(int nx, int ny, double W, double H, double q, const double*
     y[2 * n2 + k] = fluid_gather_vertex(out.data(), nx, ny, int(k % (nx + 1)), int(k / (nx + 1)), kFluidOut, 12);
 }
 
+// the operator by output node (unclamped rows, pm off the pressure)
+void emu_fluid_apply_nodes(int nx, int ny, double W, double H, double q, double pm, const double* rho, const double* x,
+                           double* y) {
+  FluidTables E;
+  fluid_tables(W / nx, H / ny, E);
+  const FluidPenal pen = emu_fluid_penal(q);
+  const size_t nt = size_t(2) * nx * ny, n2 = size_t(2 * nx + 1) * (2 * ny + 1), nv = size_t(nx + 1) * (ny + 1);
+  std::vector<double> mk(nt * kFluidMass);
+  for (size_t t = 0; t < nt; ++t) {
+    double r[3];
+    fluid_tri_rho(rho, nx, t, r);
+    fluid_tri_mass(E, pen, r, mk.data() + t * kFluidMass);
+    for (int i = 0; i < 6; ++i)
+      for (int j = i; j < 6; ++j) mk[t * kFluidMass + fluid_mass_index(i, j)] += E.lap[t & 1][i][j];
+  }
+  for (size_t i = 0; i < n2 + nv; ++i) {
+    const FluidNode F = fluid_output(i, nx, ny);
+    double v[2];
+    fluid_node_rows(E, mk.data(), nx, ny, F, x, x + 2 * n2, pm, v);
+    if (F.cls == 4) {
+      y[2 * n2 + size_t(F.j) * (nx + 1) + F.i] = v[0];
+    } else {
+      const size_t node = size_t(2 * F.j + (F.cls >> 1)) * (2 * nx + 1) + 2 * F.i + (F.cls & 1);
+      y[2 * node] = v[0];
+      y[2 * node + 1] = v[1];
+    }
+  }
+}
+
 double emu_fluid_objective(int nx, int ny, double W, double H, double q, double mu, const double* rho,
                            const double* u) {
   FluidTables E;

@@ -11,7 +11,12 @@
 // preconditioned with the block-diagonal
 //   diag( P1-iso-P2 V-cycles of K + alpha M on the (2nx)x(2ny) lattice, one per component,
 //         lumped-mass inverse + V-cycle of the 1/alpha-weighted P1 Laplacian )
-// (a variable-coefficient Cahouet-Chabard Schur-complement approximation).
+// (a variable-coefficient Cahouet-Chabard Schur-complement approximation).  The Krylov basis,
+// directions, operator and Gram-Schmidt are FP64; the V-cycles run in FP32, both velocity
+// components in one batch, the pressure's beside them: flexible GMRES keeps A Z = V H in FP64
+// for whatever directions it is given, and this GPU issues FP64 at 1/64 of its FP32 rate.  One
+// restart cycle is one CUDA graph whose WHILE body is an iteration; the Givens rotations and
+// the stopping test run on the device.
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
@@ -28,6 +33,7 @@
 #include "topo_setup.h"
 
 namespace topo {
+extern template class MG<float>;
 extern template class MG<double>;
 }  // namespace topo
 
@@ -35,7 +41,11 @@ using namespace topo;
 
 namespace {
 
-constexpr int kFluidRestart = 30;
+// Restart length: the long one unless its 2 m + 1 vectors pass kFluidBasisMax bytes.
+constexpr int kFluidRestart = 30, kFluidRestartMax = 60;
+constexpr size_t kFluidBasisMax = size_t(16) << 30;
+constexpr int kDotGroup = 8;  // basis vectors of one block of the Gram-Schmidt products
+constexpr int kDotGroups = (kFluidRestartMax + kDotGroup) / kDotGroup;
 constexpr double kLaplaceShift = 1e-3;  // mass shift of the pressure Laplacian (its constant mode)
 
 // ---------------------------------------------------------------------------
@@ -47,43 +57,63 @@ __global__ void k_fluid_mass(int nx, int ny, const FluidTables* __restrict__ E, 
   TOPO_GRID_STRIDE(t, nt) {
     double r[3];
     fluid_tri_rho(rho, nx, t, r);
-    fluid_tri_mass(*E, pen, r, mass + t * kFluidMass);
+    double* m = mass + t * kFluidMass;
+    fluid_tri_mass(*E, pen, r, m);
+    for (int i = 0; i < 6; ++i)
+      for (int j = i; j < 6; ++j) m[fluid_mass_index(i, j)] += E->lap[t & 1][i][j];
   }
 }
 
-// x = [u (2 n2, interleaved) | p (nv)]
-__global__ void k_fluid_tri(int nx, int ny, const FluidTables* __restrict__ E, const double* __restrict__ mass,
-                            const double* __restrict__ x, double* __restrict__ out) {
-  const size_t nt = size_t(2) * nx * ny;
-  const size_t n2 = size_t(2 * nx + 1) * (2 * ny + 1);
-  TOPO_GRID_STRIDE(t, nt) {
-    size_t nd[6], vt[3];
-    fluid_tri_nodes(nx, t, nd);
-    fluid_tri_vertices(nx, t, vt);
-    double ue[6][2], pe[3];
-    for (int k = 0; k < 6; ++k) {
-      ue[k][0] = x[2 * nd[k]];
-      ue[k][1] = x[2 * nd[k] + 1];
-    }
-    for (int k = 0; k < 3; ++k) pe[k] = x[2 * n2 + vt[k]];
-    fluid_tri_apply(*E, int(t & 1), mass + t * kFluidMass, ue, pe, out + t * kFluidOut);
-  }
-}
+// Device-side state of one restart cycle.  v_0 .. v_j are the basis so far, column j of the
+// Hessenberg matrix is being formed.
+struct FluidKrylov {
+  int j, it, maxit, status;  // status: 1 running, 0 done, 4 non-finite
+  int second, pad;           // the column needs a second Gram-Schmidt pass
+  double target;             // residual norm to reach
+  double psum, zsum;         // sums of the pressure parts of v_j and of z_j
+  double ww, hn;             // |w|^2 before and |w| after the orthogonalisation
+  double h[kFluidRestartMax + 1], hp[kFluidRestartMax + 1];  // the column, and a pass's products
+  double cs[kFluidRestartMax], sn[kFluidRestartMax], gv[kFluidRestartMax + 1], y[kFluidRestartMax];
+  double H[(kFluidRestartMax + 1) * kFluidRestartMax];
+};
 
-__global__ void k_fluid_gather(int nx, int ny, const double* __restrict__ tri_out, const double* __restrict__ x,
-                               double* __restrict__ y, int clamp) {
-  const int NX = 2 * nx + 1, NY = 2 * ny + 1, VX = nx + 1;
+// y = A x, x = [u (2 n2, interleaved) | p (nv)], by output node: the element matrices' rows are
+// formed where they are needed, each once.  With K: x = z_j with its pressure's mean taken off
+// (and written back), y = v_(j+1).  clamp: boundary velocity rows are the identity.
+// Bound: FP64, 72 products per P2 node, and the latency of up to six triangles' loads.
+// (A thread per triangle into a 128-byte buffer and a gather took 16 + 4 us at 40x40 and
+// 16 + 6 at 128x128.)
+constexpr int kFluidThreads = 128;
+template <bool KRYLOV>
+__global__ void __launch_bounds__(kFluidThreads)
+    k_fluid_apply(int nx, int ny, const FluidTables* __restrict__ E, const double* __restrict__ mk, const double* xin,
+                  double* yout, int clamp, const FluidKrylov* K, size_t n, double* zc) {
+  TOPO_PDL_ENTRY();
+  const int NX = 2 * nx + 1, NY = 2 * ny + 1;
   const size_t n2 = size_t(NX) * NY, nv = size_t(nx + 1) * (ny + 1);
-  TOPO_GRID_STRIDE(i, n2 + nv) {
-    if (i < n2) {
-      double v[2];
-      fluid_gather_node(tri_out, nx, ny, int(i % NX), int(i / NX), clamp != 0, x, v);
-      y[2 * i] = v[0];
-      y[2 * i + 1] = v[1];
+  const double* x = KRYLOV ? xin + size_t(K->j) * n : xin;
+  double* y = KRYLOV ? yout + size_t(K->j + 1) * n : yout;
+  const double pm = KRYLOV ? K->zsum / double(nv) : 0.0;
+  const size_t i = size_t(blockIdx.x) * kFluidThreads + threadIdx.x;
+  if (i >= n2 + nv) return;
+  const FluidNode F = fluid_output(i, nx, ny);
+  double v[2];
+  if (F.cls < 4) {
+    const int a = 2 * F.i + (F.cls & 1), b = 2 * F.j + (F.cls >> 1);
+    const size_t node = size_t(b) * NX + a;
+    if (clamp && fluid_boundary_node(a, b, NX, NY)) {
+      v[0] = x[2 * node];
+      v[1] = x[2 * node + 1];
     } else {
-      const size_t k = i - n2;
-      y[2 * n2 + k] = fluid_gather_vertex(tri_out, nx, ny, int(k % VX), int(k / VX), kFluidOut, 12);
+      fluid_node_rows(*E, mk, nx, ny, F, x, x + 2 * n2, pm, v);
     }
+    y[2 * node] = v[0];
+    y[2 * node + 1] = v[1];
+  } else {
+    const size_t k = size_t(F.j) * (nx + 1) + F.i;
+    fluid_node_rows(*E, mk, nx, ny, F, x, x + 2 * n2, pm, v);
+    y[2 * n2 + k] = v[0];
+    if (KRYLOV) zc[k] = x[2 * n2 + k] - pm;  // the centred pressure, moved into z_j by k_fluid_dot
   }
 }
 
@@ -172,37 +202,232 @@ __global__ void k_fluid_coarsen(const double* __restrict__ kf, int nxf, int nyf,
   }
 }
 
-// planar components of the interleaved velocity, zero on the boundary nodes
-__global__ void k_fluid_split(int NX, int NY, const double* __restrict__ v, double* __restrict__ c0,
-                              double* __restrict__ c1) {
-  const size_t n = size_t(NX) * NY;
-  TOPO_GRID_STRIDE(i, n) {
-    const bool bd = fluid_boundary_node(int(i % NX), int(i / NX), NX, NY);
-    c0[i] = bd ? 0.0 : v[2 * i];
-    c1[i] = bd ? 0.0 : v[2 * i + 1];
-  }
-}
-
-__global__ void k_fluid_merge(int NX, int NY, const double* __restrict__ c0, const double* __restrict__ c1,
-                              double* __restrict__ v) {
-  const size_t n = size_t(NX) * NY;
-  TOPO_GRID_STRIDE(i, n) {
-    const bool bd = fluid_boundary_node(int(i % NX), int(i / NX), NX, NY);
-    v[2 * i] = bd ? 0.0 : c0[i];
-    v[2 * i + 1] = bd ? 0.0 : c1[i];
-  }
-}
-
 // y = x - sum(x)/n with the sum a device scalar (one reduction before); y may be x
 __global__ void k_fluid_center(const double* x, double* y, size_t n, const double* __restrict__ sum) {
   const double m = *sum / double(n);
   TOPO_GRID_STRIDE(i, n) y[i] = x[i] - m;
 }
 
-// z = r / m_lumped + zl
-__global__ void k_fluid_pcombine(const double* __restrict__ r, const double* __restrict__ ml,
-                                 const double* __restrict__ zl, double* __restrict__ z, size_t n) {
-  TOPO_GRID_STRIDE(i, n) z[i] = r[i] / ml[i] + zl[i];
+// ---------------------------------------------------------------------------
+// one flexible-GMRES iteration
+// ---------------------------------------------------------------------------
+// FP32 right-hand sides of the preconditioner: the planar velocity components of v_j (zero on
+// the boundary) and its pressure less the mean
+__global__ void k_fluid_split(int NX, int NY, const double* V, size_t n, size_t nv, const FluidKrylov* K,
+                              float* c, float* pt) {
+  TOPO_PDL_ENTRY();
+  const size_t n2 = size_t(NX) * NY;
+  const double* v = V + size_t(K->j) * n;
+  const double pm = K->psum / double(nv);
+  TOPO_GRID_STRIDE(i, n2 + nv) {
+    if (i < n2) {
+      const bool bd = fluid_boundary_node(int(i % NX), int(i / NX), NX, NY);
+      c[i] = bd ? 0.0f : float(v[2 * i]);
+      c[n2 + i] = bd ? 0.0f : float(v[2 * i + 1]);
+    } else {
+      pt[i - n2] = float(v[n2 + i] - pm);  // (pressure entry k at 2 n2 + k = n2 + i)
+    }
+  }
+}
+
+// z_j = the V-cycles' velocity, and pressure r / m_lumped + the V-cycle's; sums the pressure
+__global__ void k_fluid_merge(int NX, int NY, const double* V, double* Z, size_t n, size_t nv, const float* c,
+                              const float* pz, const double* ml, double* partials, unsigned* counter, FluidKrylov* K) {
+  TOPO_PDL_ENTRY();
+  const size_t n2 = size_t(NX) * NY;
+  const double* v = V + size_t(K->j) * n + 2 * n2;
+  double* z = Z + size_t(K->j) * n;
+  double s[1] = {0.0};
+  TOPO_GRID_STRIDE(i, n2 + nv) {
+    if (i < n2) {
+      const bool bd = fluid_boundary_node(int(i % NX), int(i / NX), NX, NY);
+      z[2 * i] = bd ? 0.0 : double(c[i]);
+      z[2 * i + 1] = bd ? 0.0 : double(c[n2 + i]);
+    } else {
+      const size_t k = i - n2;
+      const double p = v[k] / ml[k] + double(pz[k]);
+      z[2 * n2 + k] = p;
+      s[0] += p;
+    }
+  }
+  double tot[1];
+  if (finish_reduction<1>(s, partials, counter, tot)) K->zsum = tot[0];
+}
+
+// A pass's products hp_i = v_i . w, i <= j, and |w|^2 (w = v_(j+1)): blockIdx.y takes eight basis
+// vectors, blockIdx.x a share of the entries.  The first pass also moves the centred
+// pressure into z_j (k_fluid_apply could not: other blocks read the uncentred one).
+__global__ void __launch_bounds__(kVecThreads)
+    k_fluid_dot(const double* V, double* Z, size_t n, size_t nv, const double* zc, int pass, double* partials,
+                unsigned* counters, FluidKrylov* K) {
+  TOPO_PDL_ENTRY();
+  const int j = K->j, i0 = blockIdx.y * kDotGroup;
+  if (pass == 1 && !K->second) return;
+  if (pass == 0 && blockIdx.y == 0) {
+    double* z = Z + size_t(j) * n + (n - nv);
+    TOPO_GRID_STRIDE(k, nv) z[k] = zc[k];
+  }
+  if (i0 > j) return;
+  const double* w = V + size_t(j + 1) * n;
+  const double* v = V + size_t(i0) * n;
+  const int count = min(kDotGroup, j + 1 - i0);
+  double s[kDotGroup + 1];
+#pragma unroll
+  for (int k = 0; k <= kDotGroup; ++k) s[k] = 0.0;
+  if (count == kDotGroup) {
+    TOPO_GRID_STRIDE(i, n) {
+      const double wi = w[i];
+#pragma unroll
+      for (int k = 0; k < kDotGroup; ++k) s[k] += v[size_t(k) * n + i] * wi;
+      if (i0 == 0) s[kDotGroup] += wi * wi;
+    }
+  } else {
+    TOPO_GRID_STRIDE(i, n) {
+      const double wi = w[i];
+#pragma unroll
+      for (int k = 0; k < kDotGroup; ++k)
+        if (k < count) s[k] += v[size_t(k) * n + i] * wi;
+      if (i0 == 0) s[kDotGroup] += wi * wi;
+    }
+  }
+  double tot[kDotGroup + 1];
+  if (finish_reduction<kDotGroup + 1>(s, partials + size_t(blockIdx.y) * (kDotGroup + 1) * gridDim.x,
+                                      counters + blockIdx.y, tot, blockIdx.x, gridDim.x)) {
+    for (int k = 0; k < count; ++k) K->hp[i0 + k] = tot[k];
+    if (i0 == 0) K->ww = tot[kDotGroup];
+  }
+}
+
+// w -= sum hp_i v_i.  The first pass (classical Gram-Schmidt) decides on the second: it is needed
+// where more than half of |w|^2 cancelled (Kahan's "twice is enough"); the second sums |w|^2.
+__global__ void __launch_bounds__(kVecThreads)
+    k_fluid_sub(double* V, size_t n, int pass, double* partials, unsigned* counter, FluidKrylov* K) {
+  TOPO_PDL_ENTRY();
+  __shared__ double h[kFluidRestartMax + 1];
+  const int j = K->j;
+  if (pass == 1 && !K->second) return;
+  for (int i = threadIdx.x; i <= j; i += blockDim.x) h[i] = K->hp[i];
+  __syncthreads();
+  double* w = V + size_t(j + 1) * n;
+  double s[1] = {0.0};
+  TOPO_GRID_STRIDE(i, n) {
+    double a = w[i];
+    int k = 0;
+    for (; k + 8 <= j + 1; k += 8) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a -= h[k + q] * V[size_t(k + q) * n + i];
+    }
+    for (; k <= j; ++k) a -= h[k] * V[size_t(k) * n + i];
+    w[i] = a;
+    s[0] += a * a;
+  }
+  if (pass == 0) {
+    // (a kernel after this one reads `second`; none of this grid does)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      double hh = 0.0;
+      for (int i = 0; i <= j; ++i) {
+        K->h[i] = h[i];
+        hh += h[i] * h[i];
+      }
+      const double ww = K->ww, est = ww - hh;
+      K->second = !(est >= 0.5 * ww);
+      K->hn = sqrt(est);
+    }
+    return;
+  }
+  double tot[1];
+  if (finish_reduction<1>(s, partials, counter, tot)) {
+    for (int i = 0; i <= j; ++i) K->h[i] += h[i];
+    K->hn = sqrt(tot[0]);
+  }
+}
+
+// v_(j+1) = w / |w| and the sum of its pressure; then the last block rotates the column into
+// the triangular factor, updates the residual norm and decides whether the cycle goes on
+__global__ void __launch_bounds__(kVecThreads)
+    k_fluid_next(double* V, size_t n, size_t nv, int m, double* partials, unsigned* counter, FluidKrylov* K,
+                 cudaGraphConditionalHandle cond, int use_cond) {
+  TOPO_PDL_ENTRY();
+  __shared__ double hs[kFluidRestartMax + 1], cs[kFluidRestartMax], sn[kFluidRestartMax];
+  const int j = K->j;
+  for (int i = threadIdx.x; i <= j; i += blockDim.x) {
+    hs[i] = K->h[i];
+    if (i < j) {
+      cs[i] = K->cs[i];
+      sn[i] = K->sn[i];
+    }
+  }
+  const double hn = K->hn, f = hn > 0 ? 1.0 / hn : 1.0;
+  double* w = V + size_t(j + 1) * n;
+  double s[1] = {0.0};
+  TOPO_GRID_STRIDE(i, n) {
+    const double v = w[i] * f;
+    w[i] = v;
+    if (i >= n - nv) s[0] += v;
+  }
+  double tot[1];
+  if (!finish_reduction<1>(s, partials, counter, tot)) return;
+  K->psum = tot[0];
+  double up = hs[0];
+  for (int i = 0; i < j; ++i) {
+    const double lo = hs[i + 1], c = cs[i], t = sn[i];
+    K->H[i * kFluidRestartMax + j] = c * up + t * lo;
+    up = -t * up + c * lo;
+  }
+  const double den = hypot(up, hn);
+  const double c = den > 0 ? up / den : 1.0, t = den > 0 ? hn / den : 0.0;
+  K->cs[j] = c;
+  K->sn[j] = t;
+  K->H[j * kFluidRestartMax + j] = den;
+  const double g = K->gv[j];
+  K->gv[j + 1] = -t * g;
+  K->gv[j] = c * g;
+  K->j = j + 1;
+  K->it += 1;
+  int st = 1;
+  if (!isfinite(hn)) st = 4;
+  else if (fabs(t * g) <= K->target || hn == 0.0 || j + 1 >= m || K->it >= K->maxit) st = 0;
+  K->status = st;
+  if (use_cond) cudaGraphSetConditional(cond, st == 1 ? 1u : 0u);
+}
+
+__global__ void k_fluid_start(FluidKrylov* K, double beta, double target, int it, int maxit) {
+  K->j = 0;
+  K->it = it;
+  K->maxit = maxit;
+  K->status = 1;
+  K->target = target;
+  K->gv[0] = beta;
+}
+
+// y = R^-1 g by one warp: column by column, the lanes hold the remaining right-hand side
+__global__ void __launch_bounds__(32) k_fluid_backsolve(FluidKrylov* K) {
+  constexpr int P = (kFluidRestartMax + 31) / 32;
+  const int k = K->j, lane = threadIdx.x;
+  double g[P];
+  for (int q = 0; q < P; ++q) g[q] = lane + 32 * q < k ? K->gv[lane + 32 * q] : 0.0;
+  for (int i = k - 1; i >= 0; --i) {
+    const double d = K->H[i * kFluidRestartMax + i];
+    const double y = __shfl_sync(0xffffffffu, i < 32 ? g[0] : g[P - 1], i & 31) / d;
+    const double yi = d != 0.0 ? y : 0.0;
+    if (lane == 0) K->y[i] = yi;
+    for (int q = 0; q < P; ++q)
+      if (lane + 32 * q < i) g[q] -= K->H[(lane + 32 * q) * kFluidRestartMax + i] * yi;
+  }
+}
+static_assert(kFluidRestartMax <= 64, "two values per lane");
+
+// x += sum_i y_i z_i over the cycle's directions
+__global__ void k_fluid_update(double* x, const double* Z, size_t n, const FluidKrylov* K) {
+  __shared__ double y[kFluidRestartMax];
+  const int k = K->j;
+  for (int i = threadIdx.x; i < k; i += blockDim.x) y[i] = K->y[i];
+  __syncthreads();
+  TOPO_GRID_STRIDE(i, n) {
+    double a = x[i];
+    for (int q = 0; q < k; ++q) a += y[q] * Z[size_t(q) * n + i];
+    x[i] = a;
+  }
 }
 
 // zero the boundary velocity rows: b[2i+c] = 0 at boundary nodes
@@ -234,33 +459,50 @@ struct topo_fluid_ctx {
   FluidTables host_tab{};
   FluidTables* tab = nullptr;  // device copy
   double* ub = nullptr;        // boundary data (interleaved, zero inside)
-  double* mass = nullptr;      // [tri][21]
-  double* tri_out = nullptr;   // [tri][16]
+  double* mass = nullptr;      // [tri][21], the Laplacian added
   double* tri3 = nullptr;      // [tri][3]
   double* ml = nullptr;        // lumped CG1 mass (vertex weights)
   double* ones = nullptr;      // nv ones (sums by a dot)
   double* rhs = nullptr;       // n
   double* x = nullptr;         // n (interior velocity | pressure)
+  int m = kFluidRestart;       // restart length
   double* V = nullptr;         // (m + 1) n
   double* Z = nullptr;         // m n
+  FluidKrylov* kry = nullptr;
+  double* dots = nullptr;      // partial sums and counters of the Gram-Schmidt products
+  unsigned* dot_counters = nullptr;
+  int* hstat = nullptr;        // pinned: j, it, maxit, status of the cycle
+  double* zc = nullptr;        // nv: z_j's centred pressure
   double* t = nullptr;         // n
-  double* c0 = nullptr;        // planar velocity components (n2 each)
-  double* c1 = nullptr;
-  double* z0 = nullptr;
-  double* z1 = nullptr;
-  double* pt = nullptr;        // nv scratch
-  double* pz = nullptr;
+  float* c = nullptr;          // preconditioner: planar velocity components (2 n2) in
+  float* z = nullptr;          // and out,
+  float* pt = nullptr;         // pressure (nv) in
+  float* pz = nullptr;         // and out
   double* gb = nullptr;        // gradient right-hand side (nv)
   // preconditioner hierarchies
   std::vector<LevelSpec> uspec, pspec;
   std::vector<ElemRefs> urefs, prefs;
   std::vector<double*> uK, uM, pK, pM;
-  MG<double> mgu, mgp;
+  MG<float> mgu, mgp;
+  // graph of one restart cycle, its recording stream, and the pressure's V-cycle beside the
+  // velocity's
+  cudaGraphExec_t graph = nullptr;
+  bool use_graph = true;
+  int graph_levels[2] = {-1, -1};  // the coarse solves' levels it was recorded with
+  long long body_nodes = 0;  // kernels of one recorded iteration
+  cudaStream_t cap = nullptr, side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   topo_ctx* proj = nullptr;  // the CG1 projection (mass-matrix solve: a filter of radius 0)
 
   ~topo_fluid_ctx() {
+    if (graph) cudaGraphExecDestroy(graph);
+    for (cudaStream_t c : {cap, side})
+      if (c) cudaStreamDestroy(c);
+    for (cudaEvent_t e : {fork, join})
+      if (e) cudaEventDestroy(e);
     if (proj) topo_destroy(proj);
     if (red.host) cudaFreeHost(red.host);
+    if (hstat) cudaFreeHost(hstat);
   }
   int fail(int code, const char* fmt, ...) {
     char buf[512];
@@ -294,27 +536,112 @@ struct topo_fluid_ctx {
     k_fluid_center<<<grid(nv), kVecThreads, 0, s>>>(xp, yp, nv, red.out);
     launches += 2;
   }
-  // y = A x: per-triangle rows, then the node / vertex gathers
+  // y = A x
   void apply(const double* xin, double* y, bool clamp, cudaStream_t s) {
-    const size_t nt = size_t(2) * nx * ny;
-    k_fluid_tri<<<grid(nt), kVecThreads, 0, s>>>(nx, ny, tab, mass, xin, tri_out);
-    k_fluid_gather<<<grid(n2 + nv), kVecThreads, 0, s>>>(nx, ny, tri_out, xin, y, clamp ? 1 : 0);
-    launches += 2;
+    const unsigned g = unsigned((n2 + nv + kFluidThreads - 1) / kFluidThreads);
+    k_fluid_apply<false><<<g, kFluidThreads, 0, s>>>(nx, ny, tab, mass, xin, y, clamp ? 1 : 0, nullptr, n, nullptr);
+    ++launches;
   }
-  // z = P r (block-diagonal preconditioner)
-  void precond(const double* r, double* z, cudaStream_t s) {
-    k_fluid_split<<<grid(n2), kVecThreads, 0, s>>>(NX(), NY(), r, c0, c1);
-    mgu.vcycle(c0, z0, s);
-    mgu.vcycle(c1, z1, s);
-    k_fluid_merge<<<grid(n2), kVecThreads, 0, s>>>(NX(), NY(), z0, z1, z);
-    const double* rp = r + 2 * n2;
-    center(rp, pt, s);
-    mgp.vcycle(pt, pz, s);
-    k_fluid_pcombine<<<grid(nv), kVecThreads, 0, s>>>(rp, ml, pz, pp(z), nv);
-    center(pp(z), pp(z), s);
-    launches += 3;
+  // one iteration of the cycle in kry, on s
+  void iteration(cudaStream_t s, cudaGraphConditionalHandle cond, int use_cond) {
+    const unsigned gn = unsigned(grid(n2 + nv)), ga = unsigned((n2 + nv + kFluidThreads - 1) / kFluidThreads);
+    const unsigned gd = unsigned(red.blocks_for(n)), gv = unsigned(grid(n));
+    const double *Vc = V, *mlc = ml, *zcc = zc, *mkc = mass;
+    const FluidTables* tc = tab;
+    const FluidKrylov* kc = kry;
+    launch_pdl(k_fluid_split, gn, kVecThreads, 0, s, NX(), NY(), Vc, n, nv, kc, c, pt);
+    cudaEventRecord(fork, s);
+    cudaStreamWaitEvent(side, fork, 0);
+    mgp.vcycle(pt, pz, side);
+    cudaEventRecord(join, side);
+    mgu.vcycle(c, z, s);
+    cudaStreamWaitEvent(s, join, 0);
+    k_fluid_merge<<<red.blocks_for(n2 + nv), kVecThreads, 0, s>>>(NX(), NY(), Vc, Z, n, nv, z, pz, mlc, red.partials,
+                                                                 red.counter, kry);
+    const double* Zc = Z;
+    launch_pdl(k_fluid_apply<true>, ga, kFluidThreads, 0, s, nx, ny, tc, mkc, Zc, V, 1, kc, n, zc);
+    for (int pass = 0; pass < 2; ++pass) {
+      launch_pdl(k_fluid_dot, dim3(gd, unsigned((m + kDotGroup - 1) / kDotGroup)), kVecThreads, 0, s, Vc, Z, n, nv, zcc, pass,
+                 dots, dot_counters, kry);
+      launch_pdl(k_fluid_sub, gv, kVecThreads, 0, s, V, n, pass, red.partials, red.counter, kry);
+    }
+    launch_pdl(k_fluid_next, gd, kVecThreads, 0, s, V, n, nv, m, red.partials, red.counter, kry, cond, use_cond);
+    launches += 9;
   }
+  int record();
+  int cycle(cudaStream_t s);
 };
+
+// Records one restart cycle: a WHILE node whose body is an iteration (k_fluid_next decides
+// on the device whether it runs again).  Nothing is launched unless every step succeeded.
+int topo_fluid_ctx::record() {
+  std::lock_guard<std::recursive_mutex> lock(device_lock());
+  cudaGetLastError();
+  const long long l0 = launches + mgu.launches + mgp.launches;
+  cudaGraph_t graph_ = nullptr, body = nullptr;
+  if (cudaGraphCreate(&graph_, 0) != cudaSuccess) return -5;
+  cudaGraphConditionalHandle h = 0;
+  bool ok = cudaGraphConditionalHandleCreate(&h, graph_, 1, cudaGraphCondAssignDefault) == cudaSuccess;
+  cudaGraphNode_t node = nullptr;
+  cudaGraphNodeParams cp = {};
+  if (ok) {
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = h;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    ok = cudaGraphAddNode(&node, graph_, nullptr, nullptr, 0, &cp) == cudaSuccess &&
+         cp.conditional.phGraph_out != nullptr;
+  }
+  if (ok) {
+    body = cp.conditional.phGraph_out[0];
+    ok = cudaStreamBeginCaptureToGraph(cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) == cudaSuccess;
+  }
+  if (ok) {
+    iteration(cap, h, 1);
+    ok = cudaStreamEndCapture(cap, &body) == cudaSuccess;
+  }
+  if (ok) ok = cudaGraphInstantiate(&graph, graph_, 0) == cudaSuccess;
+  cudaGraphDestroy(graph_);
+  ok = cudaGetLastError() == cudaSuccess && ok;
+  body_nodes = launches + mgu.launches + mgp.launches - l0;
+  launches -= body_nodes;  // recording is not execution
+  if (!ok && graph) {
+    cudaGraphExecDestroy(graph);
+    graph = nullptr;
+  }
+  return ok ? 0 : -5;
+}
+
+// Runs the cycle set up in kry to its end and reads its counters back (hstat).  Without a graph
+// (TOPO_GRAPHS=0, or a recording that another thread's device-wide work spoiled) the host
+// launches the same kernels, one round trip per iteration.
+int topo_fluid_ctx::cycle(cudaStream_t s) {
+  const int levels[2] = {mgu.coarse_cheb_level(), mgp.coarse_cheb_level()};
+  if (graph && std::memcmp(levels, graph_levels, sizeof(levels))) {
+    cudaGraphExecDestroy(graph);
+    graph = nullptr;
+  }
+  if (use_graph && !graph) {
+    std::memcpy(graph_levels, levels, sizeof(levels));
+    if (cudaStreamSynchronize(s) != cudaSuccess) return -5;  // the recording must not see queued work
+    if (record() != 0) cudaGetLastError();
+  }
+  const int before = hstat[1];
+  if (use_graph && graph) {
+    if (cudaGraphLaunch(graph, s) != cudaSuccess) return -5;
+  } else {
+    do {
+      iteration(s, 0, 0);
+      cudaMemcpyAsync(hstat, kry, 4 * sizeof(int), cudaMemcpyDeviceToHost, s);
+      if (cudaStreamSynchronize(s) != cudaSuccess) return -5;
+    } while (hstat[3] == 1);
+    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  }
+  cudaMemcpyAsync(hstat, kry, 4 * sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (cudaStreamSynchronize(s) != cudaSuccess) return -5;
+  launches += body_nodes * std::max(0, hstat[1] - before);
+  return 0;
+}
 
 namespace {
 
@@ -345,54 +672,10 @@ int fluid_setup(topo_fluid_ctx* C, const double* rho, cudaStream_t s) {
   return C->cuda_check("fluid set-up");
 }
 
-// chunked classical Gram-Schmidt helpers over the Krylov basis (at most 8 vectors a launch)
-void multidot(topo_fluid_ctx* C, int count, const double* w, double* h, double& ww, cudaStream_t s) {
-  for (int i0 = 0; i0 < count; i0 += 8) {
-    const int c = std::min(8, count - i0);
-    const double* Vb = C->V + size_t(i0) * C->n;
-#define TOPO_MD(K) \
-  k_multidot<double, double, K><<<C->red.blocks_for(C->n), kVecThreads, 0, s>>>(Vb, C->n, w, C->n, C->red.partials, C->red.counter, C->red.out)
-    TOPO_DISPATCH_COUNT(c, TOPO_MD)
-#undef TOPO_MD
-    ++C->launches;
-    cudaMemcpyAsync(C->red.host, C->red.out, (c + 1) * sizeof(double), cudaMemcpyDeviceToHost, s);
-    cudaStreamSynchronize(s);
-    for (int k = 0; k < c; ++k) h[i0 + k] = C->red.host[k];
-    ww = C->red.host[c];
-  }
-}
-
-void sub_multi(topo_fluid_ctx* C, int count, const double* h, double* w, cudaStream_t s) {
-  for (int i0 = 0; i0 < count; i0 += 8) {
-    const int c = std::min(8, count - i0);
-    MultiCoef cf{};
-    for (int k = 0; k < c; ++k) cf.c[k] = h[i0 + k];
-    const double* Vb = C->V + size_t(i0) * C->n;
-#define TOPO_SM(K) k_sub_multi<double, double, K><<<C->grid(C->n), kVecThreads, 0, s>>>(w, Vb, C->n, cf, C->n)
-    TOPO_DISPATCH_COUNT(c, TOPO_SM)
-#undef TOPO_SM
-    ++C->launches;
-  }
-}
-
-void add_multi(topo_fluid_ctx* C, int count, const double* y, double* x, cudaStream_t s) {
-  for (int i0 = 0; i0 < count; i0 += 8) {
-    const int c = std::min(8, count - i0);
-    MultiCoef cf{};
-    for (int k = 0; k < c; ++k) cf.c[k] = y[i0 + k];
-    const double* Zb = C->Z + size_t(i0) * C->n;
-#define TOPO_AM(K) k_add_multi<double, double, K><<<C->grid(C->n), kVecThreads, 0, s>>>(x, Zb, C->n, cf, C->n)
-    TOPO_DISPATCH_COUNT(c, TOPO_AM)
-#undef TOPO_AM
-    ++C->launches;
-  }
-}
-
 // Flexible GMRES(m), right preconditioned, on the clamped operator from x = 0;
 // stops on the true residual |b - A x| <= rtol |b|.
 int fluid_fgmres(topo_fluid_ctx* C, const double* b, double* x, double rtol, int maxit, int& iters, double& relres,
                  cudaStream_t s) {
-  constexpr int m = kFluidRestart;
   const size_t n = C->n;
   const int g = C->grid(n);
   iters = 0;
@@ -402,8 +685,6 @@ int fluid_fgmres(topo_fluid_ctx* C, const double* b, double* x, double rtol, int
   const double bn = std::sqrt(C->dot(b, b, n, s));
   if (!std::isfinite(bn)) return C->fail(TOPO_ERR_NAN, "non-finite right-hand side");
   if (bn == 0.0) return TOPO_OK;
-  std::vector<double> H((m + 1) * m), cs(m), sn(m), gv(m + 1), h(m + 1), y(m);
-  auto Hij = [&](int i, int j) -> double& { return H[size_t(i) * m + j]; };
   for (int cycle = 0;; ++cycle) {
     double* r = C->V;
     if (cycle == 0) {
@@ -421,65 +702,17 @@ int fluid_fgmres(topo_fluid_ctx* C, const double* b, double* x, double rtol, int
       return C->fail(TOPO_ERR_NOT_CONVERGED, "fluid state solve did not converge (relres %.3g after %d iterations)",
                      relres, iters);
     k_scale<double><<<g, kVecThreads, 0, s>>>(r, 1.0 / beta, n);
-    ++C->launches;
-    std::fill(gv.begin(), gv.end(), 0.0);
-    gv[0] = beta;
-    int k = 0;
-    for (int j = 0; j < m && iters < maxit; ++j) {
-      double* vj = C->V + size_t(j) * n;
-      double* zj = C->Z + size_t(j) * n;
-      double* w = C->V + size_t(j + 1) * n;
-      C->precond(vj, zj, s);
-      C->apply(zj, w, true, s);
-      ++iters;
-      // classical Gram-Schmidt, a second pass when the first cancelled more than half of w
-      std::fill(h.begin(), h.end(), 0.0);
-      double hn = 0.0;
-      for (int pass = 0; pass < 2; ++pass) {
-        std::vector<double> hp(j + 1);
-        double ww = 0.0;
-        multidot(C, j + 1, w, hp.data(), ww, s);
-        double hh = 0.0;
-        for (int i = 0; i <= j; ++i) {
-          h[i] += hp[i];
-          hh += hp[i] * hp[i];
-        }
-        sub_multi(C, j + 1, hp.data(), w, s);
-        const double est = ww - hh;
-        if (pass == 0 && est >= 0.5 * ww) {
-          hn = std::sqrt(est);
-          break;
-        }
-        if (pass == 1) hn = std::sqrt(C->dot(w, w, n, s));
-      }
-      if (!std::isfinite(hn)) return C->fail(TOPO_ERR_NAN, "non-finite Krylov vector in the fluid solve");
-      for (int i = 0; i <= j; ++i) Hij(i, j) = h[i];
-      Hij(j + 1, j) = hn;
-      if (hn > 0) {
-        k_scale<double><<<g, kVecThreads, 0, s>>>(w, 1.0 / hn, n);
-        ++C->launches;
-      }
-      for (int i = 0; i < j; ++i) {
-        const double t0 = cs[i] * Hij(i, j) + sn[i] * Hij(i + 1, j);
-        Hij(i + 1, j) = -sn[i] * Hij(i, j) + cs[i] * Hij(i + 1, j);
-        Hij(i, j) = t0;
-      }
-      const double den = std::hypot(Hij(j, j), Hij(j + 1, j));
-      cs[j] = den > 0 ? Hij(j, j) / den : 1.0;
-      sn[j] = den > 0 ? Hij(j + 1, j) / den : 0.0;
-      Hij(j, j) = den;
-      Hij(j + 1, j) = 0.0;
-      gv[j + 1] = -sn[j] * gv[j];
-      gv[j] = cs[j] * gv[j];
-      k = j + 1;
-      if (std::fabs(gv[j + 1]) <= 0.5 * rtol * bn || hn == 0.0) break;
-    }
-    for (int i = k - 1; i >= 0; --i) {
-      double acc = gv[i];
-      for (int l = i + 1; l < k; ++l) acc -= Hij(i, l) * y[l];
-      y[i] = Hij(i, i) != 0.0 ? acc / Hij(i, i) : 0.0;
-    }
-    add_multi(C, k, y.data(), x, s);
+    k_dot<double, double><<<C->red.blocks_for(C->nv), kVecThreads, 0, s>>>(C->pp(r), C->ones, C->nv, C->red.partials,
+                                                                         C->red.counter, &C->kry->psum);
+    k_fluid_start<<<1, 1, 0, s>>>(C->kry, beta, 0.5 * rtol * bn, iters, maxit);
+    C->hstat[1] = iters;
+    const int rc = C->cycle(s);
+    if (rc) return C->fail(TOPO_ERR_CUDA, "fluid solve: CUDA error");
+    k_fluid_backsolve<<<1, 32, 0, s>>>(C->kry);
+    k_fluid_update<<<g, kVecThreads, 0, s>>>(x, C->Z, n, C->kry);
+    C->launches += 5;
+    iters = C->hstat[1];
+    if (C->hstat[3] == 4) return C->fail(TOPO_ERR_NAN, "non-finite Krylov vector in the fluid solve");
   }
 }
 
@@ -526,21 +759,30 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
   C->tab = C->arena.alloc_n<FluidTables>(1);
   C->ub = C->arena.alloc_n<double>(2 * C->n2);
   C->mass = C->arena.alloc_n<double>(nt * kFluidMass);
-  C->tri_out = C->arena.alloc_n<double>(nt * kFluidOut);
   C->tri3 = C->arena.alloc_n<double>(3 * nt);
   C->ml = C->arena.alloc_n<double>(C->nv);
   C->ones = C->arena.alloc_n<double>(C->nv);
   C->rhs = C->arena.alloc_n<double>(C->n);
   C->x = C->arena.alloc_n<double>(C->n);
-  C->V = C->arena.alloc_n<double>(size_t(kFluidRestart + 1) * C->n);
-  C->Z = C->arena.alloc_n<double>(size_t(kFluidRestart) * C->n);
+  if (C->n * sizeof(double) * (2 * kFluidRestartMax + 1) <= kFluidBasisMax) C->m = kFluidRestartMax;
+  C->V = C->arena.alloc_n<double>(size_t(C->m + 1) * C->n);
+  C->Z = C->arena.alloc_n<double>(size_t(C->m) * C->n);
   C->t = C->arena.alloc_n<double>(C->n);
-  C->c0 = C->arena.alloc_n<double>(C->n2);
-  C->c1 = C->arena.alloc_n<double>(C->n2);
-  C->z0 = C->arena.alloc_n<double>(C->n2);
-  C->z1 = C->arena.alloc_n<double>(C->n2);
-  C->pt = C->arena.alloc_n<double>(C->nv);
-  C->pz = C->arena.alloc_n<double>(C->nv);
+  C->kry = C->arena.alloc_n<FluidKrylov>(1);
+  C->dots = C->arena.alloc_n<double>(size_t(C->red.blocks) * (kDotGroup + 1) * kDotGroups);
+  C->dot_counters = C->arena.alloc_n<unsigned>(kDotGroups);
+  C->zc = C->arena.alloc_n<double>(C->nv);
+  C->c = C->arena.alloc_n<float>(2 * C->n2);
+  C->z = C->arena.alloc_n<float>(2 * C->n2);
+  C->pt = C->arena.alloc_n<float>(C->nv);
+  C->pz = C->arena.alloc_n<float>(C->nv);
+  if (cudaMallocHost(&C->hstat, 4 * sizeof(int)) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "out of host memory");
+  std::memset(C->hstat, 0, 4 * sizeof(int));
+  for (cudaStream_t* c : {&C->cap, &C->side})
+    if (cudaStreamCreateWithFlags(c, cudaStreamNonBlocking) != cudaSuccess) return C->cuda_check("fluid streams");
+  for (cudaEvent_t* e : {&C->fork, &C->join})
+    if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return C->cuda_check("fluid events");
+  if (const char* e = std::getenv("TOPO_GRAPHS")) C->use_graph = e[0] != '0';
   C->gb = C->arena.alloc_n<double>(C->nv);
   if (C->arena.failed()) return C->fail(TOPO_ERR_CUDA, "out of device memory");
   const std::vector<double> w = vertex_weights(C->nx, C->ny, C->hx, C->hy);
@@ -579,9 +821,11 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
   for (size_t l = 0; l < C->pspec.size(); ++l)
     k_fill<double><<<C->grid(C->pspec[l].ntri()), kVecThreads, 0, s>>>(C->pM[l], kLaplaceShift, C->pspec[l].ntri());
   for (auto* mg : {&C->mgu, &C->mgp}) {
-    mg->use_graphs = false;  // only V-cycles are used, launched from the host
+    mg->use_graphs = false;  // only V-cycles are used
     mg->profile_levels = false;
+    mg->element_bounds = true;
   }
+  C->mgu.batch = 2;
   C->mgu.init(C->uspec, C->urefs.data(), 0.0, 0.0, C->arena, &C->red);
   C->mgu.set_coefficients(std::vector<const double*>(C->uK.begin(), C->uK.end()),
                           std::vector<const double*>(C->uM.begin(), C->uM.end()));

@@ -228,4 +228,72 @@ TOPO_HD double fluid_gather_vertex(const double* tri_out, int nx, int ny, int a,
   return s;
 }
 
+// ---------------------------------------------------------------------------
+// the operator by output node
+// ---------------------------------------------------------------------------
+// Output i of [0, n2 + nv): the P2 nodes by class -- vertices, midpoints of horizontal, of
+// vertical and of diagonal edges, so that the lanes of a warp have the same number of
+// incident triangles (six, or two) -- and then the pressure vertices.
+struct FluidNode {
+  int cls;   // 0 vertex, 1 horizontal, 2 vertical, 3 diagonal edge, 4 pressure vertex
+  int i, j;  // cell column and row of the vertex, or of the edge's lower left vertex
+};
+
+TOPO_HD FluidNode fluid_output(size_t i, int nx, int ny) {
+  const size_t n[4] = {size_t(nx + 1) * (ny + 1), size_t(nx) * (ny + 1), size_t(nx + 1) * ny, size_t(nx) * ny};
+  const int w[4] = {nx + 1, nx, nx + 1, nx};
+  int c = 0;
+  while (c < 4 && i >= n[c]) i -= n[c++];
+  const int width = c < 4 ? w[c] : nx + 1;
+  return FluidNode{c, int(i % width), int(i / width)};
+}
+
+// the element rows of one triangle: mk its matrix M + K (upper triangle), local row r
+TOPO_HD void fluid_row(const FluidTables& E, int o, int r, const double* mk, const double (&ue)[6][2],
+                       const double (&pe)[3], double (&y)[2]) {
+  for (int j = 0; j < 6; ++j) {
+    const double m = r <= j ? mk[fluid_mass_index(r, j)] : mk[fluid_mass_index(j, r)];
+    y[0] += m * ue[j][0];
+    y[1] += m * ue[j][1];
+  }
+  for (int k = 0; k < 3; ++k) {
+    y[0] += E.grad[o][r][0][k] * pe[k];
+    y[1] += E.grad[o][r][1][k] * pe[k];
+  }
+}
+
+// Rows of the operator at output F.  mk: [tri][kFluidMass] with the Laplacian added; u, p the
+// velocity and pressure, pm a constant taken off the pressure.  Fills y[2] (velocity) or y[0]
+// (pressure vertex).  Boundary velocity nodes are the caller's.
+TOPO_HD void fluid_node_rows(const FluidTables& E, const double* mk, int nx, int ny, const FluidNode& F,
+                             const double* u, const double* p, double pm, double (&y)[2]) {
+  // incident triangles of each class, a byte each: column offset + 1 | (row offset + 1) << 1 |
+  // orientation << 2 | local index << 3
+  const int c = F.cls == 4 ? 0 : F.cls, count = c == 0 ? 6 : 2;
+  const unsigned long long inc = c == 0 ? 0x07030a0d1410ull : c == 1 ? 0x2b1dull : c == 2 ? 0x2f1aull : 0x2723ull;
+  y[0] = y[1] = 0.0;
+  for (int e = 0; e < count; ++e) {
+    const unsigned f = unsigned(inc >> (8 * e)) & 255u;
+    const int ci = F.i + int(f & 1u) - 1, cj = F.j + int((f >> 1) & 1u) - 1, o = int((f >> 2) & 1u), r = int(f >> 3);
+    if (ci < 0 || ci >= nx || cj < 0 || cj >= ny) continue;
+    const size_t t = (size_t(cj) * nx + ci) * 2 + o;
+    double ue[6][2];
+    const int NX = 2 * nx + 1;
+    for (int k = 0; k < 6; ++k) {
+      const size_t nd = size_t(2 * cj + p2_off_b(o, k)) * NX + 2 * ci + p2_off_a(o, k);
+      ue[k][0] = u[2 * nd];
+      ue[k][1] = u[2 * nd + 1];
+    }
+    if (F.cls == 4) {
+      double s = 0.0;
+      for (int k = 0; k < 6; ++k) s += E.div[o][r][k][0] * ue[k][0] + E.div[o][r][k][1] * ue[k][1];
+      y[0] -= s;
+    } else {
+      double pe[3];
+      for (int k = 0; k < 3; ++k) pe[k] = p[size_t(cj + p1_off_b(o, k)) * (nx + 1) + ci + p1_off_a(o, k)] - pm;
+      fluid_row(E, o, r, mk + t * kFluidMass, ue, pe, y);
+    }
+  }
+}
+
 }  // namespace topo

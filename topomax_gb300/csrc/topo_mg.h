@@ -78,6 +78,8 @@ struct ElemRefs {
 ElemRefs make_elem_refs(double hx, double hy, double lmbda, double mu);
 double p1_elasticity_bound(const ElemRefs& R);
 void p1_helmholtz_bounds(const ElemRefs& R, double t, double& lo, double& hi);
+// largest eigenvalue of D_e^-1 A_e over A_e = s K_e + t M_e, s, t >= 0 (bounds the assembled one)
+double p1_scalar_bound(const ElemRefs& R);
 // Interval [lo, hi] holding the spectrum of Dinv A for P1 levels assembled from
 // t K_e + M_e with t in [tmin, tmax], and the Chebyshev degree reaching a
 // residual reduction tol on it.
@@ -192,6 +194,13 @@ class MG {
   int coarse_cheb_max_degree = 16;
   int coarse_cheb_level() const { return cheb_coarse_; }
   int coarse_cheb_deg = 0;
+  // V-cycles act on `batch` right-hand sides stored one after the other (scalar hierarchies
+  // whose levels all have stencils; set before init, the Krylov solves take one)
+  int batch = 1;
+  // scalar levels >= 0 take the element bound of lambda_max(D^-1 A) -- the largest of the
+  // stiffness's and the mass's, for any coefficients -- instead of a power iteration, and
+  // no level is searched for a shared interior row: hierarchies set up for every solve
+  bool element_bounds = false;
   long long capture_failures = 0;  // recordings that failed (those solves ran host-driven)
   // opt-in level timing (host-driven mode only): inclusive ms per level, summed
   bool profile_levels = false;

@@ -225,6 +225,14 @@ void p1_helmholtz_bounds(const ElemRefs& R, double t, double& lo, double& hi) {
   }
 }
 
+// x^T (s K + t M) x / x^T (s D_K + t D_M) x is at most the larger of the two quotients
+double p1_scalar_bound(const ElemRefs& R) {
+  double lo, mass, stiff;
+  p1_helmholtz_bounds(R, 0.0, lo, mass);
+  p1_helmholtz_bounds(R, 1e12, lo, stiff);
+  return std::max(mass, stiff);
+}
+
 int coarse_cheb_plan(const ElemRefs& R, double tmin, double tmax, double tol, double& lo, double& hi) {
   lo = 1e300;
   hi = 0.0;

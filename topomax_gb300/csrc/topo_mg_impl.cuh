@@ -247,6 +247,9 @@ __global__ void __launch_bounds__(kSweepThreads)
   T* sx = reinterpret_cast<T*>(sweep_raw);
   T* sd = sx + NC * P.down_w() * P.down_h();
   const int tid = threadIdx.x, nt = blockDim.x, I0 = blockIdx.x * P.cx, J0 = blockIdx.y * P.cy;
+  b += blockIdx.z * size_t(NC) * P.NX * P.NY;  // the batch's vectors
+  x += blockIdx.z * size_t(NC) * P.NX * P.NY;
+  bc += blockIdx.z * size_t(NC) * P.NXc * P.NYc;
   TOPO_PDL_LAUNCH();
   LevelNode<T, NC> N;
   const bool on = LevelDown<T, NC>::start(P, I0, J0, tid, N);
@@ -268,6 +271,10 @@ __global__ void __launch_bounds__(kSweepThreads)
   T* sd = reinterpret_cast<T*>(sweep_raw);
   T* sx = sd + NC * P.up_w() * P.up_h();
   const int tid = threadIdx.x, nt = blockDim.x, I0 = blockIdx.x * P.cx, J0 = blockIdx.y * P.cy;
+  b += blockIdx.z * size_t(NC) * P.NX * P.NY;
+  x += blockIdx.z * size_t(NC) * P.NX * P.NY;
+  xin += blockIdx.z * size_t(NC) * P.NX * P.NY;
+  xc += blockIdx.z * size_t(NC) * P.NXc * P.NYc;
   TOPO_PDL_LAUNCH();
   typename LevelUp<T, NC>::Node N;
   const bool on = LevelUp<T, NC>::start(P, I0, J0, tid, N);
@@ -403,14 +410,20 @@ __global__ void __launch_bounds__(32) k_coarse_inverse(int nx, int ny, Dir dir, 
   if (j == 0) *status = bad;
 }
 
+// x = Ainv b on the coarsest level, n <= kCoarseMaxDofs (Ainv symmetric: column reads)
 template <class T>
-__global__ void k_dense_matvec(const T* __restrict__ Ainv, const T* __restrict__ b, T* __restrict__ x, int n) {
-  TOPO_PDL_ENTRY();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    T s = T(0);
-    for (int j = 0; j < n; ++j) s += Ainv[size_t(i) * n + j] * b[j];
-    x[i] = s;
-  }
+__global__ void __launch_bounds__(kCoarseMaxDofs) k_dense_matvec(const T* Ainv, const T* b, T* x, int n) {
+  __shared__ T A[kCoarseMaxDofs * kCoarseMaxDofs], v[kCoarseMaxDofs];
+  TOPO_PDL_LAUNCH();
+  const int i = threadIdx.x;
+  for (int k = i; k < n * n; k += blockDim.x) A[k] = Ainv[k];
+  TOPO_PDL_WAIT();
+  if (i < n) v[i] = b[blockIdx.x * size_t(n) + i];
+  __syncthreads();
+  if (i >= n) return;
+  T s = T(0);
+  for (int j = 0; j < n; ++j) s = fma_t(A[j * n + i], v[j], s);
+  x[blockIdx.x * size_t(n) + i] = s;
 }
 
 constexpr int kCoarseThreads = 1024;                   // one-CTA coarse Chebyshev solve
@@ -425,6 +438,8 @@ __global__ void __launch_bounds__(kTailNodes)
   extern __shared__ __align__(16) unsigned char sweep_raw[];
   T* sm = reinterpret_cast<T*>(sweep_raw);
   const int tid = threadIdx.x, nt = blockDim.x;
+  b += blockIdx.x * size_t(NC) * P.lv[0].NX * P.lv[0].NY;
+  x += blockIdx.x * size_t(NC) * P.lv[0].NX * P.lv[0].NY;
   TOPO_PDL_LAUNCH();
   // what no solve changes: rows, inverse diagonals, the coarsest inverse
   for (int i = tid; i < P.vectors; i += nt) sm[i] = T(0);
@@ -573,8 +588,8 @@ constexpr int coarse_cheb_npt() {
 
 template <class T>
 __global__ void __launch_bounds__(kCoarseThreads)
-    k_coarse_cheb(const CoarseChebDesc<T, 1>* __restrict__ D, const T* __restrict__ b, T* __restrict__ x_out) {
-  TOPO_PDL_ENTRY();
+    k_coarse_cheb(const CoarseChebDesc<T, 1>* D, const T* b, T* x_out) {
+  TOPO_PDL_LAUNCH();
   constexpr int NP = coarse_cheb_npt<T>(), SW = StencilLayout<1>::stride;
   extern __shared__ __align__(16) unsigned char cc_raw[];
   T* d0 = reinterpret_cast<T*>(cc_raw);
@@ -582,7 +597,9 @@ __global__ void __launch_bounds__(kCoarseThreads)
   const int nn = D->nn, NX = D->NX;
   T* d1 = d0 + nn;
   const CoarseCheb<T>& C = D->C;  // read in place (uniform loads)
-  const T* __restrict__ sg = D->S.s;
+  const T* sg = D->S.s;
+  b += blockIdx.x * size_t(nn);
+  x_out += blockIdx.x * size_t(nn);
   T st[NP][7], dv[NP], r[NP], x[NP];
 #pragma unroll
   for (int q = 0; q < NP; ++q) {
@@ -591,6 +608,12 @@ __global__ void __launch_bounds__(kCoarseThreads)
 #pragma unroll
     for (int k = 0; k < 7; ++k) st[q][k] = on ? sg[size_t(n) * SW + k] : T(0);
     dv[q] = on ? D->dinv[n] : T(0);
+  }
+  TOPO_PDL_WAIT();  // the rows above are fixed during a solve
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    const int n = tid + q * nt;
+    const bool on = n < nn;
     r[q] = on ? b[n] : T(0);
     x[q] = T(0);
     if (on) d0[n] = C.c0 * dv[q] * r[q];
@@ -981,16 +1004,16 @@ void MG<T>::init(const std::vector<LevelSpec>& specs, const ElemRefs* refs, doub
   }
   lv_.assign(specs.size(), Lev{});
   for (size_t l = 0; l < specs.size(); ++l) {
-    const size_t n = specs[l].ndof();
+    const size_t n = specs[l].ndof(), nb = n * batch;
     Lev& v = lv_[l];
     if (l > 0) {
-      v.x = arena.alloc_n<T>(n);
-      v.b = arena.alloc_n<T>(n);
+      v.x = arena.alloc_n<T>(nb);
+      v.b = arena.alloc_n<T>(nb);
     }
     v.r = arena.alloc_n<T>(n);
     v.d = arena.alloc_n<T>(n);
     v.t = arena.alloc_n<T>(n);
-    v.x2 = arena.alloc_n<T>(n);
+    v.x2 = arena.alloc_n<T>(nb);
     v.diag = arena.alloc_n<T>(n);
     v.dinv = arena.alloc_n<T>(n);
     if (!specs[l].p2) {
@@ -1329,6 +1352,9 @@ int MG<T>::setup(cudaStream_t s) {
     if (!S.p2 && S.NC == 2) {
       lv_[l].lmax = p1_elasticity_bound(refs_[l]);
       lv_[l].bound = true;
+    } else if (!S.p2 && element_bounds) {
+      lv_[l].lmax = p1_scalar_bound(refs_[l]);
+      lv_[l].bound = true;
     } else {
       lv_[l].lmax = estimate_lmax(l, s);
       lv_[l].bound = false;
@@ -1351,7 +1377,7 @@ int MG<T>::setup(cudaStream_t s) {
   if (!cc_selected_) {  // the coefficients of a hierarchy with a mass term do not change
     cudaStreamSynchronize(s);
     select_coarse_cheb(s);
-    detect_uniform_levels(s);
+    if (!element_bounds) detect_uniform_levels(s);
     cc_selected_ = true;
   }
   for (int l = 1; l + 1 < L; ++l) bounds(l);
@@ -1417,7 +1443,7 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
   const LevelSpec& S = specs_[l];
   if (l == cheb_coarse_ && cc_desc_) {
     KClock kc(s, "coarse Chebyshev (one CTA)", l, 0.0);
-    launch_pdl(k_coarse_cheb<T>, 1, kCoarseThreads, cc_smem_, s, static_cast<const CoarseChebDesc<T, 1>*>(cc_desc_), b, x);
+    launch_pdl(k_coarse_cheb<T>, batch, kCoarseThreads, cc_smem_, s, static_cast<const CoarseChebDesc<T, 1>*>(cc_desc_), b, x);
     ++launches;
     return;
   }
@@ -1425,14 +1451,14 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
     if (l == tail_ && use_tail) {
       KClock kc(s, "V-cycle tail (one CTA)", l, 0.0);
       const dim3 nt(unsigned(S.nn() + 31) / 32 * 32);
-      if (S.NC == 2) launch_pdl(k_level_tail<T, 2>, 1, nt, tail2_.shared * sizeof(T), s, tail2_, b, x);
-      else launch_pdl(k_level_tail<T, 1>, 1, nt, tail1_.shared * sizeof(T), s, tail1_, b, x);
+      if (S.NC == 2) launch_pdl(k_level_tail<T, 2>, batch, nt, tail2_.shared * sizeof(T), s, tail2_, b, x);
+      else launch_pdl(k_level_tail<T, 1>, batch, nt, tail1_.shared * sizeof(T), s, tail1_, b, x);
       ++launches;
       return;
     }
   }
   if (l == L - 1) {
-    launch_pdl(k_dense_matvec<T>, 1, 256, 0, s, static_cast<const T*>(cinv_), b, x, int(S.ndof()));
+    launch_pdl(k_dense_matvec<T>, batch, kCoarseMaxDofs, 0, s, static_cast<const T*>(cinv_), b, x, int(S.ndof()));
     ++launches;
     return;
   }
@@ -1481,7 +1507,7 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
   auto run = [&](auto nc_tag) {
     constexpr int NC = decltype(nc_tag)::value;
     const LevelSweep<T, NC> P = level_sweep<T, NC>(S, X, v.st, v.inner, v.dinv, cheb_ + 8 * l);
-    const dim3 g((X.NXc + P.cx - 1) / P.cx, (X.NYc + P.cy - 1) / P.cy);
+    const dim3 g((X.NXc + P.cx - 1) / P.cx, (X.NYc + P.cy - 1) / P.cy, batch);
     auto threads = [](int nodes) { return dim3(unsigned(nodes + 31) / 32 * 32); };
     {
       KClock kc(s, "P1 level down", l, row + (3 * nf + ncrs) * sizeof(T));

@@ -117,11 +117,12 @@ __device__ __forceinline__ void block_sums(const R (&v)[NV], double* res) {
 // most kVecThreads threads).  Returns true in thread 0 of the last block, with the totals
 // in tot[].  The in-block sums run in R (float for FP32 data) up to the warps, the
 // combination of warps and blocks in FP64, always in the same order.
+// bid, nb: the block and the blocks of the reduction (several may share a grid).
 template <int NV, class R>
-__device__ bool finish_reduction(const R (&v)[NV], double* partials, unsigned* counter, double (&tot)[NV]) {
+__device__ bool finish_reduction(const R (&v)[NV], double* partials, unsigned* counter, double (&tot)[NV], unsigned bid,
+                                 unsigned nb) {
   __shared__ double res[NV];
   __shared__ bool last;
-  const unsigned bid = blockIdx.y * gridDim.x + blockIdx.x, nb = gridDim.x * gridDim.y;
   block_sums<NV, R>(v, res);
   if (nb > 1) {
     if (threadIdx.x < NV) {
@@ -146,6 +147,11 @@ __device__ bool finish_reduction(const R (&v)[NV], double* partials, unsigned* c
 #pragma unroll
   for (int k = 0; k < NV; ++k) tot[k] = res[k];
   return true;
+}
+
+template <int NV, class R>
+__device__ bool finish_reduction(const R (&v)[NV], double* partials, unsigned* counter, double (&tot)[NV]) {
+  return finish_reduction<NV, R>(v, partials, counter, tot, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
 }
 
 // out[0] = sum a_i b_i (or sum a_i^2 when b == nullptr)
