@@ -298,6 +298,10 @@ int topo_dem_enforce(topo_dem_ctx* ctx, const float* u_hat, float* u, topo_strea
 int topo_dem_energy(topo_dem_ctx* ctx, const float* u, const float* density, int masked, double* energy,
                     topo_stream_t stream);
 
+/* The same energy rounded to a device float scalar. */
+int topo_dem_energy_f32(topo_dem_ctx* ctx, const float* u, const float* density, int masked, float* energy,
+                        topo_stream_t stream);
+
 /* Gradient of topo_dem_energy times the device float scalar *scale: du float32 [nn][2]
  * (d psi / d u, or d psi / d u_hat when masked) and/or ddensity float32 [ny][nx]
  * (0.5 r'(rho) SE detJ); either may be NULL.  No counterpart in the reference (torch autograd
@@ -310,6 +314,10 @@ int topo_dem_energy_backward(topo_dem_ctx* ctx, const float* u, const float* den
  * (device float32 [ny][nx]). */
 int topo_dem_objective_gradient(topo_dem_ctx* ctx, const float* u, const float* density, double* objective,
                                 float* gradient, topo_stream_t stream);
+
+/* The same with the objective rounded to a device float scalar. */
+int topo_dem_objective_gradient_f32(topo_dem_ctx* ctx, const float* u, const float* density, float* objective,
+                                    float* gradient, topo_stream_t stream);
 
 /* ---- DEM density filter: replaces create_density_filter (DEM_src/filter.py:8-31) and
  * its two uses, W @ rho and W.T @ g (DEM_src/elasisity_problem.py:148, 162, 171). ------

@@ -33,7 +33,8 @@ EXPORTED = [
     "topo_launch_count", "topo_kernel_clock", "topo_kernel_clock_report", "topo_march_tiles_report", "topo_sensitivity_rhs_noalloc", "topo_mass_apply",
     "topo_dem_create", "topo_dem_destroy", "topo_dem_last_error", "topo_dem_set_penalization",
     "topo_dem_set_external", "topo_dem_set_mask", "topo_dem_enforce", "topo_dem_energy",
-    "topo_dem_energy_backward", "topo_dem_objective_gradient",
+    "topo_dem_energy_backward", "topo_dem_objective_gradient", "topo_dem_energy_f32",
+    "topo_dem_objective_gradient_f32",
     "topo_density_filter_create", "topo_density_filter_destroy", "topo_density_filter_nnz",
     "topo_density_filter_apply",
     "topo_fluid_create", "topo_fluid_destroy", "topo_fluid_last_error", "topo_fluid_sizes",
@@ -144,6 +145,8 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
     lib.topo_dem_energy.argtypes = [P, P, P, I, P, P]
     lib.topo_dem_energy_backward.argtypes = [P, P, P, I, P, P, P, P]
     lib.topo_dem_objective_gradient.argtypes = [P, P, P, P, P, P]
+    lib.topo_dem_energy_f32.argtypes = [P, P, P, I, P, P]
+    lib.topo_dem_objective_gradient_f32.argtypes = [P, P, P, P, P, P]
     lib.topo_density_filter_create.restype = P
     lib.topo_density_filter_create.argtypes = [I, I, D, D, D, PI]
     lib.topo_density_filter_destroy.restype = None

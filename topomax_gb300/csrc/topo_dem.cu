@@ -158,16 +158,17 @@ enum DemMode { kDemEnergy = 0, kDemObjective = 1, kDemDensityGrad = 2 };
 // One pass over the cells (and, for the energy, over the nodes for the external
 // work).  kDemEnergy: out = 0.5 * sum r*SE*detJ - sum w.u ;  kDemObjective:
 // out = sum r*(SE*detJ), cellv = -r' * (SE*detJ) ;  kDemDensityGrad:
-// cellv = scale * 0.5 * r' * SE * detJ.
+// cellv = scale * 0.5 * r' * SE * detJ.  block, blocks: the block's share of the cells.
+// The sum goes to out (FP64) or outf (rounded to FP32), whichever is given.
 template <int MODE, bool MASK>
-__global__ void __launch_bounds__(kDemThreads)
-    k_dem_cells(DemK K, const float* __restrict__ u, const float* __restrict__ mask, const float* __restrict__ rho,
-                const float* __restrict__ wext, const float* __restrict__ scale, float* __restrict__ cellv,
-                double* partials, unsigned* counter, double* out) {
+__device__ __forceinline__ void
+    dem_cells(const DemK& K, const float* __restrict__ u, const float* __restrict__ mask, const float* __restrict__ rho,
+              const float* __restrict__ wext, const float* __restrict__ scale, float* __restrict__ cellv,
+              double* partials, unsigned* counter, double* out, float* outf, unsigned block, unsigned blocks) {
   const size_t ncell = size_t(K.nx) * K.ny;
   double acc = 0.0;
   const float sc = (MODE == kDemDensityGrad) ? *scale : 0.0f;
-  for (size_t c = size_t(blockIdx.x) * blockDim.x + threadIdx.x; c < ncell; c += size_t(gridDim.x) * blockDim.x) {
+  for (size_t c = size_t(block) * blockDim.x + threadIdx.x; c < ncell; c += size_t(blocks) * blockDim.x) {
     const int iy = int(c / K.nx), ix = int(c - size_t(iy) * K.nx);
     float U[4][2];
     load_cell<MASK>(K, u, mask, ix, iy, U);
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kDemThreads)
   double ext = 0.0;
   if (MODE == kDemEnergy && wext) {
     const size_t nn = size_t(K.nx + 1) * (K.ny + 1);
-    for (size_t n = size_t(blockIdx.x) * blockDim.x + threadIdx.x; n < nn; n += size_t(gridDim.x) * blockDim.x)
+    for (size_t n = size_t(block) * blockDim.x + threadIdx.x; n < nn; n += size_t(blocks) * blockDim.x)
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         float v = u[2 * n + j];
@@ -197,21 +198,33 @@ __global__ void __launch_bounds__(kDemThreads)
   }
   const double v[2] = {acc, ext};
   double tot[2];
-  if (finish_reduction<2>(v, partials, counter, tot))
-    *out = (MODE == kDemEnergy) ? 0.5 * tot[0] - tot[1] : tot[0];
+  if (finish_reduction<2>(v, partials, counter, tot)) {
+    const double r = (MODE == kDemEnergy) ? 0.5 * tot[0] - tot[1] : tot[0];
+    if (out) *out = r;
+    if (outf) *outf = float(r);
+  }
+}
+
+template <int MODE, bool MASK>
+__global__ void __launch_bounds__(kDemThreads)
+    k_dem_cells(DemK K, const float* __restrict__ u, const float* __restrict__ mask, const float* __restrict__ rho,
+                const float* __restrict__ wext, float* __restrict__ cellv, double* partials, unsigned* counter,
+                double* out, float* outf) {
+  dem_cells<MODE, MASK>(K, u, mask, rho, wext, nullptr, cellv, partials, counter, out, outf, blockIdx.x, gridDim.x);
 }
 
 // d psi / d u at every node: sum over the node's cells of
 // r * detJ * sum_g sum_k sigma_g[j][k] * D[i][g][k], minus the external
 // weight, times *scale (and times the mask when u is the network output).
 template <bool MASK>
-__global__ void __launch_bounds__(kDemThreads)
-    k_dem_du(DemK K, const float* __restrict__ u, const float* __restrict__ mask, const float* __restrict__ rho,
-             const float* __restrict__ wext, const float* __restrict__ scale, float* __restrict__ du) {
+__device__ __forceinline__ void
+    dem_du(const DemK& K, const float* __restrict__ u, const float* __restrict__ mask, const float* __restrict__ rho,
+           const float* __restrict__ wext, const float* __restrict__ scale, float* __restrict__ du, unsigned block,
+           unsigned blocks) {
   const int NX = K.nx + 1, NY = K.ny + 1;
   const size_t nn = size_t(NX) * NY;
   const float sc = *scale;
-  for (size_t n = size_t(blockIdx.x) * blockDim.x + threadIdx.x; n < nn; n += size_t(gridDim.x) * blockDim.x) {
+  for (size_t n = size_t(block) * blockDim.x + threadIdx.x; n < nn; n += size_t(blocks) * blockDim.x) {
     const int ix = int(n / NY), iy = int(n - size_t(ix) * NY);
     float g0 = 0.0f, g1 = 0.0f;
 #pragma unroll
@@ -247,6 +260,20 @@ __global__ void __launch_bounds__(kDemThreads)
     du[2 * n] = sc * g0;
     du[2 * n + 1] = sc * g1;
   }
+}
+
+// Both gradients in one launch: the first `nodes` blocks take d psi / d u, the others
+// d psi / d rho (either share may be empty).
+template <bool MASK>
+__global__ void __launch_bounds__(kDemThreads)
+    k_dem_backward(DemK K, const float* __restrict__ u, const float* __restrict__ mask, const float* __restrict__ rho,
+                   const float* __restrict__ wext, const float* __restrict__ scale, float* __restrict__ du,
+                   float* __restrict__ drho, unsigned nodes) {
+  if (blockIdx.x < nodes)
+    dem_du<MASK>(K, u, mask, rho, wext, scale, du, blockIdx.x, nodes);
+  else
+    dem_cells<kDemDensityGrad, MASK>(K, u, mask, rho, nullptr, scale, drho, nullptr, nullptr, nullptr, nullptr,
+                                     blockIdx.x - nodes, gridDim.x - nodes);
 }
 
 __global__ void k_dem_enforce(const float* __restrict__ uh, const float* __restrict__ mask, float* __restrict__ u,
@@ -622,25 +649,33 @@ int topo_dem_enforce(topo_dem_ctx* ctx, const float* u_hat, float* u, topo_strea
   });
 }
 
-int topo_dem_energy(topo_dem_ctx* ctx, const float* u, const float* density, int masked, double* energy,
-                    topo_stream_t stream) {
+static int dem_energy(topo_dem_ctx* ctx, const float* u, const float* density, int masked, double* e64, float* e32,
+                      topo_stream_t stream) {
   return guarded(ctx, [&]() {
-    if (!u || !density || !energy) return ctx->fail(TOPO_ERR_ARG, "null array");
+    if (!u || !density || (!e64 && !e32)) return ctx->fail(TOPO_ERR_ARG, "null array");
     if (!ctx->penal_set) return ctx->fail(TOPO_ERR_STATE, "You must set penalization before calling penalizer");
     if (masked && !ctx->mask) return ctx->fail(TOPO_ERR_STATE, "no Dirichlet mask set");
     const DemK K = make_k(ctx);
     const size_t n = std::max(size_t(K.nx) * K.ny, size_t(K.nx + 1) * (K.ny + 1));
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (masked)
-      k_dem_cells<kDemEnergy, true><<<grid_for(ctx, n), kDemThreads, 0, s>>>(K, u, ctx->mask, density, ctx->wext,
-                                                                             nullptr, nullptr, ctx->partials,
-                                                                             ctx->counter, energy);
+      k_dem_cells<kDemEnergy, true><<<grid_for(ctx, n), kDemThreads, 0, s>>>(K, u, ctx->mask, density, ctx->wext, nullptr,
+                                                                             ctx->partials, ctx->counter, e64, e32);
     else
-      k_dem_cells<kDemEnergy, false><<<grid_for(ctx, n), kDemThreads, 0, s>>>(K, u, nullptr, density, ctx->wext,
-                                                                              nullptr, nullptr, ctx->partials,
-                                                                              ctx->counter, energy);
+      k_dem_cells<kDemEnergy, false><<<grid_for(ctx, n), kDemThreads, 0, s>>>(K, u, nullptr, density, ctx->wext, nullptr,
+                                                                              ctx->partials, ctx->counter, e64, e32);
     return ctx->cuda_check("energy");
   });
+}
+
+int topo_dem_energy(topo_dem_ctx* ctx, const float* u, const float* density, int masked, double* energy,
+                    topo_stream_t stream) {
+  return dem_energy(ctx, u, density, masked, energy, nullptr, stream);
+}
+
+int topo_dem_energy_f32(topo_dem_ctx* ctx, const float* u, const float* density, int masked, float* energy,
+                        topo_stream_t stream) {
+  return dem_energy(ctx, u, density, masked, nullptr, energy, stream);
 }
 
 int topo_dem_energy_backward(topo_dem_ctx* ctx, const float* u, const float* density, int masked, const float* scale,
@@ -651,36 +686,40 @@ int topo_dem_energy_backward(topo_dem_ctx* ctx, const float* u, const float* den
     if (masked && !ctx->mask) return ctx->fail(TOPO_ERR_STATE, "no Dirichlet mask set");
     const DemK K = make_k(ctx);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const size_t nc = size_t(K.nx) * K.ny, nn = size_t(K.nx + 1) * (K.ny + 1);
-    if (ddensity) {
-      if (masked)
-        k_dem_cells<kDemDensityGrad, true><<<grid_for(ctx, nc), kDemThreads, 0, s>>>(
-            K, u, ctx->mask, density, nullptr, scale, ddensity, nullptr, nullptr, nullptr);
-      else
-        k_dem_cells<kDemDensityGrad, false><<<grid_for(ctx, nc), kDemThreads, 0, s>>>(
-            K, u, nullptr, density, nullptr, scale, ddensity, nullptr, nullptr, nullptr);
-    }
-    if (du) {
-      if (masked)
-        k_dem_du<true><<<grid_for(ctx, nn), kDemThreads, 0, s>>>(K, u, ctx->mask, density, ctx->wext, scale, du);
-      else
-        k_dem_du<false><<<grid_for(ctx, nn), kDemThreads, 0, s>>>(K, u, nullptr, density, ctx->wext, scale, du);
-    }
+    const unsigned nodes = du ? unsigned(grid_for(ctx, size_t(K.nx + 1) * (K.ny + 1))) : 0u;
+    const unsigned cells = ddensity ? unsigned(grid_for(ctx, size_t(K.nx) * K.ny)) : 0u;
+    if (nodes + cells == 0) return ctx->cuda_check("energy backward");
+    if (masked)
+      k_dem_backward<true><<<nodes + cells, kDemThreads, 0, s>>>(K, u, ctx->mask, density, ctx->wext, scale, du, ddensity,
+                                                                 nodes);
+    else
+      k_dem_backward<false><<<nodes + cells, kDemThreads, 0, s>>>(K, u, nullptr, density, ctx->wext, scale, du, ddensity,
+                                                                  nodes);
     return ctx->cuda_check("energy backward");
+  });
+}
+
+static int dem_objective(topo_dem_ctx* ctx, const float* u, const float* density, double* o64, float* o32,
+                         float* gradient, topo_stream_t stream) {
+  return guarded(ctx, [&]() {
+    if (!u || !density || (!o64 && !o32) || !gradient) return ctx->fail(TOPO_ERR_ARG, "null array");
+    if (!ctx->penal_set) return ctx->fail(TOPO_ERR_STATE, "You must set penalization before calling penalizer");
+    const DemK K = make_k(ctx);
+    const size_t nc = size_t(K.nx) * K.ny;
+    k_dem_cells<kDemObjective, false><<<grid_for(ctx, nc), kDemThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        K, u, nullptr, density, nullptr, gradient, ctx->partials, ctx->counter, o64, o32);
+    return ctx->cuda_check("objective and gradient");
   });
 }
 
 int topo_dem_objective_gradient(topo_dem_ctx* ctx, const float* u, const float* density, double* objective,
                                 float* gradient, topo_stream_t stream) {
-  return guarded(ctx, [&]() {
-    if (!u || !density || !objective || !gradient) return ctx->fail(TOPO_ERR_ARG, "null array");
-    if (!ctx->penal_set) return ctx->fail(TOPO_ERR_STATE, "You must set penalization before calling penalizer");
-    const DemK K = make_k(ctx);
-    const size_t nc = size_t(K.nx) * K.ny;
-    k_dem_cells<kDemObjective, false><<<grid_for(ctx, nc), kDemThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        K, u, nullptr, density, nullptr, nullptr, gradient, ctx->partials, ctx->counter, objective);
-    return ctx->cuda_check("objective and gradient");
-  });
+  return dem_objective(ctx, u, density, objective, nullptr, gradient, stream);
+}
+
+int topo_dem_objective_gradient_f32(topo_dem_ctx* ctx, const float* u, const float* density, float* objective,
+                                    float* gradient, topo_stream_t stream) {
+  return dem_objective(ctx, u, density, nullptr, objective, gradient, stream);
 }
 
 }  // extern "C"

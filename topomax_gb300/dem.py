@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes
 from dataclasses import dataclass
+import itertools
 import math
 from typing import Iterable
 
@@ -331,6 +332,7 @@ class _DemContext:
             raise RuntimeError(f"topo_dem_create failed ({st.value})")
         self.mesh = mesh
         self.detJ = detJ
+        self.mask_version = None  # the version of the Dirichlet mask on the device
 
     def check(self, rc: int) -> None:
         if rc == _capi.TOPO_OK:
@@ -412,15 +414,26 @@ def create_density_filter(radius: float, mesh: Mesh) -> DensityFilter:
     return DensityFilter(radius, mesh)
 
 
+def _as_f32(t: torch.Tensor) -> torch.Tensor:
+    """t detached, as contiguous float32 on the current device (itself where it is that: an
+    evaluation is a handful of microseconds of kernels, a conversion call costs as much)."""
+    d = t.detach()
+    if d.dtype is torch.float32 and d.is_cuda and d.is_contiguous() and d.get_device() == torch.cuda.current_device():
+        return d
+    return d.to(device="cuda", dtype=torch.float32).contiguous()
+
+
 def _as_u(u: torch.Tensor, mesh: Mesh) -> torch.Tensor:
     nn = (mesh.Nx + 1) * (mesh.Ny + 1)
     if u.shape != (nn, 2):
         raise ValueError(f"u must have shape ({nn}, 2), got {tuple(u.shape)}")
-    return u.detach().to(device="cuda", dtype=torch.float32).contiguous()
+    return _as_f32(u)
 
 
 def _as_density(rho: torch.Tensor, mesh: Mesh) -> torch.Tensor:
-    r = rho.detach().to(device="cuda", dtype=torch.float32).contiguous()
+    r = _as_f32(rho)
+    if r.shape == mesh.intervals:
+        return r
     if r.numel() != mesh.Nx * mesh.Ny:
         raise ValueError(f"density must have {mesh.Nx * mesh.Ny} cells, got {r.numel()}")
     return r.reshape(mesh.intervals)
@@ -432,24 +445,26 @@ class _EnergyFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, u, rho, dem, masked):
         uu, rr = _as_u(u, dem.mesh), _as_density(rho, dem.mesh)
-        out = torch.empty((), dtype=torch.float64, device="cuda")
-        dem.check(dem.lib.topo_dem_energy(dem.ptr, _ptr(uu), _ptr(rr), int(masked), _ptr(out), _stream()))
+        out = uu.new_empty(())
+        dem.check(dem.lib.topo_dem_energy_f32(dem.ptr, _ptr(uu), _ptr(rr), int(masked), _ptr(out), _stream()))
         ctx.save_for_backward(uu, rr)
         ctx.dem, ctx.masked = dem, masked
         ctx.rho_shape = rho.shape
-        return out.to(torch.float32)
+        return out
 
     @staticmethod
     def backward(ctx, grad):
         uu, rr = ctx.saved_tensors
         dem = ctx.dem
-        scale = grad.detach().to(device="cuda", dtype=torch.float32).reshape(()).contiguous()
+        scale = _as_f32(grad)
         du = torch.empty_like(uu) if ctx.needs_input_grad[0] else None
         dr = torch.empty_like(rr) if ctx.needs_input_grad[1] else None
         dem.check(dem.lib.topo_dem_energy_backward(dem.ptr, _ptr(uu), _ptr(rr), int(ctx.masked), _ptr(scale),
                                                    _ptr(du) if du is not None else None,
                                                    _ptr(dr) if dr is not None else None, _stream()))
-        return du, (dr.reshape(ctx.rho_shape) if dr is not None else None), None, None
+        if dr is not None and dr.shape != ctx.rho_shape:
+            dr = dr.reshape(ctx.rho_shape)
+        return du, dr, None, None
 
 
 class StrainEnergy:
@@ -500,11 +515,14 @@ class StrainEnergy:
         """(sum r(rho) SE detJ, -r'(rho) SE detJ) as float32 tensors (gradient shaped like density)."""
         self._check_shape(shape)
         uu, rr = _as_u(u, self.mesh), _as_density(density, self.mesh)
-        obj = torch.empty((), dtype=torch.float64, device="cuda")
+        obj = uu.new_empty(())
         grad = torch.empty_like(rr)
-        self._dem.check(self._dem.lib.topo_dem_objective_gradient(self._dem.ptr, _ptr(uu), _ptr(rr), _ptr(obj),
-                                                                  _ptr(grad), _stream()))
-        return obj.to(torch.float32), grad.reshape(density.shape)
+        self._dem.check(self._dem.lib.topo_dem_objective_gradient_f32(self._dem.ptr, _ptr(uu), _ptr(rr), _ptr(obj),
+                                                                      _ptr(grad), _stream()))
+        return obj, (grad if grad.shape == density.shape else grad.reshape(density.shape))
+
+
+_mask_versions = itertools.count(1)  # one per mask: contexts tell by it which they hold
 
 
 class ElasticityEnforcer:
@@ -527,12 +545,24 @@ class ElasticityEnforcer:
                 z = z * ny
             else:
                 raise ValueError(f"Unknown side: '{side}'")
-        self.mask_host = np.ascontiguousarray(z.astype(np.float32))
-        self.zero_enforcer = torch.from_numpy(self.mask_host).to(device or "cuda")
+        self._mask = np.ascontiguousarray(z.astype(np.float32))
+        self._mask_version = next(_mask_versions)
+        self.zero_enforcer = torch.from_numpy(self._mask).to(device or "cuda")
         self._dem = None
 
+    @property
+    def mask_host(self) -> np.ndarray:
+        """The mask's host array.  Whoever takes it may write to it: from then on it is
+        uploaded for every use."""
+        self._mask_version = None
+        return self._mask
+
     def _install(self, dem: _DemContext) -> None:
-        dem.check(dem.lib.topo_dem_set_mask(dem.ptr, self.mask_host.ctypes.data))
+        # the upload waits for the device: once per mask and context, not per evaluation
+        if self._mask_version is None or dem.mask_version != self._mask_version:
+            dem.mask_version = None
+            dem.check(dem.lib.topo_dem_set_mask(dem.ptr, self._mask.ctypes.data))
+            dem.mask_version = self._mask_version
         self._dem = dem
 
     def __call__(self, u: torch.Tensor) -> torch.Tensor:
