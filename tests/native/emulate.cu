@@ -218,44 +218,50 @@ P2Params<T> p2params(int nx, int ny, double hx, double hy, double lam, double mu
 namespace {
 // Both sweeps of a stencil level over all blocks, every thread of a phase before any of the
 // next; shared memory starts as NaN.
-template <class T, int NC>
+template <class T, int NC, int D>
 void level_sweeps(LevelSweep<T, NC> P, const T* b, const T* xin, const T* xc, T* xpre, T* bc, T* xpost) {
+  using Ph = LevelPhases<T, NC>;
   const T nan = std::numeric_limits<T>::quiet_NaN();
-  const int nt = 256;
   for (int J0 = 0; J0 < P.NYc; J0 += P.cy)
-    for (int I0 = 0; I0 < P.NXc; I0 += P.cx) {
-      std::vector<T> sm(P.down_shared(), nan);
-      T *sx = sm.data(), *sd = sx + NC * P.down_w() * P.down_h();
-      std::vector<LevelNode<T, NC>> N(nt);
-      std::vector<char> on(nt);
-      for (int t = 0; t < nt; ++t) on[t] = LevelDown<T, NC>::start(P, I0, J0, t, N[t]);
-      for (int t = 0; t < nt; ++t) {
-        LevelDown<T, NC>::first(P, I0, J0, t, nt, b, sd);
-        if (on[t]) N[t].load_b(P, b);
+    for (int I0 = 0; I0 < P.NXc; I0 += P.cx)
+      for (int up = 0; up < 2; ++up) {
+        const int w = up ? up_w<D>(P) : down_w<D>(P), h = up ? up_h<D>(P) : down_h<D>(P);
+        const int ring = up ? D - 1 : D, a0 = 2 * I0 - ring, b0 = 2 * J0 - ring, nt = (w * h + 31) / 32 * 32;
+        std::vector<T> sm(sweep_shared(w, h, NC), nan);
+        T *s = sm.data(), *sn = s + NC * (w + 2) * (h + 2);
+        std::vector<typename Ph::Node> N(nt);
+        std::vector<char> on(nt);
+        for (int t = 0; t < nt; ++t) on[t] = Ph::start(P, a0, b0, w, h, t, N[t]);
+        auto each = [&](auto&& f) {
+          for (int t = 0; t < nt; ++t)
+            if (on[t]) f(t, N[t]);
+        };
+        for (int t = 0; t < nt; ++t) {
+          if (up) Ph::up_first(P, a0, b0, w, h, t, nt, xin, xc, s);
+          else Ph::down_first(P, a0, b0, w, h, t, nt, b, s);
+        }
+        each([&](int, auto& n) { n.load_b(P, b); });
+        if (!up) each([&](int, auto& n) { Ph::down_own(s, n); });
+        if (up) {
+          each([&](int, auto& n) { Ph::up_residual(P, w, s, sn, n); });
+          std::swap(s, sn);
+        }
+        for (int k = 1; k < D; ++k) {
+          each([&](int, auto& n) {
+            if (k + 1 < D) Ph::step(P, k, w, s, sn, n);
+            else Ph::last(P, k, w, s, up ? nullptr : sn, n);
+          });
+          std::swap(s, sn);
+        }
+        each([&](int t, auto& n) { Ph::store(P, w, ring, t, n, up ? xpost : xpre); });
+        if (up) continue;
+        each([&](int, auto& n) { Ph::down_residual(w, s, sn, n); });
+        for (int t = 0; t < nt; ++t) Ph::restrict_to(P, I0, J0, w, ring, t, nt, sn, bc);
       }
-      for (int t = 0; t < nt; ++t)
-        if (on[t]) LevelDown<T, NC>::smooth(P, t, N[t], sd, sx, xpre);
-      for (int t = 0; t < nt; ++t)
-        if (on[t]) LevelDown<T, NC>::residual(P, t, N[t], sx, sd);
-      for (int t = 0; t < nt; ++t) LevelDown<T, NC>::restrict_to(P, I0, J0, t, nt, sd, bc);
-      sm.assign(P.up_shared(), nan);
-      sd = sm.data();
-      sx = sd + NC * P.up_w() * P.up_h();
-      std::vector<typename LevelUp<T, NC>::Node> U(nt);
-      for (int t = 0; t < nt; ++t) on[t] = LevelUp<T, NC>::start(P, I0, J0, t, U[t]);
-      for (int t = 0; t < nt; ++t) {
-        LevelUp<T, NC>::correct(P, I0, J0, t, nt, xin, xc, sx);
-        if (on[t]) U[t].load_b(P, b);
-      }
-      for (int t = 0; t < nt; ++t)
-        if (on[t]) LevelUp<T, NC>::first(P, t, U[t], sx, sd);
-      for (int t = 0; t < nt; ++t)
-        if (on[t] && LevelUp<T, NC>::owned(P, t, U[t])) LevelUp<T, NC>::second(P, t, U[t], sd, xpost);
-    }
 }
 
 template <class T, int NC>
-int emu_sweeps(int nx, int ny, double hx, double hy, double lam, double mu, const int* dir, const double* kK,
+int emu_sweeps(int D, int nx, int ny, double hx, double hy, double lam, double mu, const int* dir, const double* kK,
                const double* kM, const double* cheb, int NXc, int NYc, const int* dirc, int cx, int cy,
                const double* b, const double* dinv, const double* xin, const double* xc, double* xpre, double* bc,
                double* xpost) {
@@ -283,7 +289,7 @@ int emu_sweeps(int nx, int ny, double hx, double hy, double lam, double mu, cons
     for (int i = 0; i < NX; ++i) p1_stencil_node<T, NC>(i, j, Q, st.data() + (size_t(j) * NX + i) * SW);
   LevelSweep<T, NC> P;
   std::memset(&P, 0, sizeof(P));
-  const std::vector<T> ch = cast(cheb, 3), di = cast(dinv, n * NC), bb = cast(b, n * NC), xi = cast(xin, n * NC),
+  const std::vector<T> ch = cast(cheb, 2 * D - 1), di = cast(dinv, n * NC), bb = cast(b, n * NC), xi = cast(xin, n * NC),
                        xcc = cast(xc, size_t(NXc) * NYc * NC);
   P.NX = NX;
   P.NY = NY;
@@ -297,7 +303,12 @@ int emu_sweeps(int nx, int ny, double hx, double hy, double lam, double mu, cons
   P.dirf = Q.dir;
   P.dirc = dir_from(dirc);
   std::vector<T> o1(n * NC, T(-7)), o2(size_t(NXc) * NYc * NC, T(-7)), o3(n * NC, T(-7));
-  level_sweeps<T, NC>(P, bb.data(), xi.data(), xcc.data(), o1.data(), o2.data(), o3.data());
+  auto run = [&](auto d) {
+    level_sweeps<T, NC, decltype(d)::value>(P, bb.data(), xi.data(), xcc.data(), o1.data(), o2.data(), o3.data());
+  };
+  if (D == 2) run(std::integral_constant<int, 2>{});
+  else if (D == 3) run(std::integral_constant<int, 3>{});
+  else run(std::integral_constant<int, 4>{});
   std::copy(o1.begin(), o1.end(), xpre);
   std::copy(o2.begin(), o2.end(), bc);
   std::copy(o3.begin(), o3.end(), xpost);
@@ -307,13 +318,13 @@ int emu_sweeps(int nx, int ny, double hx, double hy, double lam, double mu, cons
 
 extern "C" {
 
-// down and up sweep of a stencil level (prec 0 FP64, 1 FP32) with cx x cy coarse nodes a block
-int emu_level_sweeps(int prec, int NC, int nx, int ny, double hx, double hy, double lam, double mu, const int* dir,
+// down and up sweep of D steps of a stencil level (prec 0 FP64, 1 FP32), cx x cy coarse nodes a block
+int emu_level_sweeps(int prec, int NC, int D, int nx, int ny, double hx, double hy, double lam, double mu, const int* dir,
                      const double* kK, const double* kM, const double* cheb, int NXc, int NYc, const int* dirc, int cx,
                      int cy, const double* b, const double* dinv, const double* xin, const double* xc, double* xpre,
                      double* bc, double* xpost) {
 #define TOPO_EMU_SWEEP(T, K) \
-  emu_sweeps<T, K>(nx, ny, hx, hy, lam, mu, dir, kK, kM, cheb, NXc, NYc, dirc, cx, cy, b, dinv, xin, xc, xpre, bc, xpost)
+  emu_sweeps<T, K>(D, nx, ny, hx, hy, lam, mu, dir, kK, kM, cheb, NXc, NYc, dirc, cx, cy, b, dinv, xin, xc, xpre, bc, xpost)
   if (NC == 2) return prec ? TOPO_EMU_SWEEP(float, 2) : TOPO_EMU_SWEEP(double, 2);
   return prec ? TOPO_EMU_SWEEP(float, 1) : TOPO_EMU_SWEEP(double, 1);
 #undef TOPO_EMU_SWEEP

@@ -2,8 +2,8 @@
 
 On the CPU the phases run over all blocks with NaN-filled shared memory and are compared with
 the same steps composed from plain operator applies and the transfers; on the GPU a V-cycle
-with the one-block tail is compared with one launch per level.  FP64 steps chain three
-applications of a 7-point operator of O(1) values: 1e-12; FP32 likewise at 2^-24: 1e-5.
+with the one-block tail is compared with one launch per level.  FP64 steps chain up to
+five applications of a 7-point operator of O(1) values: 1e-12; FP32 likewise at 2^-24: 1e-5.
 """
 import ctypes
 
@@ -39,8 +39,9 @@ def _free(dirv, NX, NY, NC):
 @pytest.mark.parametrize("prec,tol", [(0, 1e-12), (1, 1e-5)])
 @pytest.mark.parametrize("NC,sides", [(2, ["Left"]), (2, ["Left", "Right"]), (1, []),
                                       (1, ["Left", "Right", "Top", "Bottom"])])
+@pytest.mark.parametrize("D", [2, 3, 4])
 @pytest.mark.parametrize("nx,ny", SIZES)
-def test_sweeps_match_composed_steps(nx, ny, NC, sides, prec, tol):
+def test_sweeps_match_composed_steps(nx, ny, D, NC, sides, prec, tol):
     rng = np.random.default_rng(100 * nx + ny)
     lam, mu, hx, hy, dirv, f, c, kK, kM = _level(NC, nx, ny, sides, rng)
     A = lambda u: emu.p1_apply(NC, nx, ny, hx, hy, lam, mu, dirv, kK, kM, u)  # noqa: E731
@@ -49,26 +50,32 @@ def test_sweeps_match_composed_steps(nx, ny, NC, sides, prec, tol):
     b, x = rng.standard_normal(n) * free, rng.standard_normal(n) * free
     xc = rng.standard_normal(nc) * freec
     dinv = np.where(free, rng.uniform(0.5, 2.0, n), 1.0)
-    cheb = np.array([0.7, 0.3, 0.9])
+    cheb = np.array([0.7, 0.3, 0.9, 0.2, 0.6, 0.25, 0.5])[:2 * D - 1]
     xpre, bc, xpost = np.zeros(n), np.zeros(nc), np.zeros(n)
-    P, I, D = emu.P_D, ctypes.c_int, ctypes.c_double
+    P, I, F = emu.P_D, ctypes.c_int, ctypes.c_double
     E = emu.lib()
-    E.emu_level_sweeps.argtypes = [I, I, I, I, D, D, D, D, emu.P_I, P, P, P, I, I, emu.P_I, I, I] + [P] * 7
-    assert E.emu_level_sweeps(prec, NC, nx, ny, hx, hy, lam, mu, emu.ip(dirv), emu.dp(kK), emu.dp(kM), emu.dp(cheb),
+    E.emu_level_sweeps.argtypes = [I, I, I, I, I, F, F, F, F, emu.P_I, P, P, P, I, I, emu.P_I, I, I] + [P] * 7
+    assert E.emu_level_sweeps(prec, NC, D, nx, ny, hx, hy, lam, mu, emu.ip(dirv), emu.dp(kK), emu.dp(kM), emu.dp(cheb),
                               c["NX"], c["NY"], emu.ip(c["dir"]), 10, 4, emu.dp(b), emu.dp(dinv), emu.dp(x),
                               emu.dp(xc), emu.dp(xpre), emu.dp(bc), emu.dp(xpost)) == 0
 
     def close(got, want):
         assert np.max(np.abs(got - want)) <= tol * max(np.max(np.abs(want)), 1e-30)
 
-    d0 = cheb[0] * dinv * b
-    ref = d0 + cheb[1] * d0 + cheb[2] * dinv * (b - A(d0))
+    def chebyshev(r, x):
+        d = cheb[0] * dinv * r
+        x = x + d
+        for k in range(1, D):
+            r = r - A(d)
+            d = cheb[2 * k - 1] * d + cheb[2 * k] * dinv * r
+            x = x + d
+        return x
+
+    ref = chebyshev(b, np.zeros(n))
     close(xpre, ref)
     close(bc, emu.restrict(NC, f["NX"], f["NY"], f["dir"], c["NX"], c["NY"], c["dir"], b - A(ref)))
     u = x + emu.prolong(NC, f["NX"], f["NY"], f["dir"], c["NX"], c["NY"], c["dir"], xc)
-    r0 = b - A(u)
-    e0 = cheb[0] * dinv * r0
-    close(xpost, u + e0 + cheb[1] * e0 + cheb[2] * dinv * (r0 - A(e0)))
+    close(xpost, chebyshev(b - A(u), u))
 
 
 @pytest.mark.gpu

@@ -838,6 +838,8 @@ topo_ctx* topo_create(const topo_grid_desc* grid, const topo_material* mat, cons
         C->smg32.use_graphs = graphs_enabled();
         C->smg32.fp64_solution = true;
         C->smg32.cheb_lo_frac = C->cheb_lo_state;
+        C->smg32.deep_degree = kCoarseDegree;
+        C->smg32.cheb_lo_deep = 0.008;
         C->smg32.trace_setup = C->trace_solves;
         C->smg32.use_tail = env_flag("TOPO_TAIL", true);
         C->smg32.profile_levels = env_flag("TOPO_PROFILE", false);

@@ -824,6 +824,9 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
     mg->use_graphs = false;  // only V-cycles are used
     mg->profile_levels = false;
     mg->element_bounds = true;
+    mg->deep_degree = kScalarDegree;
+    mg->deep_from = 0;
+    mg->cheb_lo_deep = 0.3;
   }
   C->mgu.batch = 2;
   C->mgu.init(C->uspec, C->urefs.data(), 0.0, 0.0, C->arena, &C->red);

@@ -21,6 +21,7 @@
 namespace topo {
 
 constexpr int kCoarseMaxDofs = 32;
+constexpr int kCoarseDegree = 4, kScalarDegree = 3;  // FP32 sweeps of MG::deep_degree steps
 
 // Device memory owner: everything allocated here is freed with the arena.
 class Arena {
@@ -178,7 +179,22 @@ class MG {
   // the FP32 operator arithmetic alone is consistent to ~1e-4.  Set before init().
   bool fp64_solution = false;
 
-  int cheb_degree = 2;  // the fused smoothing kernels implement degree 2
+  // Chebyshev steps of a smoothing sweep: two on level 0 of a P2 hierarchy, on the levels
+  // without a stencil (march kernels) and above deep_from; deep_degree on the others (2, or
+  // FP32 kCoarseDegree for elasticity and kScalarDegree for scalar levels).
+  //
+  // State hierarchy, FP32: the iterations of a solve grow with the design's contrast through
+  // the P1 levels below the first, and a further step inside a sweep costs less there than
+  // what it saves: with 2, 3 and 4 steps from level 2 on, design evaluations took 5.46, 5.25
+  // and 5.07 ms (80x40), 16.8, 15.4 and 13.9 (303x101), 18.1, 16.8 and 15.3 (1000x500), 45.8,
+  // 41.9 and 37.9 (2000x1000).  The interval's lower end between 0.005 and 0.03 lambda_max
+  // is within 3 %.  FP64 sweeps are bound by the FP64 pipe: two steps (59.4 ms against 58.5
+  // with three and 80 with four before their tiles were fitted).
+  // Fluid preconditioner: 11.3, 10.5 and 10.6 ms (40x40), 21.3, 19.7 and 20.5 (128x128).
+  // Filter: no difference (1.36 ms at 1000x500).
+  int deep_degree = 2, deep_from = 2;
+  double cheb_lo_deep = 0.1;  // their interval's lower end, times lambda_max
+  int level_degree(int l) const { return l >= deep_from && lv_[l].st ? deep_degree : 2; }
   double cheb_lo_frac = 0.1;   // smoothing interval [lo_frac, 1.1] * lambda_max
   int power_iters = 10;
   int power_iters_warm = 4;  // level 0 of a P2 hierarchy, started from the previous set-up's vector
@@ -227,6 +243,14 @@ class MG {
   void vcycle_level(int l, const T* b, T* x, cudaStream_t s);
   void tune_marches(cudaStream_t s);
   void vcycle_level_body(int l, const T* b, T* x, cudaStream_t s);
+  template <int NC, int D>
+  void sweep_level(int l, const T* b, T* x, cudaStream_t s);
+  template <int NC>
+  void sweep_level(int l, const T* b, T* x, cudaStream_t s);
+  template <int NC, int D>
+  void launch_tail(const TailSweep<T, NC>& P, int nodes, const T* b, T* x, cudaStream_t s);
+  template <int NC>
+  void launch_tail(const TailSweep<T, NC>& P, int l, const T* b, T* x, cudaStream_t s);
   int prof_depth_ = 0;
   int capture_pcg(bool warm);
   void pcg_prologue(bool warm, cudaStream_t s);

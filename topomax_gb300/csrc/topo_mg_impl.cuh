@@ -238,53 +238,80 @@ __global__ void __launch_bounds__(P2M_THREADS) k_p1_march(P1Params<T, NC> P, P1I
 // 18.6, 6 x 6 19.2, 14 x 2 18.9; FP64 at 160x80 63.9 ms against 76.8, 66.1 and 66.2 (a tile's
 // recomputed ring costs FP64-pipe time, a large tile leaves SMs without a block).
 constexpr int kSweepTileX = 10, kSweepTileY = 4;
-constexpr int kSweepThreads = 256;
+template <int D>
+constexpr int sweep_threads() {  // the down sweep's region, the larger one
+  return ((2 * kSweepTileX + 2 * D - 1) * (2 * kSweepTileY + 2 * D - 1) + 31) / 32 * 32;
+}
 
-template <class T, int NC>
-__global__ void __launch_bounds__(kSweepThreads)
-    k_level_down(LevelSweep<T, NC> P, const T* b, T* x, T* bc) {
+template <class T, int NC, int D>
+__global__ void __launch_bounds__(sweep_threads<D>()) k_level_down(LevelSweep<T, NC> P, const T* b, T* x, T* bc) {
+  using Ph = LevelPhases<T, NC>;
   extern __shared__ __align__(16) unsigned char sweep_raw[];
-  T* sx = reinterpret_cast<T*>(sweep_raw);
-  T* sd = sx + NC * P.down_w() * P.down_h();
+  const int w = down_w<D>(P), h = down_h<D>(P);
+  T* s = reinterpret_cast<T*>(sweep_raw);
+  T* sn = s + NC * (w + 2) * (h + 2);
   const int tid = threadIdx.x, nt = blockDim.x, I0 = blockIdx.x * P.cx, J0 = blockIdx.y * P.cy;
   b += blockIdx.z * size_t(NC) * P.NX * P.NY;  // the batch's vectors
   x += blockIdx.z * size_t(NC) * P.NX * P.NY;
   bc += blockIdx.z * size_t(NC) * P.NXc * P.NYc;
   TOPO_PDL_LAUNCH();
-  LevelNode<T, NC> N;
-  const bool on = LevelDown<T, NC>::start(P, I0, J0, tid, N);
+  const int a0 = 2 * I0 - D, b0 = 2 * J0 - D;
+  typename Ph::Node N;
+  const bool on = Ph::start(P, a0, b0, w, h, tid, N);
   TOPO_PDL_WAIT();
-  LevelDown<T, NC>::first(P, I0, J0, tid, nt, b, sd);
+  Ph::down_first(P, a0, b0, w, h, tid, nt, b, s);
   if (on) N.load_b(P, b);
   __syncthreads();
-  if (on) LevelDown<T, NC>::smooth(P, tid, N, sd, sx, x);
+  if (on) Ph::down_own(s, N);
+#pragma unroll
+  for (int k = 1; k < D; ++k) {
+    if (on && k + 1 < D) Ph::step(P, k, w, s, sn, N);
+    if (on && k + 1 == D) Ph::last(P, k, w, s, sn, N);
+    T* const t = s;
+    s = sn;
+    sn = t;
+    __syncthreads();
+  }
+  if (on) {
+    Ph::store(P, w, D, tid, N, x);
+    Ph::down_residual(w, s, sn, N);
+  }
   __syncthreads();
-  if (on) LevelDown<T, NC>::residual(P, tid, N, sx, sd);
-  __syncthreads();
-  LevelDown<T, NC>::restrict_to(P, I0, J0, tid, nt, sd, bc);
+  Ph::restrict_to(P, I0, J0, w, D, tid, nt, sn, bc);
 }
 
-template <class T, int NC>
-__global__ void __launch_bounds__(kSweepThreads)
+template <class T, int NC, int D>
+__global__ void __launch_bounds__(sweep_threads<D>())
     k_level_up(LevelSweep<T, NC> P, const T* b, const T* xin, const T* xc, T* x) {
+  using Ph = LevelPhases<T, NC>;
   extern __shared__ __align__(16) unsigned char sweep_raw[];
-  T* sd = reinterpret_cast<T*>(sweep_raw);
-  T* sx = sd + NC * P.up_w() * P.up_h();
+  const int w = up_w<D>(P), h = up_h<D>(P);
+  T* s = reinterpret_cast<T*>(sweep_raw);
+  T* sn = s + NC * (w + 2) * (h + 2);
   const int tid = threadIdx.x, nt = blockDim.x, I0 = blockIdx.x * P.cx, J0 = blockIdx.y * P.cy;
   b += blockIdx.z * size_t(NC) * P.NX * P.NY;
   x += blockIdx.z * size_t(NC) * P.NX * P.NY;
   xin += blockIdx.z * size_t(NC) * P.NX * P.NY;
   xc += blockIdx.z * size_t(NC) * P.NXc * P.NYc;
   TOPO_PDL_LAUNCH();
-  typename LevelUp<T, NC>::Node N;
-  const bool on = LevelUp<T, NC>::start(P, I0, J0, tid, N);
+  const int a0 = 2 * I0 - (D - 1), b0 = 2 * J0 - (D - 1);
+  typename Ph::Node N;
+  const bool on = Ph::start(P, a0, b0, w, h, tid, N);
   TOPO_PDL_WAIT();
-  LevelUp<T, NC>::correct(P, I0, J0, tid, nt, xin, xc, sx);
+  Ph::up_first(P, a0, b0, w, h, tid, nt, xin, xc, s);
   if (on) N.load_b(P, b);
   __syncthreads();
-  if (on) LevelUp<T, NC>::first(P, tid, N, sx, sd);
-  __syncthreads();
-  if (on && LevelUp<T, NC>::owned(P, tid, N)) LevelUp<T, NC>::second(P, tid, N, sd, x);
+  if (on) Ph::up_residual(P, w, s, sn, N);
+#pragma unroll
+  for (int k = 1; k < D; ++k) {
+    T* const t = s;
+    s = sn;
+    sn = t;
+    __syncthreads();
+    if (on && k + 1 < D) Ph::step(P, k, w, s, sn, N);
+    if (on && k + 1 == D) Ph::last(P, k, w, s, static_cast<T*>(nullptr), N);
+  }
+  if (on) Ph::store(P, w, D - 1, tid, N, x);
 }
 
 template <class T, int NC>
@@ -411,12 +438,13 @@ __global__ void __launch_bounds__(32) k_coarse_inverse(int nx, int ny, Dir dir, 
 }
 
 // x = Ainv b on the coarsest level, n <= kCoarseMaxDofs (Ainv symmetric: column reads)
+constexpr int kDenseThreads = 256;
 template <class T>
-__global__ void __launch_bounds__(kCoarseMaxDofs) k_dense_matvec(const T* Ainv, const T* b, T* x, int n) {
+__global__ void __launch_bounds__(kDenseThreads) k_dense_matvec(const T* Ainv, const T* b, T* x, int n) {
   __shared__ T A[kCoarseMaxDofs * kCoarseMaxDofs], v[kCoarseMaxDofs];
   TOPO_PDL_LAUNCH();
   const int i = threadIdx.x;
-  for (int k = i; k < n * n; k += blockDim.x) A[k] = Ainv[k];
+  for (int k = i; k < n * n; k += kDenseThreads) A[k] = Ainv[k];
   TOPO_PDL_WAIT();
   if (i < n) v[i] = b[blockIdx.x * size_t(n) + i];
   __syncthreads();
@@ -429,9 +457,133 @@ __global__ void __launch_bounds__(kCoarseMaxDofs) k_dense_matvec(const T* Ainv, 
 constexpr int kCoarseThreads = 1024;                   // one-CTA coarse Chebyshev solve
 constexpr size_t kCoarseSharedBudget = 196 * 1024;
 
-// The last levels of the V-cycle (see TailSweep): x = V-cycle(b) from its level 0 down.
-// Latency-bound: seven barriers per level.
+// Phases of the tail.  A thread's node of a level: its row, inverse diagonal, right-hand side.
 template <class T, int NC>
+struct TailNode {
+  __align__(16) T st[StencilLayout<NC>::stride];
+  T di[NC], b[NC];
+};
+
+// D - 1 steps from the direction d in shared vector s; the direction goes to sn and back in turn,
+// r and v are the residual and the iterate.  The last step stores the iterate instead.
+// Returns its vector (the stores followed by a barrier).
+template <class T, int NC, int D>
+__device__ __forceinline__ T* tail_steps(const T* cheb, bool on, int w, int p, const TailNode<T, NC>& N, T (&r)[NC],
+                                         T (&v)[NC], T (&d)[NC], T* s, T* sn) {
+#pragma unroll
+  for (int k = 1; k < D; ++k) {
+    if (on) {
+      T t[NC];
+      level_apply<T, NC>(N.st, s, w, p, t);
+      const T c1 = cheb[2 * k - 1], c2 = cheb[2 * k];
+      for (int c = 0; c < NC; ++c) {
+        if (k + 1 < D) {
+          r[c] -= t[c];
+          d[c] = level_direction(c1, d[c], c2, N.di[c], r[c]);
+          v[c] += d[c];
+          sn[NC * p + c] = d[c];
+        } else {
+          v[c] = level_last(v[c], c1, d[c], c2, N.di[c], r[c] - t[c]);
+          sn[NC * p + c] = v[c];
+        }
+      }
+    }
+    T* const q = s;
+    s = sn;
+    sn = q;
+    __syncthreads();
+  }
+  return s;
+}
+
+// Level l from its right-hand side to the next level's; leaves x in L.x.
+template <class T, int NC, int D>
+__device__ __forceinline__ void tail_down(const TailSweep<T, NC>& P, int l, int tid, T* sm, const TailNode<T, NC>& N) {
+  const auto& L = P.lv[l];
+  const auto& K = P.lv[l + 1];
+  const bool on = tid < L.NX * L.NY;
+  const int j = tid / L.NX, i = tid - j * L.NX, w = L.NX + 2, p = on ? (j + 1) * w + i + 1 : 0;
+  T r[NC], v[NC], d[NC], t[NC];
+  const T c0 = L.cheb[0];
+  for (int c = 0; c < NC; ++c) {
+    r[c] = N.b[c];
+    v[c] = d[c] = (c0 * N.di[c]) * N.b[c];
+    if (on) sm[L.d + NC * p + c] = d[c];
+  }
+  __syncthreads();
+  const T* s = tail_steps<T, NC, D>(L.cheb, on, w, p, N, r, v, d, sm + L.d, sm + L.x);
+  if (on) level_apply<T, NC>(N.st, s, w, p, t);
+  __syncthreads();  // the iterate has been read
+  if (on)
+    for (int c = 0; c < NC; ++c) {
+      sm[L.d + NC * p + c] = N.b[c] - t[c];
+      sm[L.x + NC * p + c] = v[c];
+    }
+  __syncthreads();
+  if (tid < K.NX * K.NY) {
+    const int J = tid / K.NX, I = tid - J * K.NX;
+    const bool zero = is_clamped(K.dir, I, J);
+    const T* q = sm + L.d + NC * ((2 * J + 1) * w + 2 * I + 1);
+    for (int c = 0; c < NC; ++c) sm[K.b + NC * tid + c] = zero ? T(0) : level_restrict<T, NC>(q + c, w);
+  }
+  __syncthreads();
+}
+
+// Level l from x and the next level's correction to its solution: to xg (level 0) or L.x.
+template <class T, int NC, int D>
+__device__ __forceinline__ void tail_up(const TailSweep<T, NC>& P, int l, int tid, T* sm, const TailNode<T, NC>& N,
+                                        T* xg) {
+  const auto& L = P.lv[l];
+  const auto& K = P.lv[l + 1];
+  const bool on = tid < L.NX * L.NY;
+  const int j = tid / L.NX, i = tid - j * L.NX, w = L.NX + 2, p = on ? (j + 1) * w + i + 1 : 0;
+  T r[NC], v[NC], d[NC];
+  for (int c = 0; c < NC; ++c) r[c] = v[c] = d[c] = T(0);
+  if (on && !is_clamped(L.dir, i, j)) {
+    const int wc = K.NX + 2;
+    const int m0 = ((j >> 1) + 1) * wc + (i >> 1) + 1, m1 = (((j + 1) >> 1) + 1) * wc + ((i + 1) >> 1) + 1;
+    for (int c = 0; c < NC; ++c) {
+      const T u = sm[K.x + NC * m0 + c], q = sm[K.x + NC * m1 + c];
+      sm[L.x + NC * p + c] += m0 == m1 ? u : T(0.5) * (u + q);
+    }
+  }
+  __syncthreads();
+  if (on) {
+    T t[NC];
+    level_apply<T, NC>(N.st, sm + L.x, w, p, t);
+    const T c0 = L.cheb[0];
+    for (int c = 0; c < NC; ++c) {
+      r[c] = N.b[c] - t[c];
+      d[c] = (c0 * N.di[c]) * r[c];
+      v[c] = sm[L.x + NC * p + c] + d[c];
+      sm[L.d + NC * p + c] = d[c];
+    }
+  }
+  __syncthreads();
+  tail_steps<T, NC, D>(L.cheb, on, w, p, N, r, v, d, sm + L.d, sm + L.x);
+  if (on)
+    for (int c = 0; c < NC; ++c) {
+      if (l == 0) xg[NC * tid + c] = v[c];
+      else sm[L.x + NC * p + c] = v[c];
+    }
+  if (l) __syncthreads();
+}
+
+// a level >= 1's node from shared memory
+template <class T, int NC>
+__device__ __forceinline__ void tail_node(const TailSweep<T, NC>& P, int l, int tid, const T* sm, TailNode<T, NC>& N) {
+  const auto& L = P.lv[l];
+  const int n = tid < L.NX * L.NY ? tid : 0;
+  copy_row<T, StencilLayout<NC>::stride>(sm + L.row + n * StencilLayout<NC>::stride, N.st);
+  for (int c = 0; c < NC; ++c) {
+    N.di[c] = sm[L.di + NC * n + c];
+    N.b[c] = sm[L.b + NC * n + c];
+  }
+}
+
+// The last levels of the V-cycle (see TailSweep): x = V-cycle(b) from its level 0 down, D
+// Chebyshev steps each way.  Latency-bound: 2 D + 4 barriers a level.
+template <class T, int NC, int D>
 __global__ void __launch_bounds__(kTailNodes)
     k_level_tail(const __grid_constant__ TailSweep<T, NC> P, const T* b, T* x) {
   constexpr int SW = StencilLayout<NC>::stride;
@@ -457,67 +609,20 @@ __global__ void __launch_bounds__(kTailNodes)
   const int m = C.NX * C.NY * NC;
   for (int i = tid; i < m * m; i += nt) sm[P.inv + i] = P.cinv[i];
   const auto& L0 = P.lv[0];
-  const bool on0 = tid < L0.NX * L0.NY;
-  const int n0 = on0 ? tid : 0;
-  T st0[SW], di0[NC], b0[NC];
-  load_row(L0.st + size_t(n0) * SW, st0);
-  level_row<T, NC>(st0);
-  for (int c = 0; c < NC; ++c) di0[c] = L0.dinv[NC * n0 + c];
+  const int n0 = tid < L0.NX * L0.NY ? tid : 0;
+  TailNode<T, NC> N0;
+  load_row(L0.st + size_t(n0) * SW, N0.st);
+  level_row<T, NC>(N0.st);
+  for (int c = 0; c < NC; ++c) N0.di[c] = L0.dinv[NC * n0 + c];
   TOPO_PDL_WAIT();
-  for (int c = 0; c < NC; ++c) b0[c] = b[NC * n0 + c];
+  for (int c = 0; c < NC; ++c) N0.b[c] = b[NC * n0 + c];
   __syncthreads();  // the zeros are in place
-  // level l's node of this thread: rows and so on from registers (level 0) or shared memory
-  auto with_node = [&](int l, auto&& f) {
-    const auto& L = P.lv[l];
-    const int n = tid;
-    if (n >= L.NX * L.NY) return;
-    const int j = n / L.NX, i = n - j * L.NX, w = L.NX + 2, p = (j + 1) * w + i + 1;
-    if (l == 0) {
-      f(L, n, i, j, w, p, st0, di0, b0);
-    } else {
-      __align__(16) T st[SW];
-      T di[NC], bl[NC];
-      copy_row<T, SW>(sm + L.row + n * SW, st);
-      for (int c = 0; c < NC; ++c) {
-        di[c] = sm[L.di + NC * n + c];
-        bl[c] = sm[L.b + NC * n + c];
-      }
-      f(L, n, i, j, w, p, st, di, bl);
-    }
-  };
-  auto down = [&](int l) {
-    with_node(l, [&](const auto& L, int, int, int, int, int p, const auto&, const auto& di, const auto& bl) {
-      const T c0 = L.cheb[0];
-      for (int c = 0; c < NC; ++c) sm[L.d + NC * p + c] = (c0 * di[c]) * bl[c];
-    });
-    __syncthreads();
-    with_node(l, [&](const auto& L, int, int, int, int w, int p, const auto& st, const auto& di, const auto& bl) {
-      T t[NC];
-      level_apply<T, NC>(st, sm + L.d, w, p, t);
-      const T c1 = L.cheb[1], c2 = L.cheb[2];
-      for (int c = 0; c < NC; ++c) {
-        const T u = sm[L.d + NC * p + c];
-        sm[L.x + NC * p + c] = level_step(u, c1, u, c2, di[c], bl[c] - t[c]);
-      }
-    });
-    __syncthreads();
-    with_node(l, [&](const auto& L, int, int, int, int w, int p, const auto& st, const auto&, const auto& bl) {
-      T t[NC];
-      level_apply<T, NC>(st, sm + L.x, w, p, t);
-      for (int c = 0; c < NC; ++c) sm[L.d + NC * p + c] = bl[c] - t[c];
-    });
-    __syncthreads();
-    const auto& L = P.lv[l];
-    const auto& K = P.lv[l + 1];
-    if (tid < K.NX * K.NY) {
-      const int J = tid / K.NX, I = tid - J * K.NX, w = L.NX + 2;
-      const bool zero = is_clamped(K.dir, I, J);
-      const T* r = sm + L.d + NC * ((2 * J + 1) * w + 2 * I + 1);
-      for (int c = 0; c < NC; ++c) sm[K.b + NC * tid + c] = zero ? T(0) : level_restrict<T, NC>(r + c, w);
-    }
-    __syncthreads();
-  };
-  for (int l = 0; l < P.nlev; ++l) down(l);
+  tail_down<T, NC, D>(P, 0, tid, sm, N0);
+  for (int l = 1; l < P.nlev; ++l) {
+    TailNode<T, NC> N;
+    tail_node(P, l, tid, sm, N);
+    tail_down<T, NC, D>(P, l, tid, sm, N);
+  }
   if (tid < m) {  // the inverse is symmetric: column reads, one line per step
     T s = T(0);
     for (int k = 0; k < m; ++k) s = fma_t(sm[P.inv + k * m + tid], sm[C.b + k], s);
@@ -525,43 +630,12 @@ __global__ void __launch_bounds__(kTailNodes)
     sm[C.x + NC * ((j + 1) * (C.NX + 2) + i + 1) + tid % NC] = s;
   }
   __syncthreads();
-  for (int l = P.nlev - 1; l >= 0; --l) {
-    T r0[NC], d0[NC], x2[NC];
-    with_node(l, [&](const auto& L, int, int i, int j, int, int p, const auto&, const auto&, const auto&) {
-      const auto& K = P.lv[l + 1];
-      if (is_clamped(L.dir, i, j)) return;
-      const int wc = K.NX + 2;
-      const int m0 = ((j >> 1) + 1) * wc + (i >> 1) + 1, m1 = (((j + 1) >> 1) + 1) * wc + ((i + 1) >> 1) + 1;
-      for (int c = 0; c < NC; ++c) {
-        const T u = sm[K.x + NC * m0 + c], v = sm[K.x + NC * m1 + c];
-        sm[L.x + NC * p + c] += m0 == m1 ? u : T(0.5) * (u + v);
-      }
-    });
-    __syncthreads();
-    with_node(l, [&](const auto& L, int, int, int, int w, int p, const auto& st, const auto& di, const auto& bl) {
-      T t[NC];
-      level_apply<T, NC>(st, sm + L.x, w, p, t);
-      const T c0 = L.cheb[0];
-      for (int c = 0; c < NC; ++c) {
-        r0[c] = bl[c] - t[c];
-        d0[c] = (c0 * di[c]) * r0[c];
-        x2[c] = sm[L.x + NC * p + c] + d0[c];
-        sm[L.d + NC * p + c] = d0[c];
-      }
-    });
-    __syncthreads();
-    with_node(l, [&](const auto& L, int n, int, int, int w, int p, const auto& st, const auto& di, const auto&) {
-      T t[NC];
-      level_apply<T, NC>(st, sm + L.d, w, p, t);
-      const T c1 = L.cheb[1], c2 = L.cheb[2];
-      for (int c = 0; c < NC; ++c) {
-        const T v = level_step(x2[c], c1, d0[c], c2, di[c], r0[c] - t[c]);
-        if (l == 0) x[NC * n + c] = v;
-        else sm[L.x + NC * p + c] = v;
-      }
-    });
-    if (l) __syncthreads();
+  for (int l = P.nlev - 1; l >= 1; --l) {
+    TailNode<T, NC> N;
+    tail_node(P, l, tid, sm, N);
+    tail_up<T, NC, D>(P, l, tid, sm, N, x);
   }
+  tail_up<T, NC, D>(P, 0, tid, sm, N0, x);
 }
 
 template <class T, int NC>
@@ -583,7 +657,13 @@ struct CoarseChebDesc {
 // nodes per thread: what the registers of a 1024-thread block hold without spilling
 template <class T>
 constexpr int coarse_cheb_npt() {
-  return sizeof(T) == 4 ? 3 : 2;
+  return sizeof(T) == 4 ? 3 : 1;
+}
+// most nodes of the level: an FP64 step of a block issues at two products a clock, so above
+// 512 nodes a level's own sweeps over all SMs cost less (861 nodes: 37 us)
+template <class T>
+constexpr size_t coarse_cheb_nodes() {
+  return sizeof(T) == 4 ? size_t(kCoarseThreads) * coarse_cheb_npt<T>() : 512;
 }
 
 template <class T>
@@ -596,7 +676,8 @@ __global__ void __launch_bounds__(kCoarseThreads)
   const int tid = threadIdx.x, nt = blockDim.x;
   const int nn = D->nn, NX = D->NX;
   T* d1 = d0 + nn;
-  const CoarseCheb<T>& C = D->C;  // read in place (uniform loads)
+  __shared__ CoarseCheb<T> C;
+  if (tid == 0) C = D->C;
   const T* sg = D->S.s;
   b += blockIdx.x * size_t(nn);
   x_out += blockIdx.x * size_t(nn);
@@ -607,8 +688,13 @@ __global__ void __launch_bounds__(kCoarseThreads)
     const bool on = n < nn;
 #pragma unroll
     for (int k = 0; k < 7; ++k) st[q][k] = on ? sg[size_t(n) * SW + k] : T(0);
+    if constexpr (sizeof(T) == 8) {  // plain rows for FP64 (level_row)
+#pragma unroll
+      for (int k = 1; k < 7; ++k) st[q][0] -= st[q][k];
+    }
     dv[q] = on ? D->dinv[n] : T(0);
   }
+  __syncthreads();
   TOPO_PDL_WAIT();  // the rows above are fixed during a solve
 #pragma unroll
   for (int q = 0; q < NP; ++q) {
@@ -633,7 +719,7 @@ __global__ void __launch_bounds__(kCoarseThreads)
 #pragma unroll
         for (int e = 1; e < 7; ++e) {
           const int m = min(max(n + st_da(e) + st_db(e) * NX, 0), nn - 1);
-          t += st[q][e] * (dc[m] - dn0);
+          t += st[q][e] * (sizeof(T) == 8 ? dc[m] : dc[m] - dn0);
         }
         x[q] += dn0;
         r[q] -= t;
@@ -898,6 +984,21 @@ inline LevelSweep<T, NC> level_sweep(const LevelSpec& S, const Transfer& X, cons
   P.NYc = X.NYc;
   P.cx = kSweepTileX;
   P.cy = kSweepTileY;
+  if (sizeof(T) == 8) {
+    // FP64: a block's time is its warps' (the SM's FP64 pipe takes two products a clock), so
+    // the tile is the one whose waves of blocks hold the fewest warps per SM
+    const int tiles[][2] = {{10, 4}, {9, 3}, {6, 4}, {6, 3}, {4, 3}, {6, 2}, {4, 2}, {3, 2}, {2, 2}, {2, 1}};
+    int best = 1 << 30;
+    for (const auto& t : tiles) {
+      const int blocks = ((X.NXc + t[0] - 1) / t[0]) * ((X.NYc + t[1] - 1) / t[1]), sms = device_sms();
+      const int warps = ((2 * t[0] + 3) * (2 * t[1] + 3) + 31) / 32, cost = (blocks + sms - 1) / sms * warps;
+      if (cost < best) {
+        best = cost;
+        P.cx = t[0];
+        P.cy = t[1];
+      }
+    }
+  }
   P.st = st;
   P.inner = inner;
   P.dinv = dinv;
@@ -1097,7 +1198,7 @@ void MG<T>::select_coarse_cheb(cudaStream_t s) {
     const LevelSpec& S = specs_[l];
     if (S.p2 || S.NC != 1 || !lv_[l].st || !kK64_[l] || !kM64_[l]) continue;
     const size_t smem = 2 * S.nn() * sizeof(T);  // the two direction buffers
-    if (S.nn() > size_t(kCoarseThreads) * coarse_cheb_npt<T>() || smem > kCoarseSharedBudget) continue;
+    if (S.nn() > coarse_cheb_nodes<T>() || smem > kCoarseSharedBudget) continue;
     const size_t nt = S.ntri();
     std::vector<double> kk(nt), km(nt);
     if (cudaMemcpyAsync(kk.data(), kK64_[l], nt * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -1172,7 +1273,7 @@ void MG<T>::build_tail() {
   };
   if (sizeof(T) == 8) return;
   for (int l = std::max(1, L - 1 - kTailMaxLevels); l + 1 < L && tail_ < 0; ++l) {
-    if (specs_[l].nn() > size_t(kTailNodes)) continue;
+    if (specs_[l].nn() > size_t(kTailNodes) || level_degree(l) != level_degree(L - 1)) continue;
     bool ok = true;
     for (int k = l; k < L; ++k) ok &= !specs_[k].p2 && lv_[k].st;
     if (ok && (specs_[l].NC == 2 ? plan(tail2_, l) : plan(tail1_, l))) tail_ = l;
@@ -1359,12 +1460,14 @@ int MG<T>::setup(cudaStream_t s) {
       lv_[l].lmax = estimate_lmax(l, s);
       lv_[l].bound = false;
     }
-    const double hi = (lv_[l].bound ? 1.0 : 1.1) * lv_[l].lmax, lo = cheb_lo_frac * lv_[l].lmax;
+    const int degree = level_degree(l);
+    const double hi = (lv_[l].bound ? 1.0 : 1.1) * lv_[l].lmax;
+    const double lo = (degree > 2 ? cheb_lo_deep : cheb_lo_frac) * lv_[l].lmax;
     const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), sigma = theta / delta;
     double* c = cc.data() + 8 * l;
     c[0] = 1.0 / theta;
     double rho_old = 1.0 / sigma;
-    for (int k = 1; k < cheb_degree && k < 4; ++k) {
+    for (int k = 1; k < degree; ++k) {
       const double rho_new = 1.0 / (2.0 * sigma - rho_old);
       c[2 * k - 1] = rho_new * rho_old;
       c[2 * k] = 2.0 * rho_new / delta;
@@ -1434,6 +1537,62 @@ void MG<T>::vcycle_level(int l, const T* b, T* x, cudaStream_t s) {
   vcycle_level_body(l, b, x, s);
 }
 
+// Both sweeps of stencil level l with D Chebyshev steps, the coarser levels between them.
+template <class T>
+template <int NC, int D>
+void MG<T>::sweep_level(int l, const T* b, T* x, cudaStream_t s) {
+  Lev& v = lv_[l];
+  Lev& c = lv_[l + 1];
+  const LevelSpec& S = specs_[l];
+  const Transfer X = make_transfer(S, specs_[l + 1]);
+  const double nf = double(S.nn()) * NC, ncrs = double(X.NXc) * X.NYc * NC;
+  // the stencil row of every node (7 NC x NC blocks, padded to 16 bytes; one row where the
+  // level shares it); down b, D^-1 read, x and the coarse residual written; up b, D^-1, x and
+  // the coarse correction read, x written
+  const double row = v.inner ? 0.0 : double((7 * NC * NC * sizeof(T) + 15) / 16 * 16) * double(S.nn());
+  const LevelSweep<T, NC> P = level_sweep<T, NC>(S, X, v.st, v.inner, v.dinv, cheb_ + 8 * l);
+  const dim3 g((X.NXc + P.cx - 1) / P.cx, (X.NYc + P.cy - 1) / P.cy, batch);
+  const int dw = down_w<D>(P), dh = down_h<D>(P), uw = up_w<D>(P), uh = up_h<D>(P);
+  {
+    KClock kc(s, "P1 level down", l, row + (3 * nf + ncrs) * sizeof(T));
+    launch_pdl(k_level_down<T, NC, D>, g, dim3(unsigned(dw * dh + 31) / 32 * 32), sweep_shared(dw, dh, NC) * sizeof(T), s,
+               P, b, v.x2, c.b);
+  }
+  vcycle_level(l + 1, c.b, c.x, s);
+  {
+    KClock kc(s, "P1 level up", l, row + (4 * nf + ncrs) * sizeof(T));
+    launch_pdl(k_level_up<T, NC, D>, g, dim3(unsigned(uw * uh + 31) / 32 * 32), sweep_shared(uw, uh, NC) * sizeof(T), s, P,
+               b, static_cast<const T*>(v.x2), static_cast<const T*>(c.x), x);
+  }
+  launches += 2;
+}
+
+template <class T>
+template <int NC>
+void MG<T>::sweep_level(int l, const T* b, T* x, cudaStream_t s) {
+  // (the degrees in use: see level_degree)
+  if constexpr (sizeof(T) == 4) {
+    constexpr int D = NC == 2 ? kCoarseDegree : kScalarDegree;
+    if (level_degree(l) == D) return sweep_level<NC, D>(l, b, x, s);
+  }
+  sweep_level<NC, 2>(l, b, x, s);
+}
+
+template <class T>
+template <int NC, int D>
+void MG<T>::launch_tail(const TailSweep<T, NC>& P, int nodes, const T* b, T* x, cudaStream_t s) {
+  launch_pdl(k_level_tail<T, NC, D>, batch, dim3(unsigned(nodes + 31) / 32 * 32), P.shared * sizeof(T), s, P, b, x);
+}
+
+template <class T>
+template <int NC>
+void MG<T>::launch_tail(const TailSweep<T, NC>& P, int l, const T* b, T* x, cudaStream_t s) {
+  const int nodes = int(specs_[l].nn());
+  constexpr int D = NC == 2 ? kCoarseDegree : kScalarDegree;
+  if (level_degree(l) == D) launch_tail<NC, D>(P, nodes, b, x, s);
+  else launch_tail<NC, 2>(P, nodes, b, x, s);
+}
+
 // One V-cycle from level l down: fused degree-2 Chebyshev pre-smoothing from
 // x = 0, residual restriction, coarse correction, fused post-smoothing.
 template <class T>
@@ -1443,22 +1602,21 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
   const LevelSpec& S = specs_[l];
   if (l == cheb_coarse_ && cc_desc_) {
     KClock kc(s, "coarse Chebyshev (one CTA)", l, 0.0);
-    launch_pdl(k_coarse_cheb<T>, batch, kCoarseThreads, cc_smem_, s, static_cast<const CoarseChebDesc<T, 1>*>(cc_desc_), b, x);
+    launch_pdl(k_coarse_cheb<T>, batch, sizeof(T) == 4 ? kCoarseThreads : 512, cc_smem_, s, static_cast<const CoarseChebDesc<T, 1>*>(cc_desc_), b, x);
     ++launches;
     return;
   }
   if constexpr (sizeof(T) == 4) {
     if (l == tail_ && use_tail) {
       KClock kc(s, "V-cycle tail (one CTA)", l, 0.0);
-      const dim3 nt(unsigned(S.nn() + 31) / 32 * 32);
-      if (S.NC == 2) launch_pdl(k_level_tail<T, 2>, batch, nt, tail2_.shared * sizeof(T), s, tail2_, b, x);
-      else launch_pdl(k_level_tail<T, 1>, batch, nt, tail1_.shared * sizeof(T), s, tail1_, b, x);
+      if (S.NC == 2) launch_tail<2>(tail2_, l, b, x, s);
+      else launch_tail<1>(tail1_, l, b, x, s);
       ++launches;
       return;
     }
   }
   if (l == L - 1) {
-    launch_pdl(k_dense_matvec<T>, batch, kCoarseMaxDofs, 0, s, static_cast<const T*>(cinv_), b, x, int(S.ndof()));
+    launch_pdl(k_dense_matvec<T>, batch, kDenseThreads, 0, s, static_cast<const T*>(cinv_), b, x, int(S.ndof()));
     ++launches;
     return;
   }
@@ -1500,28 +1658,6 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
   // algorithmic bytes of the transfers
   const double nf = double(S.nn()) * S.NC, ncrs = double(X.NXc) * X.NYc * S.NC;
   const double rbytes = (nf + ncrs) * sizeof(T), pbytes = (2 * nf + ncrs) * sizeof(T);
-  // per sweep: the stencil row of every node (7 NC x NC blocks, padded to 16 bytes; one row
-  // where the level shares it), down b, D^-1 read, x and the coarse residual written, up
-  // b, D^-1, x and the coarse correction read, x written
-  const double row = v.inner ? 0.0 : double((7 * S.NC * S.NC * sizeof(T) + 15) / 16 * 16) * double(S.nn());
-  auto run = [&](auto nc_tag) {
-    constexpr int NC = decltype(nc_tag)::value;
-    const LevelSweep<T, NC> P = level_sweep<T, NC>(S, X, v.st, v.inner, v.dinv, cheb_ + 8 * l);
-    const dim3 g((X.NXc + P.cx - 1) / P.cx, (X.NYc + P.cy - 1) / P.cy, batch);
-    auto threads = [](int nodes) { return dim3(unsigned(nodes + 31) / 32 * 32); };
-    {
-      KClock kc(s, "P1 level down", l, row + (3 * nf + ncrs) * sizeof(T));
-      launch_pdl(k_level_down<T, NC>, g, threads(P.down_w() * P.down_h()), P.down_shared() * sizeof(T), s, P, b, v.x2,
-                 c.b);
-    }
-    vcycle_level(l + 1, c.b, c.x, s);
-    {
-      KClock kc(s, "P1 level up", l, row + (4 * nf + ncrs) * sizeof(T));
-      launch_pdl(k_level_up<T, NC>, g, threads(P.up_w() * P.up_h()), P.up_shared() * sizeof(T), s, P, b,
-                 static_cast<const T*>(v.x2), static_cast<const T*>(c.x), x);
-    }
-    launches += 2;
-  };
   // large levels without a stencil: the column march (element products per cell)
   auto run_march = [&](auto nc_tag, const auto& P) {
     constexpr int NC = decltype(nc_tag)::value;
@@ -1549,10 +1685,10 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
   using I2 = std::integral_constant<int, 2>;
   using I1 = std::integral_constant<int, 1>;
   if (S.NC == 2) {
-    if (v.st) run(I2{});
+    if (v.st) sweep_level<2>(l, b, x, s);
     else run_march(I2{}, make_p1<T, 2>(S, refs_[l], v.kK, nullptr));
   } else {
-    if (v.st) run(I1{});
+    if (v.st) sweep_level<1>(l, b, x, s);
     else run_march(I1{}, make_p1<T, 1>(S, refs_[l], v.kK, v.kM));
   }
 }

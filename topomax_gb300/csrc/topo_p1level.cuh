@@ -1,15 +1,16 @@
 // The V-cycle's two sweeps of a P1 level with an assembled stencil, one launch each:
-//   down:  x = two Chebyshev steps from zero, r = b - A x, b_c = P^T r
-//   up:    x += P x_c, two Chebyshev steps
+//   down:  x = D Chebyshev steps from zero, r = b - A x, b_c = P^T r
+//   up:    x += P x_c, D Chebyshev steps
 // A block owns cx x cy coarse nodes and the 2cx x 2cy fine nodes over them and
-// recomputes the ring its own results need (three nodes wide down, two up), so
-// that the steps between the loads and the stores go through shared memory.
-// Such a level is bound by latency: six launches (two smoothing, a residual, a
-// restriction, a prolongation and a smoothing step more) of 4 to 6 us each, for
-// vectors that stay in L2.  A thread keeps its node's stencil row, inverse
-// diagonal and right-hand side in registers through both operator applications;
-// the rows and diagonals, which no solve changes, are loaded before the kernel
-// waits for its predecessor.
+// recomputes the ring its own results need (D + 1 nodes wide down, D up), so that the
+// steps between the loads and the stores go through shared memory.
+// Such a level is bound by latency: as separate launches (smoothing steps, residual,
+// restriction, prolongation) each takes 4 to 6 us for vectors that stay in L2, while
+// a further step inside a sweep is a barrier and seven products.  A thread keeps its
+// node's stencil row, inverse diagonal, residual and iterate in registers; only the
+// direction, which the neighbours read, goes through shared memory.  The rows and
+// diagonals, which no solve changes, are loaded before the kernel waits for its
+// predecessor.
 #pragma once
 
 #include "topo_p1.cuh"
@@ -25,15 +26,23 @@ struct LevelSweep {
   const T* dinv;
   const T* cheb;
   Dir dirf, dirc;
-
-  TOPO_HD int down_w() const { return 2 * cx + 3; }  // region of x
-  TOPO_HD int down_h() const { return 2 * cy + 3; }
-  TOPO_HD int up_w() const { return 2 * cx + 2; }  // region of d0
-  TOPO_HD int up_h() const { return 2 * cy + 2; }
-  // shared values: the region's vector and the next wider one's
-  TOPO_HD int down_shared() const { return NC * (down_w() * down_h() + (down_w() + 2) * (down_h() + 2)); }
-  TOPO_HD int up_shared() const { return NC * (up_w() * up_h() + (up_w() + 2) * (up_h() + 2)); }
 };
+
+// the threads' region, one node each: a block's nodes with a ring of D down (1 for the
+// residual the restriction reads, D - 1 for the steps before it), of D - 1 up
+template <int D, class L>
+TOPO_HD int down_w(const L& P) { return 2 * P.cx + 2 * D - 1; }
+template <int D, class L>
+TOPO_HD int down_h(const L& P) { return 2 * P.cy + 2 * D - 1; }
+template <int D, class L>
+TOPO_HD int up_w(const L& P) { return 2 * P.cx + 2 * D - 2; }
+template <int D, class L>
+TOPO_HD int up_h(const L& P) { return 2 * P.cy + 2 * D - 2; }
+
+// Two shared vectors over the region and a ring around it; the direction alternates
+// between them.  Positions outside the part that a step still needs hold stale or no
+// values; they are read (in bounds) and never reach a result.
+TOPO_HD int sweep_shared(int w, int h, int NC) { return 2 * NC * (w + 2) * (h + 2); }
 
 // 16-byte loads of N values (source and N * sizeof(T) multiples of 16 bytes)
 template <class T, int N>
@@ -125,10 +134,15 @@ TOPO_HD void level_apply(const T (&st)[StencilLayout<NC>::stride], const T* u, i
   }
 }
 
-// u + c1 u + c2 Dinv r : the second Chebyshev step's result from the first's (pre-smoothing),
-// and x2 + c1 d + c2 Dinv r (post-smoothing)
+// the next Chebyshev direction c1 d + c2 Dinv r
 template <class T>
-TOPO_HD T level_step(T x, T c1, T d, T c2, T di, T r) {
+TOPO_HD T level_direction(T c1, T d, T c2, T di, T r) {
+  return fma_t(c2 * di, r, c1 * d);
+}
+
+// the iterate after the last direction: x + c1 d + c2 Dinv r
+template <class T>
+TOPO_HD T level_last(T x, T c1, T d, T c2, T di, T r) {
   return fma_t(c2 * di, r, fma_t(c1, d, x));
 }
 
@@ -173,86 +187,47 @@ struct LevelNode {
   }
 };
 
-// Phases of the down sweep; a barrier between one and the next.  tid, nt: the thread and the
-// block's threads (at least down_w x down_h of them).
+// Phases of a sweep, a barrier between one and the next.  tid, nt: the thread and the block's
+// threads (at least as many as the region has nodes); w: the region's width.
 template <class T, int NC>
-struct LevelDown {
-  using L = LevelSweep<T, NC>;
-  using Node = LevelNode<T, NC>;
-  // the thread's node of the x region
-  TOPO_HD static bool start(const L& P, int I0, int J0, int tid, Node& N) {
-    if (tid >= P.down_w() * P.down_h()) return false;
-    N.load(P, 2 * I0 - 2 + tid % P.down_w(), 2 * J0 - 2 + tid / P.down_w());
-    return true;
-  }
-  // d0 = c0 Dinv b on the x region and a ring around it
-  TOPO_HD static void first(const L& P, int I0, int J0, int tid, int nt, const T* b, T* sd) {
-    const int w = P.down_w() + 2, n = w * (P.down_h() + 2);
-    const T c0 = P.cheb[0];
-    for (int i = tid; i < n; i += nt) {
-      const int a = 2 * I0 - 3 + i % w, r = 2 * J0 - 3 + i / w;
-      const bool in = a >= 0 && a < P.NX && r >= 0 && r < P.NY;
-      const size_t g = in ? size_t(r) * P.NX + a : 0;
-      for (int c = 0; c < NC; ++c) sd[NC * i + c] = in ? (c0 * P.dinv[NC * g + c]) * b[NC * g + c] : T(0);
-    }
-  }
-  // x = d0 + d1, d1 = c1 d0 + c2 Dinv (b - A d0)
-  TOPO_HD static void smooth(const L& P, int tid, const Node& N, const T* sd, T* sx, T* x) {
-    const int w = P.down_w(), i = tid % w, j = tid / w;
-    const T c1 = P.cheb[1], c2 = P.cheb[2];
-    const int p = (j + 1) * (w + 2) + i + 1;
-    T t[NC];
-    level_apply<T, NC>(N.st, sd, w + 2, p, t);
-    const bool own = N.in && i >= 2 && i < 2 + 2 * P.cx && j >= 2 && j < 2 + 2 * P.cy;
-    for (int c = 0; c < NC; ++c) {
-      const T u = sd[NC * p + c], r1 = N.bv[c] - t[c];
-      const T v = level_step(u, c1, u, c2, N.di[c], r1);
-      sx[NC * tid + c] = v;
-      if (own) x[NC * N.index(P) + c] = v;
-    }
-  }
-  // r = b - A x on the x region less its outer ring (zero outside the lattice); sr in the
-  // layout of the x region
-  TOPO_HD static void residual(const L& P, int tid, const Node& N, const T* sx, T* sr) {
-    const int w = P.down_w(), i = tid % w, j = tid / w;
-    if (i < 1 || i > w - 2 || j < 1 || j > P.down_h() - 2) return;
-    T t[NC];
-    level_apply<T, NC>(N.st, sx, w, tid, t);
-    for (int c = 0; c < NC; ++c) sr[NC * tid + c] = N.bv[c] - t[c];
-  }
-  TOPO_HD static void restrict_to(const L& P, int I0, int J0, int tid, int nt, const T* sr, T* bc) {
-    const int w = P.down_w();
-    for (int i = tid; i < P.cx * P.cy; i += nt) {
-      const int ic = i % P.cx, jc = i / P.cx, I = I0 + ic, J = J0 + jc;
-      if (I >= P.NXc || J >= P.NYc) continue;
-      const int p = (2 * jc + 2) * w + 2 * ic + 2;
-      const bool zero = is_clamped(P.dirc, I, J);
-      for (int c = 0; c < NC; ++c)
-        bc[NC * (size_t(J) * P.NXc + I) + c] = zero ? T(0) : level_restrict<T, NC>(sr + NC * p + c, w);
-    }
-  }
-};
-
-// Phases of the up sweep.
-template <class T, int NC>
-struct LevelUp {
+struct LevelPhases {
   using L = LevelSweep<T, NC>;
   struct Node : LevelNode<T, NC> {
-    T r0[NC], d0[NC], x2[NC];
+    int p;              // position in the shared vectors
+    T r[NC], x[NC], d[NC];
   };
-  TOPO_HD static bool start(const L& P, int I0, int J0, int tid, Node& N) {
-    if (tid >= P.up_w() * P.up_h()) return false;
-    N.load(P, 2 * I0 - 1 + tid % P.up_w(), 2 * J0 - 1 + tid / P.up_w());
+  // the thread's node of a region of w x h nodes from lattice position (a0, b0)
+  TOPO_HD static bool start(const L& P, int a0, int b0, int w, int h, int tid, Node& N) {
+    if (tid >= w * h) return false;
+    N.load(P, a0 + tid % w, b0 + tid / w);
+    N.p = (tid / w + 1) * (w + 2) + tid % w + 1;
     return true;
   }
-  // x + P x_c on the d0 region and a ring around it (zero outside the lattice)
-  TOPO_HD static void correct(const L& P, int I0, int J0, int tid, int nt, const T* x, const T* xc, T* sx) {
-    const int w = P.up_w() + 2, n = w * (P.up_h() + 2);
-    for (int i = tid; i < n; i += nt) {
-      const int a = 2 * I0 - 2 + i % w, b = 2 * J0 - 2 + i / w;
+  // down: d0 = c0 Dinv b on the region and a ring around it
+  TOPO_HD static void down_first(const L& P, int a0, int b0, int w, int h, int tid, int nt, const T* b, T* s) {
+    const T c0 = P.cheb[0];
+    for (int i = tid; i < (w + 2) * (h + 2); i += nt) {
+      const int a = a0 - 1 + i % (w + 2), c = b0 - 1 + i / (w + 2);
+      const bool in = a >= 0 && a < P.NX && c >= 0 && c < P.NY;
+      const size_t g = in ? size_t(c) * P.NX + a : 0;
+      for (int k = 0; k < NC; ++k) s[NC * i + k] = in ? (c0 * P.dinv[NC * g + k]) * b[NC * g + k] : T(0);
+    }
+  }
+  // r = b, x = d = d0 of the thread's node, after the barrier
+  TOPO_HD static void down_own(const T* s, Node& N) {
+    for (int c = 0; c < NC; ++c) {
+      N.r[c] = N.bv[c];
+      N.x[c] = N.d[c] = s[NC * N.p + c];
+    }
+  }
+  // up: x + P x_c on the region and a ring around it (zero outside the lattice)
+  TOPO_HD static void up_first(const L& P, int a0, int b0, int w, int h, int tid, int nt, const T* x, const T* xc,
+                               T* s) {
+    for (int i = tid; i < (w + 2) * (h + 2); i += nt) {
+      const int a = a0 - 1 + i % (w + 2), b = b0 - 1 + i / (w + 2);
       const bool in = a >= 0 && a < P.NX && b >= 0 && b < P.NY;
       if (!in) {
-        for (int c = 0; c < NC; ++c) sx[NC * i + c] = T(0);
+        for (int c = 0; c < NC; ++c) s[NC * i + c] = T(0);
         continue;
       }
       // the node's two coarse neighbours, or twice the coarse node it is
@@ -261,36 +236,65 @@ struct LevelUp {
       const size_t g = size_t(b) * P.NX + a;
       for (int c = 0; c < NC; ++c) {
         const T v = m0 == m1 ? xc[NC * m0 + c] : T(0.5) * (xc[NC * m0 + c] + xc[NC * m1 + c]);
-        sx[NC * i + c] = free ? x[NC * g + c] + v : x[NC * g + c];
+        s[NC * i + c] = free ? x[NC * g + c] + v : x[NC * g + c];
       }
     }
   }
-  // r0 = b - A x, d0 = c0 Dinv r0, x2 = x + d0
-  TOPO_HD static void first(const L& P, int tid, Node& N, const T* sx, T* sd) {
-    const int w = P.up_w(), p = (tid / w + 1) * (w + 2) + tid % w + 1;
-    const T c0 = P.cheb[0];
+  // up: r = b - A x, d0 = c0 Dinv r, x += d0
+  TOPO_HD static void up_residual(const L& P, int w, const T* sx, T* sd, Node& N) {
     T t[NC];
-    level_apply<T, NC>(N.st, sx, w + 2, p, t);
+    level_apply<T, NC>(N.st, sx, w + 2, N.p, t);
+    const T c0 = P.cheb[0];
     for (int c = 0; c < NC; ++c) {
-      N.r0[c] = N.bv[c] - t[c];
-      N.d0[c] = (c0 * N.di[c]) * N.r0[c];
-      N.x2[c] = sx[NC * p + c] + N.d0[c];
-      sd[NC * tid + c] = N.d0[c];
+      N.r[c] = N.bv[c] - t[c];
+      N.d[c] = (c0 * N.di[c]) * N.r[c];
+      N.x[c] = sx[NC * N.p + c] + N.d[c];
+      sd[NC * N.p + c] = N.d[c];
     }
   }
-  // whether the thread's node is one the block writes
-  TOPO_HD static bool owned(const L& P, int tid, const Node& N) {
-    const int w = P.up_w(), i = tid % w, j = tid / w;
-    return N.in && i >= 1 && i <= 2 * P.cx && j >= 1 && j <= 2 * P.cy;
-  }
-  // x = x2 + c1 d0 + c2 Dinv (r0 - A d0)
-  TOPO_HD static void second(const L& P, int tid, const Node& N, const T* sd, T* x) {
-    const T c1 = P.cheb[1], c2 = P.cheb[2];
+  // step k >= 1: r -= A d, d = c1 d + c2 Dinv r, x += d; the direction from s to sn
+  TOPO_HD static void step(const L& P, int k, int w, const T* s, T* sn, Node& N) {
     T t[NC];
-    level_apply<T, NC>(N.st, sd, P.up_w(), tid, t);
+    level_apply<T, NC>(N.st, s, w + 2, N.p, t);
+    const T c1 = P.cheb[2 * k - 1], c2 = P.cheb[2 * k];
     for (int c = 0; c < NC; ++c) {
-      const T r1 = N.r0[c] - t[c];
-      x[NC * N.index(P) + c] = level_step(N.x2[c], c1, N.d0[c], c2, N.di[c], r1);
+      N.r[c] -= t[c];
+      N.d[c] = level_direction(c1, N.d[c], c2, N.di[c], N.r[c]);
+      N.x[c] += N.d[c];
+      sn[NC * N.p + c] = N.d[c];
+    }
+  }
+  // the last step: x alone, to sn (the residual b - A x reads it)
+  TOPO_HD static void last(const L& P, int k, int w, const T* s, T* sn, Node& N) {
+    T t[NC];
+    level_apply<T, NC>(N.st, s, w + 2, N.p, t);
+    const T c1 = P.cheb[2 * k - 1], c2 = P.cheb[2 * k];
+    for (int c = 0; c < NC; ++c) {
+      N.x[c] = level_last(N.x[c], c1, N.d[c], c2, N.di[c], N.r[c] - t[c]);
+      if (sn) sn[NC * N.p + c] = N.x[c];
+    }
+  }
+  // down, at the end: r = b - A x (zero outside the lattice), to shared memory for the restriction
+  TOPO_HD static void down_residual(int w, const T* s, T* sr, const Node& N) {
+    T t[NC];
+    level_apply<T, NC>(N.st, s, w + 2, N.p, t);
+    for (int c = 0; c < NC; ++c) sr[NC * N.p + c] = N.bv[c] - t[c];
+  }
+  // stores the block's own nodes (ring: how far they lie inside the region)
+  TOPO_HD static void store(const L& P, int w, int ring, int tid, const Node& N, T* x) {
+    const int i = tid % w - ring, j = tid / w - ring;
+    if (!N.in || i < 0 || i >= 2 * P.cx || j < 0 || j >= 2 * P.cy) return;
+    for (int c = 0; c < NC; ++c) x[NC * N.index(P) + c] = N.x[c];
+  }
+  // ring: the position of the block's first coarse node inside the region
+  TOPO_HD static void restrict_to(const L& P, int I0, int J0, int w, int ring, int tid, int nt, const T* sr, T* bc) {
+    for (int i = tid; i < P.cx * P.cy; i += nt) {
+      const int ic = i % P.cx, jc = i / P.cx, I = I0 + ic, J = J0 + jc;
+      if (I >= P.NXc || J >= P.NYc) continue;
+      const int p = (2 * jc + ring + 1) * (w + 2) + 2 * ic + ring + 1;
+      const bool zero = is_clamped(P.dirc, I, J);
+      for (int c = 0; c < NC; ++c)
+        bc[NC * (size_t(J) * P.NXc + I) + c] = zero ? T(0) : level_restrict<T, NC>(sr + NC * p + c, w + 2);
     }
   }
 };
