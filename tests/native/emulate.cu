@@ -821,18 +821,27 @@ void emu_fluid_apply_nodes(int nx, int ny, double W, double H, double q, double 
     for (int i = 0; i < 6; ++i)
       for (int j = i; j < 6; ++j) mk[t * kFluidMass + fluid_mass_index(i, j)] += E.lap[t & 1][i][j];
   }
-  for (size_t i = 0; i < n2 + nv; ++i) {
-    const FluidNode F = fluid_output(i, nx, ny);
-    double v[2];
-    fluid_node_rows(E, mk.data(), nx, ny, F, x, x + 2 * n2, pm, v);
-    if (F.cls == 4) {
-      y[2 * n2 + size_t(F.j) * (nx + 1) + F.i] = v[0];
-    } else {
-      const size_t node = size_t(2 * F.j + (F.cls >> 1)) * (2 * nx + 1) + 2 * F.i + (F.cls & 1);
-      y[2 * node] = v[0];
-      y[2 * node + 1] = v[1];
-    }
-  }
+  FluidStencils S;
+  fluid_stencils(E, S);
+  (void)nv;
+  auto velocity = [&](auto tag, int w, int h) {
+    constexpr int C = decltype(tag)::value;
+    for (int j = 0; j < h; ++j)
+      for (int i = 0; i < w; ++i) {
+        double row[kFluidNodes], v[2];
+        fluid_build_row<C>(mk.data(), nx, ny, i, j, row);
+        fluid_velocity<C>(S, row, 1, nx, ny, i, j, x, x + 2 * n2, pm, v);
+        const size_t node = size_t(2 * j + (C >> 1)) * (2 * nx + 1) + 2 * i + (C & 1);
+        y[2 * node] = v[0];
+        y[2 * node + 1] = v[1];
+      }
+  };
+  velocity(std::integral_constant<int, 0>{}, nx + 1, ny + 1);
+  velocity(std::integral_constant<int, 1>{}, nx, ny + 1);
+  velocity(std::integral_constant<int, 2>{}, nx + 1, ny);
+  velocity(std::integral_constant<int, 3>{}, nx, ny);
+  for (int j = 0; j <= ny; ++j)
+    for (int i = 0; i <= nx; ++i) y[2 * n2 + size_t(j) * (nx + 1) + i] = fluid_continuity(S, nx, ny, i, j, x);
 }
 
 double emu_fluid_objective(int nx, int ny, double W, double H, double q, double mu, const double* rho,

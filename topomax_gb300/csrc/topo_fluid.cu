@@ -44,6 +44,11 @@ namespace {
 // Restart length: the long one unless its 2 m + 1 vectors pass kFluidBasisMax bytes.
 constexpr int kFluidRestart = 30, kFluidRestartMax = 60;
 constexpr size_t kFluidBasisMax = size_t(16) << 30;
+// A column is orthogonalised again where less than this share of |w|^2 is left: the loss of
+// orthogonality is then at most ten roundings, which 60 vectors at a relative residual of
+// 1e-12 do not see (the same iterations as with 0.5, which repeats two passes in three;
+// 13.9 ms against 19.6 at 128x128, 8.1 against 10.5 at 40x40 with the finer grids).
+constexpr double kReorthogonalise = 0.01;
 constexpr int kDotGroup = 8;  // basis vectors of one block of the Gram-Schmidt products
 constexpr int kDotGroups = (kFluidRestartMax + kDotGroup) / kDotGroup;
 constexpr double kLaplaceShift = 1e-3;  // mass shift of the pressure Laplacian (its constant mode)
@@ -77,43 +82,89 @@ struct FluidKrylov {
   double H[(kFluidRestartMax + 1) * kFluidRestartMax];
 };
 
-// y = A x, x = [u (2 n2, interleaved) | p (nv)], by output node: the element matrices' rows are
-// formed where they are needed, each once.  With K: x = z_j with its pressure's mean taken off
-// (and written back), y = v_(j+1).  clamp: boundary velocity rows are the identity.
-// Bound: FP64, 72 products per P2 node, and the latency of up to six triangles' loads.
-// (A thread per triangle into a 128-byte buffer and a gather took 16 + 4 us at 40x40 and
-// 16 + 6 at 128x128.)
-constexpr int kFluidThreads = 128;
+// Blocks of the operator's kernels by class (topo_fluid.cuh): class c has blocks [start[c], start[c + 1])
+constexpr int kFluidThreads = 64;
+struct FluidGrid {
+  unsigned start[6];
+  FluidGrid(int nx, int ny) {
+    const FluidRows R(nx, ny);
+    start[0] = 0;
+    for (int c = 0; c < 5; ++c)
+      start[c + 1] = start[c] + unsigned((R.count[c < 4 ? c : 0] + kFluidThreads - 1) / kFluidThreads);
+  }
+};
+
+// the thread's class and index among the class's nodes; false past the last one
+__device__ __forceinline__ bool fluid_thread(const FluidGrid& G, const FluidRows& R, int& cls, size_t& k) {
+  cls = 0;
+  while (cls < 4 && blockIdx.x >= G.start[cls + 1]) ++cls;
+  k = size_t(blockIdx.x - G.start[cls]) * kFluidThreads + threadIdx.x;
+  return k < R.count[cls < 4 ? cls : 0];
+}
+
+// the velocity rows of the design, from the triangles' matrices (once per solve)
+__global__ void __launch_bounds__(kFluidThreads)
+    k_fluid_rows(int nx, int ny, FluidGrid G, const double* __restrict__ mk, double* __restrict__ rows) {
+  const FluidRows R(nx, ny);
+  int cls;
+  size_t k;
+  if (!fluid_thread(G, R, cls, k)) return;
+  const int w = cls & 1 ? nx : nx + 1, i = int(k % w), j = int(k / w);
+  double row[kFluidNodes];
+  switch (cls) {
+    case 0: fluid_build_row<0>(mk, nx, ny, i, j, row); break;
+    case 1: fluid_build_row<1>(mk, nx, ny, i, j, row); break;
+    case 2: fluid_build_row<2>(mk, nx, ny, i, j, row); break;
+    default: fluid_build_row<3>(mk, nx, ny, i, j, row); break;
+  }
+  for (int e = 0; e < fluid_nodes(cls); ++e) rows[R.first[cls] + size_t(e) * R.count[cls] + k] = row[e];
+}
+
+// y = A x, x = [u (2 n2, interleaved) | p (nv)], by output node: assembled velocity rows, and
+// gradient and divergence coefficients by node type.  KRYLOV: x = z_j with its pressure's mean
+// taken off, y = v_(j+1).  clamp: boundary velocity rows are the identity.
+// Bound: FP64, 42 products per P2 node on average (the triangles' matrices applied where they are
+// needed take 72), all loads of a row in flight at once: 10.4 us at 128x128, 6.0 at 40x40; by
+// triangle rows 19.6 and 17.4, through a per-triangle buffer and a gather 22 and 20.
+template <int CLS>
+__device__ __forceinline__ void fluid_apply_class(int nx, int ny, const FluidStencils& S, const double* rows,
+                                                  const FluidRows& R, size_t k, const double* x, double pm, bool clamp,
+                                                  double* y) {
+  const int NX = 2 * nx + 1, NY = 2 * ny + 1, w = CLS & 1 ? nx : nx + 1;
+  const int i = int(k % w), j = int(k / w), a = 2 * i + (CLS & 1), b = 2 * j + (CLS >> 1);
+  const size_t node = size_t(b) * NX + a;
+  double v[2];
+  if (clamp && fluid_boundary_node(a, b, NX, NY)) {
+    v[0] = x[2 * node];
+    v[1] = x[2 * node + 1];
+  } else {
+    fluid_velocity<CLS>(S, rows + R.first[CLS] + k, R.count[CLS], nx, ny, i, j, x, x + 2 * size_t(NX) * NY, pm, v);
+  }
+  y[2 * node] = v[0];
+  y[2 * node + 1] = v[1];
+}
+
 template <bool KRYLOV>
 __global__ void __launch_bounds__(kFluidThreads)
-    k_fluid_apply(int nx, int ny, const FluidTables* __restrict__ E, const double* __restrict__ mk, const double* xin,
-                  double* yout, int clamp, const FluidKrylov* K, size_t n, double* zc) {
+    k_fluid_apply(int nx, int ny, FluidGrid G, const FluidStencils* __restrict__ S, const double* __restrict__ rows,
+                  const double* xin, double* yout, int clamp, const FluidKrylov* K, size_t n, double* zc) {
   TOPO_PDL_ENTRY();
-  const int NX = 2 * nx + 1, NY = 2 * ny + 1;
-  const size_t n2 = size_t(NX) * NY, nv = size_t(nx + 1) * (ny + 1);
+  const FluidRows R(nx, ny);
+  const size_t n2 = size_t(2 * nx + 1) * (2 * ny + 1), nv = R.count[0];
+  int cls;
+  size_t k;
+  if (!fluid_thread(G, R, cls, k)) return;
   const double* x = KRYLOV ? xin + size_t(K->j) * n : xin;
   double* y = KRYLOV ? yout + size_t(K->j + 1) * n : yout;
   const double pm = KRYLOV ? K->zsum / double(nv) : 0.0;
-  const size_t i = size_t(blockIdx.x) * kFluidThreads + threadIdx.x;
-  if (i >= n2 + nv) return;
-  const FluidNode F = fluid_output(i, nx, ny);
-  double v[2];
-  if (F.cls < 4) {
-    const int a = 2 * F.i + (F.cls & 1), b = 2 * F.j + (F.cls >> 1);
-    const size_t node = size_t(b) * NX + a;
-    if (clamp && fluid_boundary_node(a, b, NX, NY)) {
-      v[0] = x[2 * node];
-      v[1] = x[2 * node + 1];
-    } else {
-      fluid_node_rows(*E, mk, nx, ny, F, x, x + 2 * n2, pm, v);
-    }
-    y[2 * node] = v[0];
-    y[2 * node + 1] = v[1];
-  } else {
-    const size_t k = size_t(F.j) * (nx + 1) + F.i;
-    fluid_node_rows(*E, mk, nx, ny, F, x, x + 2 * n2, pm, v);
-    y[2 * n2 + k] = v[0];
-    if (KRYLOV) zc[k] = x[2 * n2 + k] - pm;  // the centred pressure, moved into z_j by k_fluid_dot
+  switch (cls) {
+    case 0: fluid_apply_class<0>(nx, ny, *S, rows, R, k, x, pm, clamp != 0, y); break;
+    case 1: fluid_apply_class<1>(nx, ny, *S, rows, R, k, x, pm, clamp != 0, y); break;
+    case 2: fluid_apply_class<2>(nx, ny, *S, rows, R, k, x, pm, clamp != 0, y); break;
+    case 3: fluid_apply_class<3>(nx, ny, *S, rows, R, k, x, pm, clamp != 0, y); break;
+    default:
+      y[2 * n2 + k] = fluid_continuity(*S, nx, ny, int(k % (nx + 1)), int(k / (nx + 1)), x);
+      if (KRYLOV) zc[k] = x[2 * n2 + k] - pm;  // the centred pressure, moved into z_j by k_fluid_dot
   }
 }
 
@@ -299,7 +350,8 @@ __global__ void __launch_bounds__(kVecThreads)
 }
 
 // w -= sum hp_i v_i.  The first pass (classical Gram-Schmidt) decides on the second: it is needed
-// where more than half of |w|^2 cancelled (Kahan's "twice is enough"); the second sums |w|^2.
+// where the products took nearly all of |w|^2 (kReorthogonalise; Kahan's "twice is enough"); the
+// second sums |w|^2.
 __global__ void __launch_bounds__(kVecThreads)
     k_fluid_sub(double* V, size_t n, int pass, double* partials, unsigned* counter, FluidKrylov* K) {
   TOPO_PDL_ENTRY();
@@ -330,7 +382,7 @@ __global__ void __launch_bounds__(kVecThreads)
         hh += h[i] * h[i];
       }
       const double ww = K->ww, est = ww - hh;
-      K->second = !(est >= 0.5 * ww);
+      K->second = !(est >= kReorthogonalise * ww);
       K->hn = sqrt(est);
     }
     return;
@@ -342,53 +394,78 @@ __global__ void __launch_bounds__(kVecThreads)
   }
 }
 
-// v_(j+1) = w / |w| and the sum of its pressure; then the last block rotates the column into
-// the triangular factor, updates the residual norm and decides whether the cycle goes on
+// v_(j+1) = w / |w| and the sum of its pressure, in all blocks but the first, whose first warp
+// rotates the column into the triangular factor, updates the residual norm and decides
+// whether the cycle goes on.  The rotations' recurrence up' = -s_i up + c_i h_(i+1) is affine in
+// up: a warp scan of two maps a lane (a thread's loop took ~10 us at 30 columns).
 __global__ void __launch_bounds__(kVecThreads)
     k_fluid_next(double* V, size_t n, size_t nv, int m, double* partials, unsigned* counter, FluidKrylov* K,
                  cudaGraphConditionalHandle cond, int use_cond) {
   TOPO_PDL_ENTRY();
-  __shared__ double hs[kFluidRestartMax + 1], cs[kFluidRestartMax], sn[kFluidRestartMax];
   const int j = K->j;
-  for (int i = threadIdx.x; i <= j; i += blockDim.x) {
-    hs[i] = K->h[i];
-    if (i < j) {
-      cs[i] = K->cs[i];
-      sn[i] = K->sn[i];
+  const double hn = K->hn, f = hn > 0 ? 1.0 / hn : 1.0;
+  double s[1] = {0.0};
+  if (blockIdx.x > 0) {
+    double* w = V + size_t(j + 1) * n;
+    for (size_t i = size_t(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x - 1) * blockDim.x) {
+      const double v = w[i] * f;
+      w[i] = v;
+      if (i >= n - nv) s[0] += v;
+    }
+  } else if (threadIdx.x < 32) {
+    const int e = 2 * int(threadIdx.x);
+    double c[2], t[2], h[2], a[2], b[2];
+    for (int q = 0; q < 2; ++q) {
+      const bool on = e + q < j;
+      c[q] = on ? K->cs[e + q] : 1.0;
+      t[q] = on ? K->sn[e + q] : 0.0;
+      h[q] = on ? K->h[e + q + 1] : 0.0;
+      a[q] = on ? -t[q] : 1.0;
+      b[q] = c[q] * h[q];
+    }
+    const double h0 = K->h[0];
+    double A = a[1] * a[0], B = a[1] * b[0] + b[1];
+    for (int o = 1; o < 32; o <<= 1) {
+      const double pa = __shfl_up_sync(0xffffffffu, A, o), pb = __shfl_up_sync(0xffffffffu, B, o);
+      if (int(threadIdx.x) >= o) {
+        B = A * pb + B;
+        A = A * pa;
+      }
+    }
+    double Ea = __shfl_up_sync(0xffffffffu, A, 1), Eb = __shfl_up_sync(0xffffffffu, B, 1);
+    if (threadIdx.x == 0) {
+      Ea = 1.0;
+      Eb = 0.0;
+    }
+    double up = Ea * h0 + Eb;
+    for (int q = 0; q < 2; ++q) {
+      if (e + q < j) K->H[(e + q) * kFluidRestartMax + j] = c[q] * up + t[q] * h[q];
+      up = a[q] * up + b[q];
+    }
+    up = __shfl_sync(0xffffffffu, up, 31);
+    if (threadIdx.x == 0) {
+      const double den = hypot(up, hn);
+      const double cj = den > 0 ? up / den : 1.0, tj = den > 0 ? hn / den : 0.0;
+      K->cs[j] = cj;
+      K->sn[j] = tj;
+      K->H[j * kFluidRestartMax + j] = den;
+      const double g = K->gv[j];
+      K->gv[j + 1] = -tj * g;
+      K->gv[j] = cj * g;
+      const int it = K->it + 1;
+      K->it = it;
+      int st = 1;
+      if (!isfinite(hn)) st = 4;
+      else if (fabs(tj * g) <= K->target || hn == 0.0 || j + 1 >= m || it >= K->maxit) st = 0;
+      K->status = st;
+      if (use_cond) cudaGraphSetConditional(cond, st == 1 ? 1u : 0u);
     }
   }
-  const double hn = K->hn, f = hn > 0 ? 1.0 / hn : 1.0;
-  double* w = V + size_t(j + 1) * n;
-  double s[1] = {0.0};
-  TOPO_GRID_STRIDE(i, n) {
-    const double v = w[i] * f;
-    w[i] = v;
-    if (i >= n - nv) s[0] += v;
-  }
   double tot[1];
-  if (!finish_reduction<1>(s, partials, counter, tot)) return;
-  K->psum = tot[0];
-  double up = hs[0];
-  for (int i = 0; i < j; ++i) {
-    const double lo = hs[i + 1], c = cs[i], t = sn[i];
-    K->H[i * kFluidRestartMax + j] = c * up + t * lo;
-    up = -t * up + c * lo;
+  if (finish_reduction<1>(s, partials, counter, tot)) {
+    K->psum = tot[0];
+    K->j = j + 1;  // every block has read it
   }
-  const double den = hypot(up, hn);
-  const double c = den > 0 ? up / den : 1.0, t = den > 0 ? hn / den : 0.0;
-  K->cs[j] = c;
-  K->sn[j] = t;
-  K->H[j * kFluidRestartMax + j] = den;
-  const double g = K->gv[j];
-  K->gv[j + 1] = -t * g;
-  K->gv[j] = c * g;
-  K->j = j + 1;
-  K->it += 1;
-  int st = 1;
-  if (!isfinite(hn)) st = 4;
-  else if (fabs(t * g) <= K->target || hn == 0.0 || j + 1 >= m || K->it >= K->maxit) st = 0;
-  K->status = st;
-  if (use_cond) cudaGraphSetConditional(cond, st == 1 ? 1u : 0u);
 }
 
 __global__ void k_fluid_start(FluidKrylov* K, double beta, double target, int it, int maxit) {
@@ -415,7 +492,7 @@ __global__ void __launch_bounds__(32) k_fluid_backsolve(FluidKrylov* K) {
       if (lane + 32 * q < i) g[q] -= K->H[(lane + 32 * q) * kFluidRestartMax + i] * yi;
   }
 }
-static_assert(kFluidRestartMax <= 64, "two values per lane");
+static_assert(kFluidRestartMax <= 64, "two values per lane, here and in k_fluid_next");
 
 // x += sum_i y_i z_i over the cycle's directions
 __global__ void k_fluid_update(double* x, const double* Z, size_t n, const FluidKrylov* K) {
@@ -460,6 +537,8 @@ struct topo_fluid_ctx {
   FluidTables* tab = nullptr;  // device copy
   double* ub = nullptr;        // boundary data (interleaved, zero inside)
   double* mass = nullptr;      // [tri][21], the Laplacian added
+  FluidStencils* sten = nullptr;  // device copy
+  double* rows = nullptr;      // velocity rows (FluidRows)
   double* tri3 = nullptr;      // [tri][3]
   double* ml = nullptr;        // lumped CG1 mass (vertex weights)
   double* ones = nullptr;      // nv ones (sums by a dot)
@@ -536,18 +615,28 @@ struct topo_fluid_ctx {
     k_fluid_center<<<grid(nv), kVecThreads, 0, s>>>(xp, yp, nv, red.out);
     launches += 2;
   }
-  // y = A x
+  // y = A x (the rows are the last design's)
   void apply(const double* xin, double* y, bool clamp, cudaStream_t s) {
-    const unsigned g = unsigned((n2 + nv + kFluidThreads - 1) / kFluidThreads);
-    k_fluid_apply<false><<<g, kFluidThreads, 0, s>>>(nx, ny, tab, mass, xin, y, clamp ? 1 : 0, nullptr, n, nullptr);
+    const FluidGrid G(nx, ny);
+    k_fluid_apply<false><<<G.start[5], kFluidThreads, 0, s>>>(nx, ny, G, sten, rows, xin, y, clamp ? 1 : 0, nullptr, n,
+                                                              nullptr);
     ++launches;
+  }
+  // the operator of design rho
+  void set_design(const double* rho, cudaStream_t s) {
+    const size_t nt = size_t(2) * nx * ny;
+    const FluidGrid G(nx, ny);
+    k_fluid_mass<<<grid(nt), kVecThreads, 0, s>>>(nx, ny, tab, pen, rho, mass);
+    k_fluid_rows<<<G.start[4], kFluidThreads, 0, s>>>(nx, ny, G, mass, rows);
+    launches += 2;
   }
   // one iteration of the cycle in kry, on s
   void iteration(cudaStream_t s, cudaGraphConditionalHandle cond, int use_cond) {
-    const unsigned gn = unsigned(grid(n2 + nv)), ga = unsigned((n2 + nv + kFluidThreads - 1) / kFluidThreads);
-    const unsigned gd = unsigned(red.blocks_for(n)), gv = unsigned(grid(n));
-    const double *Vc = V, *mlc = ml, *zcc = zc, *mkc = mass;
-    const FluidTables* tc = tab;
+    const FluidGrid G(nx, ny);
+    const unsigned gn = unsigned(grid(n2 + nv)), gv = unsigned(grid(n));
+    const unsigned gd = unsigned(red.spread(n)), gm = unsigned(red.spread(n2 + nv));
+    const double *Vc = V, *mlc = ml, *zcc = zc, *rc = rows;
+    const FluidStencils* sc = sten;
     const FluidKrylov* kc = kry;
     launch_pdl(k_fluid_split, gn, kVecThreads, 0, s, NX(), NY(), Vc, n, nv, kc, c, pt);
     cudaEventRecord(fork, s);
@@ -556,16 +645,16 @@ struct topo_fluid_ctx {
     cudaEventRecord(join, side);
     mgu.vcycle(c, z, s);
     cudaStreamWaitEvent(s, join, 0);
-    k_fluid_merge<<<red.blocks_for(n2 + nv), kVecThreads, 0, s>>>(NX(), NY(), Vc, Z, n, nv, z, pz, mlc, red.partials,
+    k_fluid_merge<<<gm, kVecThreads, 0, s>>>(NX(), NY(), Vc, Z, n, nv, z, pz, mlc, red.partials,
                                                                  red.counter, kry);
     const double* Zc = Z;
-    launch_pdl(k_fluid_apply<true>, ga, kFluidThreads, 0, s, nx, ny, tc, mkc, Zc, V, 1, kc, n, zc);
+    launch_pdl(k_fluid_apply<true>, G.start[5], kFluidThreads, 0, s, nx, ny, G, sc, rc, Zc, V, 1, kc, n, zc);
     for (int pass = 0; pass < 2; ++pass) {
       launch_pdl(k_fluid_dot, dim3(gd, unsigned((m + kDotGroup - 1) / kDotGroup)), kVecThreads, 0, s, Vc, Z, n, nv, zcc, pass,
                  dots, dot_counters, kry);
       launch_pdl(k_fluid_sub, gv, kVecThreads, 0, s, V, n, pass, red.partials, red.counter, kry);
     }
-    launch_pdl(k_fluid_next, gd, kVecThreads, 0, s, V, n, nv, m, red.partials, red.counter, kry, cond, use_cond);
+    launch_pdl(k_fluid_next, gd + 1, kVecThreads, 0, s, V, n, nv, m, red.partials, red.counter, kry, cond, use_cond);
     launches += 9;
   }
   int record();
@@ -647,10 +736,10 @@ namespace {
 
 int fluid_setup(topo_fluid_ctx* C, const double* rho, cudaStream_t s) {
   const size_t nt = size_t(2) * C->nx * C->ny;
-  k_fluid_mass<<<C->grid(nt), kVecThreads, 0, s>>>(C->nx, C->ny, C->tab, C->pen, rho, C->mass);
+  C->set_design(rho, s);
   k_fluid_refined_alpha<<<C->grid(C->uspec[0].ntri()), kVecThreads, 0, s>>>(C->nx, C->ny, C->pen, rho, C->uM[0]);
   k_fluid_inv_alpha<<<C->grid(nt), kVecThreads, 0, s>>>(C->nx, C->ny, C->pen, rho, C->pK[0]);
-  C->launches += 3;
+  C->launches += 2;
   for (size_t l = 1; l < C->uspec.size(); ++l) {
     const LevelSpec &F = C->uspec[l - 1], &Cc = C->uspec[l];
     k_fluid_coarsen<<<C->grid(Cc.ntri()), kVecThreads, 0, s>>>(C->uM[l - 1], F.nx, F.ny, C->uM[l], Cc.nx, Cc.ny);
@@ -759,6 +848,8 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
   C->tab = C->arena.alloc_n<FluidTables>(1);
   C->ub = C->arena.alloc_n<double>(2 * C->n2);
   C->mass = C->arena.alloc_n<double>(nt * kFluidMass);
+  C->sten = C->arena.alloc_n<FluidStencils>(1);
+  C->rows = C->arena.alloc_n<double>(FluidRows(C->nx, C->ny).size);
   C->tri3 = C->arena.alloc_n<double>(3 * nt);
   C->ml = C->arena.alloc_n<double>(C->nv);
   C->ones = C->arena.alloc_n<double>(C->nv);
@@ -769,7 +860,7 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
   C->Z = C->arena.alloc_n<double>(size_t(C->m) * C->n);
   C->t = C->arena.alloc_n<double>(C->n);
   C->kry = C->arena.alloc_n<FluidKrylov>(1);
-  C->dots = C->arena.alloc_n<double>(size_t(C->red.blocks) * (kDotGroup + 1) * kDotGroups);
+  C->dots = C->arena.alloc_n<double>(size_t(C->red.spread(C->n)) * (kDotGroup + 1) * kDotGroups);
   C->dot_counters = C->arena.alloc_n<unsigned>(kDotGroups);
   C->zc = C->arena.alloc_n<double>(C->nv);
   C->c = C->arena.alloc_n<float>(2 * C->n2);
@@ -786,7 +877,10 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
   C->gb = C->arena.alloc_n<double>(C->nv);
   if (C->arena.failed()) return C->fail(TOPO_ERR_CUDA, "out of device memory");
   const std::vector<double> w = vertex_weights(C->nx, C->ny, C->hx, C->hy);
-  if (cudaMemcpy(C->tab, &C->host_tab, sizeof(FluidTables), cudaMemcpyHostToDevice) != cudaSuccess ||
+  FluidStencils st{};
+  fluid_stencils(C->host_tab, st);
+  if (cudaMemcpy(C->sten, &st, sizeof(st), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(C->tab, &C->host_tab, sizeof(FluidTables), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(C->ub, ub.data(), ub.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(C->ml, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
     return C->cuda_check("fluid set-up copies");
@@ -836,9 +930,9 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
   C->mgp.set_coefficients(std::vector<const double*>(C->pK.begin(), C->pK.end()),
                           std::vector<const double*>(C->pM.begin(), C->pM.end()));
   if (C->arena.failed()) return C->fail(TOPO_ERR_CUDA, "out of device memory");
-  int st = 0;
-  C->proj = topo_create_filter(g, 0.0, TOPO_PREC_FP64, &st);
-  if (!C->proj) return C->fail(st ? st : TOPO_ERR_CUDA, "CG1 projection set-up failed");
+  int rc = 0;
+  C->proj = topo_create_filter(g, 0.0, TOPO_PREC_FP64, &rc);
+  if (!C->proj) return C->fail(rc ? rc : TOPO_ERR_CUDA, "CG1 projection set-up failed");
   return C->cuda_check("fluid set-up");
 }
 
@@ -908,9 +1002,7 @@ int topo_fluid_apply(topo_fluid_ctx* ctx, const double* rho, const double* x, do
     if (!ctx->penal_set) return ctx->fail(TOPO_ERR_STATE, "You must set penalization before calling penalizer");
     if (!rho || !x || !y || x == y) return ctx->fail(TOPO_ERR_ARG, "invalid apply arguments");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const size_t nt = size_t(2) * ctx->nx * ctx->ny;
-    k_fluid_mass<<<ctx->grid(nt), kVecThreads, 0, s>>>(ctx->nx, ctx->ny, ctx->tab, ctx->pen, rho, ctx->mass);
-    ++ctx->launches;
+    ctx->set_design(rho, s);
     ctx->apply(x, y, clamp != 0, s);
     return ctx->cuda_check("fluid apply");
   });

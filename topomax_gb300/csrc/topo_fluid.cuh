@@ -231,69 +231,159 @@ TOPO_HD double fluid_gather_vertex(const double* tri_out, int nx, int ny, int a,
 // ---------------------------------------------------------------------------
 // the operator by output node
 // ---------------------------------------------------------------------------
-// Output i of [0, n2 + nv): the P2 nodes by class -- vertices, midpoints of horizontal, of
-// vertical and of diagonal edges, so that the lanes of a warp have the same number of
-// incident triangles (six, or two) -- and then the pressure vertices.
-struct FluidNode {
-  int cls;   // 0 vertex, 1 horizontal, 2 vertical, 3 diagonal edge, 4 pressure vertex
-  int i, j;  // cell column and row of the vertex, or of the edge's lower left vertex
+// P2 nodes by class: 0 vertices, midpoints of 1 horizontal, 2 vertical and 3 diagonal edges, so
+// that the threads of a block do the same work; (i, j): column and row of the vertex, or of
+// the edge's lower left vertex.  (Class 4 in the kernels: the pressure vertices.)
+
+// Incident triangles of a class's nodes, a byte each: column offset + 1 | (row offset + 1) << 1 |
+// orientation << 2 | local index << 3 (six of a vertex, two of an edge)
+TOPO_HD constexpr unsigned long long fluid_incidence(int cls) {
+  return cls == 0 ? 0x07030a0d1410ull : cls == 1 ? 0x2b1dull : cls == 2 ? 0x2f1aull : 0x2723ull;
+}
+TOPO_HD constexpr int fluid_incidences(int cls) { return cls == 0 ? 6 : 2; }
+
+// Offsets (in lattice steps) of the P2 nodes a class's node couples to: 19 of a vertex, 9 of an
+// edge, and of the CG1 vertices (in cells, from (i, j)) its gradient row reads: 7 and 4.
+constexpr int kFluidNodes = 19, kFluidEdgeNodes = 9, kFluidVerts = 7, kFluidEdgeVerts = 4;
+TOPO_HD constexpr int fluid_nodes(int cls) { return cls == 0 ? kFluidNodes : kFluidEdgeNodes; }
+TOPO_HD constexpr int fluid_verts(int cls) { return cls == 0 ? kFluidVerts : kFluidEdgeVerts; }
+struct FluidOffset {
+  signed char a, b;
+};
+template <int CLS>
+TOPO_HD constexpr FluidOffset fluid_node_offset(int k) {
+  if (CLS == 0) {  // both cells on the diagonal, then the two corners the other triangles add
+    const FluidOffset t[kFluidNodes] = {{0, 0},   {1, 0},   {2, 0},   {0, 1},   {1, 1},  {2, 1},  {0, 2},
+                                        {1, 2},   {2, 2},   {-1, 0},  {-2, 0},  {0, -1}, {-1, -1}, {-2, -1},
+                                        {0, -2},  {-1, -2}, {-2, -2}, {1, -1},  {-1, 1}};
+    return t[k];
+  }
+  if (CLS == 1) {  // triangle above (0: from the left vertex) and below the edge
+    const FluidOffset t[kFluidEdgeNodes] = {{0, 0}, {-1, 0}, {1, 0}, {1, 1}, {0, 1}, {1, 2}, {-1, -1}, {-1, -2}, {0, -1}};
+    return t[k];
+  }
+  if (CLS == 2) {
+    const FluidOffset t[kFluidEdgeNodes] = {{0, 0}, {0, -1}, {0, 1}, {1, 1}, {1, 0}, {2, 1}, {-1, -1}, {-2, -1}, {-1, 0}};
+    return t[k];
+  }
+  const FluidOffset t[kFluidEdgeNodes] = {{0, 0}, {-1, -1}, {1, 1}, {1, -1}, {0, -1}, {1, 0}, {-1, 1}, {-1, 0}, {0, 1}};
+  return t[k];
+}
+template <int CLS>
+TOPO_HD constexpr FluidOffset fluid_vert_offset(int k) {
+  if (CLS == 0) {
+    const FluidOffset t[kFluidVerts] = {{0, 0}, {1, 0}, {0, 1}, {1, 1}, {-1, 0}, {0, -1}, {-1, -1}};
+    return t[k];
+  }
+  if (CLS == 1) {
+    const FluidOffset t[kFluidEdgeVerts] = {{0, 0}, {1, 0}, {1, 1}, {0, -1}};
+    return t[k];
+  }
+  if (CLS == 2) {
+    const FluidOffset t[kFluidEdgeVerts] = {{0, 0}, {0, 1}, {1, 1}, {-1, 0}};
+    return t[k];
+  }
+  const FluidOffset t[kFluidEdgeVerts] = {{0, 0}, {1, 0}, {0, 1}, {1, 1}};
+  return t[k];
+}
+
+// The velocity rows' matrix entries live in memory class by class, entry k of all the class's
+// nodes together: offset of the class's entries, and the number of all.
+struct FluidRows {
+  size_t count[4];   // nodes of a class
+  size_t first[4];   // its entries
+  size_t size;
+  TOPO_HD FluidRows(int nx, int ny) : count{size_t(nx + 1) * (ny + 1), size_t(nx) * (ny + 1), size_t(nx + 1) * ny, size_t(nx) * ny} {
+    size = 0;
+    for (int c = 0; c < 4; ++c) {
+      first[c] = size;
+      size += count[c] * fluid_nodes(c);
+    }
+  }
 };
 
-TOPO_HD FluidNode fluid_output(size_t i, int nx, int ny) {
-  const size_t n[4] = {size_t(nx + 1) * (ny + 1), size_t(nx) * (ny + 1), size_t(nx + 1) * ny, size_t(nx) * ny};
-  const int w[4] = {nx + 1, nx, nx + 1, nx};
-  int c = 0;
-  while (c < 4 && i >= n[c]) i -= n[c++];
-  const int width = c < 4 ? w[c] : nx + 1;
-  return FluidNode{c, int(i % width), int(i / width)};
+// The gradient's and the divergence's coefficients depend only on which sides the node lies on:
+// type 0, 1, 2 for the first, an inner, the last column (and row).  Built by fluid_stencils.
+struct FluidStencils {
+  double gv[9][kFluidVerts][2];      // vertex velocity rows, type = column type + 3 row type
+  double ge[3][3][kFluidEdgeVerts][2];  // edges: [class - 1][type across the edge]
+  double dv[9][kFluidNodes][2];      // pressure vertices, over the vertex node offsets
+};
+
+// Row of velocity node (class CLS, position (i, j)) from the triangles' matrices M + K.
+template <int CLS>
+TOPO_HD void fluid_build_row(const double* mk, int nx, int ny, int i, int j, double (&row)[kFluidNodes]) {
+  for (int k = 0; k < fluid_nodes(CLS); ++k) row[k] = 0.0;
+  // the node's own position inside its cell-based frame: (a, b) = (2 i + da, 2 j + db)
+  const int da = CLS & 1, db = CLS >> 1;
+  for (int e = 0; e < fluid_incidences(CLS); ++e) {
+    const unsigned f = unsigned(fluid_incidence(CLS) >> (8 * e)) & 255u;
+    const int ci = int(f & 1u) - 1, cj = int((f >> 1) & 1u) - 1, o = int((f >> 2) & 1u), r = int(f >> 3);
+    if (i + ci < 0 || i + ci >= nx || j + cj < 0 || j + cj >= ny) continue;
+    const double* m = mk + ((size_t(j + cj) * nx + i + ci) * 2 + o) * kFluidMass;
+    for (int q = 0; q < 6; ++q) {
+      const int oa = 2 * ci + p2_off_a(o, q) - da, ob = 2 * cj + p2_off_b(o, q) - db;
+      for (int k = 0; k < fluid_nodes(CLS); ++k) {
+        const FluidOffset t = fluid_node_offset<CLS>(k);
+        if (t.a == oa && t.b == ob) row[k] += r <= q ? m[fluid_mass_index(r, q)] : m[fluid_mass_index(q, r)];
+      }
+    }
+  }
 }
 
-// the element rows of one triangle: mk its matrix M + K (upper triangle), local row r
-TOPO_HD void fluid_row(const FluidTables& E, int o, int r, const double* mk, const double (&ue)[6][2],
-                       const double (&pe)[3], double (&y)[2]) {
-  for (int j = 0; j < 6; ++j) {
-    const double m = r <= j ? mk[fluid_mass_index(r, j)] : mk[fluid_mass_index(j, r)];
-    y[0] += m * ue[j][0];
-    y[1] += m * ue[j][1];
-  }
-  for (int k = 0; k < 3; ++k) {
-    y[0] += E.grad[o][r][0][k] * pe[k];
-    y[1] += E.grad[o][r][1][k] * pe[k];
-  }
-}
+TOPO_HD int fluid_side(int k, int n) { return k == 0 ? 0 : k == n ? 2 : 1; }
 
-// Rows of the operator at output F.  mk: [tri][kFluidMass] with the Laplacian added; u, p the
-// velocity and pressure, pm a constant taken off the pressure.  Fills y[2] (velocity) or y[0]
-// (pressure vertex).  Boundary velocity nodes are the caller's.
-TOPO_HD void fluid_node_rows(const FluidTables& E, const double* mk, int nx, int ny, const FluidNode& F,
-                             const double* u, const double* p, double pm, double (&y)[2]) {
-  // incident triangles of each class, a byte each: column offset + 1 | (row offset + 1) << 1 |
-  // orientation << 2 | local index << 3
-  const int c = F.cls == 4 ? 0 : F.cls, count = c == 0 ? 6 : 2;
-  const unsigned long long inc = c == 0 ? 0x07030a0d1410ull : c == 1 ? 0x2b1dull : c == 2 ? 0x2f1aull : 0x2723ull;
+// Velocity rows of node (i, j) of class CLS, entry k of its matrix row at row[k * stride]: y.
+// pm: a constant taken off the pressure.
+template <int CLS>
+TOPO_HD void fluid_velocity(const FluidStencils& S, const double* row, size_t stride, int nx, int ny, int i, int j,
+                            const double* u, const double* p, double pm, double (&y)[2]) {
+  const int NX = 2 * nx + 1, NY = 2 * ny + 1, a = 2 * i + (CLS & 1), b = 2 * j + (CLS >> 1);
   y[0] = y[1] = 0.0;
-  for (int e = 0; e < count; ++e) {
-    const unsigned f = unsigned(inc >> (8 * e)) & 255u;
-    const int ci = F.i + int(f & 1u) - 1, cj = F.j + int((f >> 1) & 1u) - 1, o = int((f >> 2) & 1u), r = int(f >> 3);
-    if (ci < 0 || ci >= nx || cj < 0 || cj >= ny) continue;
-    const size_t t = (size_t(cj) * nx + ci) * 2 + o;
-    double ue[6][2];
-    const int NX = 2 * nx + 1;
-    for (int k = 0; k < 6; ++k) {
-      const size_t nd = size_t(2 * cj + p2_off_b(o, k)) * NX + 2 * ci + p2_off_a(o, k);
-      ue[k][0] = u[2 * nd];
-      ue[k][1] = u[2 * nd + 1];
-    }
-    if (F.cls == 4) {
-      double s = 0.0;
-      for (int k = 0; k < 6; ++k) s += E.div[o][r][k][0] * ue[k][0] + E.div[o][r][k][1] * ue[k][1];
-      y[0] -= s;
-    } else {
-      double pe[3];
-      for (int k = 0; k < 3; ++k) pe[k] = p[size_t(cj + p1_off_b(o, k)) * (nx + 1) + ci + p1_off_a(o, k)] - pm;
-      fluid_row(E, o, r, mk + t * kFluidMass, ue, pe, y);
-    }
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int k = 0; k < fluid_nodes(CLS); ++k) {
+    const FluidOffset t = fluid_node_offset<CLS>(k);
+    const int aa = a + t.a, bb = b + t.b;
+    if (aa < 0 || aa >= NX || bb < 0 || bb >= NY) continue;
+    const size_t nd = size_t(bb) * NX + aa;
+    const double m = row[size_t(k) * stride];
+    y[0] += m * u[2 * nd];
+    y[1] += m * u[2 * nd + 1];
   }
+  const int type = CLS == 0 ? fluid_side(i, nx) + 3 * fluid_side(j, ny) : CLS == 1 ? fluid_side(j, ny)
+                   : CLS == 2 ? fluid_side(i, nx) : 1;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int k = 0; k < fluid_verts(CLS); ++k) {
+    const FluidOffset t = fluid_vert_offset<CLS>(k);
+    const int ii = i + t.a, jj = j + t.b;
+    if (ii < 0 || ii > nx || jj < 0 || jj > ny) continue;
+    const double q = p[size_t(jj) * (nx + 1) + ii] - pm;
+    const double* g = CLS == 0 ? S.gv[type][k] : S.ge[CLS == 0 ? 0 : CLS - 1][CLS == 0 ? 0 : type][CLS == 0 ? 0 : k];
+    y[0] += g[0] * q;
+    y[1] += g[1] * q;
+  }
+}
+
+// Continuity row of vertex (i, j)
+TOPO_HD double fluid_continuity(const FluidStencils& S, int nx, int ny, int i, int j, const double* u) {
+  const int NX = 2 * nx + 1, NY = 2 * ny + 1, type = fluid_side(i, nx) + 3 * fluid_side(j, ny);
+  double s0 = 0.0, s1 = 0.0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int k = 0; k < kFluidNodes; ++k) {
+    const FluidOffset t = fluid_node_offset<0>(k);
+    const int aa = 2 * i + t.a, bb = 2 * j + t.b;
+    if (aa < 0 || aa >= NX || bb < 0 || bb >= NY) continue;
+    const size_t nd = size_t(bb) * NX + aa;
+    s0 += S.dv[type][k][0] * u[2 * nd];
+    s1 += S.dv[type][k][1] * u[2 * nd + 1];
+  }
+  return -(s0 + s1);
 }
 
 }  // namespace topo

@@ -240,4 +240,45 @@ inline int fluid_boundary_values(int nx, int ny, double W, double H, const topo_
   return 0;
 }
 
+// The gradient's and divergence's coefficients per node type, summed over the triangles that a
+// node of the type has: the types of a 2 x 2 mesh (a first, an inner, a last column and row).
+inline void fluid_stencils(const FluidTables& E, FluidStencils& S) {
+  std::memset(&S, 0, sizeof(S));
+  const int nx = 2, ny = 2;
+  auto triangles = [&](int cls, int i, int j, auto&& f) {
+    for (int e = 0; e < fluid_incidences(cls); ++e) {
+      const unsigned v = unsigned(fluid_incidence(cls) >> (8 * e)) & 255u;
+      const int ci = int(v & 1u) - 1, cj = int((v >> 1) & 1u) - 1;
+      if (i + ci >= 0 && i + ci < nx && j + cj >= 0 && j + cj < ny) f(ci, cj, int((v >> 2) & 1u), int(v >> 3));
+    }
+  };
+  auto vert = [](int cls, int k) {
+    return cls == 0 ? fluid_vert_offset<0>(k) : cls == 1 ? fluid_vert_offset<1>(k) : cls == 2 ? fluid_vert_offset<2>(k)
+                                                                                               : fluid_vert_offset<3>(k);
+  };
+  auto gradient = [&](int cls, int i, int j, double (*g)[2]) {
+    triangles(cls, i, j, [&](int ci, int cj, int o, int r) {
+      for (int q = 0; q < 3; ++q)
+        for (int k = 0; k < fluid_verts(cls); ++k)
+          if (vert(cls, k).a == ci + p1_off_a(o, q) && vert(cls, k).b == cj + p1_off_b(o, q))
+            for (int c = 0; c < 2; ++c) g[k][c] += E.grad[o][r][c][q];
+    });
+  };
+  for (int j = 0; j < 3; ++j)
+    for (int i = 0; i < 3; ++i) {
+      gradient(0, i, j, S.gv[i + 3 * j]);
+      triangles(0, i, j, [&](int ci, int cj, int o, int r) {
+        for (int q = 0; q < 6; ++q)
+          for (int k = 0; k < kFluidNodes; ++k)
+            if (fluid_node_offset<0>(k).a == 2 * ci + p2_off_a(o, q) && fluid_node_offset<0>(k).b == 2 * cj + p2_off_b(o, q))
+              for (int c = 0; c < 2; ++c) S.dv[i + 3 * j][k][c] += E.div[o][r][q][c];
+      });
+    }
+  for (int t = 0; t < 3; ++t) {
+    gradient(1, 0, t, S.ge[0][t]);
+    gradient(2, t, 0, S.ge[1][t]);
+    gradient(3, 0, 0, S.ge[2][t]);
+  }
+}
+
 }  // namespace topo

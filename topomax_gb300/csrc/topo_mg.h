@@ -101,6 +101,13 @@ struct Reducer {
     const size_t b = (n + 1023) / 1024;
     return b < 1 ? 1 : b < size_t(blocks) ? int(b) : blocks;
   }
+  // the same for a latency-bound chain: one value a thread while that leaves at most two blocks
+  // per SM
+  int spread(size_t n) const {
+    const size_t one = (n + 255) / 256, two = size_t(2) * sms;
+    const int b = blocks_for(n);
+    return one < 1 ? 1 : size_t(b) >= two ? b : int(one < two ? one : two);
+  }
 };
 
 // Device-resident scalars of one preconditioned-CG solve (read back once at the end).
