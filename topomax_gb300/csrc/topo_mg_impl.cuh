@@ -1775,11 +1775,12 @@ void MG<T>::tune_marches(cudaStream_t s) {
       choose(march_family(true, sizeof(T), 2), S.nx, S.ny, p2_march_bps<T, kP2Apply>(), max_blocks,
              [&](int seg) { launch_p2_mode<T, kP2Apply>(p2_op_, xi_, io, s, seg); });
     } else if (!v.st && l + 1 < L) {
-      cudaMemsetAsync(v.x, 0, S.ndof() * sizeof(T), s);
+      T* x = l > 0 ? v.x : pcg_[8];  // level 0 works on its caller's vector and owns none
+      cudaMemsetAsync(x, 0, S.ndof() * sizeof(T), s);
       P1Io<T> io;
       std::memset(&io, 0, sizeof(io));
       io.mode = kP2Apply;
-      io.u = v.x;
+      io.u = x;
       io.y = v.t;
       if (S.NC == 2) {
         const auto P = make_p1<T, 2>(S, refs_[l], v.kK, nullptr);
