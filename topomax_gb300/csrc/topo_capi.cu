@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "topomax_gb300.h"
+#include "topo_krylov.cuh"
 #include "topo_mg_impl.cuh"
 #include "topo_setup.h"
 #include "topo_sens.cuh"
@@ -42,12 +43,59 @@ struct Fgmres {
   double* V = nullptr;         // (m+1) x n Krylov basis (FP64)
   double* Z = nullptr;         // m x n preconditioned directions (inner solutions, accumulated in FP64)
   double* t = nullptr;         // n
-  void init(Arena& a, size_t n) {
+  // a restart cycle as one graph (fgmres_device): its scalars, scratch, and what it was recorded for
+  KrylovDev* K = nullptr;
+  double* dots = nullptr;
+  unsigned* counters = nullptr;
+  KrylovDev* host = nullptr;  // pinned: the scalars up to KrylovDev::res
+  cudaGraphExec_t graph = nullptr;
+  long long epoch = -1;
+  std::vector<unsigned char> op;                // the FP64 operator's parameters
+  long long outer_nodes = 0, inner_nodes = 0;  // launches of an outer and of an inner iteration
+  void init(Arena& a, size_t n, const Reducer& red) {
     V = a.alloc_n<double>((m + 1) * n);
     Z = a.alloc_n<double>(m * n);
     t = a.alloc_n<double>(n);
+    K = a.alloc_n<KrylovDev>(1);
+    dots = a.alloc_n<double>(krylov_dots(red.spread(n)));
+    counters = a.alloc_n<unsigned>(kDotGroups);
+    cudaMallocHost(&host, sizeof(KrylovDev));
+  }
+  ~Fgmres() {
+    if (graph) cudaGraphExecDestroy(graph);
+    if (host) cudaFreeHost(host);
   }
 };
+
+// r = f b, the first basis vector (in place, or from the right-hand side of a cold start)
+__global__ void k_scaled_copy(double* r, const double* b, double f, size_t n) {
+  TOPO_GRID_STRIDE(i, n) r[i] = b[i] * f;
+}
+
+// Right-hand side of the inner solve for column j: v_j in FP32, and its tolerance (squared) and
+// iteration cap.  The inner solve aims at what is left of the target, but need not go much
+// below what one refinement step can use (see fgmres_ir).
+__global__ void k_refine_rhs(const double* V, size_t n, const KrylovDev* K, float* b, PcgDev* dv) {
+  TOPO_PDL_ENTRY();
+  const double* v = V + size_t(K->j) * n;
+  TOPO_GRID_STRIDE(i, n) b[i] = float(v[i]);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const double tol = fmin(0.1, fmax(K->inner_floor, K->inner_tol / K->res));
+    dv->tol2 = tol * tol;
+    dv->maxit = K->inner_maxit;
+  }
+}
+
+// z_j = the inner solution; its iterations and status
+__global__ void k_refine_direction(const double* x64, double* Z, size_t n, KrylovDev* K, const PcgDev* dv) {
+  TOPO_PDL_ENTRY();
+  double* z = Z + size_t(K->j) * n;
+  TOPO_GRID_STRIDE(i, n) z[i] = x64[i];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    K->inner += dv->it;
+    if (dv->status == 3 || dv->status == 4) K->bad = dv->status;
+  }
+}
 
 __device__ __forceinline__ double expit_d(double x) { return 1.0 / (1.0 + exp(-x)); }
 
@@ -447,7 +495,7 @@ int init_filter(topo_ctx* C, double eps) {
     C->fmg32.init(C->fspec, C->frefs.data(), 0.0, 0.0, C->arena, &C->red);
     C->fmg32.set_coefficients(kK, kM);
     C->fd32 = C->arena.alloc_n<float>(C->nv);
-    C->fgm.init(C->arena, C->nv);
+    C->fgm.init(C->arena, C->nv, C->red);
     if (C->arena.failed()) return C->fail(TOPO_ERR_CUDA, "out of device memory");
     st = C->fmg32.setup(s);
   } else {
@@ -647,6 +695,148 @@ int fgmres_ir(topo_ctx* C, MG<float>& mg, Apply64 apply64, const double* b, doub
                  rtol, st.relres, st.iterations);
 }
 
+// Records one restart cycle of the refinement into W.graph: a WHILE node whose body is an outer
+// iteration -- inner FP32 solve (a WHILE node of its own), FP64 operator, Gram-Schmidt and
+// test.  apply64 must read and write fixed device addresses only.
+template <class Apply64>
+bool record_refinement(topo_ctx* C, MG<float>& mg, Apply64 apply64, size_t n, Fgmres& W) {
+  std::lock_guard<std::recursive_mutex> lock(device_lock());
+  cudaGetLastError();
+  const long long l0 = mg.launches;
+  cudaStream_t s = mg.recording_stream(0), sb = mg.recording_stream(1);
+  cudaGraph_t g = nullptr;
+  if (cudaGraphCreate(&g, 0) != cudaSuccess) return false;
+  cudaGraphConditionalHandle h = 0;
+  cudaGraphNode_t node = nullptr;
+  cudaGraphNodeParams cp = {};
+  bool ok = cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) == cudaSuccess;
+  if (ok) {
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = h;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    ok = cudaGraphAddNode(&node, g, nullptr, nullptr, 0, &cp) == cudaSuccess && cp.conditional.phGraph_out != nullptr;
+  }
+  cudaGraph_t body = ok ? cp.conditional.phGraph_out[0] : nullptr;
+  if (ok) ok = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) == cudaSuccess;
+  if (ok) {
+    const int gv = C->grid(n), gd = C->red.spread(n);
+    k_refine_rhs<<<gv, kVecThreads, 0, s>>>(W.V, n, W.K, mg.scratch0(5), mg.device_scalars());
+    long long l1 = 0, l2 = 0;
+    const bool rec = mg.record_solve(false, s, sb, l1, l2);
+    W.outer_nodes = l1 - l0 + 9;
+    W.inner_nodes = l2 - l1;
+    k_refine_direction<<<gv, kVecThreads, 0, s>>>(mg.solution64(), W.Z, n, W.K, mg.device_scalars());
+    apply64(mg.solution64(), W.t, s);
+    krylov_column(KrylovSpace{W.V, W.t, W.Z, nullptr, n, 0, Fgmres::m, W.dots, W.counters, C->red.partials,
+                              C->red.counter, W.K},
+                  gd, gv, h, 1, s);
+    ok = cudaStreamEndCapture(s, &body) == cudaSuccess && rec;
+  }
+  if (ok) ok = cudaGraphInstantiate(&W.graph, g, 0) == cudaSuccess;
+  cudaGraphDestroy(g);
+  ok = cudaGetLastError() == cudaSuccess && ok;
+  mg.launches = l0;  // recording is not execution
+  if (!ok && W.graph) {
+    cudaGraphExecDestroy(W.graph);
+    W.graph = nullptr;
+  }
+  return ok;
+}
+
+// fgmres_ir with the outer iterations on the device as well: two host round trips a restart cycle
+// instead of five an outer iteration (12 to 14 us each).  Loop from the host against this: state
+// solve 80x40 5.34 to 4.61 ms per evaluation, 303x101 13.28 to 12.57, 1000x500 16.09 to 15.65,
+// 2000x1000 38.4 to 38.0; filter 1000x500 1.37 to 1.28.  Returns 1, with x the guess or an
+// improved iterate, where fgmres_ir has to take over: no graphs, a recording that failed, or an
+// operator that is indefinite in FP32 (its inner solves are MINRES, driven by the host).
+template <class Apply64>
+int fgmres_device(topo_ctx* C, MG<float>& mg, Apply64 apply64, const void* op, size_t op_bytes, const double* b,
+                  double* x, bool warm, size_t n, double rtol, Fgmres& W, int maxit, double inner_floor,
+                  SolveStats& st, cudaStream_t s) {
+  st = SolveStats{};
+  if (!mg.use_graphs || !W.host || C->iter_limit > 0 || C->trace_solves || C->verify_residual) return 1;
+  const int g = C->grid(n);
+  const unsigned char* key = static_cast<const unsigned char*>(op);
+  if (W.graph && (W.epoch != mg.epoch() || W.op.size() != op_bytes || !std::equal(key, key + op_bytes, W.op.begin()))) {
+    cudaGraphExecDestroy(W.graph);
+    W.graph = nullptr;
+  }
+  if (!W.graph) {
+    // the recording streams must not see work still queued on s
+    if (cudaStreamSynchronize(s) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "refinement: CUDA error");
+    if (!record_refinement(C, mg, apply64, n, W)) {
+      cudaGetLastError();
+      ++mg.capture_failures;
+      return 1;
+    }
+    W.epoch = mg.epoch();
+    W.op.assign(key, key + op_bytes);
+  }
+  if (!warm) k_fill<double><<<g, kVecThreads, 0, s>>>(x, 0.0, n);
+  const double bn = std::sqrt(C->dot64(b, b, n, s));
+  if (!std::isfinite(bn)) return C->fail(TOPO_ERR_NAN, "non-finite right-hand side");
+  if (bn == 0.0) {
+    k_fill<double><<<g, kVecThreads, 0, s>>>(x, 0.0, n);
+    return TOPO_OK;
+  }
+  double prev = 0.0;
+  for (int cycle = 0; cycle < kMaxOuter; ++cycle) {
+    C->launches += 4;
+    double beta = bn;
+    const bool zero = cycle == 0 && !warm;  // x = 0: the residual is b
+    if (!zero) {
+      apply64(x, W.t, s);
+      k_sub<double><<<g, kVecThreads, 0, s>>>(W.V, b, W.t, n);
+      beta = std::sqrt(C->dot64(W.V, W.V, n, s));
+    }
+    st.relres = beta / bn;
+    if (!std::isfinite(beta)) return C->fail(TOPO_ERR_NAN, "non-finite residual");
+    if (beta <= rtol * bn) return TOPO_OK;
+    if (cycle > 0 && beta > 0.9 * prev) break;  // stagnation at the FP64 residual floor
+    prev = beta;
+    k_scaled_copy<<<g, kVecThreads, 0, s>>>(W.V, zero ? b : W.V, 1.0 / beta, n);
+    k_krylov_start<<<1, 1, 0, s>>>(W.K, beta, 0.5 * rtol * bn, 0, kMaxOuter * Fgmres::m, 0.3 * rtol * bn, inner_floor,
+                                   maxit);
+    if (cudaGraphLaunch(W.graph, s) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "refinement: graph launch failed");
+    cudaMemcpyAsync(W.host, W.K, offsetof(KrylovDev, res) + sizeof(double), cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "refinement: CUDA error");
+    const KrylovDev& K = *W.host;
+    st.iterations += K.inner;
+    st.outer += K.j;
+    mg.launches += K.j * W.outer_nodes + K.inner * W.inner_nodes;
+    if (K.status == 4) return C->fail(TOPO_ERR_NAN, "non-finite value in the FP32 inner solve or its Krylov vector");
+    k_krylov_backsolve<<<1, 32, 0, s>>>(W.K);
+    k_krylov_update<<<g, kVecThreads, 0, s>>>(x, W.Z, n, W.K);
+    if (K.status == 3) return 1;
+    if (K.res <= 0.5 * rtol * bn) {  // (see fgmres_ir)
+      st.relres = K.res / bn;
+      return TOPO_OK;
+    }
+  }
+  apply64(x, W.t, s);
+  k_sub<double><<<g, kVecThreads, 0, s>>>(W.V, b, W.t, n);
+  st.relres = std::sqrt(C->dot64(W.V, W.V, n, s)) / bn;
+  if (st.relres <= rtol) return TOPO_OK;
+  return C->fail(TOPO_ERR_NOT_CONVERGED, "refinement did not reach rtol %.3g (relres %.3g after %d inner iterations)",
+                 rtol, st.relres, st.iterations);
+}
+
+// The refinement: on the device where that can be, else from the host.  op: the bytes that
+// determine apply64's launches, besides mg's own parameters.
+template <class Apply64>
+int refine(topo_ctx* C, MG<float>& mg, Apply64 apply64, const void* op, size_t op_bytes, const double* b, double* x,
+           bool warm, size_t n, double rtol, Fgmres& W, int maxit, double inner_floor, SolveStats& st, cudaStream_t s) {
+  const int rc = fgmres_device(C, mg, apply64, op, op_bytes, b, x, warm, n, rtol, W, maxit, inner_floor, st, s);
+  if (rc != 1) return rc;
+  SolveStats more;
+  const int again = fgmres_ir(C, mg, apply64, b, x, warm || st.outer > 0, n, rtol, W, maxit, inner_floor, more, s);
+  more.iterations += st.iterations;
+  more.outer += st.outer;
+  st = more;
+  return again;
+}
+
 // channel: 0 design filter, 1 sensitivity filter (warm-started from the channel's last
 // solution when topo_set_filter_warm_start is on), -1 no warm start
 int filter_solve_impl(topo_ctx* C, const double* b, double* xi, double rtol, int* iters, cudaStream_t s,
@@ -675,8 +865,8 @@ int filter_solve_impl(topo_ctx* C, const double* b, double* xi, double rtol, int
   if (channel >= 0) C->fwarm_hist[channel] = 0;  // until this solve succeeds
   if (C->filter_mixed) {
     auto ap = [C](const double* x, double* y, cudaStream_t ss) { filter_apply64(C, x, y, true, ss); };
-    rc = fgmres_ir(C, C->fmg32, ap, b, xi, warm, C->nv, rtol, C->fgm, C->max_iterations(kFilterMaxIt),
-                   C->inner_floor_filter, st, s);
+    rc = refine(C, C->fmg32, ap, nullptr, 0, b, xi, warm, C->nv, rtol, C->fgm, C->max_iterations(kFilterMaxIt),
+                C->inner_floor_filter, st, s);
   } else {
     rc = C->fmg64.pcg(b, xi, warm, rtol, C->max_iterations(kFilterMaxIt), st, s);
     if (rc == -4) rc = C->fail(TOPO_ERR_NAN, "non-finite value in the filter solve");
@@ -847,7 +1037,7 @@ topo_ctx* topo_create(const topo_grid_desc* grid, const topo_material* mat, cons
         C->smg32.set_coefficients(kK, kM);
         C->xi32 = C->arena.alloc_n<float>(C->nv);
         C->d32 = C->arena.alloc_n<float>(n);
-        C->sgm.init(C->arena, n);
+        C->sgm.init(C->arena, n, C->red);
         C->sens_tri = C->arena.alloc_n<float>(size_t(3) * C->sspec[0].ntri());
       } else {
         C->smg64.use_graphs = graphs_enabled();
@@ -996,8 +1186,8 @@ int topo_state_solve(topo_ctx* ctx, const double* xi, double* u, double rtol, in
       if (ctx->op_dd) {
         const P2Params<dd> Pdd = ctx->p2params<dd>(0, reinterpret_cast<const dd*>(ctx->rm_op64));
         auto ap = [Pdd](const double* x, double* y, cudaStream_t ss) { p2_apply_dd(Pdd, x, y, ss); };
-        rc = fgmres_ir(ctx, ctx->smg32, ap, ctx->load, u, warm, n, rtol, ctx->sgm,
-                       ctx->max_iterations(kStateMaxIt), ctx->inner_floor_state, st, s);
+        rc = refine(ctx, ctx->smg32, ap, &Pdd, sizeof(Pdd), ctx->load, u, warm, n, rtol, ctx->sgm,
+                    ctx->max_iterations(kStateMaxIt), ctx->inner_floor_state, st, s);
       } else {
         const P2Params<double> P64 = ctx->p2params<double>(0, ctx->rm_op64);
         auto ap = [P64, xi](const double* x, double* y, cudaStream_t ss) { p2_apply_f64(P64, xi, x, y, ss); };

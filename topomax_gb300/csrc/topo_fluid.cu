@@ -29,6 +29,7 @@
 #include "topo_fluid.cuh"
 #include "topo_mg_impl.cuh"
 #include "topo_fluid_setup.h"
+#include "topo_krylov.cuh"
 #include "topo_sens.cuh"
 #include "topo_setup.h"
 
@@ -41,16 +42,9 @@ using namespace topo;
 
 namespace {
 
-// Restart length: the long one unless its 2 m + 1 vectors pass kFluidBasisMax bytes.
-constexpr int kFluidRestart = 30, kFluidRestartMax = 60;
+// Restart length: kKrylovMax unless its 2 m + 1 vectors pass kFluidBasisMax bytes.
+constexpr int kFluidRestart = 30;
 constexpr size_t kFluidBasisMax = size_t(16) << 30;
-// A column is orthogonalised again where less than this share of |w|^2 is left: the loss of
-// orthogonality is then at most ten roundings, which 60 vectors at a relative residual of
-// 1e-12 do not see (the same iterations as with 0.5, which repeats two passes in three;
-// 13.9 ms against 19.6 at 128x128, 8.1 against 10.5 at 40x40 with the finer grids).
-constexpr double kReorthogonalise = 0.01;
-constexpr int kDotGroup = 8;  // basis vectors of one block of the Gram-Schmidt products
-constexpr int kDotGroups = (kFluidRestartMax + kDotGroup) / kDotGroup;
 constexpr double kLaplaceShift = 1e-3;  // mass shift of the pressure Laplacian (its constant mode)
 
 // ---------------------------------------------------------------------------
@@ -68,19 +62,6 @@ __global__ void k_fluid_mass(int nx, int ny, const FluidTables* __restrict__ E, 
       for (int j = i; j < 6; ++j) m[fluid_mass_index(i, j)] += E->lap[t & 1][i][j];
   }
 }
-
-// Device-side state of one restart cycle.  v_0 .. v_j are the basis so far, column j of the
-// Hessenberg matrix is being formed.
-struct FluidKrylov {
-  int j, it, maxit, status;  // status: 1 running, 0 done, 4 non-finite
-  int second, pad;           // the column needs a second Gram-Schmidt pass
-  double target;             // residual norm to reach
-  double psum, zsum;         // sums of the pressure parts of v_j and of z_j
-  double ww, hn;             // |w|^2 before and |w| after the orthogonalisation
-  double h[kFluidRestartMax + 1], hp[kFluidRestartMax + 1];  // the column, and a pass's products
-  double cs[kFluidRestartMax], sn[kFluidRestartMax], gv[kFluidRestartMax + 1], y[kFluidRestartMax];
-  double H[(kFluidRestartMax + 1) * kFluidRestartMax];
-};
 
 // Blocks of the operator's kernels by class (topo_fluid.cuh): class c has blocks [start[c], start[c + 1])
 constexpr int kFluidThreads = 64;
@@ -147,7 +128,7 @@ __device__ __forceinline__ void fluid_apply_class(int nx, int ny, const FluidSte
 template <bool KRYLOV>
 __global__ void __launch_bounds__(kFluidThreads)
     k_fluid_apply(int nx, int ny, FluidGrid G, const FluidStencils* __restrict__ S, const double* __restrict__ rows,
-                  const double* xin, double* yout, int clamp, const FluidKrylov* K, size_t n, double* zc) {
+                  const double* xin, double* yout, int clamp, const KrylovDev* K, size_t n, double* zc) {
   TOPO_PDL_ENTRY();
   const FluidRows R(nx, ny);
   const size_t n2 = size_t(2 * nx + 1) * (2 * ny + 1), nv = R.count[0];
@@ -164,7 +145,7 @@ __global__ void __launch_bounds__(kFluidThreads)
     case 3: fluid_apply_class<3>(nx, ny, *S, rows, R, k, x, pm, clamp != 0, y); break;
     default:
       y[2 * n2 + k] = fluid_continuity(*S, nx, ny, int(k % (nx + 1)), int(k / (nx + 1)), x);
-      if (KRYLOV) zc[k] = x[2 * n2 + k] - pm;  // the centred pressure, moved into z_j by k_fluid_dot
+      if (KRYLOV) zc[k] = x[2 * n2 + k] - pm;  // the centred pressure, moved into z_j by k_krylov_dot
   }
 }
 
@@ -264,7 +245,7 @@ __global__ void k_fluid_center(const double* x, double* y, size_t n, const doubl
 // ---------------------------------------------------------------------------
 // FP32 right-hand sides of the preconditioner: the planar velocity components of v_j (zero on
 // the boundary) and its pressure less the mean
-__global__ void k_fluid_split(int NX, int NY, const double* V, size_t n, size_t nv, const FluidKrylov* K,
+__global__ void k_fluid_split(int NX, int NY, const double* V, size_t n, size_t nv, const KrylovDev* K,
                               float* c, float* pt) {
   TOPO_PDL_ENTRY();
   const size_t n2 = size_t(NX) * NY;
@@ -283,7 +264,7 @@ __global__ void k_fluid_split(int NX, int NY, const double* V, size_t n, size_t 
 
 // z_j = the V-cycles' velocity, and pressure r / m_lumped + the V-cycle's; sums the pressure
 __global__ void k_fluid_merge(int NX, int NY, const double* V, double* Z, size_t n, size_t nv, const float* c,
-                              const float* pz, const double* ml, double* partials, unsigned* counter, FluidKrylov* K) {
+                              const float* pz, const double* ml, double* partials, unsigned* counter, KrylovDev* K) {
   TOPO_PDL_ENTRY();
   const size_t n2 = size_t(NX) * NY;
   const double* v = V + size_t(K->j) * n + 2 * n2;
@@ -303,208 +284,6 @@ __global__ void k_fluid_merge(int NX, int NY, const double* V, double* Z, size_t
   }
   double tot[1];
   if (finish_reduction<1>(s, partials, counter, tot)) K->zsum = tot[0];
-}
-
-// A pass's products hp_i = v_i . w, i <= j, and |w|^2 (w = v_(j+1)): blockIdx.y takes eight basis
-// vectors, blockIdx.x a share of the entries.  The first pass also moves the centred
-// pressure into z_j (k_fluid_apply could not: other blocks read the uncentred one).
-__global__ void __launch_bounds__(kVecThreads)
-    k_fluid_dot(const double* V, double* Z, size_t n, size_t nv, const double* zc, int pass, double* partials,
-                unsigned* counters, FluidKrylov* K) {
-  TOPO_PDL_ENTRY();
-  const int j = K->j, i0 = blockIdx.y * kDotGroup;
-  if (pass == 1 && !K->second) return;
-  if (pass == 0 && blockIdx.y == 0) {
-    double* z = Z + size_t(j) * n + (n - nv);
-    TOPO_GRID_STRIDE(k, nv) z[k] = zc[k];
-  }
-  if (i0 > j) return;
-  const double* w = V + size_t(j + 1) * n;
-  const double* v = V + size_t(i0) * n;
-  const int count = min(kDotGroup, j + 1 - i0);
-  double s[kDotGroup + 1];
-#pragma unroll
-  for (int k = 0; k <= kDotGroup; ++k) s[k] = 0.0;
-  if (count == kDotGroup) {
-    TOPO_GRID_STRIDE(i, n) {
-      const double wi = w[i];
-#pragma unroll
-      for (int k = 0; k < kDotGroup; ++k) s[k] += v[size_t(k) * n + i] * wi;
-      if (i0 == 0) s[kDotGroup] += wi * wi;
-    }
-  } else {
-    TOPO_GRID_STRIDE(i, n) {
-      const double wi = w[i];
-#pragma unroll
-      for (int k = 0; k < kDotGroup; ++k)
-        if (k < count) s[k] += v[size_t(k) * n + i] * wi;
-      if (i0 == 0) s[kDotGroup] += wi * wi;
-    }
-  }
-  double tot[kDotGroup + 1];
-  if (finish_reduction<kDotGroup + 1>(s, partials + size_t(blockIdx.y) * (kDotGroup + 1) * gridDim.x,
-                                      counters + blockIdx.y, tot, blockIdx.x, gridDim.x)) {
-    for (int k = 0; k < count; ++k) K->hp[i0 + k] = tot[k];
-    if (i0 == 0) K->ww = tot[kDotGroup];
-  }
-}
-
-// w -= sum hp_i v_i.  The first pass (classical Gram-Schmidt) decides on the second: it is needed
-// where the products took nearly all of |w|^2 (kReorthogonalise; Kahan's "twice is enough"); the
-// second sums |w|^2.
-__global__ void __launch_bounds__(kVecThreads)
-    k_fluid_sub(double* V, size_t n, int pass, double* partials, unsigned* counter, FluidKrylov* K) {
-  TOPO_PDL_ENTRY();
-  __shared__ double h[kFluidRestartMax + 1];
-  const int j = K->j;
-  if (pass == 1 && !K->second) return;
-  for (int i = threadIdx.x; i <= j; i += blockDim.x) h[i] = K->hp[i];
-  __syncthreads();
-  double* w = V + size_t(j + 1) * n;
-  double s[1] = {0.0};
-  TOPO_GRID_STRIDE(i, n) {
-    double a = w[i];
-    int k = 0;
-    for (; k + 8 <= j + 1; k += 8) {
-#pragma unroll
-      for (int q = 0; q < 8; ++q) a -= h[k + q] * V[size_t(k + q) * n + i];
-    }
-    for (; k <= j; ++k) a -= h[k] * V[size_t(k) * n + i];
-    w[i] = a;
-    s[0] += a * a;
-  }
-  if (pass == 0) {
-    // (a kernel after this one reads `second`; none of this grid does)
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      double hh = 0.0;
-      for (int i = 0; i <= j; ++i) {
-        K->h[i] = h[i];
-        hh += h[i] * h[i];
-      }
-      const double ww = K->ww, est = ww - hh;
-      K->second = !(est >= kReorthogonalise * ww);
-      K->hn = sqrt(est);
-    }
-    return;
-  }
-  double tot[1];
-  if (finish_reduction<1>(s, partials, counter, tot)) {
-    for (int i = 0; i <= j; ++i) K->h[i] += h[i];
-    K->hn = sqrt(tot[0]);
-  }
-}
-
-// v_(j+1) = w / |w| and the sum of its pressure, in all blocks but the first, whose first warp
-// rotates the column into the triangular factor, updates the residual norm and decides
-// whether the cycle goes on.  The rotations' recurrence up' = -s_i up + c_i h_(i+1) is affine in
-// up: a warp scan of two maps a lane (a thread's loop took ~10 us at 30 columns).
-__global__ void __launch_bounds__(kVecThreads)
-    k_fluid_next(double* V, size_t n, size_t nv, int m, double* partials, unsigned* counter, FluidKrylov* K,
-                 cudaGraphConditionalHandle cond, int use_cond) {
-  TOPO_PDL_ENTRY();
-  const int j = K->j;
-  const double hn = K->hn, f = hn > 0 ? 1.0 / hn : 1.0;
-  double s[1] = {0.0};
-  if (blockIdx.x > 0) {
-    double* w = V + size_t(j + 1) * n;
-    for (size_t i = size_t(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x - 1) * blockDim.x) {
-      const double v = w[i] * f;
-      w[i] = v;
-      if (i >= n - nv) s[0] += v;
-    }
-  } else if (threadIdx.x < 32) {
-    const int e = 2 * int(threadIdx.x);
-    double c[2], t[2], h[2], a[2], b[2];
-    for (int q = 0; q < 2; ++q) {
-      const bool on = e + q < j;
-      c[q] = on ? K->cs[e + q] : 1.0;
-      t[q] = on ? K->sn[e + q] : 0.0;
-      h[q] = on ? K->h[e + q + 1] : 0.0;
-      a[q] = on ? -t[q] : 1.0;
-      b[q] = c[q] * h[q];
-    }
-    const double h0 = K->h[0];
-    double A = a[1] * a[0], B = a[1] * b[0] + b[1];
-    for (int o = 1; o < 32; o <<= 1) {
-      const double pa = __shfl_up_sync(0xffffffffu, A, o), pb = __shfl_up_sync(0xffffffffu, B, o);
-      if (int(threadIdx.x) >= o) {
-        B = A * pb + B;
-        A = A * pa;
-      }
-    }
-    double Ea = __shfl_up_sync(0xffffffffu, A, 1), Eb = __shfl_up_sync(0xffffffffu, B, 1);
-    if (threadIdx.x == 0) {
-      Ea = 1.0;
-      Eb = 0.0;
-    }
-    double up = Ea * h0 + Eb;
-    for (int q = 0; q < 2; ++q) {
-      if (e + q < j) K->H[(e + q) * kFluidRestartMax + j] = c[q] * up + t[q] * h[q];
-      up = a[q] * up + b[q];
-    }
-    up = __shfl_sync(0xffffffffu, up, 31);
-    if (threadIdx.x == 0) {
-      const double den = hypot(up, hn);
-      const double cj = den > 0 ? up / den : 1.0, tj = den > 0 ? hn / den : 0.0;
-      K->cs[j] = cj;
-      K->sn[j] = tj;
-      K->H[j * kFluidRestartMax + j] = den;
-      const double g = K->gv[j];
-      K->gv[j + 1] = -tj * g;
-      K->gv[j] = cj * g;
-      const int it = K->it + 1;
-      K->it = it;
-      int st = 1;
-      if (!isfinite(hn)) st = 4;
-      else if (fabs(tj * g) <= K->target || hn == 0.0 || j + 1 >= m || it >= K->maxit) st = 0;
-      K->status = st;
-      if (use_cond) cudaGraphSetConditional(cond, st == 1 ? 1u : 0u);
-    }
-  }
-  double tot[1];
-  if (finish_reduction<1>(s, partials, counter, tot)) {
-    K->psum = tot[0];
-    K->j = j + 1;  // every block has read it
-  }
-}
-
-__global__ void k_fluid_start(FluidKrylov* K, double beta, double target, int it, int maxit) {
-  K->j = 0;
-  K->it = it;
-  K->maxit = maxit;
-  K->status = 1;
-  K->target = target;
-  K->gv[0] = beta;
-}
-
-// y = R^-1 g by one warp: column by column, the lanes hold the remaining right-hand side
-__global__ void __launch_bounds__(32) k_fluid_backsolve(FluidKrylov* K) {
-  constexpr int P = (kFluidRestartMax + 31) / 32;
-  const int k = K->j, lane = threadIdx.x;
-  double g[P];
-  for (int q = 0; q < P; ++q) g[q] = lane + 32 * q < k ? K->gv[lane + 32 * q] : 0.0;
-  for (int i = k - 1; i >= 0; --i) {
-    const double d = K->H[i * kFluidRestartMax + i];
-    const double y = __shfl_sync(0xffffffffu, i < 32 ? g[0] : g[P - 1], i & 31) / d;
-    const double yi = d != 0.0 ? y : 0.0;
-    if (lane == 0) K->y[i] = yi;
-    for (int q = 0; q < P; ++q)
-      if (lane + 32 * q < i) g[q] -= K->H[(lane + 32 * q) * kFluidRestartMax + i] * yi;
-  }
-}
-static_assert(kFluidRestartMax <= 64, "two values per lane, here and in k_fluid_next");
-
-// x += sum_i y_i z_i over the cycle's directions
-__global__ void k_fluid_update(double* x, const double* Z, size_t n, const FluidKrylov* K) {
-  __shared__ double y[kFluidRestartMax];
-  const int k = K->j;
-  for (int i = threadIdx.x; i < k; i += blockDim.x) y[i] = K->y[i];
-  __syncthreads();
-  TOPO_GRID_STRIDE(i, n) {
-    double a = x[i];
-    for (int q = 0; q < k; ++q) a += y[q] * Z[size_t(q) * n + i];
-    x[i] = a;
-  }
 }
 
 // zero the boundary velocity rows: b[2i+c] = 0 at boundary nodes
@@ -547,7 +326,7 @@ struct topo_fluid_ctx {
   int m = kFluidRestart;       // restart length
   double* V = nullptr;         // (m + 1) n
   double* Z = nullptr;         // m n
-  FluidKrylov* kry = nullptr;
+  KrylovDev* kry = nullptr;
   double* dots = nullptr;      // partial sums and counters of the Gram-Schmidt products
   unsigned* dot_counters = nullptr;
   int* hstat = nullptr;        // pinned: j, it, maxit, status of the cycle
@@ -637,7 +416,7 @@ struct topo_fluid_ctx {
     const unsigned gd = unsigned(red.spread(n)), gm = unsigned(red.spread(n2 + nv));
     const double *Vc = V, *mlc = ml, *zcc = zc, *rc = rows;
     const FluidStencils* sc = sten;
-    const FluidKrylov* kc = kry;
+    const KrylovDev* kc = kry;
     launch_pdl(k_fluid_split, gn, kVecThreads, 0, s, NX(), NY(), Vc, n, nv, kc, c, pt);
     cudaEventRecord(fork, s);
     cudaStreamWaitEvent(side, fork, 0);
@@ -649,12 +428,8 @@ struct topo_fluid_ctx {
                                                                  red.counter, kry);
     const double* Zc = Z;
     launch_pdl(k_fluid_apply<true>, G.start[5], kFluidThreads, 0, s, nx, ny, G, sc, rc, Zc, V, 1, kc, n, zc);
-    for (int pass = 0; pass < 2; ++pass) {
-      launch_pdl(k_fluid_dot, dim3(gd, unsigned((m + kDotGroup - 1) / kDotGroup)), kVecThreads, 0, s, Vc, Z, n, nv, zcc, pass,
-                 dots, dot_counters, kry);
-      launch_pdl(k_fluid_sub, gv, kVecThreads, 0, s, V, n, pass, red.partials, red.counter, kry);
-    }
-    launch_pdl(k_fluid_next, gd + 1, kVecThreads, 0, s, V, n, nv, m, red.partials, red.counter, kry, cond, use_cond);
+    krylov_column(KrylovSpace{V, nullptr, Z, zcc, n, nv, m, dots, dot_counters, red.partials, red.counter, kry},
+                  int(gd), int(gv), cond, use_cond, s);
     launches += 9;
   }
   int record();
@@ -793,12 +568,12 @@ int fluid_fgmres(topo_fluid_ctx* C, const double* b, double* x, double rtol, int
     k_scale<double><<<g, kVecThreads, 0, s>>>(r, 1.0 / beta, n);
     k_dot<double, double><<<C->red.blocks_for(C->nv), kVecThreads, 0, s>>>(C->pp(r), C->ones, C->nv, C->red.partials,
                                                                          C->red.counter, &C->kry->psum);
-    k_fluid_start<<<1, 1, 0, s>>>(C->kry, beta, 0.5 * rtol * bn, iters, maxit);
+    k_krylov_start<<<1, 1, 0, s>>>(C->kry, beta, 0.5 * rtol * bn, iters, maxit, 0.0, 0.0, 0);
     C->hstat[1] = iters;
     const int rc = C->cycle(s);
     if (rc) return C->fail(TOPO_ERR_CUDA, "fluid solve: CUDA error");
-    k_fluid_backsolve<<<1, 32, 0, s>>>(C->kry);
-    k_fluid_update<<<g, kVecThreads, 0, s>>>(x, C->Z, n, C->kry);
+    k_krylov_backsolve<<<1, 32, 0, s>>>(C->kry);
+    k_krylov_update<<<g, kVecThreads, 0, s>>>(x, C->Z, n, C->kry);
     C->launches += 5;
     iters = C->hstat[1];
     if (C->hstat[3] == 4) return C->fail(TOPO_ERR_NAN, "non-finite Krylov vector in the fluid solve");
@@ -855,12 +630,12 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
   C->ones = C->arena.alloc_n<double>(C->nv);
   C->rhs = C->arena.alloc_n<double>(C->n);
   C->x = C->arena.alloc_n<double>(C->n);
-  if (C->n * sizeof(double) * (2 * kFluidRestartMax + 1) <= kFluidBasisMax) C->m = kFluidRestartMax;
+  if (C->n * sizeof(double) * (2 * kKrylovMax + 1) <= kFluidBasisMax) C->m = kKrylovMax;
   C->V = C->arena.alloc_n<double>(size_t(C->m + 1) * C->n);
   C->Z = C->arena.alloc_n<double>(size_t(C->m) * C->n);
   C->t = C->arena.alloc_n<double>(C->n);
-  C->kry = C->arena.alloc_n<FluidKrylov>(1);
-  C->dots = C->arena.alloc_n<double>(size_t(C->red.spread(C->n)) * (kDotGroup + 1) * kDotGroups);
+  C->kry = C->arena.alloc_n<KrylovDev>(1);
+  C->dots = C->arena.alloc_n<double>(krylov_dots(C->red.spread(C->n)));
   C->dot_counters = C->arena.alloc_n<unsigned>(kDotGroups);
   C->zc = C->arena.alloc_n<double>(C->nv);
   C->c = C->arena.alloc_n<float>(2 * C->n2);

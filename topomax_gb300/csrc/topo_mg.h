@@ -139,7 +139,7 @@ class MG {
   void set_p2(const P2Params<T>& op, const P2Params<T>& pc, const T* xi) {
     // kernel parameters are baked into the captured solve graphs
     if (std::memcmp(&op, &p2_op_, sizeof(op)) || std::memcmp(&pc, &p2_, sizeof(pc)) || xi != xi_)
-      graph_valid_ = false;
+      invalidate();
     p2_op_ = op;
     p2_ = pc;
     xi_ = xi;
@@ -174,6 +174,15 @@ class MG {
   // receives the result.  Returns -5 when the object was set up without it.
   int pcg_x64(const T* b, double* x64, bool x_nonzero, double rtol, int maxit, SolveStats& st, cudaStream_t s);
   int minres(const T* b, T* x, double rtol, int maxit, SolveStats& st, cudaStream_t s);
+  // For a caller that records the solve into a graph of its own: from x = 0, the right-hand side
+  // in scratch0(5), the tolerance squared and the iteration cap in device_scalars(), the
+  // result in solution64(), status and iterations in device_scalars().  epoch() changes when
+  // a recording is no longer valid.
+  bool record_solve(bool warm, cudaStream_t s, cudaStream_t sb, long long& l1, long long& l2);
+  PcgDev* device_scalars() { return dev_; }
+  const double* solution64() const { return xacc_; }
+  cudaStream_t recording_stream(int k) const { return cap_[k]; }
+  long long epoch() const { return epoch_; }
   const LevelSpec& spec(int l) const { return specs_[l]; }
   int levels() const { return int(specs_.size()); }
   double lmax(int l) const { return lv_[l].lmax; }
@@ -291,6 +300,11 @@ class MG {
     long long prologue_nodes = 0, body_nodes = 0;
   } graph_[2];
   bool graph_valid_ = false;
+  long long epoch_ = 0;
+  void invalidate() {
+    graph_valid_ = false;
+    ++epoch_;
+  }
   void build_tail();
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> prof_events_;
   // truncated hierarchy: the V-cycle stops at level cheb_coarse_ and solves it

@@ -1179,7 +1179,7 @@ void MG<T>::detect_uniform_levels(cudaStream_t s) {
     }
     v.inner = dst;
   }
-  graph_valid_ = false;
+  invalidate();
 }
 
 // Picks the truncation level (see CoarseCheb): the finest level l >= 1 with a
@@ -1246,7 +1246,7 @@ void MG<T>::select_coarse_cheb(cudaStream_t s) {
     coarse_cheb_deg = deg;
     break;
   }
-  if (cheb_coarse_ != prev) graph_valid_ = false;
+  if (cheb_coarse_ != prev) invalidate();
 }
 
 // Chooses the levels of k_level_tail (FP32): from the first level with at most kTailNodes
@@ -1899,6 +1899,51 @@ void MG<T>::pcg_body(cudaStream_t s, cudaGraphConditionalHandle h, int use_cond)
   launches += 5;
 }
 
+// Captures a solve on s, which must be capturing: the prologue, then a WHILE node (its body on
+// sb) running the iterations.  l1, l2: the launch counter before and after the body.
+template <class T>
+bool MG<T>::record_solve(bool warm, cudaStream_t s, cudaStream_t sb, long long& l1, long long& l2) {
+  bool ok = true;
+  cudaGraphNode_t wnode = nullptr;
+  pcg_prologue(warm, s);
+  cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
+  cudaGraph_t cg = nullptr;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t ndeps = 0;
+  ok &= cudaStreamGetCaptureInfo(s, &cst, nullptr, &cg, &deps, nullptr, &ndeps) == cudaSuccess;
+  ok &= (cst == cudaStreamCaptureStatusActive) && cg != nullptr;
+  cudaGraphConditionalHandle h = 0;
+  if (ok) ok &= cudaGraphConditionalHandleCreate(&h, cg, 1, cudaGraphCondAssignDefault) == cudaSuccess;
+  if (ok) {
+    k_pcg_start<<<1, 1, 0, s>>>(dev_, h, 1);
+    ok &= cudaStreamGetCaptureInfo(s, &cst, nullptr, &cg, &deps, nullptr, &ndeps) == cudaSuccess;
+    ok &= (cst == cudaStreamCaptureStatusActive);
+  }
+  cudaGraphNodeParams cp = {};
+  if (ok) {
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = h;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    ok &= cudaGraphAddNode(&wnode, cg, deps, nullptr, ndeps, &cp) == cudaSuccess;
+    ok &= cp.conditional.phGraph_out != nullptr;
+  }
+  if (ok) {
+    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    l1 = launches;
+    ok &= cudaStreamBeginCaptureToGraph(sb, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) ==
+          cudaSuccess;
+    if (ok) {
+      pcg_body(sb, h, 1);
+      ok &= cudaStreamEndCapture(sb, &body) == cudaSuccess;
+    }
+    l2 = launches;
+    if (ok) ok &= cudaStreamUpdateCaptureDependencies(s, &wnode, nullptr, 1, cudaStreamSetCaptureDependencies) ==
+                  cudaSuccess;
+  }
+  return ok;
+}
+
 // Records the CG solve into a graph: a prologue (initial residual, first
 // preconditioned direction, start test) followed by a WHILE conditional node
 // whose body is one CG iteration; the body's last kernel decides whether the
@@ -1919,47 +1964,8 @@ int MG<T>::capture_pcg(bool warm) {
   cudaGetLastError();
   const long long l0 = launches;
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return -5;
-  bool ok = true;
-  cudaGraphNode_t wnode = nullptr;
   long long l1 = 0, l2 = 0;
-  {
-    pcg_prologue(warm, s);
-    cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
-    cudaGraph_t cg = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    ok &= cudaStreamGetCaptureInfo(s, &cst, nullptr, &cg, &deps, nullptr, &ndeps) == cudaSuccess;
-    ok &= (cst == cudaStreamCaptureStatusActive) && cg != nullptr;
-    cudaGraphConditionalHandle h = 0;
-    if (ok) ok &= cudaGraphConditionalHandleCreate(&h, cg, 1, cudaGraphCondAssignDefault) == cudaSuccess;
-    if (ok) {
-      k_pcg_start<<<1, 1, 0, s>>>(dev_, h, 1);
-      ok &= cudaStreamGetCaptureInfo(s, &cst, nullptr, &cg, &deps, nullptr, &ndeps) == cudaSuccess;
-      ok &= (cst == cudaStreamCaptureStatusActive);
-    }
-    cudaGraphNodeParams cp = {};
-    if (ok) {
-      cp.type = cudaGraphNodeTypeConditional;
-      cp.conditional.handle = h;
-      cp.conditional.type = cudaGraphCondTypeWhile;
-      cp.conditional.size = 1;
-      ok &= cudaGraphAddNode(&wnode, cg, deps, nullptr, ndeps, &cp) == cudaSuccess;
-      ok &= cp.conditional.phGraph_out != nullptr;
-    }
-    if (ok) {
-      cudaGraph_t body = cp.conditional.phGraph_out[0];
-      l1 = launches;
-      ok &= cudaStreamBeginCaptureToGraph(sb, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) ==
-            cudaSuccess;
-      if (ok) {
-        pcg_body(sb, h, 1);
-        ok &= cudaStreamEndCapture(sb, &body) == cudaSuccess;
-      }
-      l2 = launches;
-      if (ok) ok &= cudaStreamUpdateCaptureDependencies(s, &wnode, nullptr, 1, cudaStreamSetCaptureDependencies) ==
-                    cudaSuccess;
-    }
-  }
+  bool ok = record_solve(warm, s, sb, l1, l2);
   cudaGraph_t graph = nullptr;
   const cudaError_t ee = cudaStreamEndCapture(s, &graph);
   ok &= (ee == cudaSuccess) && graph != nullptr;
