@@ -339,6 +339,7 @@ struct P2Lane {
   T X[2][2];      // density at vertices (i+c, j+r)
   T A[3][3][2];   // element results at the same nodes
   T M[12];        // r-weighted mass matrices of the cell (when precomputed), [o][k]
+  T C[2][2][2];   // First: coarse correction at vertices (i+c, j+r)
 };
 
 // The loads of the next step, issued before the current step's arithmetic so
@@ -348,6 +349,12 @@ struct P2Next {
   T U[2][3][2];   // operand rows 1, 2 of the next step
   T X[2];         // density row 1 of the next step
   T M[12];        // mass matrices of the next cell
+  // Nothing is computed from a load before the current step's arithmetic (the warp would wait for
+  // it there): Pre's operand c0 Dinv b is formed in take(), First's prolongation in compute().
+  T D[2][3][2];   // Pre: Dinv (U holds b)
+  T c0;
+  bool scaled;    // U is to be multiplied by c0 D
+  T C[2][2];      // First: row 1 of the coarse correction
 };
 
 template <class T>
@@ -378,24 +385,36 @@ struct P2March {
     }
   }
 
-  // P1 -> P2 prolongation of the coarse correction at node (a,b): the coarse
-  // hat functions are 1 at vertex (a/2, b/2) and 1/2 at the edge midpoints
-  TOPO_HD static void prolong(const P2Params<T>& P, const T* xc, int a, int b, T (&v)[2]) {
-    const int NXc = P.nx + 1;
-    const int pa = a & 1, pb = b & 1, I0 = a >> 1, J0 = b >> 1;
-    const size_t m0 = size_t(J0) * NXc + I0;
-    T x0[2];
-    ld2(xc + 2 * m0, x0);
-    if (pa | pb) {
-      const size_t m1 = size_t(J0 + pb) * NXc + I0 + pa;
-      T x1[2];
-      ld2(xc + 2 * m1, x1);
-      v[0] += T(0.5) * (x0[0] + x1[0]);
-      v[1] += T(0.5) * (x0[1] + x1[1]);
-    } else {
-      v[0] += x0[0];
-      v[1] += x0[1];
+  // Coarse correction (P1) at vertices (i, j) and (i+1, j), zero outside the lattice
+  template <bool LEAN = false>
+  TOPO_HD static void coarse(const P2Params<T>& P, const P2Io<T>& io, const P2Mask& K, int i, int j, T (&v)[2][2]) {
+    for (int c = 0; c < 2; ++c) {
+      v[c][0] = v[c][1] = T(0);
+      if (io.xc && (LEAN || K.vcol[c])) ld2(io.xc + 2 * size_t(unsigned(j) * unsigned(P.nx + 1) + unsigned(i + c)), v[c]);
     }
+  }
+
+  // P1 -> P2 prolongation of the coarse correction, added to the operand's rows R0..R1 at free
+  // nodes: the coarse hat functions are 1 at their vertex and 1/2 at the adjacent edge midpoints.
+  // Each lane takes its two vertices of a row from memory once per step, where a node by node
+  // prolongation took up to two loads for each of four nodes.
+  template <int R0, int R1, bool LEAN = false>
+  TOPO_HD static void prolong(const P2Params<T>& P, P2Lane<T>& L, int j) {
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int r = R0; r <= R1; ++r)
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+      for (int c = 0; c < 3; ++c) {
+        if (!LEAN && (!L.K.col[c] || clamped(P, L.K, c, 2 * L.i + c, 2 * j + r))) continue;
+        const int r0 = r >> 1, c0 = c >> 1, r1 = (r + 1) >> 1, c1 = (c + 1) >> 1;
+        for (int d = 0; d < 2; ++d) {
+          if (r0 == r1 && c0 == c1) L.U[r][c][d] += L.C[r0][c0][d];
+          else L.U[r][c][d] += T(0.5) * (L.C[r0][c0][d] + L.C[r1][c1][d]);
+        }
+      }
   }
 
   // Whether a warp's whole march runs on the lean path: every cell it touches
@@ -420,9 +439,9 @@ struct P2March {
     return K.ccl[c] || row_clamped(P, b) || (K.pts && is_clamped(P.dir, a, b));
   }
 
-  // Operand at node (a, b) = (2i + c, b) of the lane, zero outside the lattice.
-  // At a clamped node it is the raw operand (without the First mode's coarse
-  // correction): the element phase zeroes it (tri), and the finish phase uses it
+  // Operand at node (a, b) = (2i + c, b) of the lane, zero outside the lattice,
+  // without the First mode's coarse correction (prolong).  At a clamped node the
+  // element phase zeroes it (tri), and the finish phase uses it
   // as the identity row's value without loading it again.  LEAN: the node is
   // known to be inside and free.
   template <bool LEAN = false>
@@ -434,7 +453,21 @@ struct P2March {
       return;
     }
     operand(io, unsigned(b) * unsigned(NX) + unsigned(a), v);
-    if (io.mode == kP2First && io.xc && (LEAN || !clamped(P, K, c, a, b))) prolong(P, io.xc, a, b, v);
+  }
+
+  // the prefetched form of fetch: Pre's b and Dinv instead of their product
+  template <bool LEAN = false>
+  TOPO_HD static void fetch_raw(const P2Params<T>& P, const P2Io<T>& io, const P2Mask& K, int c, int a, int b,
+                                P2Next<T>& N, int r) {
+    if (io.mode != kP2Pre) {
+      fetch<LEAN>(P, io, K, c, a, b, N.U[r][c]);
+      return;
+    }
+    for (int d = 0; d < 2; ++d) N.U[r][c][d] = N.D[r][c][d] = T(0);
+    if (!LEAN && !K.col[c]) return;
+    const size_t i = 2 * size_t(unsigned(b) * unsigned(2 * P.nx + 1) + unsigned(a));
+    ld2(io.B.b + i, N.U[r][c]);
+    ld2(io.B.dinv + i, N.D[r][c]);
   }
 
   // density at vertex (i + c, j) of the lane (rows j <= ny always)
@@ -459,6 +492,11 @@ struct P2March {
         fetch<LEAN>(P, io, L.K, 1, 2 * L.i + 1, b, L.U[r][1]);
         if (L.edge) fetch<LEAN>(P, io, L.K, 2, 2 * L.i + 2, b, L.U[r][2]);
       }
+    }
+    if (io.mode == kP2First) {  // row 0 here, rows 1 and 2 in compute()
+      coarse<LEAN>(P, io, L.K, L.i, j, L.C[0]);
+      coarse<LEAN>(P, io, L.K, L.i, j + 1, L.C[1]);
+      prolong<0, 0, LEAN>(P, L, j);
     }
 #if defined(__CUDA_ARCH__)
 #pragma unroll
@@ -571,11 +609,14 @@ struct P2March {
 #endif
       for (int r = 1; r <= 2; ++r) {
         const int b = 2 * j + r;
-        fetch<LEAN>(P, io, L.K, 0, 2 * L.i, b, N.U[r - 1][0]);
-        fetch<LEAN>(P, io, L.K, 1, 2 * L.i + 1, b, N.U[r - 1][1]);
-        if (L.edge) fetch<LEAN>(P, io, L.K, 2, 2 * L.i + 2, b, N.U[r - 1][2]);
+        fetch_raw<LEAN>(P, io, L.K, 0, 2 * L.i, b, N, r - 1);
+        fetch_raw<LEAN>(P, io, L.K, 1, 2 * L.i + 1, b, N, r - 1);
+        if (L.edge) fetch_raw<LEAN>(P, io, L.K, 2, 2 * L.i + 2, b, N, r - 1);
       }
     }
+    if (io.mode == kP2First) coarse<LEAN>(P, io, L.K, L.i, j + 1, N.C);
+    N.scaled = io.mode == kP2Pre;
+    N.c0 = io.cf[0];
     N.X[0] = density<LEAN>(P, xi, L.K, 0, L.i, j + 1);
     if (L.edge) N.X[1] = density<LEAN>(P, xi, L.K, 1, L.i, j + 1);
     if constexpr (!IsDD<T>::value) load_mass<LEAN>(P, L.K, L.i, j, N.M);  // (dd: loaded at compute time)
@@ -585,7 +626,11 @@ struct P2March {
   TOPO_HD static void take(P2Lane<T>& L, const P2Next<T>& N) {
     for (int r = 1; r <= 2; ++r)
       for (int c = 0; c < 3; ++c)
-        for (int d = 0; d < 2; ++d) L.U[r][c][d] = N.U[r - 1][c][d];
+        for (int d = 0; d < 2; ++d) {
+          if (!IsDD<T>::value && N.scaled) L.U[r][c][d] = N.c0 * N.D[r - 1][c][d] * N.U[r - 1][c][d];
+          else L.U[r][c][d] = N.U[r - 1][c][d];
+          L.C[1][c & 1][d] = N.C[c & 1][d];
+        }
     L.X[1][0] = N.X[0];
     L.X[1][1] = N.X[1];
     if constexpr (!IsDD<T>::value)
@@ -595,6 +640,8 @@ struct P2March {
   // element results of cell (L.i, j), both triangles (0 <= j < ny always)
   template <bool LEAN = false>
   TOPO_HD static void compute(const P2Params<T>& P, P2Lane<T>& L, int j, int mode) {
+    if constexpr (!IsDD<T>::value)
+      if (mode == kP2First) prolong<1, 2, LEAN>(P, L, j);
     if (!LEAN && !L.K.cell) return;
     bool Z[3][3] = {};
     if (!LEAN)
@@ -778,6 +825,8 @@ struct P2March {
       }
     L.X[0][0] = L.X[1][0];
     L.X[0][1] = L.X[1][1];
+    for (int c = 0; c < 2; ++c)
+      for (int d = 0; d < 2; ++d) L.C[0][c][d] = L.C[1][c][d];
   }
 
   TOPO_HD static void begin(const P2Params<T>& P, P2Lane<T>& L, int i, bool edge) {
@@ -797,6 +846,8 @@ struct P2March {
       for (int c = 0; c < 3; ++c)
         for (int d = 0; d < 2; ++d) L.U[r][c][d] = L.A[r][c][d] = T(0);
     L.X[0][0] = L.X[0][1] = L.X[1][0] = L.X[1][1] = T(0);
+    for (int c = 0; c < 2; ++c)
+      for (int d = 0; d < 2; ++d) L.C[0][c][d] = L.C[1][c][d] = T(0);
     for (int k = 0; k < 12; ++k) L.M[k] = T(0);
   }
 };
