@@ -231,17 +231,20 @@ void level_sweeps(LevelSweep<T, NC> P, const T* b, const T* xin, const T* xc, T*
         T *s = sm.data(), *sn = s + NC * (w + 2) * (h + 2);
         std::vector<typename Ph::Node> N(nt);
         std::vector<char> on(nt);
-        for (int t = 0; t < nt; ++t) on[t] = Ph::start(P, a0, b0, w, h, t, N[t]);
+        for (int t = 0; t < nt; ++t) on[t] = Ph::template start<D>(P, a0, b0, w, h, t, N[t]);
         auto each = [&](auto&& f) {
           for (int t = 0; t < nt; ++t)
             if (on[t]) f(t, N[t]);
         };
+        each([&](int, auto& n) {
+          n.load(P);
+          n.load_b(P, b);
+          if (up) Ph::up_own(P, xin, xc, n);
+        });
         for (int t = 0; t < nt; ++t) {
-          if (up) Ph::up_first(P, a0, b0, w, h, t, nt, xin, xc, s);
-          else Ph::down_first(P, a0, b0, w, h, t, nt, b, s);
+          if (up) Ph::up_first(P, a0, b0, w, h, t, nt, xin, xc, s, on[t], N[t]);
+          else Ph::down_first(P, a0, b0, w, h, t, nt, b, s, on[t], N[t]);
         }
-        each([&](int, auto& n) { n.load_b(P, b); });
-        if (!up) each([&](int, auto& n) { Ph::down_own(s, n); });
         if (up) {
           each([&](int, auto& n) { Ph::up_residual(P, w, s, sn, n); });
           std::swap(s, sn);
@@ -253,10 +256,10 @@ void level_sweeps(LevelSweep<T, NC> P, const T* b, const T* xin, const T* xc, T*
           });
           std::swap(s, sn);
         }
-        each([&](int t, auto& n) { Ph::store(P, w, ring, t, n, up ? xpost : xpre); });
+        each([&](int, auto& n) { Ph::store(P, a0, b0, ring, n, up ? xpost : xpre); });
         if (up) continue;
         each([&](int, auto& n) { Ph::down_residual(w, s, sn, n); });
-        for (int t = 0; t < nt; ++t) Ph::restrict_to(P, I0, J0, w, ring, t, nt, sn, bc);
+        for (int t = 0; t < nt; ++t) Ph::restrict_to(P, P.cx, P.cy, I0, J0, w, ring, t, nt, sn, bc);
       }
 }
 
@@ -314,9 +317,49 @@ int emu_sweeps(int D, int nx, int ny, double hx, double hy, double lam, double m
   std::copy(o3.begin(), o3.end(), xpost);
   return 0;
 }
+// Every node's row as stored (p1_stencil_node) and as built in the sweeps (level_row_free).
+template <class T, int NC>
+int emu_rows(int nx, int ny, double hx, double hy, double lam, double mu, const int* dir, const double* kK,
+             const double* kM, double* stored, double* built) {
+  constexpr int SW = StencilLayout<NC>::stride;
+  const ElemRefs R = make_elem_refs(hx, hy, lam, mu);
+  P1Params<T, NC> Q;
+  std::memset(&Q, 0, sizeof(Q));
+  Q.nx = nx;
+  Q.ny = ny;
+  Q.dir = dir_from(dir);
+  for (int o = 0; o < 2; ++o) {
+    for (int a = 0; a < 3 * NC; ++a)
+      for (int c = 0; c < 3 * NC; ++c) Q.K[o][a][c] = T(NC == 2 ? R.K2[o][a][c] : R.K1[o][a][c]);
+    for (int a = 0; a < 3; ++a)
+      for (int c = 0; c < 3; ++c) Q.Mm[o][a][c] = T(R.M1[o][a][c]);
+  }
+  const std::vector<T> k(kK, kK + size_t(2) * nx * ny), m(kM, kM + (NC == 1 ? size_t(2) * nx * ny : 0));
+  Q.kK = k.data();
+  Q.kM = NC == 1 ? m.data() : nullptr;
+  for (int b = 0; b <= ny; ++b)
+    for (int a = 0; a <= nx; ++a) {
+      T s[SW], f[SW];
+      p1_stencil_node<T, NC>(a, b, Q, s);
+      level_row_free<T, NC>(Q, a, b, f);
+      const size_t n = (size_t(b) * (nx + 1) + a) * SW;
+      std::copy(s, s + SW, stored + n);
+      std::copy(f, f + SW, built + n);
+    }
+  return SW;
+}
 }  // namespace
 
 extern "C" {
+
+int emu_level_rows(int prec, int NC, int nx, int ny, double hx, double hy, double lam, double mu, const int* dir,
+                   const double* kK, const double* kM, double* stored, double* built) {
+  if (NC == 2)
+    return prec ? emu_rows<float, 2>(nx, ny, hx, hy, lam, mu, dir, kK, kM, stored, built)
+                : emu_rows<double, 2>(nx, ny, hx, hy, lam, mu, dir, kK, kM, stored, built);
+  return prec ? emu_rows<float, 1>(nx, ny, hx, hy, lam, mu, dir, kK, kM, stored, built)
+              : emu_rows<double, 1>(nx, ny, hx, hy, lam, mu, dir, kK, kM, stored, built);
+}
 
 // down and up sweep of D steps of a stencil level (prec 0 FP64, 1 FP32), cx x cy coarse nodes a block
 int emu_level_sweeps(int prec, int NC, int D, int nx, int ny, double hx, double hy, double lam, double mu, const int* dir,

@@ -195,8 +195,8 @@ class MG {
   // the FP32 operator arithmetic alone is consistent to ~1e-4.  Set before init().
   bool fp64_solution = false;
 
-  // Chebyshev steps of a smoothing sweep: two on level 0 of a P2 hierarchy, on the levels
-  // without a stencil (march kernels) and above deep_from; deep_degree on the others (2, or
+  // Chebyshev steps of a smoothing sweep: two on level 0 of a P2 hierarchy and
+  // above deep_from; deep_degree on the others (2, or
   // FP32 kCoarseDegree for elasticity and kScalarDegree for scalar levels).
   //
   // State hierarchy, FP32: the iterations of a solve grow with the design's contrast through
@@ -210,7 +210,7 @@ class MG {
   // Filter: no difference (1.36 ms at 1000x500).
   int deep_degree = 2, deep_from = 2;
   double cheb_lo_deep = 0.1;  // their interval's lower end, times lambda_max
-  int level_degree(int l) const { return l >= deep_from && lv_[l].st ? deep_degree : 2; }
+  int level_degree(int l) const { return l >= deep_from ? deep_degree : 2; }
   double cheb_lo_frac = 0.1;   // smoothing interval [lo_frac, 1.1] * lambda_max
   int power_iters = 10;
   int power_iters_warm = 4;  // level 0 of a P2 hierarchy, started from the previous set-up's vector
@@ -259,8 +259,8 @@ class MG {
   void vcycle_level(int l, const T* b, T* x, cudaStream_t s);
   void tune_marches(cudaStream_t s);
   void vcycle_level_body(int l, const T* b, T* x, cudaStream_t s);
-  template <int NC, int D>
-  void sweep_level(int l, const T* b, T* x, cudaStream_t s);
+  template <int NC, int D, class ROWS>
+  void sweep_level(int l, const ROWS& Q, const T* b, T* x, cudaStream_t s);
   template <int NC>
   void sweep_level(int l, const T* b, T* x, cudaStream_t s);
   template <int NC, int D>

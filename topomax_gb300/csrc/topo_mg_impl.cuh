@@ -27,9 +27,10 @@ namespace topo {
 // Lattice kernels use a 2D grid: blockIdx.y is the row, x covers the columns.
 constexpr int kRowThreads = 128;
 // P1 levels keep an assembled stencil up to a node count: elasticity levels
-// up to 2^18 nodes (a larger one streams 112 B per node per pass, more than
-// evaluating its element matrices on the fly costs), filter levels always
-// (32 B per node).  TOPO_STENCIL_NODES overrides both limits.
+// up to 2^18 nodes (a larger one streams 112 B per node and sweep, more than
+// building the rows from its triangles' coefficients costs: level_row_free; at 126 k nodes stored
+// rows and built ones measured the same, 10 and 11 us a sweep, at 31 k 3.2 and 4.8), filter levels
+// always (32 B per node).  TOPO_STENCIL_NODES overrides both limits.
 inline size_t stencil_max_nodes(int NC) {
   if (const char* e = std::getenv("TOPO_STENCIL_NODES")) return size_t(std::strtoull(e, nullptr, 10));
   return NC == 2 ? (size_t(1) << 18) : (size_t(1) << 40);
@@ -233,36 +234,62 @@ __global__ void __launch_bounds__(P2M_THREADS) k_p1_march(P1Params<T, NC> P, P1I
 // Measured on design evaluations (us): the six launches per level and the earlier one-block
 // tail of 30 to 35 us took 8,490 at 80x40, 31,000 at 303x101 and 25,470 at 1000x500; sweeps
 // and tail take 5,520, 17,100 and 18,300.
-// Tile: 10 x 4 coarse nodes, 253 threads for 160 fine nodes of its own down, 220 up.  On the
-// 1000x500 design evaluation 14 x 6 (465 threads, less recomputed) measured 18.8 ms against
-// 18.6, 6 x 6 19.2, 14 x 2 18.9; FP64 at 160x80 63.9 ms against 76.8, 66.1 and 66.2 (a tile's
+// Tile: 10 x 4 coarse nodes, 253 threads for 160 fine nodes of its own down, 220 up (two steps).
+// With the tile a constant in FP32, coefficients read before the wait, two values per access and
+// the ring apart from the nodes of its own, a down sweep of two steps is 460 instructions a warp
+// (707 before): 80x40 4.51 to 4.37 ms, 303x101 14.95 to 13.92, filter 1000x500 1.28 to 1.15,
+// FP64 160x80 60.5 to 53.3.  On the 1000x500 design evaluation 14 x 6 measured 18.8 ms against
+// 18.6, 6 x 6 19.2, 14 x 2 18.9; FP64 tiles: see level_sweep (a tile's
 // recomputed ring costs FP64-pipe time, a large tile leaves SMs without a block).
+// Levels with built rows fill the chip many times over and take 14 x 6 (31 x 15 nodes for 28 x 12)
+// at two steps: 67.9 us down against 70.9 at two million nodes.  Their loads are issued together
+// before the row is built (59.4).  Level 1 of 1000x500 takes 17 + 16 us for what were six launches
+// of 59 us (column march, restriction, prolongation), of 2000x1000 59 + 64 for 160.
 constexpr int kSweepTileX = 10, kSweepTileY = 4;
-template <int D>
+// ROWS: StoredRows, or the P1Params that the rows are built from.
+struct StoredRows {};
+template <class ROWS, int D>
+constexpr int sweep_tile_x() {
+  return std::is_same<ROWS, StoredRows>::value || D > 2 ? kSweepTileX : 14;
+}
+template <class ROWS, int D>
+constexpr int sweep_tile_y() {
+  return std::is_same<ROWS, StoredRows>::value || D > 2 ? kSweepTileY : 6;
+}
+template <class ROWS, int D>
 constexpr int sweep_threads() {  // the down sweep's region, the larger one
-  return ((2 * kSweepTileX + 2 * D - 1) * (2 * kSweepTileY + 2 * D - 1) + 31) / 32 * 32;
+  return ((2 * sweep_tile_x<ROWS, D>() + 2 * D - 1) * (2 * sweep_tile_y<ROWS, D>() + 2 * D - 1) + 31) / 32 * 32;
 }
 
-template <class T, int NC, int D>
-__global__ void __launch_bounds__(sweep_threads<D>()) k_level_down(LevelSweep<T, NC> P, const T* b, T* x, T* bc) {
+template <class T, int NC>
+__device__ __forceinline__ const P1Params<T, NC>* row_source(const P1Params<T, NC>& Q) { return &Q; }
+template <class T, int NC>
+__device__ __forceinline__ const P1Params<T, NC>* row_source(const StoredRows&) { return nullptr; }
+
+// FP32 blocks have one tile (level_sweep), so their index arithmetic divides by constants.
+template <class T, int NC, int D, class ROWS>
+__global__ void __launch_bounds__(sweep_threads<ROWS, D>())
+    k_level_down(LevelSweep<T, NC> P, const ROWS Q, const T* b, T* x, T* bc) {
   using Ph = LevelPhases<T, NC>;
   extern __shared__ __align__(16) unsigned char sweep_raw[];
-  const int w = down_w<D>(P), h = down_h<D>(P);
+  constexpr bool F = sizeof(T) == 4, stored = std::is_same<ROWS, StoredRows>::value;
+  const int cx = F ? sweep_tile_x<ROWS, D>() : P.cx, cy = F ? sweep_tile_y<ROWS, D>() : P.cy, w = 2 * cx + 2 * D - 1, h = 2 * cy + 2 * D - 1;
   T* s = reinterpret_cast<T*>(sweep_raw);
   T* sn = s + NC * (w + 2) * (h + 2);
-  const int tid = threadIdx.x, nt = blockDim.x, I0 = blockIdx.x * P.cx, J0 = blockIdx.y * P.cy;
+  const int tid = threadIdx.x, nt = blockDim.x, I0 = blockIdx.x * cx, J0 = blockIdx.y * cy;
   b += blockIdx.z * size_t(NC) * P.NX * P.NY;  // the batch's vectors
   x += blockIdx.z * size_t(NC) * P.NX * P.NY;
   bc += blockIdx.z * size_t(NC) * P.NXc * P.NYc;
   TOPO_PDL_LAUNCH();
   const int a0 = 2 * I0 - D, b0 = 2 * J0 - D;
   typename Ph::Node N;
-  const bool on = Ph::start(P, a0, b0, w, h, tid, N);
+  const bool on = Ph::template start<D>(P, a0, b0, w, h, tid, N);
+  if (on && stored) N.load(P);
   TOPO_PDL_WAIT();
-  Ph::down_first(P, a0, b0, w, h, tid, nt, b, s);
   if (on) N.load_b(P, b);
+  if (on && !stored) N.load(P, row_source<T, NC>(Q));
+  Ph::down_first(P, a0, b0, w, h, tid, nt, b, s, on, N);
   __syncthreads();
-  if (on) Ph::down_own(s, N);
 #pragma unroll
   for (int k = 1; k < D; ++k) {
     if (on && k + 1 < D) Ph::step(P, k, w, s, sn, N);
@@ -273,22 +300,23 @@ __global__ void __launch_bounds__(sweep_threads<D>()) k_level_down(LevelSweep<T,
     __syncthreads();
   }
   if (on) {
-    Ph::store(P, w, D, tid, N, x);
+    Ph::store(P, a0, b0, D, N, x);
     Ph::down_residual(w, s, sn, N);
   }
   __syncthreads();
-  Ph::restrict_to(P, I0, J0, w, D, tid, nt, sn, bc);
+  Ph::restrict_to(P, cx, cy, I0, J0, w, D, tid, nt, sn, bc);
 }
 
-template <class T, int NC, int D>
-__global__ void __launch_bounds__(sweep_threads<D>())
-    k_level_up(LevelSweep<T, NC> P, const T* b, const T* xin, const T* xc, T* x) {
+template <class T, int NC, int D, class ROWS>
+__global__ void __launch_bounds__(sweep_threads<ROWS, D>())
+    k_level_up(LevelSweep<T, NC> P, const ROWS Q, const T* b, const T* xin, const T* xc, T* x) {
   using Ph = LevelPhases<T, NC>;
   extern __shared__ __align__(16) unsigned char sweep_raw[];
-  const int w = up_w<D>(P), h = up_h<D>(P);
+  constexpr bool F = sizeof(T) == 4, stored = std::is_same<ROWS, StoredRows>::value;
+  const int cx = F ? sweep_tile_x<ROWS, D>() : P.cx, cy = F ? sweep_tile_y<ROWS, D>() : P.cy, w = 2 * cx + 2 * D - 2, h = 2 * cy + 2 * D - 2;
   T* s = reinterpret_cast<T*>(sweep_raw);
   T* sn = s + NC * (w + 2) * (h + 2);
-  const int tid = threadIdx.x, nt = blockDim.x, I0 = blockIdx.x * P.cx, J0 = blockIdx.y * P.cy;
+  const int tid = threadIdx.x, nt = blockDim.x, I0 = blockIdx.x * cx, J0 = blockIdx.y * cy;
   b += blockIdx.z * size_t(NC) * P.NX * P.NY;
   x += blockIdx.z * size_t(NC) * P.NX * P.NY;
   xin += blockIdx.z * size_t(NC) * P.NX * P.NY;
@@ -296,10 +324,15 @@ __global__ void __launch_bounds__(sweep_threads<D>())
   TOPO_PDL_LAUNCH();
   const int a0 = 2 * I0 - (D - 1), b0 = 2 * J0 - (D - 1);
   typename Ph::Node N;
-  const bool on = Ph::start(P, a0, b0, w, h, tid, N);
+  const bool on = Ph::template start<D>(P, a0, b0, w, h, tid, N);
+  if (on && stored) N.load(P);
   TOPO_PDL_WAIT();
-  Ph::up_first(P, a0, b0, w, h, tid, nt, xin, xc, s);
-  if (on) N.load_b(P, b);
+  if (on) {
+    N.load_b(P, b);
+    Ph::up_own(P, xin, xc, N);
+    if (!stored) N.load(P, row_source<T, NC>(Q));
+  }
+  Ph::up_first(P, a0, b0, w, h, tid, nt, xin, xc, s, on, N);
   __syncthreads();
   if (on) Ph::up_residual(P, w, s, sn, N);
 #pragma unroll
@@ -311,7 +344,7 @@ __global__ void __launch_bounds__(sweep_threads<D>())
     if (on && k + 1 < D) Ph::step(P, k, w, s, sn, N);
     if (on && k + 1 == D) Ph::last(P, k, w, s, static_cast<T*>(nullptr), N);
   }
-  if (on) Ph::store(P, w, D - 1, tid, N, x);
+  if (on) Ph::store(P, a0, b0, D - 1, N, x);
 }
 
 template <class T, int NC>
@@ -824,15 +857,17 @@ inline void prime_march_occupancy() {
   (void)p2_march_bps<T, kP2First>();
   (void)p2_march_bps<T, kP2Post2>();
   (void)p1_march_bps<T, 1, kP2Apply>();
-  (void)p1_march_bps<T, 1, kP2Pre>();
-  (void)p1_march_bps<T, 1, kP2Res>();
-  (void)p1_march_bps<T, 1, kP2First>();
-  (void)p1_march_bps<T, 1, kP2Post2>();
   (void)p1_march_bps<T, 2, kP2Apply>();
-  (void)p1_march_bps<T, 2, kP2Pre>();
-  (void)p1_march_bps<T, 2, kP2Res>();
-  (void)p1_march_bps<T, 2, kP2First>();
-  (void)p1_march_bps<T, 2, kP2Post2>();
+  if constexpr (sizeof(T) == 8) {  // (FP32 levels are smoothed by the sweeps)
+    (void)p1_march_bps<T, 1, kP2Pre>();
+    (void)p1_march_bps<T, 1, kP2Res>();
+    (void)p1_march_bps<T, 1, kP2First>();
+    (void)p1_march_bps<T, 1, kP2Post2>();
+    (void)p1_march_bps<T, 2, kP2Pre>();
+    (void)p1_march_bps<T, 2, kP2Res>();
+    (void)p1_march_bps<T, 2, kP2First>();
+    (void)p1_march_bps<T, 2, kP2Post2>();
+  }
 }
 
 // Kernel-clock names and algorithmic bytes of one launch (topo_kclock.h).  A mode
@@ -1304,7 +1339,7 @@ void MG<T>::apply(int l, const T* x, T* y, cudaStream_t s, bool op) {
       io.mode = kP2Apply;
       io.u = x;
       io.y = y;
-      launch_p1_march<T, 2>(make_p1<T, 2>(L, refs_[l], v.kK, nullptr), io, s);
+      launch_p1_mode<T, 2, kP2Apply>(make_p1<T, 2>(L, refs_[l], v.kK, nullptr), io, s);
     }
   } else {
     if (v.st && stencils_ready_) {
@@ -1315,7 +1350,7 @@ void MG<T>::apply(int l, const T* x, T* y, cudaStream_t s, bool op) {
       io.mode = kP2Apply;
       io.u = x;
       io.y = y;
-      launch_p1_march<T, 1>(make_p1<T, 1>(L, refs_[l], v.kK, v.kM), io, s);
+      launch_p1_mode<T, 1, kP2Apply>(make_p1<T, 1>(L, refs_[l], v.kK, v.kM), io, s);
     }
   }
 }
@@ -1537,32 +1572,39 @@ void MG<T>::vcycle_level(int l, const T* b, T* x, cudaStream_t s) {
   vcycle_level_body(l, b, x, s);
 }
 
-// Both sweeps of stencil level l with D Chebyshev steps, the coarser levels between them.
+// Both sweeps of level l with D Chebyshev steps, the coarser levels between them.
 template <class T>
-template <int NC, int D>
-void MG<T>::sweep_level(int l, const T* b, T* x, cudaStream_t s) {
+template <int NC, int D, class ROWS>
+void MG<T>::sweep_level(int l, const ROWS& Q, const T* b, T* x, cudaStream_t s) {
   Lev& v = lv_[l];
   Lev& c = lv_[l + 1];
   const LevelSpec& S = specs_[l];
   const Transfer X = make_transfer(S, specs_[l + 1]);
   const double nf = double(S.nn()) * NC, ncrs = double(X.NXc) * X.NYc * NC;
   // the stencil row of every node (7 NC x NC blocks, padded to 16 bytes; one row where the
-  // level shares it); down b, D^-1 read, x and the coarse residual written; up b, D^-1, x and
-  // the coarse correction read, x written
-  const double row = v.inner ? 0.0 : double((7 * NC * NC * sizeof(T) + 15) / 16 * 16) * double(S.nn());
-  const LevelSweep<T, NC> P = level_sweep<T, NC>(S, X, v.st, v.inner, v.dinv, cheb_ + 8 * l);
+  // level shares it; the triangles' coefficients where the rows are built from them); down b, D^-1
+  // read, x and the coarse residual written; up b, D^-1, x and the coarse correction read, x written
+  const double row = !v.st ? double(S.ntri() * sizeof(T) * (NC == 1 ? 2 : 1))
+                     : v.inner ? 0.0
+                               : double((7 * NC * NC * sizeof(T) + 15) / 16 * 16) * double(S.nn());
+  LevelSweep<T, NC> P = level_sweep<T, NC>(S, X, v.st, v.inner, v.dinv, cheb_ + 8 * l);
+  if (sizeof(T) == 4) {
+    P.cx = sweep_tile_x<ROWS, D>();
+    P.cy = sweep_tile_y<ROWS, D>();
+  }
   const dim3 g((X.NXc + P.cx - 1) / P.cx, (X.NYc + P.cy - 1) / P.cy, batch);
   const int dw = down_w<D>(P), dh = down_h<D>(P), uw = up_w<D>(P), uh = up_h<D>(P);
   {
     KClock kc(s, "P1 level down", l, row + (3 * nf + ncrs) * sizeof(T));
-    launch_pdl(k_level_down<T, NC, D>, g, dim3(unsigned(dw * dh + 31) / 32 * 32), sweep_shared(dw, dh, NC) * sizeof(T), s,
-               P, b, v.x2, c.b);
+    launch_pdl(k_level_down<T, NC, D, ROWS>, g, dim3(unsigned(dw * dh + 31) / 32 * 32),
+               sweep_shared(dw, dh, NC) * sizeof(T), s, P, Q, b, v.x2, c.b);
   }
   vcycle_level(l + 1, c.b, c.x, s);
   {
     KClock kc(s, "P1 level up", l, row + (4 * nf + ncrs) * sizeof(T));
-    launch_pdl(k_level_up<T, NC, D>, g, dim3(unsigned(uw * uh + 31) / 32 * 32), sweep_shared(uw, uh, NC) * sizeof(T), s, P,
-               b, static_cast<const T*>(v.x2), static_cast<const T*>(c.x), x);
+    launch_pdl(k_level_up<T, NC, D, ROWS>, g, dim3(unsigned(uw * uh + 31) / 32 * 32),
+               sweep_shared(uw, uh, NC) * sizeof(T), s, P, Q, b, static_cast<const T*>(v.x2),
+               static_cast<const T*>(c.x), x);
   }
   launches += 2;
 }
@@ -1573,9 +1615,14 @@ void MG<T>::sweep_level(int l, const T* b, T* x, cudaStream_t s) {
   // (the degrees in use: see level_degree)
   if constexpr (sizeof(T) == 4) {
     constexpr int D = NC == 2 ? kCoarseDegree : kScalarDegree;
-    if (level_degree(l) == D) return sweep_level<NC, D>(l, b, x, s);
+    if (!lv_[l].st) {
+      const P1Params<T, NC> Q = make_p1<T, NC>(specs_[l], refs_[l], lv_[l].kK, lv_[l].kM);
+      if (level_degree(l) == D) return sweep_level<NC, D>(l, Q, b, x, s);
+      return sweep_level<NC, 2>(l, Q, b, x, s);
+    }
+    if (level_degree(l) == D) return sweep_level<NC, D>(l, StoredRows{}, b, x, s);
   }
-  sweep_level<NC, 2>(l, b, x, s);
+  sweep_level<NC, 2>(l, StoredRows{}, b, x, s);
 }
 
 template <class T>
@@ -1655,41 +1702,41 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
     launches += 2;
     return;
   }
-  // algorithmic bytes of the transfers
-  const double nf = double(S.nn()) * S.NC, ncrs = double(X.NXc) * X.NYc * S.NC;
-  const double rbytes = (nf + ncrs) * sizeof(T), pbytes = (2 * nf + ncrs) * sizeof(T);
-  // large levels without a stencil: the column march (element products per cell)
-  auto run_march = [&](auto nc_tag, const auto& P) {
-    constexpr int NC = decltype(nc_tag)::value;
-    P1Io<T> io;
-    std::memset(&io, 0, sizeof(io));
-    io.B = B;
-    io.u = x;
-    io.mode = kP2Pre;
-    launch_p1_march<T, NC>(P, io, s);
-    io.mode = kP2Res;
-    launch_p1_march<T, NC>(P, io, s);
-    {
-      KClock kc(s, "restriction", l, rbytes);
-      launch_pdl(k_restrict<T, NC>, gc, kRowThreads, 0, s, X, static_cast<const T*>(v.r), c.b, static_cast<const T*>(nullptr));
-    }
-    launches += 3;
-    vcycle_level(l + 1, c.b, c.x, s);
-    { KClock kc(s, "prolongation", l, pbytes); launch_pdl(k_prolong_add<T, NC>, gf, kRowThreads, 0, s, X, static_cast<const T*>(c.x), x); }
-    io.mode = kP2First;
-    launch_p1_march<T, NC>(P, io, s);
-    io.mode = kP2Post2;
-    launch_p1_march<T, NC>(P, io, s);
-    launches += 3;
-  };
-  using I2 = std::integral_constant<int, 2>;
-  using I1 = std::integral_constant<int, 1>;
-  if (S.NC == 2) {
-    if (v.st) sweep_level<2>(l, b, x, s);
-    else run_march(I2{}, make_p1<T, 2>(S, refs_[l], v.kK, nullptr));
-  } else {
-    if (v.st) sweep_level<1>(l, b, x, s);
-    else run_march(I1{}, make_p1<T, 1>(S, refs_[l], v.kK, v.kM));
+  if (sizeof(T) == 4 || v.st) {
+    if (S.NC == 2) sweep_level<2>(l, b, x, s);
+    else sweep_level<1>(l, b, x, s);
+    return;
+  }
+  // FP64 levels without a stencil: the column march (element products per cell; the ring that a
+  // sweep's blocks recompute would cost FP64-pipe time)
+  if constexpr (sizeof(T) == 8) {
+    const double nf = double(S.nn()) * S.NC, ncrs = double(X.NXc) * X.NYc * S.NC;
+    const double rbytes = (nf + ncrs) * sizeof(T), pbytes = (2 * nf + ncrs) * sizeof(T);
+    auto run_march = [&](auto nc_tag, const auto& P) {
+      constexpr int NC = decltype(nc_tag)::value;
+      P1Io<T> io;
+      std::memset(&io, 0, sizeof(io));
+      io.B = B;
+      io.u = x;
+      io.mode = kP2Pre;
+      launch_p1_march<T, NC>(P, io, s);
+      io.mode = kP2Res;
+      launch_p1_march<T, NC>(P, io, s);
+      {
+        KClock kc(s, "restriction", l, rbytes);
+        launch_pdl(k_restrict<T, NC>, gc, kRowThreads, 0, s, X, static_cast<const T*>(v.r), c.b, static_cast<const T*>(nullptr));
+      }
+      launches += 3;
+      vcycle_level(l + 1, c.b, c.x, s);
+      { KClock kc(s, "prolongation", l, pbytes); launch_pdl(k_prolong_add<T, NC>, gf, kRowThreads, 0, s, X, static_cast<const T*>(c.x), x); }
+      io.mode = kP2First;
+      launch_p1_march<T, NC>(P, io, s);
+      io.mode = kP2Post2;
+      launch_p1_march<T, NC>(P, io, s);
+      launches += 3;
+    };
+    if (S.NC == 2) run_march(std::integral_constant<int, 2>{}, make_p1<T, 2>(S, refs_[l], v.kK, nullptr));
+    else run_march(std::integral_constant<int, 1>{}, make_p1<T, 1>(S, refs_[l], v.kK, v.kM));
   }
 }
 

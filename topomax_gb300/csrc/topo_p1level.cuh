@@ -1,4 +1,4 @@
-// The V-cycle's two sweeps of a P1 level with an assembled stencil, one launch each:
+// The V-cycle's two sweeps of a P1 level, one launch each:
 //   down:  x = D Chebyshev steps from zero, r = b - A x, b_c = P^T r
 //   up:    x += P x_c, D Chebyshev steps
 // A block owns cx x cy coarse nodes and the 2cx x 2cy fine nodes over them and
@@ -10,10 +10,12 @@
 // node's stencil row, inverse diagonal, residual and iterate in registers; only the
 // direction, which the neighbours read, goes through shared memory.  The rows and
 // diagonals, which no solve changes, are loaded before the kernel waits for its
-// predecessor.
+// predecessor.  A level too large for an assembled stencil builds its rows from the
+// triangles' coefficients instead (level_row_free).
 #pragma once
 
 #include "topo_p1.cuh"
+#include "topo_p2.cuh"
 
 namespace topo {
 
@@ -69,6 +71,18 @@ TOPO_HD void load_row(const T* src, T (&dst)[N]) {
 #endif
 }
 
+// one node's values (NC = 2: both at once, an address of twice their size)
+template <class T, int NC>
+TOPO_HD void load_node(const T* p, T (&v)[NC]) {
+  if constexpr (NC == 2) ld2(p, v);
+  else v[0] = p[0];
+}
+template <class T, int NC>
+TOPO_HD void store_node(T* p, const T (&v)[NC]) {
+  if constexpr (NC == 2) st2(p, v[0], v[1]);
+  else p[0] = v[0];
+}
+
 // the same copy within shared memory's address space (generic loads and stores)
 template <class T, int N>
 TOPO_HD void copy_row(const T* src, T* dst) {
@@ -117,7 +131,7 @@ TOPO_HD void level_row(T (&st)[StencilLayout<NC>::stride]) {
 template <class T, int NC>
 TOPO_HD void level_apply(const T (&st)[StencilLayout<NC>::stride], const T* u, int w, int p, T (&acc)[NC]) {
   T un[NC];
-  for (int c = 0; c < NC; ++c) un[c] = u[NC * p + c];
+  load_node<T, NC>(u + NC * p, un);
   for (int c = 0; c < NC; ++c) {
     acc[c] = st[c * NC] * un[0];
     for (int d = 1; d < NC; ++d) acc[c] = fma_t(st[c * NC + d], un[d], acc[c]);
@@ -128,7 +142,9 @@ TOPO_HD void level_apply(const T (&st)[StencilLayout<NC>::stride], const T* u, i
   for (int k = 1; k < 7; ++k) {
     const int q = p + st_db(k) * w + st_da(k);
     T ul[NC];
-    for (int c = 0; c < NC; ++c) ul[c] = sizeof(T) == 8 ? u[NC * q + c] : u[NC * q + c] - un[c];
+    load_node<T, NC>(u + NC * q, ul);
+    if constexpr (sizeof(T) == 4)
+      for (int c = 0; c < NC; ++c) ul[c] -= un[c];
     for (int c = 0; c < NC; ++c)
       for (int d = 0; d < NC; ++d) acc[c] = fma_t(st[k * NC * NC + c * NC + d], ul[d], acc[c]);
   }
@@ -158,6 +174,71 @@ TOPO_HD T level_restrict(const T* r, int w) {
   return fma_t(T(0.5), h, r[0]);
 }
 
+// The row (not yet level_row) of node (a, b) from the coefficients of the level's triangles: what
+// p1_stencil_node stores, in the level's precision.  A triangle's stiffness rows sum to zero, so
+// the row sum of block 0 is the mass's, less the couplings that a clamped neighbour takes out.
+// 48 products and 48 bytes of coefficients (shared with the neighbours) take the place of a load of
+// 112 bytes: the rows of a level too large for L2.
+template <class T, int NC>
+TOPO_HD void level_row_free(const P1Params<T, NC>& Q, int a, int b, T (&st)[StencilLayout<NC>::stride]) {
+  constexpr int SB = NC * NC;
+  for (int i = 0; i < StencilLayout<NC>::stride; ++i) st[i] = T(0);
+  // both triangles of the four cells around the node, zero outside the mesh
+  T kk4[4][2], km4[4][2];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int q = 0; q < 4; ++q) {
+    const int ci = a - 1 + (q & 1), cj = b - 1 + (q >> 1);
+    kk4[q][0] = kk4[q][1] = km4[q][0] = km4[q][1] = T(0);
+    if (ci < 0 || ci >= Q.nx || cj < 0 || cj >= Q.ny) continue;
+    const unsigned t = 2u * (unsigned(cj) * unsigned(Q.nx) + unsigned(ci));
+    if (Q.kK) ld2(Q.kK + t, kk4[q]);
+    else kk4[q][0] = kk4[q][1] = Q.kK_c;
+    if constexpr (NC == 1) {
+      if (Q.kM) ld2(Q.kM + t, km4[q]);
+      else km4[q][0] = km4[q][1] = Q.kM_c;
+    }
+  }
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int e = 0; e < 6; ++e) {
+    int dci, dcj, o, loc;
+    p1_incidence(e, dci, dcj, o, loc);
+    const T kk = kk4[dci + 1 + 2 * (dcj + 1)][o], km = km4[dci + 1 + 2 * (dcj + 1)][o];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int L = 0; L < 3; ++L) {
+      if constexpr (NC == 1) st[0] = fma_t(km, Q.Mm[o][loc][L], st[0]);
+      if (L == loc) continue;
+      T* bk = st + st_block(dci + p1_off_a(o, L), dcj + p1_off_b(o, L)) * SB;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+      for (int i = 0; i < SB; ++i) {
+        bk[i] = fma_t(kk, Q.K[o][loc * NC + i / NC][L * NC + i % NC], bk[i]);
+        if constexpr (NC == 1) bk[i] = fma_t(km, Q.Mm[o][loc][L], bk[i]);
+      }
+    }
+  }
+  if (!P1Kern<T, NC>::near_clamped(Q.dir, a, b)) return;
+  const bool self = is_clamped(Q.dir, a, b);
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int k = 1; k < 7; ++k) {
+    if (!self && !is_clamped(Q.dir, a + st_da(k), b + st_db(k))) continue;
+    for (int i = 0; i < SB; ++i) {
+      st[i] -= st[k * SB + i];
+      st[k * SB + i] = T(0);
+    }
+  }
+  if (self)
+    for (int i = 0; i < SB; ++i) st[i] = i / NC == i % NC ? T(1) : T(0);
+}
+
 // A thread's node: what the two operator applications share.
 template <class T, int NC>
 struct LevelNode {
@@ -166,24 +247,31 @@ struct LevelNode {
   T st[StencilLayout<NC>::stride];
   T di[NC], bv[NC];
 
-  // row and inverse diagonal (zero outside the lattice)
-  TOPO_HD void load(const LevelSweep<T, NC>& L, int a_, int b_) {
+  TOPO_HD void place(const LevelSweep<T, NC>& L, int a_, int b_) {
     a = a_;
     b = b_;
     in = a >= 0 && a < L.NX && b >= 0 && b < L.NY;
-    const size_t n = in ? size_t(b) * L.NX + a : 0;
-    const bool interior = L.inner && a > 0 && b > 0 && a < L.NX - 1 && b < L.NY - 1;
-    load_row(interior ? L.inner : L.st + n * StencilLayout<NC>::stride, st);
-    for (int c = 0; c < NC; ++c) di[c] = L.dinv[NC * n + c];
+  }
+  // row and inverse diagonal (zero outside the lattice); Q: the row from its coefficients
+  TOPO_HD void load(const LevelSweep<T, NC>& L, const P1Params<T, NC>* Q = nullptr) {
+    const unsigned n = in ? unsigned(b) * unsigned(L.NX) + unsigned(a) : 0u;
+    load_node<T, NC>(L.dinv + NC * size_t(n), di);
+    if (Q) {
+      level_row_free<T, NC>(*Q, a, b, st);
+    } else {
+      const bool interior = L.inner && a > 0 && b > 0 && a < L.NX - 1 && b < L.NY - 1;
+      load_row(interior ? L.inner : L.st + size_t(n) * StencilLayout<NC>::stride, st);
+    }
     if (!in) {
       for (int i = 0; i < StencilLayout<NC>::stride; ++i) st[i] = T(0);
       for (int c = 0; c < NC; ++c) di[c] = T(0);
     }
     level_row<T, NC>(st);
   }
-  TOPO_HD size_t index(const LevelSweep<T, NC>& L) const { return size_t(b) * L.NX + a; }
+  TOPO_HD size_t index(const LevelSweep<T, NC>& L) const { return unsigned(b) * unsigned(L.NX) + unsigned(a); }
   TOPO_HD void load_b(const LevelSweep<T, NC>& L, const T* bg) {
-    for (int c = 0; c < NC; ++c) bv[c] = in ? bg[NC * index(L) + c] : T(0);
+    for (int c = 0; c < NC; ++c) bv[c] = T(0);
+    if (in) load_node<T, NC>(bg + NC * index(L), bv);
   }
 };
 
@@ -195,106 +283,143 @@ struct LevelPhases {
   struct Node : LevelNode<T, NC> {
     int p;              // position in the shared vectors
     T r[NC], x[NC], d[NC];
+    T cf[7];            // smoothing coefficients
   };
-  // the thread's node of a region of w x h nodes from lattice position (a0, b0)
+  // the thread's node of a region of w x h nodes from lattice position (a0, b0), and the
+  // coefficients of D steps (its row and vectors come with load, load_b and up_own)
+  template <int D>
   TOPO_HD static bool start(const L& P, int a0, int b0, int w, int h, int tid, Node& N) {
+    for (int k = 0; k < 2 * D - 1; ++k) N.cf[k] = P.cheb[k];
     if (tid >= w * h) return false;
-    N.load(P, a0 + tid % w, b0 + tid / w);
-    N.p = (tid / w + 1) * (w + 2) + tid % w + 1;
+    const int i = int(unsigned(tid) % unsigned(w)), j = int(unsigned(tid) / unsigned(w));
+    N.place(P, a0 + i, b0 + j);
+    N.p = (j + 1) * (w + 2) + i + 1;
     return true;
   }
-  // down: d0 = c0 Dinv b on the region and a ring around it
-  TOPO_HD static void down_first(const L& P, int a0, int b0, int w, int h, int tid, int nt, const T* b, T* s) {
-    const T c0 = P.cheb[0];
-    for (int i = tid; i < (w + 2) * (h + 2); i += nt) {
-      const int a = a0 - 1 + i % (w + 2), c = b0 - 1 + i / (w + 2);
-      const bool in = a >= 0 && a < P.NX && c >= 0 && c < P.NY;
-      const size_t g = in ? size_t(c) * P.NX + a : 0;
-      for (int k = 0; k < NC; ++k) s[NC * i + k] = in ? (c0 * P.dinv[NC * g + k]) * b[NC * g + k] : T(0);
+  // position i of the ring around the region, 0 <= i < ring_size: (column, row) of the shared vectors
+  TOPO_HD static int ring_size(int w, int h) { return 2 * (w + 2) + 2 * h; }
+  TOPO_HD static void ring_position(int i, int w, int h, int& u, int& v) {
+    if (i < 2 * (w + 2)) {
+      u = i < w + 2 ? i : i - (w + 2);
+      v = i < w + 2 ? 0 : h + 1;
+    } else {
+      u = (i & 1) ? w + 1 : 0;
+      v = ((i - 2 * (w + 2)) >> 1) + 1;
     }
   }
-  // r = b, x = d = d0 of the thread's node, after the barrier
-  TOPO_HD static void down_own(const T* s, Node& N) {
-    for (int c = 0; c < NC; ++c) {
-      N.r[c] = N.bv[c];
-      N.x[c] = N.d[c] = s[NC * N.p + c];
-    }
-  }
-  // up: x + P x_c on the region and a ring around it (zero outside the lattice)
-  TOPO_HD static void up_first(const L& P, int a0, int b0, int w, int h, int tid, int nt, const T* x, const T* xc,
-                               T* s) {
-    for (int i = tid; i < (w + 2) * (h + 2); i += nt) {
-      const int a = a0 - 1 + i % (w + 2), b = b0 - 1 + i / (w + 2);
-      const bool in = a >= 0 && a < P.NX && b >= 0 && b < P.NY;
-      if (!in) {
-        for (int c = 0; c < NC; ++c) s[NC * i + c] = T(0);
-        continue;
-      }
-      // the node's two coarse neighbours, or twice the coarse node it is
-      const size_t m0 = size_t(b >> 1) * P.NXc + (a >> 1), m1 = size_t((b + 1) >> 1) * P.NXc + ((a + 1) >> 1);
-      const bool free = !is_clamped(P.dirf, a, b);
-      const size_t g = size_t(b) * P.NX + a;
+  // down: d0 = c0 Dinv b, at the thread's node (on) and in the ring around the region
+  TOPO_HD static void down_first(const L& P, int a0, int b0, int w, int h, int tid, int nt, const T* b, T* s, bool on,
+                                 Node& N) {
+    const T c0 = N.cf[0];
+    if (on) {
       for (int c = 0; c < NC; ++c) {
-        const T v = m0 == m1 ? xc[NC * m0 + c] : T(0.5) * (xc[NC * m0 + c] + xc[NC * m1 + c]);
-        s[NC * i + c] = free ? x[NC * g + c] + v : x[NC * g + c];
+        N.r[c] = N.bv[c];
+        N.x[c] = N.d[c] = (c0 * N.di[c]) * N.bv[c];
       }
+      store_node<T, NC>(s + NC * N.p, N.d);
+    }
+    for (int i = tid; i < ring_size(w, h); i += nt) {
+      int u, v;
+      ring_position(i, w, h, u, v);
+      const int a = a0 - 1 + u, c = b0 - 1 + v;
+      T d[NC], bv[NC];
+      for (int k = 0; k < NC; ++k) d[k] = T(0);
+      if (a >= 0 && a < P.NX && c >= 0 && c < P.NY) {
+        const size_t g = unsigned(c) * unsigned(P.NX) + unsigned(a);
+        load_node<T, NC>(P.dinv + NC * g, d);
+        load_node<T, NC>(b + NC * g, bv);
+        for (int k = 0; k < NC; ++k) d[k] = (c0 * d[k]) * bv[k];
+      }
+      store_node<T, NC>(s + NC * (v * (w + 2) + u), d);
+    }
+  }
+  // (x + P x_c) at node (a, b), zero outside the lattice
+  TOPO_HD static void up_value(const L& P, int a, int b, const T* x, const T* xc, T (&v)[NC]) {
+    for (int c = 0; c < NC; ++c) v[c] = T(0);
+    if (a < 0 || a >= P.NX || b < 0 || b >= P.NY) return;
+    // the node's two coarse neighbours, or twice the coarse node it is
+    const unsigned m0 = unsigned(b >> 1) * unsigned(P.NXc) + unsigned(a >> 1),
+                   m1 = unsigned((b + 1) >> 1) * unsigned(P.NXc) + unsigned((a + 1) >> 1);
+    T y0[NC], y1[NC];
+    load_node<T, NC>(x + NC * size_t(unsigned(b) * unsigned(P.NX) + unsigned(a)), v);
+    load_node<T, NC>(xc + NC * size_t(m0), y0);
+    load_node<T, NC>(xc + NC * size_t(m1), y1);
+    const bool free = surely_free(P.dirf, a, b) || !is_clamped(P.dirf, a, b);
+    for (int c = 0; c < NC; ++c) {
+      const T y = m0 == m1 ? y0[c] : T(0.5) * (y0[c] + y1[c]);
+      v[c] = free ? v[c] + y : v[c];
+    }
+  }
+  // up: x + P x_c at the thread's node
+  TOPO_HD static void up_own(const L& P, const T* x, const T* xc, Node& N) { up_value(P, N.a, N.b, x, xc, N.x); }
+  // ... and in the ring around the region, to shared memory
+  TOPO_HD static void up_first(const L& P, int a0, int b0, int w, int h, int tid, int nt, const T* x, const T* xc, T* s,
+                               bool on, const Node& N) {
+    if (on) store_node<T, NC>(s + NC * N.p, N.x);
+    for (int i = tid; i < ring_size(w, h); i += nt) {
+      int u, v;
+      ring_position(i, w, h, u, v);
+      T y[NC];
+      up_value(P, a0 - 1 + u, b0 - 1 + v, x, xc, y);
+      store_node<T, NC>(s + NC * (v * (w + 2) + u), y);
     }
   }
   // up: r = b - A x, d0 = c0 Dinv r, x += d0
-  TOPO_HD static void up_residual(const L& P, int w, const T* sx, T* sd, Node& N) {
+  TOPO_HD static void up_residual(const L&, int w, const T* sx, T* sd, Node& N) {
     T t[NC];
     level_apply<T, NC>(N.st, sx, w + 2, N.p, t);
-    const T c0 = P.cheb[0];
+    const T c0 = N.cf[0];
     for (int c = 0; c < NC; ++c) {
       N.r[c] = N.bv[c] - t[c];
       N.d[c] = (c0 * N.di[c]) * N.r[c];
-      N.x[c] = sx[NC * N.p + c] + N.d[c];
-      sd[NC * N.p + c] = N.d[c];
+      N.x[c] += N.d[c];
     }
+    store_node<T, NC>(sd + NC * N.p, N.d);
   }
   // step k >= 1: r -= A d, d = c1 d + c2 Dinv r, x += d; the direction from s to sn
-  TOPO_HD static void step(const L& P, int k, int w, const T* s, T* sn, Node& N) {
+  TOPO_HD static void step(const L&, int k, int w, const T* s, T* sn, Node& N) {
     T t[NC];
     level_apply<T, NC>(N.st, s, w + 2, N.p, t);
-    const T c1 = P.cheb[2 * k - 1], c2 = P.cheb[2 * k];
+    const T c1 = N.cf[2 * k - 1], c2 = N.cf[2 * k];
     for (int c = 0; c < NC; ++c) {
       N.r[c] -= t[c];
       N.d[c] = level_direction(c1, N.d[c], c2, N.di[c], N.r[c]);
       N.x[c] += N.d[c];
-      sn[NC * N.p + c] = N.d[c];
     }
+    store_node<T, NC>(sn + NC * N.p, N.d);
   }
   // the last step: x alone, to sn (the residual b - A x reads it)
-  TOPO_HD static void last(const L& P, int k, int w, const T* s, T* sn, Node& N) {
+  TOPO_HD static void last(const L&, int k, int w, const T* s, T* sn, Node& N) {
     T t[NC];
     level_apply<T, NC>(N.st, s, w + 2, N.p, t);
-    const T c1 = P.cheb[2 * k - 1], c2 = P.cheb[2 * k];
-    for (int c = 0; c < NC; ++c) {
-      N.x[c] = level_last(N.x[c], c1, N.d[c], c2, N.di[c], N.r[c] - t[c]);
-      if (sn) sn[NC * N.p + c] = N.x[c];
-    }
+    const T c1 = N.cf[2 * k - 1], c2 = N.cf[2 * k];
+    for (int c = 0; c < NC; ++c) N.x[c] = level_last(N.x[c], c1, N.d[c], c2, N.di[c], N.r[c] - t[c]);
+    if (sn) store_node<T, NC>(sn + NC * N.p, N.x);
   }
   // down, at the end: r = b - A x (zero outside the lattice), to shared memory for the restriction
   TOPO_HD static void down_residual(int w, const T* s, T* sr, const Node& N) {
     T t[NC];
     level_apply<T, NC>(N.st, s, w + 2, N.p, t);
-    for (int c = 0; c < NC; ++c) sr[NC * N.p + c] = N.bv[c] - t[c];
+    for (int c = 0; c < NC; ++c) t[c] = N.bv[c] - t[c];
+    store_node<T, NC>(sr + NC * N.p, t);
   }
-  // stores the block's own nodes (ring: how far they lie inside the region)
-  TOPO_HD static void store(const L& P, int w, int ring, int tid, const Node& N, T* x) {
-    const int i = tid % w - ring, j = tid / w - ring;
+  // stores the block's own nodes, of a region that starts `ring` nodes before them at (a0, b0)
+  TOPO_HD static void store(const L& P, int a0, int b0, int ring, const Node& N, T* x) {
+    const int i = N.a - a0 - ring, j = N.b - b0 - ring;
     if (!N.in || i < 0 || i >= 2 * P.cx || j < 0 || j >= 2 * P.cy) return;
-    for (int c = 0; c < NC; ++c) x[NC * N.index(P) + c] = N.x[c];
+    store_node<T, NC>(x + NC * N.index(P), N.x);
   }
   // ring: the position of the block's first coarse node inside the region
-  TOPO_HD static void restrict_to(const L& P, int I0, int J0, int w, int ring, int tid, int nt, const T* sr, T* bc) {
-    for (int i = tid; i < P.cx * P.cy; i += nt) {
-      const int ic = i % P.cx, jc = i / P.cx, I = I0 + ic, J = J0 + jc;
+  TOPO_HD static void restrict_to(const L& P, int cx, int cy, int I0, int J0, int w, int ring, int tid, int nt,
+                                  const T* sr, T* bc) {
+    for (int i = tid; i < cx * cy; i += nt) {
+      const int ic = int(unsigned(i) % unsigned(cx)), jc = int(unsigned(i) / unsigned(cx)), I = I0 + ic, J = J0 + jc;
       if (I >= P.NXc || J >= P.NYc) continue;
       const int p = (2 * jc + ring + 1) * (w + 2) + 2 * ic + ring + 1;
       const bool zero = is_clamped(P.dirc, I, J);
-      for (int c = 0; c < NC; ++c)
-        bc[NC * (size_t(J) * P.NXc + I) + c] = zero ? T(0) : level_restrict<T, NC>(sr + NC * p + c, w + 2);
+      T y[NC];
+      for (int c = 0; c < NC; ++c) y[c] = zero ? T(0) : level_restrict<T, NC>(sr + NC * p + c, w + 2);
+      store_node<T, NC>(bc + NC * size_t(unsigned(J) * unsigned(P.NXc) + unsigned(I)), y);
     }
   }
 };
