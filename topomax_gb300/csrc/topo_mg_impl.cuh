@@ -84,13 +84,18 @@ __device__ __forceinline__ void p2m_exchange_up(P2Lane<T>& L, int lane) {
 __device__ inline void pcg_check_dev(PcgDev* dv, cudaGraphConditionalHandle h, int use_cond) {
   dv->it += 1;
   const double pq = dv->pq, rr = dv->rr, rzn = dv->rz_new;
-  dv->relres = sqrt(rr / dv->bb);
   int st = 1;
   if (!isfinite(pq) || !isfinite(rr) || !isfinite(rzn)) st = 4;
   else if (!(pq > 0.0) || !(dv->rz > 0.0)) st = 3;
   else if (rr <= dv->tol2) st = 0;
   else if (dv->it >= dv->maxit) st = 2;
-  dv->beta = (st == 1) ? rzn / dv->rz : 0.0;
+  // (a chain of FP64 divisions and a root takes this one thread over 1 us: only what is needed)
+  if (st == 1) {
+    dv->beta = rzn / dv->rz;
+  } else {
+    dv->beta = 0.0;
+    dv->relres = sqrt(rr / dv->bb);
+  }
   dv->rz = rzn;
   dv->status = st;
   if (use_cond) cudaGraphSetConditional(h, st == 1 ? 1u : 0u);
@@ -1056,6 +1061,14 @@ __global__ void k_pcg_r(T* __restrict__ r, const T* __restrict__ q, PcgDev* __re
   TOPO_PDL_ENTRY();
   __shared__ T alpha_s;
   __shared__ bool ok_s;
+  // the first values are on their way while thread 0 divides
+  const size_t step = size_t(gridDim.x) * blockDim.x;
+  size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  T ri = T(0), qi = T(0);
+  if (i < n) {
+    ri = r[i];
+    qi = q[i];
+  }
   if (threadIdx.x == 0) {
     const double pq = dv->pq;
     ok_s = (pq > 0.0) && isfinite(pq);
@@ -1065,7 +1078,8 @@ __global__ void k_pcg_r(T* __restrict__ r, const T* __restrict__ q, PcgDev* __re
   __syncthreads();
   if (!ok_s) return;
   const T alpha = alpha_s;
-  TOPO_GRID_STRIDE(i, n) r[i] -= alpha * q[i];
+  if (i < n) r[i] = ri - alpha * qi;
+  for (i += step; i < n; i += step) r[i] -= alpha * q[i];
 }
 
 // x += alpha p (x in T or FP64: the product of two FP32 numbers is exact in
@@ -1074,13 +1088,7 @@ template <class T, class TX>
 __global__ void k_pcg_p(T* __restrict__ p, const T* __restrict__ z, TX* __restrict__ x, const PcgDev* __restrict__ dv,
                         size_t n) {
   TOPO_PDL_ENTRY();
-  __shared__ T beta_s, alpha_s;
-  if (threadIdx.x == 0) {
-    beta_s = T(dv->beta);
-    alpha_s = T(dv->alpha);
-  }
-  __syncthreads();
-  const T beta = beta_s, alpha = alpha_s;
+  const T beta = T(dv->beta), alpha = T(dv->alpha);
   TOPO_GRID_STRIDE(i, n) {
     const T pi = p[i];
     x[i] += TX(alpha) * TX(pi);
