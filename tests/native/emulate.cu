@@ -52,12 +52,75 @@ static long lean_warps = 0;
 // Segment length of the emulated P2 marches (0: the kernel's one-wave rule).
 static int seg_override = 0;
 
+// The short form of the P2 kernel (k_p2_rows): one cell row per warp, the sums of a warp's top
+// node row handed to the next warp of its block.
+template <class T>
+void p2_rows_io(const P2Params<T>& P, const T* xi, P2Io<T> io) {
+  using M = P2March<T>;
+  M::prepare(io);
+  const bool operand = io.mode != kP2Diag;
+  T acc[2] = {T(0), T(0)};
+  for (int i0 = -1; i0 + 1 < P.nx + 1; i0 += P2M_OWN)
+    for (int J0 = 0; J0 < P.ny; J0 += P2R_ROWS) {
+      const bool lean = !IsDD<T>::value && M::lean_region(P, i0, J0 > 0 ? J0 - 1 : 0, J0 + P2R_ROWS);
+      T top[32][2][2] = {};
+      for (int w = 0; w <= P2R_ROWS; ++w) {
+        const int j = J0 - 1 + w;
+        std::vector<P2Lane<T>> L(32);
+        std::vector<typename M::Fin> F(32);
+        for (int l = 0; l < 32; ++l) M::begin(P, L[l], i0 + l, l == 31);
+        const bool row = j >= 0 && j < P.ny;
+        auto each = [&](auto&& f) {
+          for (int l = 0; l < 32; ++l)
+            if (row) f(l);
+        };
+        auto fin = [&](int l) { return w > 0 && l > 0 && L[l].i <= P.nx; };
+        each([&](int l) {
+          if (lean) {
+            M::template load_mass<true>(P, L[l].K, L[l].i, j, L[l].M);
+            M::template load<0, true>(P, io, xi, L[l], j);
+            if (fin(l)) M::template fin_load<true>(P, io, L[l], j, F[l]);
+          } else {
+            M::load_mass(P, L[l].K, L[l].i, j, L[l].M);
+            M::template load<0>(P, io, xi, L[l], j);
+            if (fin(l)) M::fin_load(P, io, L[l], j, F[l]);
+          }
+        });
+        for (int l = 0; l < 31; ++l) {
+          if (operand)
+            for (int r = 0; r <= 2; ++r)
+              for (int c = 0; c < 2; ++c) L[l].U[r][2][c] = L[l + 1].U[r][0][c];
+          for (int r = 0; r <= 1; ++r) L[l].X[r][1] = L[l + 1].X[r][0];
+        }
+        each([&](int l) {
+          if (lean) M::template compute<true>(P, L[l], j, io.mode);
+          else M::compute(P, L[l], j, io.mode);
+        });
+        for (int l = 31; l >= 1; --l)
+          for (int r = 0; r < 3; ++r)
+            for (int c = 0; c < 2; ++c) L[l].A[r][0][c] += L[l - 1].A[r][2][c];
+        for (int l = 0; l < 32; ++l) {
+          T mine[2][2];
+          for (int k = 0; k < 4; ++k) mine[k >> 1][k & 1] = L[l].A[2][k >> 1][k & 1];
+          if (row && fin(l)) {
+            if (j > 0)
+              for (int k = 0; k < 4; ++k) L[l].A[0][k >> 1][k & 1] += top[l][k >> 1][k & 1];
+            if (lean) M::template finish<true>(P, io, L[l], j, j == P.ny - 1 ? 3 : 2, F[l], acc);
+            else M::finish(P, io, L[l], j, j == P.ny - 1 ? 3 : 2, F[l], acc);
+          }
+          for (int k = 0; k < 4; ++k) top[l][k >> 1][k & 1] = mine[k >> 1][k & 1];
+        }
+      }
+    }
+}
+
 // Runs the column-march P2 kernel on the CPU: the 32 lanes of a warp execute
 // each phase in turn and the shuffles become copies between lane states.
 template <class T>
 void p2_run_io(const P2Params<T>& P, const T* xi, P2Io<T> io, int seg = 0) {
-  P2March<T>::prepare(io);
   lean_warps = 0;
+  if (seg_override == kRowsSegment) return p2_rows_io(P, xi, io);
+  P2March<T>::prepare(io);
   if (seg <= 0) seg = seg_override > 0 ? std::min(seg_override, P.ny) : p2_march_segment(P.nx, P.ny, 4, 5);
   const int nxw = (P.nx + 1 + P2M_OWN - 1) / P2M_OWN;
   const bool operand = io.mode != kP2Diag;

@@ -140,6 +140,23 @@ constexpr int p2_march_min_blocks() {
   return IsDD<T>::value ? 3 : sizeof(T) == 4 ? 4 : 2;
 }
 
+// the CG's reductions fused into a launch (P2Io::fuse)
+template <class T, int MODE>
+__device__ __forceinline__ void p2_reduce(const P2Io<T>& io, const T (&acc)[2]) {
+  if constexpr ((MODE == kP2Apply || MODE == kP2Post2) && !IsDD<T>::value) {
+    if (io.fuse == kFuseNone) return;
+    double tot[2];
+    if (!finish_reduction<2>(acc, io.partials, io.counter, tot)) return;
+    if (io.fuse == kFusePQ) {
+      io.pcg->pq = tot[0];
+    } else {
+      io.pcg->rr = tot[0];
+      io.pcg->rz_new = tot[1];
+      pcg_check_dev(io.pcg, cudaGraphConditionalHandle(io.cond), io.use_cond);
+    }
+  }
+}
+
 template <class T, int MODE>
 __global__ void __launch_bounds__(P2M_THREADS, p2_march_min_blocks<T>())
     k_p2_march(P2Params<T> P, const T* __restrict__ xi, P2Io<T> io, int seg) {
@@ -162,20 +179,63 @@ __global__ void __launch_bounds__(P2M_THREADS, p2_march_min_blocks<T>())
       p2_march_run<T, MODE, false>(P, xi, io, lane, js, je, acc);
     }
   }
-  if constexpr ((MODE == kP2Apply || MODE == kP2Post2) && !IsDD<T>::value) {
-    if (io.fuse != kFuseNone) {
-      double tot[2];
-      if (finish_reduction<2>(acc, io.partials, io.counter, tot)) {
-        if (io.fuse == kFusePQ) {
-          io.pcg->pq = tot[0];
-        } else {
-          io.pcg->rr = tot[0];
-          io.pcg->rz_new = tot[1];
-          pcg_check_dev(io.pcg, cudaGraphConditionalHandle(io.cond), io.use_cond);
-        }
-      }
-    }
+  p2_reduce<T, MODE>(io, acc);
+}
+
+// One cell row of the short form: warp 0 of a block takes the row below its own P2R_ROWS, for
+// what that row adds to their lowest node row; each warp hands its top node row's sums to the
+// next through shared memory.  top: 4 values per thread.
+template <class T, int MODE, bool LEAN>
+__device__ __forceinline__ void p2_rows_run(const P2Params<T>& P, const T* xi, P2Io<T>& io, int lane, int j, bool own,
+                                            T* top, T (&acc)[2]) {
+  P2Lane<T> L;
+  P2March<T>::begin(P, L, int(blockIdx.x) * P2M_OWN - 1 + lane, lane == 31);
+  const bool row = j >= 0 && j < P.ny;
+  const bool fin = own && row && lane > 0 && L.i <= P.nx;
+  if (io.early) {
+    P2March<T>::prepare(io);
+    if (row) P2March<T>::template load_mass<LEAN>(P, L.K, L.i, j, L.M);
   }
+  TOPO_PDL_WAIT();
+  TOPO_PDL_LAUNCH();
+  if (!io.early) {
+    P2March<T>::prepare(io);
+    if (row) P2March<T>::template load_mass<LEAN>(P, L.K, L.i, j, L.M);
+  }
+  typename P2March<T>::Fin F;
+  if (row) {  // (the whole warp)
+    P2March<T>::template load<0, LEAN>(P, io, xi, L, j);
+    if (MODE != kP2Apply && MODE != kP2Diag && fin) P2March<T>::template fin_load<LEAN>(P, io, L, j, F);
+    p2m_exchange_down<T, 0, MODE != kP2Diag>(L);
+    P2March<T>::template compute<LEAN>(P, L, j, MODE);
+    p2m_exchange_up<T>(L, lane);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) top[k * P2R_THREADS + threadIdx.x] = L.A[2][k >> 1][k & 1];
+  __syncthreads();
+  if (!fin) return;
+  if (j > 0)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) L.A[0][k >> 1][k & 1] += top[k * P2R_THREADS + threadIdx.x - 32];
+  P2March<T>::template finish<LEAN>(P, io, L, j, j == P.ny - 1 ? 3 : 2, F, acc);
+}
+
+// A march with segments of one row computes each row twice and, in FP64, is bound by the pipe that
+// a block's warps share: 160x80 has 480 warps' rows, five row steps per SM here against eight.
+template <class T, int MODE>
+__global__ void __launch_bounds__(P2R_THREADS, sizeof(T) == 4 ? 3 : 2)
+    k_p2_rows(P2Params<T> P, const T* xi, P2Io<T> io) {
+  __shared__ T top[4 * P2R_THREADS];
+  io.mode = MODE;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, J0 = blockIdx.y * P2R_ROWS, j = J0 - 1 + w;
+  T acc[2] = {T(0), T(0)};
+  // block-uniform
+  if (!IsDD<T>::value &&
+      P2March<T>::lean_region(P, int(blockIdx.x) * P2M_OWN - 1, J0 > 0 ? J0 - 1 : 0, J0 + P2R_ROWS))
+    p2_rows_run<T, MODE, true>(P, xi, io, lane, j, w > 0, top, acc);
+  else
+    p2_rows_run<T, MODE, false>(P, xi, io, lane, j, w > 0, top, acc);
+  p2_reduce<T, MODE>(io, acc);
 }
 
 // The column-march kernel of the large P1 levels (see P1March).
@@ -852,6 +912,23 @@ inline dim3 march_grid(int nx, int ny, int blocks_per_sm, int& seg, int family =
   return dim3((nx + 1 + P2M_OWN - 1) / P2M_OWN, (nseg + P2M_WARPS - 1) / P2M_WARPS);
 }
 
+// The grid of a P2 launch: its short form (seg = kRowsSegment) up to three blocks per SM (one wave
+// in FP32), else the march.  The rule looks at sizes only: the two forms add a node row's sums in a
+// different order, and which one runs must not depend on a timing.
+// Short form against the march of its best segment, us: 80x40 Apply 5.8 / 6.6, First 6.0 / 6.7,
+// Res 4.1 / 5.2; 320x160 (440 blocks) 7.5 / 8.1, 6.7 / 7.4, 4.9 / 6.0; 303x101 pair-of-FP32 13.6 /
+// 44.4; FP64 160x80 18.1 / 25.4, 22.0 / 29.4, 18.0 / 24.5; 1000x500 34.0 / 24.3, 34.0 / 26.4,
+// 17.4 / 16.6.
+inline bool p2_short_form(int nx, int ny) {
+  const long blocks = long((nx + 1 + P2M_OWN - 1) / P2M_OWN) * ((ny + P2R_ROWS - 1) / P2R_ROWS);
+  return blocks <= 3l * device_sms();
+}
+inline dim3 p2_grid(int nx, int ny, int blocks_per_sm, int& seg, int family = -1, int seg_force = 0) {
+  if (seg_force > 0 || !p2_short_form(nx, ny)) return march_grid(nx, ny, blocks_per_sm, seg, family, seg_force);
+  seg = kRowsSegment;
+  return dim3((nx + 1 + P2M_OWN - 1) / P2M_OWN, (ny + P2R_ROWS - 1) / P2R_ROWS);
+}
+
 // occupancy queries happen outside any stream capture
 template <class T>
 inline void prime_march_occupancy() {
@@ -912,13 +989,14 @@ inline int mode_vectors(int mode, bool p2, bool fused_rz) {
 template <class T, int MODE>
 inline void launch_p2_mode(const P2Params<T>& P, const T* xi, const P2Io<T>& io, cudaStream_t s, int seg_force = 0) {
   int seg = 0;
-  const dim3 g = march_grid(P.nx, P.ny, p2_march_bps<T, MODE>(), seg, march_family(true, sizeof(T), 2), seg_force);
+  const dim3 g = p2_grid(P.nx, P.ny, p2_march_bps<T, MODE>(), seg, march_family(true, sizeof(T), 2), seg_force);
   const double n = 2.0 * (2 * P.nx + 1) * (2 * P.ny + 1), nv = double(P.nx + 1) * (P.ny + 1);
   // the design (one value per vertex) plus, for First, the coarse correction (2 per vertex)
   const double bytes = (mode_vectors(MODE, true, io.fuse == kFuseRZ) * n + nv + (MODE == kP2First ? 2 * nv : 0)) *
                        sizeof(T);
   KClock kc(s, p2_family<T>(MODE), 0, bytes);
-  launch_pdl(k_p2_march<T, MODE>, g, P2M_THREADS, 0, s, P, xi, io, seg);
+  if (seg == kRowsSegment) launch_pdl(k_p2_rows<T, MODE>, g, P2R_THREADS, 0, s, P, xi, io);
+  else launch_pdl(k_p2_march<T, MODE>, g, P2M_THREADS, 0, s, P, xi, io, seg);
 }
 
 template <class T>
@@ -975,11 +1053,14 @@ inline void launch_p2_apply_dd(const P2Params<dd>& P, const double* x, double* y
   io.u = reinterpret_cast<const dd*>(x);
   io.y = reinterpret_cast<dd*>(y);
   int seg = 0;
-  const dim3 g = march_grid(P.nx, P.ny, p2_march_bps<dd, kP2Apply>(), seg);
+  const dim3 g = p2_grid(P.nx, P.ny, p2_march_bps<dd, kP2Apply>(), seg);
   // x read and y written in FP64, the mass matrices (12 pairs per cell)
   const double n = 2.0 * (2 * P.nx + 1) * (2 * P.ny + 1), nc = double(P.nx) * P.ny;
   KClock kc(s, "P2 march pair-of-FP32 Apply", 0, 2.0 * n * 8.0 + 12.0 * nc * 8.0);
-  launch_pdl(k_p2_march<dd, kP2Apply>, g, P2M_THREADS, 0, s, P, static_cast<const dd*>(nullptr), io, seg);
+  if (seg == kRowsSegment)
+    launch_pdl(k_p2_rows<dd, kP2Apply>, g, P2R_THREADS, 0, s, P, static_cast<const dd*>(nullptr), io);
+  else
+    launch_pdl(k_p2_march<dd, kP2Apply>, g, P2M_THREADS, 0, s, P, static_cast<const dd*>(nullptr), io, seg);
 }
 
 template <class T, int NC>
@@ -1684,6 +1765,7 @@ void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
     std::memset(&io, 0, sizeof(io));
     io.B = B;
     io.u = x;
+    io.early = 1;  // (a solve's launches all follow the set-up's last synchronisation)
     io.mode = kP2Pre;
     launch_p2_tile<T>(p2_, xi_, io, s);
     io.mode = kP2Res;
@@ -1817,6 +1899,7 @@ void MG<T>::tune_marches(cudaStream_t s) {
     if (l == tail_ && use_tail) break;  // the tail runs the rest
     if (l == cheb_coarse_ && cc_desc_) break;
     if (S.p2) {
+      if (p2_short_form(S.nx, S.ny)) continue;
       const size_t n = S.ndof();
       T *x = pcg_[8], *y = pcg_[9];
       cudaMemsetAsync(x, 0, n * sizeof(T), s);
@@ -1910,8 +1993,8 @@ void MG<T>::pcg_body(cudaStream_t s, cudaGraphConditionalHandle h, int use_cond)
   // both fused launches (operator and last post-smoothing) must fit the partial slots
   int seg = 0;
   const int fam = march_family(true, sizeof(T), 2);
-  const dim3 ga = march_grid(specs_[0].nx, specs_[0].ny, p2_march_bps<T, kP2Apply>(), seg, fam);
-  const dim3 gp = march_grid(specs_[0].nx, specs_[0].ny, p2_march_bps<T, kP2Post2>(), seg, fam);
+  const dim3 ga = p2_grid(specs_[0].nx, specs_[0].ny, p2_march_bps<T, kP2Apply>(), seg, fam);
+  const dim3 gp = p2_grid(specs_[0].nx, specs_[0].ny, p2_march_bps<T, kP2Post2>(), seg, fam);
   const size_t mblocks = std::max(size_t(ga.x) * ga.y, size_t(gp.x) * gp.y);
   if (specs_[0].p2 && mblocks * 2 <= size_t(red_->blocks) * 16) {
     // P2 level 0: p.q is reduced inside the operator launch, r.r / r.z and the
@@ -1922,6 +2005,7 @@ void MG<T>::pcg_body(cudaStream_t s, cudaGraphConditionalHandle h, int use_cond)
     io.u = p;
     io.y = q;
     io.fuse = kFusePQ;
+    io.early = 1;
     io.partials = red_->partials;
     io.counter = red_->counter;
     io.pcg = dev_;

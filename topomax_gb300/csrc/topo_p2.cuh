@@ -287,6 +287,11 @@ TOPO_HD void tri_diag(int o, const T (&xi)[3], const P2Params<T>& P, T (&d)[6][2
 constexpr int P2M_OWN = 31;                   // owned cell columns per warp
 constexpr int P2M_WARPS = 4;                  // warps per block, one row segment each
 constexpr int P2M_THREADS = 32 * P2M_WARPS;
+// The short form for grids that leave the chip idle: one cell row per warp, a block's warps on
+// consecutive rows, the first of them one row below the block's own (k_p2_rows).
+constexpr int P2R_ROWS = 4;
+constexpr int P2R_THREADS = 32 * (P2R_ROWS + 1);
+constexpr int kRowsSegment = -1;  // in place of a segment length
 
 // What one launch of the P2 kernel computes.
 enum P2Mode { kP2Apply = 0, kP2Diag = 1, kP2Pre = 2, kP2Res = 3, kP2First = 4, kP2Post2 = 5 };
@@ -316,6 +321,7 @@ struct P2Io {
   unsigned long long cond;  // graph conditional handle of the CG loop
   int use_cond;
   T cf[3];             // B.cheb[0..2], copied in by P2March::prepare (registers, not re-read)
+  int early;           // B.cheb and the mass matrices are from before the launch's predecessors
 };
 
 // Which of a lane's cells and nodes exist and which nodes are clamped.  A lane
