@@ -211,7 +211,8 @@ int64_t topo_kernel_clock_report(char* buf, int64_t len);
 
 /* Measurement hook (no counterpart in the reference): the tiles the march-kernel autotuner
  * chose in this process (cell rows per warp segment), as text, one line per kernel family and
- * grid: "family<TAB>nx<TAB>ny<TAB>segment<LF>", into buf when len is large enough.  Returns the
+ * grid: "family<TAB>nx<TAB>ny<TAB>segment<LF>", into buf when len is large enough.  P2 grids small
+ * enough for the short form (one cell row per warp) are not tuned and have no line.  Returns the
  * length needed including the terminating NUL. */
 int64_t topo_march_tiles_report(char* buf, int64_t len);
 
@@ -323,8 +324,10 @@ int topo_dem_objective_gradient_f32(topo_dem_ctx* ctx, const float* u, const flo
  * its two uses, W @ rho and W.T @ g (DEM_src/elasisity_problem.py:148, 162, 171). ------
  * W_ij = (radius - d_ij) / S_i for element points i, j (np.linspace(0, width, Nx) x
  * np.linspace(0, height, Ny), element i = iy*Nx + ix) within radius, S_i the row sum;
- * evaluated on the fly in FP64 with the reference's order of operations (bit-identical
- * to the scipy/sklearn product).  create computes the row sums (synchronises). */
+ * in FP64 with the reference's order of operations (bit-identical to the scipy/sklearn
+ * product): the distinct distances are tabulated and divided by an exact integer method, or
+ * evaluated per neighbour where a radius has too many of them.  create builds the table or
+ * the row sums (synchronises). */
 typedef struct topo_density_filter topo_density_filter;
 topo_density_filter* topo_density_filter_create(int Nx, int Ny, double width, double height, double radius,
                                                 int* status);
