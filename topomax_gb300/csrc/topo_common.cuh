@@ -29,6 +29,9 @@
 // grid has passed that point and overlaps its launch with this grid's drain.
 // A kernel that reads data no kernel of the chain writes may call TOPO_PDL_LAUNCH() first,
 // read them, and TOPO_PDL_WAIT() before it touches anything else.
+// What the chain writes (vectors, scalars) reaches such a kernel through pointers without
+// __restrict__: a load that the compiler takes to be from memory nobody writes may move above
+// the wait.  The qualifier is for what is fixed during a solve: tables and assembled rows.
 #if defined(__CUDA_ARCH__)
 #define TOPO_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
 #define TOPO_PDL_LAUNCH() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")

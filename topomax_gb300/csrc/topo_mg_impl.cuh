@@ -104,7 +104,7 @@ __device__ inline void pcg_check_dev(PcgDev* dv, cudaGraphConditionalHandle h, i
 // One warp's march over cell rows js .. je-1 (see P2March).  LEAN: the warp's
 // region passed P2March::lean_region, so the phases make no per-node tests.
 template <class T, int MODE, bool LEAN>
-__device__ __forceinline__ void p2_march_run(const P2Params<T>& P, const T* __restrict__ xi, const P2Io<T>& io,
+__device__ __forceinline__ void p2_march_run(const P2Params<T>& P, const T* xi, const P2Io<T>& io,
                                              int lane, int js, int je, T (&acc)[2]) {
   constexpr bool OPERAND = MODE != kP2Diag;
   P2Lane<T> L;
@@ -159,7 +159,7 @@ __device__ __forceinline__ void p2_reduce(const P2Io<T>& io, const T (&acc)[2]) 
 
 template <class T, int MODE>
 __global__ void __launch_bounds__(P2M_THREADS, p2_march_min_blocks<T>())
-    k_p2_march(P2Params<T> P, const T* __restrict__ xi, P2Io<T> io, int seg) {
+    k_p2_march(P2Params<T> P, const T* xi, P2Io<T> io, int seg) {
   TOPO_PDL_ENTRY();
   io.mode = MODE;  // compile-time mode: the per-node switches fold
   P2March<T>::prepare(io);
@@ -292,9 +292,7 @@ __global__ void __launch_bounds__(P2M_THREADS) k_p1_march(P1Params<T, NC> P, P1I
 
 // The sweeps of a stencil level (see topo_p1level.cuh).  The rows, inverse diagonals and
 // smoothing coefficients are fixed during a solve, so they are read before the wait for
-// the predecessor; the successor may start its own such reads at once.  What the
-// predecessor wrote comes through pointers without __restrict__: a load that the compiler
-// takes to be from memory nobody writes may move above the wait.
+// the predecessor; the successor may start its own such reads at once.
 //
 // Measured on design evaluations (us): the six launches per level and the earlier one-block
 // tail of 30 to 35 us took 8,490 at 80x40, 31,000 at 303x101 and 25,470 at 1000x500; sweeps
@@ -413,14 +411,14 @@ __global__ void __launch_bounds__(sweep_threads<ROWS, D>())
 }
 
 template <class T, int NC>
-__global__ void __launch_bounds__(kRowThreads_) k_prolong_add(Transfer X, const T* __restrict__ xc, T* __restrict__ xf) {
+__global__ void __launch_bounds__(kRowThreads_) k_prolong_add(Transfer X, const T* xc, T* xf) {
   TOPO_PDL_ENTRY();
   const int a = blockIdx.x * kRowThreads_ + threadIdx.x, b = blockIdx.y;
   if (a < X.NXf) TransferKern<T, NC>::node_prolong_add(a, b, X, xc, xf);
 }
 
 template <class T, int NC, class PP>
-__global__ void __launch_bounds__(kRowThreads) k_p1_apply(PP P, const T* __restrict__ u, T* __restrict__ y) {
+__global__ void __launch_bounds__(kRowThreads) k_p1_apply(PP P, const T* u, T* y) {
   TOPO_PDL_ENTRY();
   const int a = blockIdx.x * kRowThreads + threadIdx.x, b = blockIdx.y;
   if (a <= P.nx) p1_node_apply<T, NC>(a, b, P, u, y);
@@ -439,8 +437,7 @@ __global__ void __launch_bounds__(kRowThreads) k_p1_stencil(P1Params<T, NC> P, T
 }
 
 template <class T, int NC>
-__global__ void __launch_bounds__(kRowThreads) k_restrict(Transfer X, const T* __restrict__ rf, T* __restrict__ bc,
-                                                          const T* __restrict__ tf) {
+__global__ void __launch_bounds__(kRowThreads) k_restrict(Transfer X, const T* rf, T* bc, const T* tf) {
   TOPO_PDL_ENTRY();
   const int I = blockIdx.x * kRowThreads + threadIdx.x, J = blockIdx.y;
   if (I < X.NXc) TransferKern<T, NC>::node_restrict(I, J, X, rf, bc, tf);
@@ -1138,7 +1135,7 @@ inline LevelSweep<T, NC> level_sweep(const LevelSpec& S, const Transfer& X, cons
 // r -= alpha q with alpha = rz / pq; block 0 records the alpha it applied
 // (the solution update happens in k_pcg_p, which reads p anyway)
 template <class T>
-__global__ void k_pcg_r(T* __restrict__ r, const T* __restrict__ q, PcgDev* __restrict__ dv, size_t n) {
+__global__ void k_pcg_r(T* r, const T* q, PcgDev* dv, size_t n) {
   TOPO_PDL_ENTRY();
   __shared__ T alpha_s;
   __shared__ bool ok_s;
@@ -1166,14 +1163,14 @@ __global__ void k_pcg_r(T* __restrict__ r, const T* __restrict__ q, PcgDev* __re
 // x += alpha p (x in T or FP64: the product of two FP32 numbers is exact in
 // FP64), then p = z + beta p
 template <class T, class TX>
-__global__ void k_pcg_p(T* __restrict__ p, const T* __restrict__ z, TX* __restrict__ x, const PcgDev* __restrict__ dv,
-                        size_t n) {
+__global__ void k_pcg_p(T* p, const T* z, TX* x, const PcgDev* dv, size_t n) {
   TOPO_PDL_ENTRY();
   const T beta = T(dv->beta), alpha = T(dv->alpha);
   TOPO_GRID_STRIDE(i, n) {
-    const T pi = p[i];
-    x[i] += TX(alpha) * TX(pi);
-    p[i] = z[i] + beta * pi;
+    const T pi = p[i], zi = z[i];
+    const TX xi = x[i];
+    x[i] = xi + TX(alpha) * TX(pi);
+    p[i] = zi + beta * pi;
   }
 }
 

@@ -161,8 +161,7 @@ __device__ bool finish_reduction(const R (&v)[NV], double* partials, unsigned* c
 
 // out[0] = sum a_i b_i (or sum a_i^2 when b == nullptr)
 template <class TA, class TB>
-__global__ void k_dot(const TA* __restrict__ a, const TB* __restrict__ b, size_t n, double* partials,
-                      unsigned* counter, double* out) { TOPO_PDL_ENTRY();
+__global__ void k_dot(const TA* a, const TB* b, size_t n, double* partials, unsigned* counter, double* out) { TOPO_PDL_ENTRY();
   // per-thread partial in the input precision (a handful of terms), then FP64
   using Acc = typename std::conditional<sizeof(TA) == 4 && sizeof(TB) == 4, float, double>::type;
   Acc acc = Acc(0);
@@ -174,8 +173,7 @@ __global__ void k_dot(const TA* __restrict__ a, const TB* __restrict__ b, size_t
 
 // two dots at once: out[0] = a.b, out[1] = c.d
 template <class T>
-__global__ void k_dot2(const T* __restrict__ a, const T* __restrict__ b, const T* __restrict__ c,
-                       const T* __restrict__ d, size_t n, double* partials, unsigned* counter,
+__global__ void k_dot2(const T* a, const T* b, const T* c, const T* d, size_t n, double* partials, unsigned* counter,
                        double* out) { TOPO_PDL_ENTRY();
   // per-thread partials in the input precision (a handful of terms), then FP64
   T p0 = T(0), p1 = T(0);
