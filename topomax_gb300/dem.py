@@ -333,6 +333,7 @@ class _DemContext:
         self.mesh = mesh
         self.detJ = detJ
         self.mask_version = None  # the version of the Dirichlet mask on the device
+        self.mask_uploads = 0
 
     def check(self, rc: int) -> None:
         if rc == _capi.TOPO_OK:
@@ -443,12 +444,15 @@ class _EnergyFn(torch.autograd.Function):
     """psi(u, rho) with hand-written backward kernels (d psi/du, d psi/d rho)."""
 
     @staticmethod
-    def forward(ctx, u, rho, dem, masked):
+    def forward(ctx, u, rho, dem, enforcer):
         uu, rr = _as_u(u, dem.mesh), _as_density(rho, dem.mesh)
         out = uu.new_empty(())
-        dem.check(dem.lib.topo_dem_energy_f32(dem.ptr, _ptr(uu), _ptr(rr), int(masked), _ptr(out), _stream()))
+        if enforcer is not None:
+            enforcer._install(dem)
+        dem.check(dem.lib.topo_dem_energy_f32(dem.ptr, _ptr(uu), _ptr(rr), int(enforcer is not None), _ptr(out),
+                                              _stream()))
         ctx.save_for_backward(uu, rr)
-        ctx.dem, ctx.masked = dem, masked
+        ctx.dem, ctx.enforcer, ctx.mask_uploads = dem, enforcer, dem.mask_uploads
         ctx.rho_shape = rho.shape
         return out
 
@@ -459,7 +463,9 @@ class _EnergyFn(torch.autograd.Function):
         scale = _as_f32(grad)
         du = torch.empty_like(uu) if ctx.needs_input_grad[0] else None
         dr = torch.empty_like(rr) if ctx.needs_input_grad[1] else None
-        dem.check(dem.lib.topo_dem_energy_backward(dem.ptr, _ptr(uu), _ptr(rr), int(ctx.masked), _ptr(scale),
+        if ctx.enforcer is not None and dem.mask_uploads != ctx.mask_uploads:
+            ctx.enforcer._install(dem)  # another evaluation has put its mask in place since
+        dem.check(dem.lib.topo_dem_energy_backward(dem.ptr, _ptr(uu), _ptr(rr), int(ctx.enforcer is not None), _ptr(scale),
                                                    _ptr(du) if du is not None else None,
                                                    _ptr(dr) if dr is not None else None, _stream()))
         if dr is not None and dr.shape != ctx.rho_shape:
@@ -503,13 +509,12 @@ class StrainEnergy:
     def calculate_energy(self, u: torch.Tensor, shape, density: torch.Tensor) -> torch.Tensor:
         """psi(u; rho) = 1/2 int r(rho) sigma:eps dx - int f.u dx - int t.u ds."""
         self._check_shape(shape)
-        return _EnergyFn.apply(u, density, self._dem, False)
+        return _EnergyFn.apply(u, density, self._dem, None)
 
     def calculate_energy_enforced(self, u_hat: torch.Tensor, enforcer: "ElasticityEnforcer",
                                   density: torch.Tensor) -> torch.Tensor:
         """calculate_energy(enforcer(u_hat), ...) in one pass (the mask applied while loading)."""
-        enforcer._install(self._dem)
-        return _EnergyFn.apply(u_hat, density, self._dem, True)
+        return _EnergyFn.apply(u_hat, density, self._dem, enforcer)
 
     def calculate_objective_and_gradient(self, u: torch.Tensor, shape, density: torch.Tensor):
         """(sum r(rho) SE detJ, -r'(rho) SE detJ) as float32 tensors (gradient shaped like density)."""
@@ -561,6 +566,7 @@ class ElasticityEnforcer:
         # the upload waits for the device: once per mask and context, not per evaluation
         if self._mask_version is None or dem.mask_version != self._mask_version:
             dem.mask_version = None
+            dem.mask_uploads += 1
             dem.check(dem.lib.topo_dem_set_mask(dem.ptr, self._mask.ctypes.data))
             dem.mask_version = self._mask_version
         self._dem = dem
@@ -572,8 +578,8 @@ class ElasticityEnforcer:
 class _EnforceFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, u_hat, enf):
-        if enf._dem is None:
-            enf._install(_DemContext(enf.mesh, 1.0, 0.3))
+        # the context may belong to an energy whose last evaluation used another mask
+        enf._install(enf._dem or _DemContext(enf.mesh, 1.0, 0.3))
         uh = _as_u(u_hat, enf.mesh)
         out = torch.empty_like(uh)
         enf._dem.check(enf._dem.lib.topo_dem_enforce(enf._dem.ptr, _ptr(uh), _ptr(out), _stream()))
