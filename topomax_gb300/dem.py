@@ -527,7 +527,18 @@ class StrainEnergy:
         return obj, (grad if grad.shape == density.shape else grad.reshape(density.shape))
 
 
-_mask_versions = itertools.count(1)  # one per mask: contexts tell by it which they hold
+class _MaskVersion:
+    """Number of a mask's contents: contexts tell by it which they hold.  None where somebody
+    else can write to the array; it is then uploaded for every use.  Enforcers that share the
+    array (copy.copy) share this object too; a deep or unpickled copy gets a number of its own."""
+
+    _numbers = itertools.count(1)
+
+    def __init__(self, private: bool = True):
+        self.number = next(self._numbers) if private else None
+
+    def __reduce__(self):
+        return _MaskVersion, (self.number is not None,)
 
 
 class ElasticityEnforcer:
@@ -551,24 +562,34 @@ class ElasticityEnforcer:
             else:
                 raise ValueError(f"Unknown side: '{side}'")
         self._mask = np.ascontiguousarray(z.astype(np.float32))
-        self._mask_version = next(_mask_versions)
         self.zero_enforcer = torch.from_numpy(self._mask).to(device or "cuda")
+        # (on the CPU the tensor is the array)
+        self._mask_version = _MaskVersion(private=self.zero_enforcer.device.type != "cpu")
         self._dem = None
 
     @property
     def mask_host(self) -> np.ndarray:
         """The mask's host array.  Whoever takes it may write to it: from then on it is
-        uploaded for every use."""
-        self._mask_version = None
+        uploaded for every use.  Another array may take its place."""
+        self._mask_version.number = None
         return self._mask
+
+    @mask_host.setter
+    def mask_host(self, values):
+        values = np.ascontiguousarray(values, dtype=np.float32)
+        if values.size < self._mask.size:
+            raise ValueError(f"the mask has {self._mask.size} values, got {values.size}")
+        self._mask = values
+        self._mask_version = _MaskVersion(private=False)
 
     def _install(self, dem: _DemContext) -> None:
         # the upload waits for the device: once per mask and context, not per evaluation
-        if self._mask_version is None or dem.mask_version != self._mask_version:
+        number = self._mask_version.number
+        if number is None or dem.mask_version != number:
             dem.mask_version = None
             dem.mask_uploads += 1
             dem.check(dem.lib.topo_dem_set_mask(dem.ptr, self._mask.ctypes.data))
-            dem.mask_version = self._mask_version
+            dem.mask_version = number
         self._dem = dem
 
     def __call__(self, u: torch.Tensor) -> torch.Tensor:
