@@ -31,3 +31,16 @@ def test_an_enforcer_applies_its_own_mask():
         energy.calculate_energy_enforced(u, enf, rho)
     for enf in (left, top, left):
         assert torch.equal(enf(u), u * torch.from_numpy(enf._mask).cuda())
+
+
+def test_a_new_mask_waits_for_queued_evaluations():
+    """On a stream that does not wait for the default stream's copies."""
+    import torch
+    _, energy, left, top, u, rho = _setup(40, 33)
+    want = [energy.calculate_energy_enforced(u, e, rho).item() for e in (left, top)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda._sleep(20_000_000)  # some 10 ms
+        got = [energy.calculate_energy_enforced(u, e, rho) for e in (left, top, left)]
+    torch.cuda.synchronize()
+    assert [g.item() for g in got] == [want[0], want[1], want[0]]

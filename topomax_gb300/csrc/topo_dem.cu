@@ -327,6 +327,8 @@ int upload(topo_dem_ctx* C, float*& dst, const float* host) {
     return C->cuda_check("clear");
   }
   if (!dst && cudaMalloc(&dst, n * sizeof(float)) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "out of device memory");
+  // evaluations still queued read the old values; the copy below does not wait for non-blocking streams
+  if (cudaDeviceSynchronize() != cudaSuccess) return C->cuda_check("upload");
   if (cudaMemcpy(dst, host, n * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
       settle_setup_stream() != cudaSuccess)
     return C->fail(TOPO_ERR_CUDA, "copy failed");
