@@ -695,9 +695,25 @@ int fgmres_ir(topo_ctx* C, MG<float>& mg, Apply64 apply64, const double* b, doub
                  rtol, st.relres, st.iterations);
 }
 
+// One outer iteration of the refinement on s: right-hand side, inner FP32 solve (solve), its FP64
+// operator, Gram-Schmidt and test.
+template <class Apply64, class Solve>
+void refinement_step(topo_ctx* C, MG<float>& mg, Apply64 apply64, size_t n, Fgmres& W, Solve solve,
+                     cudaGraphConditionalHandle cond, int use_cond, cudaStream_t s) {
+  const int gv = C->grid(n), gd = C->red.spread(n);
+  k_refine_rhs<<<gv, kVecThreads, 0, s>>>(W.V, n, W.K, mg.scratch0(5), mg.device_scalars());
+  solve();
+  k_refine_direction<<<gv, kVecThreads, 0, s>>>(mg.solution64(), W.Z, n, W.K, mg.device_scalars());
+  apply64(mg.solution64(), W.t, s);
+  krylov_column(KrylovSpace{W.V, W.t, W.Z, nullptr, n, 0, Fgmres::m, W.dots, W.counters, C->red.partials,
+                            C->red.counter, W.K},
+                gd, gv, cond, use_cond, s);
+}
+constexpr int kRefinementLaunches = 8;  // of a step, besides the inner solve's
+
 // Records one restart cycle of the refinement into W.graph: a WHILE node whose body is an outer
-// iteration -- inner FP32 solve (a WHILE node of its own), FP64 operator, Gram-Schmidt and
-// test.  apply64 must read and write fixed device addresses only.
+// iteration, its inner solve a WHILE node of its own.  apply64 must read and write fixed
+// device addresses only.
 template <class Apply64>
 bool record_refinement(topo_ctx* C, MG<float>& mg, Apply64 apply64, size_t n, Fgmres& W) {
   std::lock_guard<std::recursive_mutex> lock(device_lock());
@@ -720,17 +736,11 @@ bool record_refinement(topo_ctx* C, MG<float>& mg, Apply64 apply64, size_t n, Fg
   cudaGraph_t body = ok ? cp.conditional.phGraph_out[0] : nullptr;
   if (ok) ok = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) == cudaSuccess;
   if (ok) {
-    const int gv = C->grid(n), gd = C->red.spread(n);
-    k_refine_rhs<<<gv, kVecThreads, 0, s>>>(W.V, n, W.K, mg.scratch0(5), mg.device_scalars());
+    bool rec = false;
     long long l1 = 0, l2 = 0;
-    const bool rec = mg.record_solve(false, s, sb, l1, l2);
-    W.outer_nodes = l1 - l0 + 9;
+    refinement_step(C, mg, apply64, n, W, [&] { rec = mg.record_solve(false, s, sb, l1, l2); }, h, 1, s);
+    W.outer_nodes = l1 - l0 + 1 + kRefinementLaunches;  // 1: the inner solve's start test
     W.inner_nodes = l2 - l1;
-    k_refine_direction<<<gv, kVecThreads, 0, s>>>(mg.solution64(), W.Z, n, W.K, mg.device_scalars());
-    apply64(mg.solution64(), W.t, s);
-    krylov_column(KrylovSpace{W.V, W.t, W.Z, nullptr, n, 0, Fgmres::m, W.dots, W.counters, C->red.partials,
-                              C->red.counter, W.K},
-                  gd, gv, h, 1, s);
     ok = cudaStreamEndCapture(s, &body) == cudaSuccess && rec;
   }
   if (ok) ok = cudaGraphInstantiate(&W.graph, g, 0) == cudaSuccess;
@@ -744,35 +754,60 @@ bool record_refinement(topo_ctx* C, MG<float>& mg, Apply64 apply64, size_t n, Fg
   return ok;
 }
 
+// Runs the cycle set up in W.K from the host: the same kernels over the same grids, so the same
+// bits, with a round trip per iteration.  Stops early at the context's iteration limit.
+// Leaves the scalars in W.host.
+template <class Apply64>
+bool refinement_cycle(topo_ctx* C, MG<float>& mg, Apply64 apply64, size_t n, Fgmres& W, int iterations,
+                      cudaStream_t s) {
+  for (;;) {
+    bool ok = true;
+    refinement_step(C, mg, apply64, n, W, [&] { ok = mg.solve_from_host(false, s); }, 0, 0, s);
+    C->launches += kRefinementLaunches;
+    const PcgDev in = mg.host_scalars();
+    const int before = W.host->inner;
+    cudaMemcpyAsync(W.host, W.K, offsetof(KrylovDev, res) + sizeof(double), cudaMemcpyDeviceToHost, s);
+    if (!ok || cudaStreamSynchronize(s) != cudaSuccess) return false;
+    if (C->trace_solves)
+      std::fprintf(stderr, "[topo solve]   inner %d: tol %.1e, %d iterations, status %d, residual then %.3e\n",
+                   W.host->j - 1, std::sqrt(in.tol2 / in.bb), W.host->inner - before, in.status, W.host->res);
+    if (W.host->status != 1) return true;
+    if (C->iter_limit > 0 && iterations + W.host->inner >= C->iter_limit) return true;
+  }
+}
+
 // fgmres_ir with the outer iterations on the device as well: two host round trips a restart cycle
 // instead of five an outer iteration (12 to 14 us each).  Loop from the host against this: state
 // solve 80x40 5.34 to 4.61 ms per evaluation, 303x101 13.28 to 12.57, 1000x500 16.09 to 15.65,
-// 2000x1000 38.4 to 38.0; filter 1000x500 1.37 to 1.28.  Returns 1, with x the guess or an
-// improved iterate, where fgmres_ir has to take over: no graphs, a recording that failed, or an
-// operator that is indefinite in FP32 (its inner solves are MINRES, driven by the host).
+// 2000x1000 38.4 to 38.0; filter 1000x500 1.37 to 1.28.  Without graphs (TOPO_GRAPHS=0, a recording
+// that another thread's work spoiled), under an iteration limit and when traced, the host launches
+// the same kernels.  Returns 1, with x the guess or an improved iterate, where fgmres_ir has
+// to take over: an operator that is indefinite in FP32 (its inner solves are MINRES).
 template <class Apply64>
 int fgmres_device(topo_ctx* C, MG<float>& mg, Apply64 apply64, const void* op, size_t op_bytes, const double* b,
                   double* x, bool warm, size_t n, double rtol, Fgmres& W, int maxit, double inner_floor,
                   SolveStats& st, cudaStream_t s) {
   st = SolveStats{};
-  if (!mg.use_graphs || !W.host || C->iter_limit > 0 || C->trace_solves || C->verify_residual) return 1;
+  if (!W.host) return 1;
   const int g = C->grid(n);
   const unsigned char* key = static_cast<const unsigned char*>(op);
   if (W.graph && (W.epoch != mg.epoch() || W.op.size() != op_bytes || !std::equal(key, key + op_bytes, W.op.begin()))) {
     cudaGraphExecDestroy(W.graph);
     W.graph = nullptr;
   }
-  if (!W.graph) {
+  const bool wanted = mg.use_graphs && C->iter_limit == 0 && !C->trace_solves;
+  if (wanted && !W.graph) {
     // the recording streams must not see work still queued on s
     if (cudaStreamSynchronize(s) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "refinement: CUDA error");
-    if (!record_refinement(C, mg, apply64, n, W)) {
+    if (record_refinement(C, mg, apply64, n, W)) {
+      W.epoch = mg.epoch();
+      W.op.assign(key, key + op_bytes);
+    } else {  // this solve from the host, the next one records again
       cudaGetLastError();
       ++mg.capture_failures;
-      return 1;
     }
-    W.epoch = mg.epoch();
-    W.op.assign(key, key + op_bytes);
   }
+  const bool graph = wanted && W.graph;
   if (!warm) k_fill<double><<<g, kVecThreads, 0, s>>>(x, 0.0, n);
   const double bn = std::sqrt(C->dot64(b, b, n, s));
   if (!std::isfinite(bn)) return C->fail(TOPO_ERR_NAN, "non-finite right-hand side");
@@ -791,6 +826,9 @@ int fgmres_device(topo_ctx* C, MG<float>& mg, Apply64 apply64, const void* op, s
       beta = std::sqrt(C->dot64(W.V, W.V, n, s));
     }
     st.relres = beta / bn;
+    if (C->trace_solves)
+      std::fprintf(stderr, "[topo solve] refinement cycle %d: |r|/|b| %.3e after %d inner iterations\n", cycle, st.relres,
+                   st.iterations);
     if (!std::isfinite(beta)) return C->fail(TOPO_ERR_NAN, "non-finite residual");
     if (beta <= rtol * bn) return TOPO_OK;
     if (cycle > 0 && beta > 0.9 * prev) break;  // stagnation at the FP64 residual floor
@@ -798,21 +836,27 @@ int fgmres_device(topo_ctx* C, MG<float>& mg, Apply64 apply64, const void* op, s
     k_scaled_copy<<<g, kVecThreads, 0, s>>>(W.V, zero ? b : W.V, 1.0 / beta, n);
     k_krylov_start<<<1, 1, 0, s>>>(W.K, beta, 0.5 * rtol * bn, 0, kMaxOuter * Fgmres::m, 0.3 * rtol * bn, inner_floor,
                                    maxit);
-    if (cudaGraphLaunch(W.graph, s) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "refinement: graph launch failed");
-    cudaMemcpyAsync(W.host, W.K, offsetof(KrylovDev, res) + sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "refinement: CUDA error");
+    W.host->inner = 0;
+    if (graph) {
+      if (cudaGraphLaunch(W.graph, s) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "refinement: graph launch failed");
+      cudaMemcpyAsync(W.host, W.K, offsetof(KrylovDev, res) + sizeof(double), cudaMemcpyDeviceToHost, s);
+      if (cudaStreamSynchronize(s) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "refinement: CUDA error");
+      mg.launches += W.host->j * W.outer_nodes + W.host->inner * W.inner_nodes;
+    } else if (!refinement_cycle(C, mg, apply64, n, W, st.iterations, s)) {
+      return C->fail(TOPO_ERR_CUDA, "refinement: CUDA error");
+    }
     const KrylovDev& K = *W.host;
     st.iterations += K.inner;
     st.outer += K.j;
-    mg.launches += K.j * W.outer_nodes + K.inner * W.inner_nodes;
     if (K.status == 4) return C->fail(TOPO_ERR_NAN, "non-finite value in the FP32 inner solve or its Krylov vector");
     k_krylov_backsolve<<<1, 32, 0, s>>>(W.K);
     k_krylov_update<<<g, kVecThreads, 0, s>>>(x, W.Z, n, W.K);
     if (K.status == 3) return 1;
-    if (K.res <= 0.5 * rtol * bn) {  // (see fgmres_ir)
+    if (K.res <= 0.5 * rtol * bn && !C->verify_residual) {  // (see fgmres_ir)
       st.relres = K.res / bn;
       return TOPO_OK;
     }
+    if (C->iter_limit > 0 && st.iterations >= C->iter_limit) break;
   }
   apply64(x, W.t, s);
   k_sub<double><<<g, kVecThreads, 0, s>>>(W.V, b, W.t, n);
@@ -822,8 +866,8 @@ int fgmres_device(topo_ctx* C, MG<float>& mg, Apply64 apply64, const void* op, s
                  rtol, st.relres, st.iterations);
 }
 
-// The refinement: on the device where that can be, else from the host.  op: the bytes that
-// determine apply64's launches, besides mg's own parameters.
+// The refinement, and where the operator proves indefinite in FP32 the form with MINRES.  op: the
+// bytes that determine apply64's launches, besides mg's own parameters.
 template <class Apply64>
 int refine(topo_ctx* C, MG<float>& mg, Apply64 apply64, const void* op, size_t op_bytes, const double* b, double* x,
            bool warm, size_t n, double rtol, Fgmres& W, int maxit, double inner_floor, SolveStats& st, cudaStream_t s) {

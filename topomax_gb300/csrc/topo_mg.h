@@ -179,6 +179,9 @@ class MG {
   // result in solution64(), status and iterations in device_scalars().  epoch() changes when
   // a recording is no longer valid.
   bool record_solve(bool warm, cudaStream_t s, cudaStream_t sb, long long& l1, long long& l2);
+  // the same from the host; false: a CUDA error.  The scalars come back in host_scalars()
+  bool solve_from_host(bool warm, cudaStream_t s);
+  const PcgDev& host_scalars() const { return *hdev_; }
   PcgDev* device_scalars() { return dev_; }
   const double* solution64() const { return xacc_; }
   cudaStream_t recording_stream(int k) const { return cap_[k]; }

@@ -2119,6 +2119,20 @@ int MG<T>::capture_pcg(bool warm) {
   return 0;
 }
 
+// The recorded solve's kernels launched one by one (a round trip per iteration).
+template <class T>
+bool MG<T>::solve_from_host(bool warm, cudaStream_t s) {
+  pcg_prologue(warm, s);
+  k_pcg_start<<<1, 1, 0, s>>>(dev_, 0, 0);
+  ++launches;
+  for (;;) {
+    cudaMemcpyAsync(hdev_, dev_, sizeof(PcgDev), cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) return false;
+    if (hdev_->status != 1) return true;
+    pcg_body(s, 0, 0);
+  }
+}
+
 // Runs the captured solve: inputs are copied into the graph's fixed buffers,
 // rtol^2 and the iteration cap are written to the device scalars the start
 // kernel reads, and the result and the scalars come back after one sync.
@@ -2162,16 +2176,7 @@ int MG<T>::graph_pcg(const T* b, T* x, double* x64, bool warm, double rtol, int 
     cudaGraphLaunch(G.exec, s);
     launches += G.prologue_nodes;
   } else {
-    // host-driven loop over the same kernels (one sync per iteration)
-    pcg_prologue(warm, s);
-    k_pcg_start<<<1, 1, 0, s>>>(dev_, 0, 0);
-    ++launches;
-    for (;;) {
-      cudaMemcpyAsync(&hdev_->status, &dev_->status, sizeof(int), cudaMemcpyDeviceToHost, s);
-      if (cudaStreamSynchronize(s) != cudaSuccess) return -5;
-      if (hdev_->status != 1) break;
-      pcg_body(s, 0, 0);
-    }
+    if (!solve_from_host(warm, s)) return -5;
   }
   if (x64) cudaMemcpyAsync(x64, xacc_, n * sizeof(double), cudaMemcpyDeviceToDevice, s);
   else cudaMemcpyAsync(x, xi, n * sizeof(T), cudaMemcpyDeviceToDevice, s);
