@@ -11,12 +11,12 @@
 // preconditioned with the block-diagonal
 //   diag( P1-iso-P2 V-cycles of K + alpha M on the (2nx)x(2ny) lattice, one per component,
 //         lumped-mass inverse + V-cycle of the 1/alpha-weighted P1 Laplacian )
-// (a variable-coefficient Cahouet-Chabard Schur-complement approximation).  The Krylov basis,
-// directions, operator and Gram-Schmidt are FP64; the V-cycles run in FP32, both velocity
-// components in one batch, the pressure's beside them: flexible GMRES keeps A Z = V H in FP64
-// for whatever directions it is given, and this GPU issues FP64 at 1/64 of its FP32 rate.  One
-// restart cycle is one CUDA graph whose WHILE body is an iteration; the Givens rotations and
-// the stopping test run on the device.
+// (a variable-coefficient Cahouet-Chabard Schur-complement approximation).  Everything is FP64;
+// the V-cycles take both velocity components in one batch, the pressure's run beside them.
+// (V-cycles in FP32 gave the same iterations and errors at 0.65 to 0.75 of the time, but the entry
+// points promise FP64 and have no precision for the caller to choose.)  One restart cycle is one
+// CUDA graph whose WHILE body is an iteration; the Givens rotations and the stopping test
+// run on the device.
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
@@ -34,7 +34,6 @@
 #include "topo_setup.h"
 
 namespace topo {
-extern template class MG<float>;
 extern template class MG<double>;
 }  // namespace topo
 
@@ -243,10 +242,10 @@ __global__ void k_fluid_center(const double* x, double* y, size_t n, const doubl
 // ---------------------------------------------------------------------------
 // one flexible-GMRES iteration
 // ---------------------------------------------------------------------------
-// FP32 right-hand sides of the preconditioner: the planar velocity components of v_j (zero on
+// Right-hand sides of the preconditioner: the planar velocity components of v_j (zero on
 // the boundary) and its pressure less the mean
 __global__ void k_fluid_split(int NX, int NY, const double* V, size_t n, size_t nv, const KrylovDev* K,
-                              float* c, float* pt) {
+                              double* c, double* pt) {
   TOPO_PDL_ENTRY();
   const size_t n2 = size_t(NX) * NY;
   const double* v = V + size_t(K->j) * n;
@@ -254,17 +253,17 @@ __global__ void k_fluid_split(int NX, int NY, const double* V, size_t n, size_t 
   TOPO_GRID_STRIDE(i, n2 + nv) {
     if (i < n2) {
       const bool bd = fluid_boundary_node(int(i % NX), int(i / NX), NX, NY);
-      c[i] = bd ? 0.0f : float(v[2 * i]);
-      c[n2 + i] = bd ? 0.0f : float(v[2 * i + 1]);
+      c[i] = bd ? 0.0 : v[2 * i];
+      c[n2 + i] = bd ? 0.0 : v[2 * i + 1];
     } else {
-      pt[i - n2] = float(v[n2 + i] - pm);  // (pressure entry k at 2 n2 + k = n2 + i)
+      pt[i - n2] = v[n2 + i] - pm;  // (pressure entry k at 2 n2 + k = n2 + i)
     }
   }
 }
 
 // z_j = the V-cycles' velocity, and pressure r / m_lumped + the V-cycle's; sums the pressure
-__global__ void k_fluid_merge(int NX, int NY, const double* V, double* Z, size_t n, size_t nv, const float* c,
-                              const float* pz, const double* ml, double* partials, unsigned* counter, KrylovDev* K) {
+__global__ void k_fluid_merge(int NX, int NY, const double* V, double* Z, size_t n, size_t nv, const double* c,
+                              const double* pz, const double* ml, double* partials, unsigned* counter, KrylovDev* K) {
   TOPO_PDL_ENTRY();
   const size_t n2 = size_t(NX) * NY;
   const double* v = V + size_t(K->j) * n + 2 * n2;
@@ -273,11 +272,11 @@ __global__ void k_fluid_merge(int NX, int NY, const double* V, double* Z, size_t
   TOPO_GRID_STRIDE(i, n2 + nv) {
     if (i < n2) {
       const bool bd = fluid_boundary_node(int(i % NX), int(i / NX), NX, NY);
-      z[2 * i] = bd ? 0.0 : double(c[i]);
-      z[2 * i + 1] = bd ? 0.0 : double(c[n2 + i]);
+      z[2 * i] = bd ? 0.0 : c[i];
+      z[2 * i + 1] = bd ? 0.0 : c[n2 + i];
     } else {
       const size_t k = i - n2;
-      const double p = v[k] / ml[k] + double(pz[k]);
+      const double p = v[k] / ml[k] + pz[k];
       z[2 * n2 + k] = p;
       s[0] += p;
     }
@@ -332,16 +331,16 @@ struct topo_fluid_ctx {
   int* hstat = nullptr;        // pinned: j, it, maxit, status of the cycle
   double* zc = nullptr;        // nv: z_j's centred pressure
   double* t = nullptr;         // n
-  float* c = nullptr;          // preconditioner: planar velocity components (2 n2) in
-  float* z = nullptr;          // and out,
-  float* pt = nullptr;         // pressure (nv) in
-  float* pz = nullptr;         // and out
+  double* c = nullptr;          // preconditioner: planar velocity components (2 n2) in
+  double* z = nullptr;          // and out,
+  double* pt = nullptr;         // pressure (nv) in
+  double* pz = nullptr;         // and out
   double* gb = nullptr;        // gradient right-hand side (nv)
   // preconditioner hierarchies
   std::vector<LevelSpec> uspec, pspec;
   std::vector<ElemRefs> urefs, prefs;
   std::vector<double*> uK, uM, pK, pM;
-  MG<float> mgu, mgp;
+  MG<double> mgu, mgp;
   // graph of one restart cycle, its recording stream, and the pressure's V-cycle beside the
   // velocity's
   cudaGraphExec_t graph = nullptr;
@@ -638,10 +637,10 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
   C->dots = C->arena.alloc_n<double>(krylov_dots(C->red.spread(C->n)));
   C->dot_counters = C->arena.alloc_n<unsigned>(kDotGroups);
   C->zc = C->arena.alloc_n<double>(C->nv);
-  C->c = C->arena.alloc_n<float>(2 * C->n2);
-  C->z = C->arena.alloc_n<float>(2 * C->n2);
-  C->pt = C->arena.alloc_n<float>(C->nv);
-  C->pz = C->arena.alloc_n<float>(C->nv);
+  C->c = C->arena.alloc_n<double>(2 * C->n2);
+  C->z = C->arena.alloc_n<double>(2 * C->n2);
+  C->pt = C->arena.alloc_n<double>(C->nv);
+  C->pz = C->arena.alloc_n<double>(C->nv);
   if (cudaMallocHost(&C->hstat, 4 * sizeof(int)) != cudaSuccess) return C->fail(TOPO_ERR_CUDA, "out of host memory");
   std::memset(C->hstat, 0, 4 * sizeof(int));
   for (cudaStream_t* c : {&C->cap, &C->side})
@@ -693,9 +692,6 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
     mg->use_graphs = false;  // only V-cycles are used
     mg->profile_levels = false;
     mg->element_bounds = true;
-    mg->deep_degree = kScalarDegree;
-    mg->deep_from = 0;
-    mg->cheb_lo_deep = 0.3;
   }
   C->mgu.batch = 2;
   C->mgu.init(C->uspec, C->urefs.data(), 0.0, 0.0, C->arena, &C->red);

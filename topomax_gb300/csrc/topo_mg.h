@@ -21,7 +21,7 @@
 namespace topo {
 
 constexpr int kCoarseMaxDofs = 32;
-constexpr int kCoarseDegree = 4, kScalarDegree = 3;  // FP32 sweeps of MG::deep_degree steps
+constexpr int kCoarseDegree = 4;  // FP32 elasticity sweeps of MG::deep_degree steps
 
 // Device memory owner: everything allocated here is freed with the arena.
 class Arena {
@@ -199,8 +199,7 @@ class MG {
   bool fp64_solution = false;
 
   // Chebyshev steps of a smoothing sweep: two on level 0 of a P2 hierarchy and
-  // above deep_from; deep_degree on the others (2, or
-  // FP32 kCoarseDegree for elasticity and kScalarDegree for scalar levels).
+  // above deep_from; deep_degree on the others (2, or kCoarseDegree for FP32 elasticity).
   //
   // State hierarchy, FP32: the iterations of a solve grow with the design's contrast through
   // the P1 levels below the first, and a further step inside a sweep costs less there than
@@ -209,7 +208,6 @@ class MG {
   // 41.9 and 37.9 (2000x1000).  The interval's lower end between 0.005 and 0.03 lambda_max
   // is within 3 %.  FP64 sweeps are bound by the FP64 pipe: two steps (59.4 ms against 58.5
   // with three and 80 with four before their tiles were fitted).
-  // Fluid preconditioner: 11.3, 10.5 and 10.6 ms (40x40), 21.3, 19.7 and 20.5 (128x128).
   // Filter: no difference (1.36 ms at 1000x500).
   int deep_degree = 2, deep_from = 2;
   double cheb_lo_deep = 0.1;  // their interval's lower end, times lambda_max

@@ -1700,13 +1700,14 @@ template <int NC>
 void MG<T>::sweep_level(int l, const T* b, T* x, cudaStream_t s) {
   // (the degrees in use: see level_degree)
   if constexpr (sizeof(T) == 4) {
-    constexpr int D = NC == 2 ? kCoarseDegree : kScalarDegree;
     if (!lv_[l].st) {
       const P1Params<T, NC> Q = make_p1<T, NC>(specs_[l], refs_[l], lv_[l].kK, lv_[l].kM);
-      if (level_degree(l) == D) return sweep_level<NC, D>(l, Q, b, x, s);
+      if constexpr (NC == 2)
+        if (level_degree(l) == kCoarseDegree) return sweep_level<NC, kCoarseDegree>(l, Q, b, x, s);
       return sweep_level<NC, 2>(l, Q, b, x, s);
     }
-    if (level_degree(l) == D) return sweep_level<NC, D>(l, StoredRows{}, b, x, s);
+    if constexpr (NC == 2)
+      if (level_degree(l) == kCoarseDegree) return sweep_level<NC, kCoarseDegree>(l, StoredRows{}, b, x, s);
   }
   sweep_level<NC, 2>(l, StoredRows{}, b, x, s);
 }
@@ -1721,9 +1722,9 @@ template <class T>
 template <int NC>
 void MG<T>::launch_tail(const TailSweep<T, NC>& P, int l, const T* b, T* x, cudaStream_t s) {
   const int nodes = int(specs_[l].nn());
-  constexpr int D = NC == 2 ? kCoarseDegree : kScalarDegree;
-  if (level_degree(l) == D) launch_tail<NC, D>(P, nodes, b, x, s);
-  else launch_tail<NC, 2>(P, nodes, b, x, s);
+  if constexpr (NC == 2)
+    if (level_degree(l) == kCoarseDegree) return launch_tail<NC, kCoarseDegree>(P, nodes, b, x, s);
+  launch_tail<NC, 2>(P, nodes, b, x, s);
 }
 
 // One V-cycle from level l down: fused degree-2 Chebyshev pre-smoothing from
