@@ -912,6 +912,8 @@ void emu_fluid_apply(int nx, int ny, double W, double H, double q, const double*
     y[2 * n2 + k] = fluid_gather_vertex(out.data(), nx, ny, int(k % (nx + 1)), int(k / (nx + 1)), kFluidOut, 12);
 }
 
+int emu_fluid_restart(long long n, long long free_bytes) { return fluid_restart(size_t(n), size_t(free_bytes)); }
+
 // the operator by output node (unclamped rows, pm off the pressure)
 void emu_fluid_apply_nodes(int nx, int ny, double W, double H, double q, double pm, const double* rho, const double* x,
                            double* y) {

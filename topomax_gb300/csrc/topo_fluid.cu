@@ -41,9 +41,7 @@ using namespace topo;
 
 namespace {
 
-// Restart length: kKrylovMax unless its 2 m + 1 vectors pass kFluidBasisMax bytes.
-constexpr int kFluidRestart = 30;
-constexpr size_t kFluidBasisMax = size_t(16) << 30;
+static_assert(kFluidRestartLong <= kKrylovMax, "the cycle's scalars");
 constexpr double kLaplaceShift = 1e-3;  // mass shift of the pressure Laplacian (its constant mode)
 
 // ---------------------------------------------------------------------------
@@ -629,7 +627,9 @@ int fluid_init(topo_fluid_ctx* C, const topo_grid_desc* g, double viscosity, con
   C->ones = C->arena.alloc_n<double>(C->nv);
   C->rhs = C->arena.alloc_n<double>(C->n);
   C->x = C->arena.alloc_n<double>(C->n);
-  if (C->n * sizeof(double) * (2 * kKrylovMax + 1) <= kFluidBasisMax) C->m = kKrylovMax;
+  size_t free_bytes = 0, total_bytes = 0;
+  if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) return C->cuda_check("device memory");
+  C->m = fluid_restart(C->n, free_bytes);
   C->V = C->arena.alloc_n<double>(size_t(C->m + 1) * C->n);
   C->Z = C->arena.alloc_n<double>(size_t(C->m) * C->n);
   C->t = C->arena.alloc_n<double>(C->n);
