@@ -427,13 +427,13 @@ struct topo_fluid_ctx {
     launch_pdl(k_fluid_apply<true>, G.start[5], kFluidThreads, 0, s, nx, ny, G, sc, rc, Zc, V, 1, kc, n, zc);
     krylov_column(KrylovSpace{V, nullptr, Z, zcc, n, nv, m, dots, dot_counters, red.partials, red.counter, kry},
                   int(gd), int(gv), cond, use_cond, s);
-    launches += 9;
+    launches += 8;
   }
   int record();
   int cycle(cudaStream_t s);
 };
 
-// Records one restart cycle: a WHILE node whose body is an iteration (k_fluid_next decides
+// Records one restart cycle: a WHILE node whose body is an iteration (k_krylov_next decides
 // on the device whether it runs again).  Nothing is launched unless every step succeeded.
 int topo_fluid_ctx::record() {
   std::lock_guard<std::recursive_mutex> lock(device_lock());
