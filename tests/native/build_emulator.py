@@ -20,7 +20,7 @@ LIB = os.path.join(HERE, "_emulate.so")
 
 def build() -> str:
     srcs = [os.path.join(HERE, "emulate.cu"), os.path.join(CSRC, "topo_mg_common.cu")]
-    deps = srcs + [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]
+    deps = srcs + [os.path.join(HERE, "reference.h")] + [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]
     if os.path.exists(LIB) and all(os.path.getmtime(d) <= os.path.getmtime(LIB) for d in deps):
         return LIB
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"

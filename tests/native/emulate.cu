@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "topo_mg.h"
+#include "reference.h"
 #include "topo_p1.cuh"
 #include "topo_p2.cuh"
 #include "topo_p1march.cuh"
@@ -877,50 +878,16 @@ double emu_fluid_alpha(double q, double rho, int derivative) {
   return derivative ? pen.da(rho) : pen.a(rho);
 }
 
-void emu_fluid_apply(int nx, int ny, double W, double H, double q, const double* rho, const double* x, double* y,
-                     int clamp) {
-  FluidTables E;
-  fluid_tables(W / nx, H / ny, E);
-  const FluidPenal pen = emu_fluid_penal(q);
-  const size_t nt = size_t(2) * nx * ny, n2 = size_t(2 * nx + 1) * (2 * ny + 1), nv = size_t(nx + 1) * (ny + 1);
-  std::vector<double> mass(nt * kFluidMass), out(nt * kFluidOut);
-  for (size_t t = 0; t < nt; ++t) {
-    double r[3];
-    fluid_tri_rho(rho, nx, t, r);
-    fluid_tri_mass(E, pen, r, mass.data() + t * kFluidMass);
-  }
-  for (size_t t = 0; t < nt; ++t) {
-    size_t nd[6], vt[3];
-    fluid_tri_nodes(nx, t, nd);
-    fluid_tri_vertices(nx, t, vt);
-    double ue[6][2], pe[3];
-    for (int k = 0; k < 6; ++k) {
-      ue[k][0] = x[2 * nd[k]];
-      ue[k][1] = x[2 * nd[k] + 1];
-    }
-    for (int k = 0; k < 3; ++k) pe[k] = x[2 * n2 + vt[k]];
-    fluid_tri_apply(E, int(t & 1), mass.data() + t * kFluidMass, ue, pe, out.data() + t * kFluidOut);
-  }
-  const int NX = 2 * nx + 1;
-  for (size_t i = 0; i < n2; ++i) {
-    double v[2];
-    fluid_gather_node(out.data(), nx, ny, int(i % NX), int(i / NX), clamp != 0, x, v);
-    y[2 * i] = v[0];
-    y[2 * i + 1] = v[1];
-  }
-  for (size_t k = 0; k < nv; ++k)
-    y[2 * n2 + k] = fluid_gather_vertex(out.data(), nx, ny, int(k % (nx + 1)), int(k / (nx + 1)), kFluidOut, 12);
-}
-
 int emu_fluid_restart(long long n, long long free_bytes) { return fluid_restart(size_t(n), size_t(free_bytes)); }
 
-// the operator by output node (unclamped rows, pm off the pressure)
-void emu_fluid_apply_nodes(int nx, int ny, double W, double H, double q, double pm, const double* rho, const double* x,
-                           double* y) {
+// the operator by output node: the kernels' rows and classes one node after the other (pm off the
+// pressure; clamp: identity rows on the boundary)
+static void fluid_apply_all(int nx, int ny, double W, double H, double q, double pm, const double* rho, const double* x,
+                            double* y, bool clamp) {
   FluidTables E;
   fluid_tables(W / nx, H / ny, E);
   const FluidPenal pen = emu_fluid_penal(q);
-  const size_t nt = size_t(2) * nx * ny, n2 = size_t(2 * nx + 1) * (2 * ny + 1), nv = size_t(nx + 1) * (ny + 1);
+  const size_t nt = size_t(2) * nx * ny, n2 = size_t(2 * nx + 1) * (2 * ny + 1);
   std::vector<double> mk(nt * kFluidMass);
   for (size_t t = 0; t < nt; ++t) {
     double r[3];
@@ -931,25 +898,34 @@ void emu_fluid_apply_nodes(int nx, int ny, double W, double H, double q, double 
   }
   FluidStencils S;
   fluid_stencils(E, S);
-  (void)nv;
-  auto velocity = [&](auto tag, int w, int h) {
+  const FluidRows R(nx, ny);
+  std::vector<double> rows(R.size);
+  auto velocity = [&](auto tag) {
     constexpr int C = decltype(tag)::value;
-    for (int j = 0; j < h; ++j)
-      for (int i = 0; i < w; ++i) {
-        double row[kFluidNodes], v[2];
-        fluid_build_row<C>(mk.data(), nx, ny, i, j, row);
-        fluid_velocity<C>(S, row, 1, nx, ny, i, j, x, x + 2 * n2, pm, v);
-        const size_t node = size_t(2 * j + (C >> 1)) * (2 * nx + 1) + 2 * i + (C & 1);
-        y[2 * node] = v[0];
-        y[2 * node + 1] = v[1];
-      }
+    const int w = C & 1 ? nx : nx + 1;
+    for (size_t k = 0; k < R.count[C]; ++k) {
+      double row[kFluidNodes];
+      fluid_build_row<C>(mk.data(), nx, ny, int(k % w), int(k / w), row);
+      for (int e = 0; e < fluid_nodes(C); ++e) rows[R.first[C] + size_t(e) * R.count[C] + k] = row[e];
+      fluid_apply_class<C>(nx, ny, S, rows.data(), R, k, x, pm, clamp, y);
+    }
   };
-  velocity(std::integral_constant<int, 0>{}, nx + 1, ny + 1);
-  velocity(std::integral_constant<int, 1>{}, nx, ny + 1);
-  velocity(std::integral_constant<int, 2>{}, nx + 1, ny);
-  velocity(std::integral_constant<int, 3>{}, nx, ny);
+  velocity(std::integral_constant<int, 0>{});
+  velocity(std::integral_constant<int, 1>{});
+  velocity(std::integral_constant<int, 2>{});
+  velocity(std::integral_constant<int, 3>{});
   for (int j = 0; j <= ny; ++j)
     for (int i = 0; i <= nx; ++i) y[2 * n2 + size_t(j) * (nx + 1) + i] = fluid_continuity(S, nx, ny, i, j, x);
+}
+
+void emu_fluid_apply(int nx, int ny, double W, double H, double q, const double* rho, const double* x, double* y,
+                     int clamp) {
+  fluid_apply_all(nx, ny, W, H, q, 0.0, rho, x, y, clamp != 0);
+}
+
+void emu_fluid_apply_nodes(int nx, int ny, double W, double H, double q, double pm, const double* rho, const double* x,
+                           double* y) {
+  fluid_apply_all(nx, ny, W, H, q, pm, rho, x, y, false);
 }
 
 double emu_fluid_objective(int nx, int ny, double W, double H, double q, double mu, const double* rho,
@@ -992,7 +968,7 @@ void emu_fluid_gradient_rhs(int nx, int ny, double W, double H, double q, const 
     for (int k = 0; k < 3; ++k) tri3[3 * t + k] = o3[k];
   }
   for (size_t v = 0; v < size_t(nx + 1) * (ny + 1); ++v)
-    b[v] = fluid_gather_vertex(tri3.data(), nx, ny, int(v % (nx + 1)), int(v / (nx + 1)), 3, 0);
+    b[v] = p1_vertex_gather3(nx, ny, tri3.data(), int(v % (nx + 1)), int(v / (nx + 1)));
 }
 
 // incident (triangle, local node) pairs of P2 node (a, b); returns the count

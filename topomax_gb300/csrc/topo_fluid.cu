@@ -104,24 +104,6 @@ __global__ void __launch_bounds__(kFluidThreads)
 // Bound: FP64, 42 products per P2 node on average (the triangles' matrices applied where they are
 // needed take 72), all loads of a row in flight at once: 10.4 us at 128x128, 6.0 at 40x40; by
 // triangle rows 19.6 and 17.4, through a per-triangle buffer and a gather 22 and 20.
-template <int CLS>
-__device__ __forceinline__ void fluid_apply_class(int nx, int ny, const FluidStencils& S, const double* rows,
-                                                  const FluidRows& R, size_t k, const double* x, double pm, bool clamp,
-                                                  double* y) {
-  const int NX = 2 * nx + 1, NY = 2 * ny + 1, w = CLS & 1 ? nx : nx + 1;
-  const int i = int(k % w), j = int(k / w), a = 2 * i + (CLS & 1), b = 2 * j + (CLS >> 1);
-  const size_t node = size_t(b) * NX + a;
-  double v[2];
-  if (clamp && fluid_boundary_node(a, b, NX, NY)) {
-    v[0] = x[2 * node];
-    v[1] = x[2 * node + 1];
-  } else {
-    fluid_velocity<CLS>(S, rows + R.first[CLS] + k, R.count[CLS], nx, ny, i, j, x, x + 2 * size_t(NX) * NY, pm, v);
-  }
-  y[2 * node] = v[0];
-  y[2 * node + 1] = v[1];
-}
-
 template <bool KRYLOV>
 __global__ void __launch_bounds__(kFluidThreads)
     k_fluid_apply(int nx, int ny, FluidGrid G, const FluidStencils* __restrict__ S, const double* __restrict__ rows,

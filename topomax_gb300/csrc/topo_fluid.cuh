@@ -1,6 +1,6 @@
 // Stokes-Brinkman state on the P2-P1 (Taylor-Hood) lattice: element tables,
-// node incidence and the per-triangle phases of the operator, the objective
-// and the gradient's right-hand side.
+// node incidence, the operator by output node and the per-triangle phases of the
+// objective and the gradient's right-hand side.
 //
 // Follows FEM_src/fluid_problem.py:48-155 and src/penalizers.py:49-67:
 //   a((u,p),(v,q)) = (alpha(rho) u, v) + (grad u, grad v) + (grad p, v) + (div u, q),
@@ -12,7 +12,7 @@
 // collapsed Gauss-Jacobi 4 x 4 rule (degree 7); the same rules are used here.
 //
 // Everything here compiles for host and device: the test emulator runs the
-// triangle phases and the incidence gathers on the CPU against the oracle.
+// operator's rows and the triangle phases on the CPU against the oracle.
 #pragma once
 
 #include <cmath>
@@ -25,7 +25,6 @@ namespace topo {
 constexpr int kFluidQ6 = 12;
 constexpr int kFluidQ7 = 16;
 constexpr int kFluidMass = 21;   // upper triangle of the 6 x 6 alpha-weighted P2 mass matrix
-constexpr int kFluidOut = 16;    // per-triangle output: 12 velocity rows, 3 pressure rows, pad
 
 // alpha(rho) and alpha'(rho) in the reference's operation order
 struct FluidPenal {
@@ -64,27 +63,6 @@ TOPO_HD void p2_values(const double (&l)[3], double (&N)[6]) {
   N[5] = 4 * l[0] * l[1];
 }
 
-// Triangles incident to P2 node (a, b) of the (2nx+1) x (2ny+1) lattice, with
-// the node's local index in each; a fixed order (cell row, cell column,
-// orientation).  Returns the count (at most 6).
-TOPO_HD int p2_node_incidence(int a, int b, int nx, int ny, size_t (&tri)[6], int (&loc)[6]) {
-  int n = 0;
-  for (int j = b / 2 - 1; j <= b / 2; ++j) {
-    if (j < 0 || j >= ny || b - 2 * j > 2) continue;
-    for (int i = a / 2 - 1; i <= a / 2; ++i) {
-      if (i < 0 || i >= nx || a - 2 * i > 2) continue;
-      for (int o = 0; o < 2; ++o)
-        for (int k = 0; k < 6; ++k)
-          if (p2_off_a(o, k) == a - 2 * i && p2_off_b(o, k) == b - 2 * j) {
-            tri[n] = (size_t(j) * nx + i) * 2 + o;
-            loc[n] = k;
-            ++n;
-          }
-    }
-  }
-  return n;
-}
-
 TOPO_HD bool fluid_boundary_node(int a, int b, int NX, int NY) {
   return a == 0 || b == 0 || a == NX - 1 || b == NY - 1;
 }
@@ -105,13 +83,6 @@ TOPO_HD void fluid_tri_nodes(int nx, size_t t, size_t (&n)[6]) {
   for (int k = 0; k < 6; ++k) n[k] = size_t(2 * j + p2_off_b(o, k)) * NX + 2 * i + p2_off_a(o, k);
 }
 
-TOPO_HD void fluid_tri_vertices(int nx, size_t t, size_t (&v)[3]) {
-  const int o = int(t & 1);
-  const size_t cell = t >> 1;
-  const int i = int(cell % nx), j = int(cell / nx);
-  for (int k = 0; k < 3; ++k) v[k] = size_t(j + p1_off_b(o, k)) * (nx + 1) + i + p1_off_a(o, k);
-}
-
 // The alpha-weighted P2 mass matrix of triangle t (upper triangle, kFluidMass values):
 // area * sum_q w_q alpha(rho_q) N_i(q) N_j(q), rho_q interpolated from the vertices.
 TOPO_HD void fluid_tri_mass(const FluidTables& E, const FluidPenal& pen, const double (&r)[3], double* m) {
@@ -126,31 +97,6 @@ TOPO_HD void fluid_tri_mass(const FluidTables& E, const FluidPenal& pen, const d
       for (int q = 0; q < kFluidQ6; ++q) s += aw[q] * E.N6[q][i] * E.N6[q][j];
       m[fluid_mass_index(i, j)] = E.area * s;
     }
-}
-
-// Local rows of the symmetric saddle-point operator on triangle t:
-//   out[2i+c] = sum_j (M_ij + K_ij) u_(j,c) + sum_k G_(i,c),k p_k   (momentum)
-//   out[12+k] = - sum_(j,c) D_k,(j,c) u_(j,c)                       (continuity, B = -D)
-// The sign of the continuity rows makes the assembled operator symmetric on
-// velocities that vanish on the boundary ((grad p, v) = -(p, div v) there).
-TOPO_HD void fluid_tri_apply(const FluidTables& E, int o, const double* m, const double (&ue)[6][2],
-                             const double (&pe)[3], double* out) {
-  for (int i = 0; i < 6; ++i)
-    for (int c = 0; c < 2; ++c) {
-      double s = 0.0;
-      for (int j = 0; j < 6; ++j) {
-        const double mij = i <= j ? m[fluid_mass_index(i, j)] : m[fluid_mass_index(j, i)];
-        s += (mij + E.lap[o][i][j]) * ue[j][c];
-      }
-      for (int k = 0; k < 3; ++k) s += E.grad[o][i][c][k] * pe[k];
-      out[2 * i + c] = s;
-    }
-  for (int k = 0; k < 3; ++k) {
-    double s = 0.0;
-    for (int j = 0; j < 6; ++j) s += E.div[o][k][j][0] * ue[j][0] + E.div[o][k][j][1] * ue[j][1];
-    out[12 + k] = -s;
-  }
-  out[15] = 0.0;
 }
 
 // Objective integrand of triangle t: area * sum_q w_q (alpha |u|^2 + mu |grad u|^2)
@@ -191,48 +137,12 @@ TOPO_HD void fluid_tri_gradient(const FluidTables& E, const FluidPenal& pen, con
   }
 }
 
-// Gathers of the per-triangle rows (kFluidOut values per triangle) onto the
-// P2 nodes and the CG1 vertices.  Velocity node rows: with clamp, boundary
-// nodes return x itself (identity rows; the Krylov vectors are zero there).
-TOPO_HD void fluid_gather_node(const double* tri_out, int nx, int ny, int a, int b, bool clamp, const double* x,
-                               double (&y)[2]) {
-  const int NX = 2 * nx + 1, NY = 2 * ny + 1;
-  const size_t node = size_t(b) * NX + a;
-  if (clamp && fluid_boundary_node(a, b, NX, NY)) {
-    y[0] = x[2 * node];
-    y[1] = x[2 * node + 1];
-    return;
-  }
-  size_t tri[6];
-  int loc[6];
-  const int n = p2_node_incidence(a, b, nx, ny, tri, loc);
-  double s0 = 0.0, s1 = 0.0;
-  for (int e = 0; e < n; ++e) {
-    s0 += tri_out[tri[e] * kFluidOut + 2 * loc[e]];
-    s1 += tri_out[tri[e] * kFluidOut + 2 * loc[e] + 1];
-  }
-  y[0] = s0;
-  y[1] = s1;
-}
-
-TOPO_HD double fluid_gather_vertex(const double* tri_out, int nx, int ny, int a, int b, int stride, int offset) {
-  // CG1 vertex (a, b): the six incidences of the right-diagonal lattice
-  const int inc[6][4] = {{-1, -1, 0, 2}, {-1, -1, 1, 2}, {0, -1, 1, 1}, {-1, 0, 0, 1}, {0, 0, 0, 0}, {0, 0, 1, 0}};
-  double s = 0.0;
-  for (int e = 0; e < 6; ++e) {
-    const int ci = a + inc[e][0], cj = b + inc[e][1];
-    if (ci < 0 || ci >= nx || cj < 0 || cj >= ny) continue;
-    const size_t t = (size_t(cj) * nx + ci) * 2 + inc[e][2];
-    s += tri_out[t * stride + offset + inc[e][3]];
-  }
-  return s;
-}
-
 // ---------------------------------------------------------------------------
 // the operator by output node
 // ---------------------------------------------------------------------------
 // P2 nodes by class: 0 vertices, midpoints of 1 horizontal, 2 vertical and 3 diagonal edges, so
-// that the threads of a block do the same work; (i, j): column and row of the vertex, or of
+// that the threads of a block do the same work.  The continuity rows are negated, which makes the
+// operator symmetric on velocities that vanish on the boundary; (i, j): column and row of the vertex, or of
 // the edge's lower left vertex.  (Class 4 in the kernels: the pressure vertices.)
 
 // Incident triangles of a class's nodes, a byte each: column offset + 1 | (row offset + 1) << 1 |
@@ -366,6 +276,26 @@ TOPO_HD void fluid_velocity(const FluidStencils& S, const double* row, size_t st
     y[0] += g[0] * q;
     y[1] += g[1] * q;
   }
+}
+
+// y at the k-th velocity node of class CLS, from the assembled rows (FluidRows).  clamp: boundary
+// rows are the identity.
+template <int CLS>
+TOPO_HD void fluid_apply_class(int nx, int ny, const FluidStencils& S, const double* rows,
+                                                  const FluidRows& R, size_t k, const double* x, double pm, bool clamp,
+                                                  double* y) {
+  const int NX = 2 * nx + 1, NY = 2 * ny + 1, w = CLS & 1 ? nx : nx + 1;
+  const int i = int(k % w), j = int(k / w), a = 2 * i + (CLS & 1), b = 2 * j + (CLS >> 1);
+  const size_t node = size_t(b) * NX + a;
+  double v[2];
+  if (clamp && fluid_boundary_node(a, b, NX, NY)) {
+    v[0] = x[2 * node];
+    v[1] = x[2 * node + 1];
+  } else {
+    fluid_velocity<CLS>(S, rows + R.first[CLS] + k, R.count[CLS], nx, ny, i, j, x, x + 2 * size_t(NX) * NY, pm, v);
+  }
+  y[2 * node] = v[0];
+  y[2 * node + 1] = v[1];
 }
 
 // Continuity row of vertex (i, j)

@@ -39,6 +39,21 @@ TOPO_HD void p1_incidence(int e, int& dci, int& dcj, int& o, int& loc) {
   loc = int(f >> 3);
 }
 
+// Sum at vertex (a, b) of its triangles' values, three per triangle.
+template <class TQ>
+TOPO_HD double p1_vertex_gather3(int nx, int ny, const TQ* tri3, int a, int b) {
+  double s = 0.0;
+  for (int e = 0; e < 6; ++e) {
+    int dci, dcj, o, loc;
+    p1_incidence(e, dci, dcj, o, loc);
+    const int ci = a + dci, cj = b + dcj;
+    if (ci < 0 || ci >= nx || cj < 0 || cj >= ny) continue;
+    const size_t t = (size_t(cj) * nx + ci) * 2 + o;
+    s += double(tri3[3 * t + loc]);
+  }
+  return s;
+}
+
 // Input of a node apply read directly from an array.
 template <class T, int NC>
 struct FetchArray {
@@ -375,9 +390,11 @@ TOPO_HD void p1_node_apply(int a, int b, const PP& P, const T* u, T* y) {
 }
 
 // ---------------------------------------------------------------------------
-// fused degree-2 Chebyshev smoothing steps of one P1 level (node-centric)
+// fused degree-2 Chebyshev smoothing steps of a level (the march kernels' modes)
 // ---------------------------------------------------------------------------
-// Buffers of one level for the fused V-cycle.
+// Buffers of one level.  Pre, from x = 0: d0 = c0 Dinv b, r1 = b - A d0, x = d0 + c1 d0 + c2 Dinv r1.
+// Res: r = b - A x.  First, after the coarse correction: r = b - A x, d = c0 Dinv r, x2 = x + d.
+// Post2: r1 = r - A d, x = x2 + c1 d + c2 Dinv r1.
 template <class T>
 struct SmoothBufs {
   const T* b;      // right-hand side
@@ -387,83 +404,6 @@ struct SmoothBufs {
   T* r;            // residual
   T* d;            // Chebyshev direction
   const T* cheb;   // c0 = 1/theta, c1, c2 of the second step (in the level's precision)
-};
-
-// PRE input: first step from x = 0, d0 = c0 Dinv b, computed per node
-template <class T, int NC>
-struct FetchPre {
-  const T* b;
-  const T* dinv;
-  T c0;
-  TOPO_HD void operator()(size_t m, int, int, T (&v)[NC]) const {
-    for (int d = 0; d < NC; ++d) v[d] = c0 * dinv[NC * m + d] * b[NC * m + d];
-  }
-};
-
-template <class T, int NC>
-struct P1Smooth {
-  // PRE: x = d0 + d1 with d0 = c0 Dinv b, r1 = b - A d0, d1 = c1 d0 + c2 Dinv r1
-  template <class PP>
-  TOPO_HD static void pre(int a, int b, const PP& P, const SmoothBufs<T>& B) {
-    const int NX = P.nx + 1;
-    const size_t n = size_t(b) * NX + a;
-    const T c0 = B.cheb[0], c1 = B.cheb[1], c2 = B.cheb[2];
-    const FetchPre<T, NC> f{B.b, B.dinv, c0};
-    T t[NC], u[NC];
-    f(n, a, b, u);
-    if (!p1_node_eval<T, NC>(a, b, P, f, t))
-      for (int c = 0; c < NC; ++c) t[c] = u[c];
-    for (int c = 0; c < NC; ++c) {
-      const size_t i = NC * n + c;
-      const T r1 = B.b[i] - t[c];
-      B.x[i] = u[c] + c1 * u[c] + c2 * B.dinv[i] * r1;
-    }
-  }
-  // RES: r = b - A x
-  template <class PP>
-  TOPO_HD static void res(int a, int b, const PP& P, const SmoothBufs<T>& B) {
-    const int NX = P.nx + 1;
-    const size_t n = size_t(b) * NX + a;
-    T t[NC];
-    if (!p1_node_eval<T, NC>(a, b, P, FetchArray<T, NC>{B.x}, t))
-      for (int c = 0; c < NC; ++c) t[c] = B.x[NC * n + c];
-    for (int c = 0; c < NC; ++c) B.r[NC * n + c] = B.b[NC * n + c] - t[c];
-  }
-  // FIRST (after the coarse correction was added to x):
-  // r0 = b - A x ; d0 = c0 Dinv r0 ; x2 = x + d0 (writes r, d, x2)
-  template <class PP>
-  TOPO_HD static void first(int a, int b, const PP& P, const SmoothBufs<T>& B) {
-    const int NX = P.nx + 1;
-    const size_t n = size_t(b) * NX + a;
-    const T c0 = B.cheb[0];
-    T t[NC];
-    if (!p1_node_eval<T, NC>(a, b, P, FetchArray<T, NC>{B.x}, t))
-      for (int c = 0; c < NC; ++c) t[c] = B.x[NC * n + c];
-    for (int c = 0; c < NC; ++c) {
-      const size_t i = NC * n + c;
-      const T r0 = B.b[i] - t[c];
-      const T d0 = c0 * B.dinv[i] * r0;
-      B.r[i] = r0;
-      B.d[i] = d0;
-      B.x2[i] = B.x[i] + d0;
-    }
-  }
-  // POST2: r1 = r0 - A d0 ; d1 = c1 d0 + c2 Dinv r1 ; x = x2 + d1
-  template <class PP>
-  TOPO_HD static void post2(int a, int b, const PP& P, const SmoothBufs<T>& B) {
-    const int NX = P.nx + 1;
-    const size_t n = size_t(b) * NX + a;
-    const T c1 = B.cheb[1], c2 = B.cheb[2];
-    const FetchArray<T, NC> f{B.d};
-    T t[NC];
-    if (!p1_node_eval<T, NC>(a, b, P, f, t))
-      for (int c = 0; c < NC; ++c) t[c] = B.d[NC * n + c];
-    for (int c = 0; c < NC; ++c) {
-      const size_t i = NC * n + c;
-      const T r1 = B.r[i] - t[c];
-      B.x[i] = B.x2[i] + c1 * B.d[i] + c2 * B.dinv[i] * r1;
-    }
-  }
 };
 
 // ---------------------------------------------------------------------------

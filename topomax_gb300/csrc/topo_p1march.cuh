@@ -6,7 +6,7 @@
 // column 0 of the next lane (operand down by a shuffle, results up), row 1 of
 // a step is row 0 of the next (registers).  After a step the lane holds the
 // complete sum at its node (i, j) and finishes it (apply or a fused smoothing
-// step, the formulas of P1Smooth).  Per cell: two element products
+// step, the formulas of SmoothBufs).  Per cell: two element products
 // y = kK Kref u (+ kM Mref u), against ~six incidences per node walked by the
 // node-centric kernel.
 #pragma once

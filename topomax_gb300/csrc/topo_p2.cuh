@@ -311,7 +311,7 @@ struct P2Io {
   int mode;
   const T* u;          // kP2Apply / kP2Res / kP2First input (x)
   T* y;                // kP2Apply / kP2Diag output
-  SmoothBufs<T> B;     // smoothing modes (see P1Smooth for the formulas)
+  SmoothBufs<T> B;     // smoothing modes
   const T* xc;         // kP2First: coarse correction on the P1 vertex lattice, added to the
                        // operand x at free nodes on the fly (the prolongation, not stored)
   int fuse;            // P2Fuse

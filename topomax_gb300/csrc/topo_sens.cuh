@@ -100,17 +100,7 @@ __global__ void k_vertex_gather3(int nx, int ny, const TQ* __restrict__ tri3, do
   const int VX = nx + 1;
   const size_t nv = size_t(nx + 1) * (ny + 1);
   TOPO_GRID_STRIDE(v, nv) {
-    const int a = int(v % VX), bb = int(v / VX);
-    double s = 0.0;
-    for (int e = 0; e < 6; ++e) {
-      int dci, dcj, o, loc;
-      p1_incidence(e, dci, dcj, o, loc);
-      const int ci = a + dci, cj = bb + dcj;
-      if (ci < 0 || ci >= nx || cj < 0 || cj >= ny) continue;
-      const size_t t = (size_t(cj) * nx + ci) * 2 + o;
-      s += double(tri3[3 * t + loc]);
-    }
-    b[v] = s;
+    b[v] = p1_vertex_gather3(nx, ny, tri3, int(v % VX), int(v / VX));
   }
 }
 
