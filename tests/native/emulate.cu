@@ -437,6 +437,8 @@ int emu_level_sweeps(int prec, int NC, int D, int nx, int ny, double hx, double 
 #undef TOPO_EMU_SWEEP
 }
 
+int emu_dens_row_alignment() { return int(alignof(DensRow)); }
+
 // density filter: w / s by the integer quotient, and y = W x or W^T x through the table
 void emu_dens_quotient(long n, const double* w, const double* s, double* q) {
   for (long i = 0; i < n; ++i) q[i] = dens_quotient(w[i], s[i], dens_reciprocal(s[i]));

@@ -437,10 +437,10 @@ __global__ void __launch_bounds__(kDensThreads)
 }
 
 // Bound: the FP64 pipe, two operations (32 issue cycles of an SM) per warp and neighbour;
-// the ~25 integer instructions of a quotient and the three loads (class and operand
-// coalesced, weights within a line or two) fit under them.  180,000 elements of 600 x 300
-// at radius 0.1732 (1.4e9 neighbours): 6.8 ms per product against the pipe's 4.6 ms; the
-// square root and division of k_dens_apply took 81 (W) and 83 ms (W^T).
+// the ~25 integer instructions of a quotient and the loads fit under them: class and operand
+// (coalesced) and weight (within a line or two), for W^T also the neighbour's row (16 bytes, coalesced).
+// 180,000 elements of 600 x 300 at radius 0.1732 (1.4e9 neighbours): 6.7 ms W, 6.9 ms W^T against the
+// pipe's 4.6 ms; the square root and division of k_dens_apply took 81 and 83 ms.
 template <bool TRANSPOSE>
 __global__ void __launch_bounds__(kDensThreads)
     k_dens_table_apply(DensTable T, const DensRow* __restrict__ rows, const double* __restrict__ x,

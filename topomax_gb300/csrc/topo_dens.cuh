@@ -120,7 +120,7 @@ inline std::vector<int> dens_half_widths(const DensAxis& X, const DensAxis& Y, d
   return h;
 }
 
-struct DensRow {  // a row's sum and its reciprocal, one 16-byte load
+struct alignas(16) DensRow {  // a row's sum and its reciprocal, one 16-byte load
   uint64_t r;
   double s;
 };
