@@ -936,8 +936,8 @@ inline void prime_march_occupancy() {
   (void)p2_march_bps<T, kP2First>();
   (void)p2_march_bps<T, kP2Post2>();
   (void)p1_march_bps<T, 1, kP2Apply>();
-  (void)p1_march_bps<T, 2, kP2Apply>();
   if constexpr (sizeof(T) == 8) {  // (FP32 levels are smoothed by the sweeps)
+    (void)p1_march_bps<T, 2, kP2Apply>();
     (void)p1_march_bps<T, 1, kP2Pre>();
     (void)p1_march_bps<T, 1, kP2Res>();
     (void)p1_march_bps<T, 1, kP2First>();
@@ -1416,28 +1416,16 @@ void MG<T>::apply(int l, const T* x, T* y, cudaStream_t s, bool op) {
                         (v.inner ? 0.0 : double((7 * L.NC * L.NC * sizeof(T) + 15) / 16 * 16) * L.nn());
   KClock kc(s, (v.st && stencils_ready_) ? "P1 stencil Apply" : "P1 march Apply (operator)", l,
             (v.st && stencils_ready_) ? abytes : 0.0);
-  if (L.NC == 2) {
-    if (v.st && stencils_ready_) {
-      launch_pdl(k_p1_apply<T, 2, P1Stencil<T, 2>>, g, kRowThreads, 0, s, P1Stencil<T, 2>{L.nx, L.ny, L.dir, v.st, v.inner}, x, y);
-    } else {
-      P1Io<T> io;
-      std::memset(&io, 0, sizeof(io));
-      io.mode = kP2Apply;
-      io.u = x;
-      io.y = y;
-      launch_p1_mode<T, 2, kP2Apply>(make_p1<T, 2>(L, refs_[l], v.kK, nullptr), io, s);
-    }
+  // (elasticity hierarchies start with a P2 level; nothing applies their P1 levels' operators)
+  if (v.st && stencils_ready_) {
+    launch_pdl(k_p1_apply<T, 1, P1Stencil<T, 1>>, g, kRowThreads, 0, s, P1Stencil<T, 1>{L.nx, L.ny, L.dir, v.st, v.inner}, x, y);
   } else {
-    if (v.st && stencils_ready_) {
-      launch_pdl(k_p1_apply<T, 1, P1Stencil<T, 1>>, g, kRowThreads, 0, s, P1Stencil<T, 1>{L.nx, L.ny, L.dir, v.st, v.inner}, x, y);
-    } else {
-      P1Io<T> io;
-      std::memset(&io, 0, sizeof(io));
-      io.mode = kP2Apply;
-      io.u = x;
-      io.y = y;
-      launch_p1_mode<T, 1, kP2Apply>(make_p1<T, 1>(L, refs_[l], v.kK, v.kM), io, s);
-    }
+    P1Io<T> io;
+    std::memset(&io, 0, sizeof(io));
+    io.mode = kP2Apply;
+    io.u = x;
+    io.y = y;
+    launch_p1_mode<T, 1, kP2Apply>(make_p1<T, 1>(L, refs_[l], v.kK, v.kM), io, s);
   }
 }
 
@@ -1910,7 +1898,8 @@ void MG<T>::tune_marches(cudaStream_t s) {
       const size_t max_blocks = red_ ? size_t(red_->blocks) * 8 : 0;
       choose(march_family(true, sizeof(T), 2), S.nx, S.ny, p2_march_bps<T, kP2Apply>(), max_blocks,
              [&](int seg) { launch_p2_mode<T, kP2Apply>(p2_op_, xi_, io, s, seg); });
-    } else if (!v.st && l + 1 < L) {
+    } else if (!v.st && l + 1 < L && (sizeof(T) == 8 || S.NC == 1)) {
+      // (FP32 elasticity levels run no march: the sweeps smooth them, their bound is the elements')
       T* x = l > 0 ? v.x : pcg_[8];  // level 0 works on its caller's vector and owns none
       cudaMemsetAsync(x, 0, S.ndof() * sizeof(T), s);
       P1Io<T> io;
@@ -1918,14 +1907,14 @@ void MG<T>::tune_marches(cudaStream_t s) {
       io.mode = kP2Apply;
       io.u = x;
       io.y = v.t;
-      if (S.NC == 2) {
-        const auto P = make_p1<T, 2>(S, refs_[l], v.kK, nullptr);
-        choose(march_family(false, sizeof(T), 2), S.nx, S.ny, p1_march_bps<T, 2, kP2Apply>(), 0,
-               [&](int seg) { launch_p1_mode<T, 2, kP2Apply>(P, io, s, seg); });
-      } else {
+      if (S.NC == 1) {
         const auto P = make_p1<T, 1>(S, refs_[l], v.kK, v.kM);
         choose(march_family(false, sizeof(T), 1), S.nx, S.ny, p1_march_bps<T, 1, kP2Apply>(), 0,
                [&](int seg) { launch_p1_mode<T, 1, kP2Apply>(P, io, s, seg); });
+      } else if constexpr (sizeof(T) == 8) {
+        const auto P = make_p1<T, 2>(S, refs_[l], v.kK, nullptr);
+        choose(march_family(false, sizeof(T), 2), S.nx, S.ny, p1_march_bps<T, 2, kP2Apply>(), 0,
+               [&](int seg) { launch_p1_mode<T, 2, kP2Apply>(P, io, s, seg); });
       }
     }
   }
