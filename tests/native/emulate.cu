@@ -437,6 +437,10 @@ int emu_level_sweeps(int prec, int NC, int D, int nx, int ny, double hx, double 
 #undef TOPO_EMU_SWEEP
 }
 
+int emu_sweep_degree(int prec, int NC, int wanted) {
+  return prec ? sweep_degree<float>(NC, wanted) : sweep_degree<double>(NC, wanted);
+}
+
 int emu_dens_row_alignment() { return int(alignof(DensRow)); }
 
 // density filter: w / s by the integer quotient, and y = W x or W^T x through the table

@@ -21,7 +21,6 @@
 namespace topo {
 
 constexpr int kCoarseMaxDofs = 32;
-constexpr int kCoarseDegree = 4;  // FP32 elasticity sweeps of MG::deep_degree steps
 
 // Device memory owner: everything allocated here is freed with the arena.
 class Arena {
@@ -211,7 +210,7 @@ class MG {
   // Filter: no difference (1.36 ms at 1000x500).
   int deep_degree = 2, deep_from = 2;
   double cheb_lo_deep = 0.1;  // their interval's lower end, times lambda_max
-  int level_degree(int l) const { return l >= deep_from ? deep_degree : 2; }
+  int level_degree(int l) const { return l >= deep_from ? sweep_degree<T>(specs_[l].NC, deep_degree) : 2; }
   double cheb_lo_frac = 0.1;   // smoothing interval [lo_frac, 1.1] * lambda_max
   int power_iters = 10;
   int power_iters_warm = 4;  // level 0 of a P2 hierarchy, started from the previous set-up's vector

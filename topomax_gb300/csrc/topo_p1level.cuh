@@ -19,6 +19,14 @@
 
 namespace topo {
 
+// Chebyshev steps of a sweep: two, or kCoarseDegree where a hierarchy asks for it (FP32 elasticity).
+// Other counts have no kernels, and the coefficients of one polynomial are no prefix of another's.
+constexpr int kCoarseDegree = 4;
+template <class T>
+constexpr int sweep_degree(int NC, int wanted) {
+  return sizeof(T) == 4 && NC == 2 && wanted == kCoarseDegree ? kCoarseDegree : 2;
+}
+
 template <class T, int NC>
 struct LevelSweep {
   int NX, NY, NXc, NYc;  // nodes of the level and of the next coarser one
