@@ -351,6 +351,18 @@ struct topo_ctx {
             std::fprintf(stderr, "[topo profile] %s level %zu (%dx%d nodes): %lld V-cycle visits, %.3f ms incl, %.2f us/visit\n",
                          name, l, mg.spec(int(l)).NX, mg.spec(int(l)).NY, mg.level_calls[l], mg.level_ms[l],
                          1e3 * mg.level_ms[l] / mg.level_calls[l]);
+        std::vector<long long> cycles;
+        mg.tail_profile(cycles);
+        if (cycles.empty() || cycles.back() == 0) return;
+        const int first = mg.tail_level(), smoothed = mg.levels() - 1 - first;
+        std::fprintf(stderr, "[topo profile] %s tail: levels %d.., %lld launches; k-cycles per phase:", name, first,
+                     cycles.back());
+        for (int k = 0; k + 1 < int(cycles.size()); ++k) {
+          const char* phase = k < smoothed ? "down" : k == smoothed ? "coarsest" : "up";
+          const int level = first + (k <= smoothed ? k : 2 * smoothed - k);
+          std::fprintf(stderr, " %s%d=%.2f", phase, level, 1e-3 * double(cycles[k]) / double(cycles.back()));
+        }
+        std::fprintf(stderr, "\n");
       };
       dump("state32", smg32);
       dump("state64", smg64);

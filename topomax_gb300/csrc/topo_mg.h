@@ -240,6 +240,10 @@ class MG {
   std::vector<double> level_ms;
   std::vector<long long> level_calls;
   void flush_level_profile();
+  // SM cycles of the tail's phases summed over its launches (down, coarsest, up), then the launches;
+  // empty without a tail or profile_levels
+  void tail_profile(std::vector<long long>& cycles) const;
+  int tail_level() const { return tail_; }
   // tune the segment length of this hierarchy's march kernels (level 0 if P2, the P1
   // levels without a stencil) once per family and grid; needs set-up data in place
   bool autotune = true;
@@ -305,7 +309,7 @@ class MG {
     graph_valid_ = false;
     ++epoch_;
   }
-  void build_tail();
+  void build_tail(Arena& arena);
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> prof_events_;
   // truncated hierarchy: the V-cycle stops at level cheb_coarse_ and solves it
   // with a fixed-degree Chebyshev iteration in one CTA (CoarseChebDesc, device)
@@ -318,6 +322,7 @@ class MG {
   T* inner_buf_ = nullptr;  // per level: one stencil row (detect_uniform_levels)
   bool cc_selected_ = false;
   int tail_ = -1;  // first level run by the one-CTA tail kernel, described by
+  long long* tail_trace_ = nullptr;
   TailSweep<T, 1> tail1_{};
   TailSweep<T, 2> tail2_{};
   // set by pcg_body around its V-cycle: the level-0 post-smoothing launch also

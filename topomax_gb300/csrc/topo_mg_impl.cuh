@@ -677,8 +677,9 @@ __device__ __forceinline__ void tail_node(const TailSweep<T, NC>& P, int l, int 
 }
 
 // The last levels of the V-cycle (see TailSweep): x = V-cycle(b) from its level 0 down, D
-// Chebyshev steps each way.  Latency-bound: 2 D + 4 barriers a level.
-template <class T, int NC, int D>
+// Chebyshev steps each way.  Latency-bound: 2 D + 4 barriers a level.  TRACE: SM cycles of every phase
+// in execution order, summed in P.trace (TOPO_PROFILE), and the launches after them.
+template <class T, int NC, int D, bool TRACE>
 __global__ void __launch_bounds__(kTailNodes)
     k_level_tail(const __grid_constant__ TailSweep<T, NC> P, const T* b, T* x) {
   constexpr int SW = StencilLayout<NC>::stride;
@@ -710,13 +711,23 @@ __global__ void __launch_bounds__(kTailNodes)
   level_row<T, NC>(N0.st);
   for (int c = 0; c < NC; ++c) N0.di[c] = L0.dinv[NC * n0 + c];
   TOPO_PDL_WAIT();
+  long long* trace = TRACE && tid == 0 && blockIdx.x == 0 ? P.trace : nullptr;
+  long long before = TRACE ? clock64() : 0;
+  auto mark = [&]() {
+    if (!TRACE || !trace) return;
+    const long long now = clock64();
+    *trace++ += now - before;
+    before = now;
+  };
   for (int c = 0; c < NC; ++c) N0.b[c] = b[NC * n0 + c];
   __syncthreads();  // the zeros are in place
   tail_down<T, NC, D>(P, 0, tid, sm, N0);
+  mark();
   for (int l = 1; l < P.nlev; ++l) {
     TailNode<T, NC> N;
     tail_node(P, l, tid, sm, N);
     tail_down<T, NC, D>(P, l, tid, sm, N);
+    mark();
   }
   if (tid < m) {  // the inverse is symmetric: column reads, one line per step
     T s = T(0);
@@ -725,12 +736,16 @@ __global__ void __launch_bounds__(kTailNodes)
     sm[C.x + NC * ((j + 1) * (C.NX + 2) + i + 1) + tid % NC] = s;
   }
   __syncthreads();
+  mark();
   for (int l = P.nlev - 1; l >= 1; --l) {
     TailNode<T, NC> N;
     tail_node(P, l, tid, sm, N);
     tail_up<T, NC, D>(P, l, tid, sm, N, x);
+    mark();
   }
   tail_up<T, NC, D>(P, 0, tid, sm, N0, x);
+  mark();
+  if (TRACE && trace) *trace += 1;
 }
 
 template <class T, int NC>
@@ -1260,7 +1275,7 @@ void MG<T>::init(const std::vector<LevelSpec>& specs, const ElemRefs* refs, doub
   for (auto& e : ev_)
     if (!e) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
   graph_valid_ = false;
-  build_tail();
+  build_tail(arena);
   cc_buf_ = arena.alloc(sizeof(CoarseChebDesc<T, 1>));
   inner_buf_ = arena.alloc_n<T>(specs.size() * StencilLayout<1>::stride);
 }
@@ -1373,7 +1388,7 @@ void MG<T>::select_coarse_cheb(cudaStream_t s) {
 // Chooses the levels of k_level_tail (FP32): from the first level with at most kTailNodes
 // nodes (never level 0) whose shared memory fits, down to the coarsest.
 template <class T>
-void MG<T>::build_tail() {
+void MG<T>::build_tail(Arena& arena) {
   tail_ = -1;
   const int L = levels();
   auto plan = [&](auto& P, int first) {
@@ -1390,9 +1405,14 @@ void MG<T>::build_tail() {
       d.dir = specs_[l].dir;
     }
     P.plan();
+    P.trace = tail_trace_;
     return size_t(P.shared) * sizeof(T) <= kTailShared;
   };
   if (sizeof(T) == 8) return;
+  if (profile_levels) {
+    tail_trace_ = static_cast<long long*>(arena.alloc(kTailPhases * sizeof(long long)));
+    if (tail_trace_) cudaMemset(tail_trace_, 0, kTailPhases * sizeof(long long));
+  }
   for (int l = std::max(1, L - 1 - kTailMaxLevels); l + 1 < L && tail_ < 0; ++l) {
     if (specs_[l].nn() > size_t(kTailNodes) || level_degree(l) != level_degree(L - 1)) continue;
     bool ok = true;
@@ -1629,6 +1649,15 @@ void MG<T>::flush_level_profile() {
 }
 
 template <class T>
+void MG<T>::tail_profile(std::vector<long long>& cycles) const {
+  cycles.clear();
+  if (!tail_trace_ || tail_ < 0) return;
+  cycles.resize(2 * (levels() - 1 - tail_) + 2);
+  if (cudaMemcpy(cycles.data(), tail_trace_, cycles.size() * sizeof(long long), cudaMemcpyDeviceToHost) != cudaSuccess)
+    cycles.clear();
+}
+
+template <class T>
 void MG<T>::vcycle_level(int l, const T* b, T* x, cudaStream_t s) {
   if (profile_levels && !use_graphs) {
     cudaEvent_t e0, e1;
@@ -1703,7 +1732,9 @@ void MG<T>::sweep_level(int l, const T* b, T* x, cudaStream_t s) {
 template <class T>
 template <int NC, int D>
 void MG<T>::launch_tail(const TailSweep<T, NC>& P, int nodes, const T* b, T* x, cudaStream_t s) {
-  launch_pdl(k_level_tail<T, NC, D>, batch, dim3(unsigned(nodes + 31) / 32 * 32), P.shared * sizeof(T), s, P, b, x);
+  const dim3 threads(unsigned(nodes + 31) / 32 * 32);
+  if (P.trace) launch_pdl(k_level_tail<T, NC, D, true>, batch, threads, P.shared * sizeof(T), s, P, b, x);
+  else launch_pdl(k_level_tail<T, NC, D, false>, batch, threads, P.shared * sizeof(T), s, P, b, x);
 }
 
 template <class T>

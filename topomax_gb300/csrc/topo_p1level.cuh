@@ -439,6 +439,7 @@ struct LevelPhases {
 // level ~2.5 us twice; here its phases are barriers and a few hundred cycles each.
 // ---------------------------------------------------------------------------
 constexpr int kTailMaxLevels = 6;                  // smoothed levels
+constexpr int kTailPhases = 2 * kTailMaxLevels + 2;  // down and up of each, the coarsest solve, the launches
 constexpr size_t kTailShared = 48 * 1024;          // (no opt-in attribute needed)
 // nodes of the first level, one per thread (1000x500: 33x17; a limit of 300 or 160 nodes
 // measured the same or up to 2 % slower).  FP32 only: an FP64 product of a warp holds the
@@ -460,6 +461,7 @@ struct TailSweep {
   int inv;         // shared offset of the inverse
   int shared;      // shared values in all
   const T* cinv;
+  long long* trace;  // cycles of the phases (null: off)
   Lev lv[kTailMaxLevels + 1];
 
   // lays the shared memory out
