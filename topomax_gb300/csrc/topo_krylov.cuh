@@ -12,11 +12,13 @@
 namespace topo {
 
 constexpr int kKrylovMax = 60;  // longest restart
-// A column is orthogonalised again where less than this share of |w|^2 is left: the loss of
-// orthogonality is then at most ten roundings, which 60 vectors at a relative residual of
-// 1e-12 do not see (the same iterations as with 0.5, which repeats two passes in three;
-// 13.9 ms against 19.6 at 128x128, 8.1 against 10.5 at 40x40 with the finer grids).
-constexpr double kReorthogonalise = 0.01;
+// A column is orthogonalised again where less than this share of |w|^2 is left (Kahan's "twice is
+// enough").  A vector keeps what the basis before it has lost, times the norm that its own
+// products took, so a lower share does not only cost a few roundings: with 0.01 no column of the
+// fluid solve was repeated, max |V^T V - I| grew to 0.015 .. 0.25 over 60 vectors (16x16 to 128x128)
+// and the residual's estimate was off by up to a third; with 0.5 the loss is 2e-15.  The
+// second passes cost 10.4 to 12.5 ms at 40x40, 20.7 to 25.2 at 128x128.
+constexpr double kReorthogonalise = 0.5;
 constexpr int kDotGroup = 8;  // basis vectors of one block of the Gram-Schmidt products
 constexpr int kDotGroups = (kKrylovMax + kDotGroup) / kDotGroup;
 
@@ -151,7 +153,7 @@ static __global__ void __launch_bounds__(kVecThreads)
 }
 
 // w -= sum hp_i v_i.  The first pass (classical Gram-Schmidt) decides on the second: it is needed
-// where the products took nearly all of |w|^2 (kReorthogonalise; Kahan's "twice is enough"); the
+// where the products took most of |w|^2 (kReorthogonalise; Kahan's "twice is enough"); the
 // second sums |w|^2.
 template <bool LARGE>
 static __global__ void __launch_bounds__(kVecThreads)
