@@ -76,9 +76,9 @@ __device__ __forceinline__ double krylov_combine(double a, const double* v, size
 }
 
 // Where a thread takes many entries (krylov_large) the loops are compiled for each count of 1 to 8
-// vectors, so that all loads of an entry are in flight together (FP64 refinement at 2000x1000 with
-// 16 M unknowns, whole solve: 42.2 to 37.3 ms per 41.6 and 38.0 of a loop from the host).  Where
-// it takes one or two, the jump costs more than it gives (fluid at 40x40 8.5 ms against 8.1).
+// vectors, so that all loads of an entry are in flight together: with loops of a run-time count the
+// state solve of 2000x1000 (16 M unknowns) was 1.5 % slower than with these.  Where it takes one
+// or two, the jump costs more than it gives (fluid at 40x40 8.5 ms against 8.1).
 #define TOPO_KRYLOV_COUNT(count, CALL) \
   switch (count) {                     \
     case 1: CALL(1); break;            \

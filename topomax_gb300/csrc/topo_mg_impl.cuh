@@ -294,20 +294,16 @@ __global__ void __launch_bounds__(P2M_THREADS) k_p1_march(P1Params<T, NC> P, P1I
 // smoothing coefficients are fixed during a solve, so they are read before the wait for
 // the predecessor; the successor may start its own such reads at once.
 //
-// Measured on design evaluations (us): the six launches per level and the earlier one-block
-// tail of 30 to 35 us took 8,490 at 80x40, 31,000 at 303x101 and 25,470 at 1000x500; sweeps
-// and tail take 5,520, 17,100 and 18,300.
-// Tile: 10 x 4 coarse nodes, 253 threads for 160 fine nodes of its own down, 220 up (two steps).
-// With the tile a constant in FP32, coefficients read before the wait, two values per access and
-// the ring apart from the nodes of its own, a down sweep of two steps is 460 instructions a warp
-// (707 before): 80x40 4.51 to 4.37 ms, 303x101 14.95 to 13.92, filter 1000x500 1.28 to 1.15,
-// FP64 160x80 60.5 to 53.3.  On the 1000x500 design evaluation 14 x 6 measured 18.8 ms against
-// 18.6, 6 x 6 19.2, 14 x 2 18.9; FP64 tiles: see level_sweep (a tile's
+// Against six launches a level (smoothing steps, residual, transfers) a design evaluation went from
+// 11.4 to 7.7 ms at 320x160 and from 22.1 to 17.8 at 1000x500.
+// Tile: 10 x 4 coarse nodes, 253 threads for 160 fine nodes of its own down, 220 up (two steps); on
+// the 1000x500 evaluation 14 x 6 measured 18.8 ms against 18.6, 6 x 6 19.2, 14 x 2 18.9.  It is
+// a constant in FP32 (index arithmetic without divisions).  FP64 tiles: see level_sweep (a tile's
 // recomputed ring costs FP64-pipe time, a large tile leaves SMs without a block).
 // Levels with built rows fill the chip many times over and take 14 x 6 (31 x 15 nodes for 28 x 12)
-// at two steps: 67.9 us down against 70.9 at two million nodes.  Their loads are issued together
-// before the row is built (59.4).  Level 1 of 1000x500 takes 17 + 16 us for what were six launches
-// of 59 us (column march, restriction, prolongation), of 2000x1000 59 + 64 for 160.
+// at two steps: 67.9 us down against 70.9 at two million nodes; their loads are issued together
+// before the row is built (59.4).  Level 1 of 1000x500 takes 17 + 16 us, of 2000x1000 59 + 64
+// (as column marches and transfers 59 and 160).
 constexpr int kSweepTileX = 10, kSweepTileY = 4;
 // ROWS: StoredRows, or the P1Params that the rows are built from.
 struct StoredRows {};
@@ -1746,8 +1742,8 @@ void MG<T>::launch_tail(const TailSweep<T, NC>& P, int l, const T* b, T* x, cuda
   launch_tail<NC, 2>(P, nodes, b, x, s);
 }
 
-// One V-cycle from level l down: fused degree-2 Chebyshev pre-smoothing from
-// x = 0, residual restriction, coarse correction, fused post-smoothing.
+// One V-cycle from level l down: Chebyshev steps (level_degree) from x = 0, restriction of the
+// residual, coarse correction, the same steps again.
 template <class T>
 void MG<T>::vcycle_level_body(int l, const T* b, T* x, cudaStream_t s) {
   Lev& v = lv_[l];
