@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kFluidThreads)
 // gradient and divergence coefficients by node type.  KRYLOV: x = z_j with its pressure's mean
 // taken off, y = v_(j+1).  clamp: boundary velocity rows are the identity.
 // Bound: FP64, 42 products per P2 node on average (the triangles' matrices applied where they are
-// needed take 72), all loads of a row in flight at once: 10.4 us at 128x128, 6.0 at 40x40; by
+// needed take 72), all loads of a row in flight at once: 10.6 us at 128x128, 6.2 at 40x40; by
 // triangle rows 19.6 and 17.4, through a per-triangle buffer and a gather 22 and 20.
 template <bool KRYLOV>
 __global__ void __launch_bounds__(kFluidThreads)
