@@ -44,3 +44,15 @@ def test_an_unreached_iteration_limit_changes_no_bit():
         prob.calculate_objective(np.random.default_rng(3).uniform(0.2, 1.0, V.dim()))
         got.append(prob.u.tensor.clone())
     assert torch.equal(*got)
+
+
+def test_the_trace_names_every_step(monkeypatch, capfd):
+    import re
+    monkeypatch.setenv("TOPO_TRACE_SOLVES", "1")
+    prob, V = _gpu_problem(_design(), 40, 20, rtol=1e-11)
+    prob.set_penalization(3.0)
+    prob.calculate_objective(np.random.default_rng(3).uniform(0.2, 1.0, V.dim()))
+    err = capfd.readouterr().err
+    inner = re.findall(r"inner (\d+): tol ([\d.e+-]+), (\d+) iterations, FP32 relres ([\d.e+-]+), rc (-?\d+)", err)
+    assert len(inner) >= 4 and all(int(i[4]) == 0 and float(i[3]) <= 1.01 * float(i[1]) for i in inner)
+    assert len(re.findall(r"fgmres cycle \d+: ", err)) >= 2 and len(re.findall(r"fgmres converged: ", err)) >= 2

@@ -781,8 +781,9 @@ bool refinement_cycle(topo_ctx* C, MG<float>& mg, Apply64 apply64, size_t n, Fgm
     cudaMemcpyAsync(W.host, W.K, offsetof(KrylovDev, res) + sizeof(double), cudaMemcpyDeviceToHost, s);
     if (!ok || cudaStreamSynchronize(s) != cudaSuccess) return false;
     if (C->trace_solves)
-      std::fprintf(stderr, "[topo solve]   inner %d: tol %.1e, %d iterations, status %d, residual then %.3e\n",
-                   W.host->j - 1, std::sqrt(in.tol2 / in.bb), W.host->inner - before, in.status, W.host->res);
+      std::fprintf(stderr, "[topo solve]   inner %d: tol %.1e, %d iterations, FP32 relres %.3e, rc %d\n",
+                   W.host->j - 1, std::sqrt(in.tol2 / in.bb), W.host->inner - before, in.relres,
+                   in.status == 5 ? 0 : -in.status);
     if (W.host->status != 1) return true;
     if (C->iter_limit > 0 && iterations + W.host->inner >= C->iter_limit) return true;
   }
@@ -839,7 +840,7 @@ int fgmres_device(topo_ctx* C, MG<float>& mg, Apply64 apply64, const void* op, s
     }
     st.relres = beta / bn;
     if (C->trace_solves)
-      std::fprintf(stderr, "[topo solve] refinement cycle %d: |r|/|b| %.3e after %d inner iterations\n", cycle, st.relres,
+      std::fprintf(stderr, "[topo solve] fgmres cycle %d: |r|/|b| %.3e after %d inner iterations\n", cycle, st.relres,
                    st.iterations);
     if (!std::isfinite(beta)) return C->fail(TOPO_ERR_NAN, "non-finite residual");
     if (beta <= rtol * bn) return TOPO_OK;
@@ -866,6 +867,9 @@ int fgmres_device(topo_ctx* C, MG<float>& mg, Apply64 apply64, const void* op, s
     if (K.status == 3) return 1;
     if (K.res <= 0.5 * rtol * bn && !C->verify_residual) {  // (see fgmres_ir)
       st.relres = K.res / bn;
+      if (C->trace_solves)
+        std::fprintf(stderr, "[topo solve] fgmres converged: estimated |r|/|b| %.3e after %d inner iterations\n",
+                     st.relres, st.iterations);
       return TOPO_OK;
     }
     if (C->iter_limit > 0 && st.iterations >= C->iter_limit) break;
