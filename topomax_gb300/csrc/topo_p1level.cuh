@@ -121,6 +121,8 @@ TOPO_HD double fma_t(double a, double b, double c) {
 
 // FP64 needs no difference form, and its pipe is the bound: block 0 becomes the node's own
 // coupling (the row sum less the neighbours'), 7 products instead of 13 operations per value.
+// Results with either form are as far from 64-bit references to four digits (FP64 designs of
+// 47x20 to 240x120: 5.533e-11, loops up to 160x80: 3.106e-12, geometric means).
 template <class T, int NC>
 TOPO_HD void level_row(T (&st)[StencilLayout<NC>::stride]) {
   if constexpr (sizeof(T) == 8) {
